@@ -6,6 +6,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include "edmd_arith.cuh"
 
 namespace edmd {
 
@@ -179,7 +180,7 @@ __device__ __forceinline__ double contact2(const Box& B, double r1, double r2) {
 }
 __device__ __forceinline__ double contact(const Box& B, double r1, double r2) {
   if (B.additive) return r1 + r2;
-  return sqrt(times4(r1) * r2);
+  return sqrt_rn(times4(r1) * r2);
 }
 
 // collisionTimeNormal src/EDMD.c:2661-2723; p1 is current at t.
@@ -199,7 +200,7 @@ __device__ __forceinline__ double coll_time_normal(const Box& B, const Disk& p1,
   double det = b * b - v2 * d2;
   if (d2 < -0.01) { *overlap = true; return NEVER; }
   if (det < 0) return NEVER;
-  return (-b - sqrt(det)) / v2;
+  return div_rn(-b - sqrt_rn(det), v2);
 }
 
 // collisionTimeGrow src/EDMD.c:2598-2659 (radii grow at vr)
@@ -219,8 +220,9 @@ __device__ __forceinline__ double coll_time_grow(const Box& B, const Disk& p1, d
   double d2 = dx * dx + dy * dy;
   double det = b * b - (v2 - dvr * dvr) * (d2 - dr * dr);
   if (det < 0) return NEVER;
-  double plus = (-b + sqrt(det)) / (v2 - dvr * dvr);
-  double minus = (-b - sqrt(det)) / (v2 - dvr * dvr);
+  const double sq = sqrt_rn(det), den = v2 - dvr * dvr;
+  double plus = div_rn(-b + sq, den);
+  double minus = div_rn(-b - sq, den);
   if (((minus > 0) && (plus > 0) && (minus < plus)) || ((minus > 0) && (plus < 0))) return minus;
   else if (((minus > 0) && (plus > 0.000000001) && (plus < minus)) ||
            ((minus < 0) && (plus > 0.000000001)))
@@ -235,10 +237,10 @@ __device__ __forceinline__ double crossing_time(const Box& B, const Disk& p, int
                                                 double t, int* dir) {
   double tx, ty;
   int xx, yy;
-  if (p.vx < 0) { tx = pbc_in_x(B, cx * B.cxs - p.x) / p.vx; xx = 1; }
-  else { tx = pbc_in_x(B, (1 + cx) * B.cxs - p.x) / p.vx; xx = 2; }
-  if (p.vy < 0) { ty = pbc_in_y(B, cy * B.cys - p.y) / p.vy; yy = 3; }
-  else { ty = pbc_in_y(B, (1 + cy) * B.cys - p.y) / p.vy; yy = 4; }
+  if (p.vx < 0) { tx = div_rn(pbc_in_x(B, cx * B.cxs - p.x), p.vx); xx = 1; }
+  else { tx = div_rn(pbc_in_x(B, (1 + cx) * B.cxs - p.x), p.vx); xx = 2; }
+  if (p.vy < 0) { ty = div_rn(pbc_in_y(B, cy * B.cys - p.y), p.vy); yy = 3; }
+  else { ty = div_rn(pbc_in_y(B, (1 + cy) * B.cys - p.y), p.vy); yy = 4; }
   if (tx < ty) { *dir = xx; return t + tx; }
   *dir = yy;
   return t + ty;
@@ -316,7 +318,7 @@ __device__ __forceinline__ double coll_time_normal_i(const Box& B, const Disk& p
   double det = b * b - v2 * d2;
   if (lt_neg(d2, 0.01)) { *overlap = true; return NEVER; }
   if (is_neg(det)) return NEVER;
-  return (-b - sqrt(det)) / v2;
+  return div_rn(-b - sqrt_rn(det), v2);
 }
 
 __device__ __forceinline__ bool key_less(uint32_t b1, uint64_t t1, uint64_t k1, int32_t i1,
@@ -336,11 +338,11 @@ __device__ __forceinline__ double crossing_time_i(const Box& B, const Disk& p, i
   if (is_neg(p.vx)) { a = cx * B.cxs - p.x; xx = 1; }
   else { a = (1 + cx) * B.cxs - p.x; xx = 2; }
   if (ge_pos(a, B.hLx)) a = a - B.Lx; else if (lt_neg(a, B.hLx)) a = a + B.Lx;
-  tx = a / p.vx;
+  tx = div_rn(a, p.vx);
   if (is_neg(p.vy)) { a = cy * B.cys - p.y; yy = 3; }
   else { a = (1 + cy) * B.cys - p.y; yy = 4; }
   if (ge_pos(a, B.hLy)) a = a - B.Ly; else if (lt_neg(a, B.hLy)) a = a + B.Ly;
-  ty = a / p.vy;
+  ty = div_rn(a, p.vy);
   if (lt_i(tx, ty)) { *dir = xx; return t + tx; }
   *dir = yy;
   return t + ty;
@@ -359,7 +361,7 @@ __device__ __forceinline__ double axis_time(const Box& B, const Disk& p, int cx,
   *dir = (ydim ? 3 : 1) + (neg ? 0 : 1);
   if (ge_pos(a, hL)) a = a - L;
   else if (lt_neg(a, hL)) a = a + L;
-  return a / v;
+  return div_rn(a, v);
 }
 
 // crossing_time_i with the two divisions on two lanes of a full warp: the

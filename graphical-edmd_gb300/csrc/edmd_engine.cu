@@ -735,7 +735,7 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
           else if (mk == sm->msum[0]) invMass = sm->inv[0];
           else if (mk == sm->msum[1]) invMass = sm->inv[1];
           else {
-            invMass = 1 / msum;
+            invMass = div_rn(1.0, msum);
             G.sync();
             if (lane == 0) {
               sm->msum[1] = sm->msum[0]; sm->inv[1] = sm->inv[0];
@@ -749,7 +749,7 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
           double collKernel = invMass * (1 + S.res) * (G.shfl(pm, 0) + G.shfl(pm, 1));
           double distSquared = contact2<ADD>(B, di.rad, dj.rad);
           double f = __double_as_longlong(distSquared) == 0x4010000000000000ll ? collKernel * 0.25
-                                                                                : collKernel / distSquared;
+                                                                                : div_rn(collKernel, distSquared);
           double ct = di.m * dj.m * f;
           // collTermX, Y, XY, YX: term lane % 4 on each lane, in shared instructions
           {
@@ -777,9 +777,9 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
           double res = 0.75 * 0 + 1;
           double dvr = S.vr[i] + S.vr[j];
           pbc(B, dx, dy);
-          double dist = sqrt(dx * dx + dy * dy);
-          double dxr = dx / dist, dyr = dy / dist;
-          double invMass = 1 / (di.m + dj.m);
+          double dist = sqrt_rn(dx * dx + dy * dy);
+          double dxr = div_rn(dx, dist), dyr = div_rn(dy, dist);
+          double invMass = div_rn(1.0, di.m + dj.m);
           double collKernel = invMass * (1 + res) * (dxr * dvx + dyr * dvy - dvr);
           di.vx += collKernel * dj.m * dxr - 2 * dj.m * invMass * delta * dxr;
           di.vy += collKernel * dj.m * dyr - 2 * dj.m * invMass * delta * dyr;

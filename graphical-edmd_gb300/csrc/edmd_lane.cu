@@ -402,12 +402,12 @@ __device__ void lane_run(const SysDev& S, const RunArgs& A) {
       if (!grow) {   // elastic branch src/EDMD.c:3802-3827
         // 1/(1+1) and x/4 are exact, so the shortcuts below round identically
         double msum = Da.m + Db.m;
-        double invMass = __double_as_longlong(msum) == 0x4000000000000000ll ? 0.5 : 1 / msum;
+        double invMass = __double_as_longlong(msum) == 0x4000000000000000ll ? 0.5 : div_rn(1.0, msum);
         pbc(B, dx, dy);
         double collKernel = invMass * (1 + S.res) * (dx * dvx + dy * dvy);
         double distSquared = contact2(B, Da.rad, Db.rad);
         double f = __double_as_longlong(distSquared) == 0x4010000000000000ll
-            ? collKernel * 0.25 : collKernel / distSquared;
+            ? collKernel * 0.25 : div_rn(collKernel, distSquared);
         double ct = Da.m * Db.m * f;
         R.collT[0] += ct * dx * dx;
         R.collT[1] += ct * dy * dy;
@@ -422,9 +422,9 @@ __device__ void lane_run(const SysDev& S, const RunArgs& A) {
         double res = 0.75 * 0 + 1;
         double dvr = S.vr[a] + S.vr[b];
         pbc(B, dx, dy);
-        double dist = sqrt(dx * dx + dy * dy);
-        double dxr = dx / dist, dyr = dy / dist;
-        double invMass = 1 / (Da.m + Db.m);
+        double dist = sqrt_rn(dx * dx + dy * dy);
+        double dxr = div_rn(dx, dist), dyr = div_rn(dy, dist);
+        double invMass = div_rn(1.0, Da.m + Db.m);
         double collKernel = invMass * (1 + res) * (dxr * dvx + dyr * dvy - dvr);
         Da.vx += collKernel * Db.m * dxr - 2 * Db.m * invMass * delta * dxr;
         Da.vy += collKernel * Db.m * dyr - 2 * Db.m * invMass * delta * dyr;

@@ -778,12 +778,12 @@ __device__ void process_event_warp(const SysDev& S, const RoundArgs& A, int s, i
         double dx = Db.x - Da.x, dy = Db.y - Da.y;
         const double dvx = Db.vx - Da.vx, dvy = Db.vy - Da.vy;
         const double msum = Da.m + Db.m;
-        const double invMass = __double_as_longlong(msum) == 0x4000000000000000ll ? 0.5 : 1 / msum;
+        const double invMass = __double_as_longlong(msum) == 0x4000000000000000ll ? 0.5 : div_rn(1.0, msum);
         pbc_i(B, dx, dy);
         const double collKernel = invMass * (1 + S.res) * (dx * dvx + dy * dvy);
         const double distSquared = contact2(B, Da.rad, Db.rad);
         const double f = __double_as_longlong(distSquared) == 0x4010000000000000ll
-            ? collKernel * 0.25 : collKernel / distSquared;
+            ? collKernel * 0.25 : div_rn(collKernel, distSquared);
         const double cf = Da.m * Db.m * f;
         // virial term q on lane q: collTermX, Y, XY, YX
         {
@@ -1026,12 +1026,12 @@ __device__ void process_event_thread(const SysDev& S, const RoundArgs& A, int s,
       double dx = Db.x - Da.x, dy = Db.y - Da.y;
       const double dvx = Db.vx - Da.vx, dvy = Db.vy - Da.vy;
       const double msum = Da.m + Db.m;
-      const double invMass = __double_as_longlong(msum) == 0x4000000000000000ll ? 0.5 : 1 / msum;
+      const double invMass = __double_as_longlong(msum) == 0x4000000000000000ll ? 0.5 : div_rn(1.0, msum);
       pbc_i(B, dx, dy);
       const double collKernel = invMass * (1 + S.res) * (dx * dvx + dy * dvy);
       const double distSquared = contact2(B, Da.rad, Db.rad);
       const double f = __double_as_longlong(distSquared) == 0x4010000000000000ll
-          ? collKernel * 0.25 : collKernel / distSquared;
+          ? collKernel * 0.25 : div_rn(collKernel, distSquared);
       const double cf = Da.m * Db.m * f;
       ct4[0] = cf * dx * dx;
       ct4[1] = cf * dy * dy;
