@@ -79,6 +79,13 @@ EDMD_HD uint32_t seed_rsqrt(uint32_t x, int ulps) {
 }
 #endif
 
+// FP32 bits of a seed of the interval (1/2, 1], which an approximation can
+// leave by a few units in the last place, brought into [1/2, 1)
+EDMD_HD uint32_t clamp_unit(uint32_t y) {
+  y = y < 0x3f000000u ? 0x3f000000u : y;
+  return y > 0x3f7fffffu ? 0x3f7fffffu : y;
+}
+
 EDMD_HD uint32_t mul_hi(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
 
 // a / b for normal a, b and a normal quotient; *other is set when that does
@@ -95,7 +102,7 @@ EDMD_HD double div_normal(double a, double b, bool* other, int seed_ulps = 0) {
   // Y = 2^32 / b, b = mb / 2^52 in [1, 2): at most 2^32 - 1, since a Newton
   // step never exceeds the value it approaches
   uint32_t y = seed_rcp(0x3f800000u | ((uint32_t)(mb >> 29) & 0x7fffffu), seed_ulps);
-  if (y > 0x3f7fffffu) y = 0x3f7fffffu;
+  y = clamp_unit(y);
   uint32_t Y = (y << 8) | 0x80000000u;
   const uint32_t B = (uint32_t)(mb >> 21);           // 2^31 b
   const int64_t er = (int64_t)((1ull << 63) - (uint64_t)Y * B);
@@ -121,7 +128,7 @@ EDMD_HD double sqrt_normal(double x, bool* other, int seed_ulps = 0) {
   const bool odd = !(ex & 1);                        // the unbiased exponent is odd
   const uint64_t M = odd ? m + m : m;                // v = M / 2^52 in [1, 4), s = sqrt(v)
   uint32_t y = seed_rsqrt((odd ? 0x40000000u : 0x3f800000u) | ((uint32_t)(m >> 29) & 0x7fffffu), seed_ulps);
-  if (y > 0x3f7fffffu) y = 0x3f7fffffu;
+  y = clamp_unit(y);
   uint32_t Y = (y << 8) | 0x80000000u;               // 2^32 / s
   const uint32_t V = (uint32_t)(M >> 22);            // 2^30 v
   const int64_t er = (int64_t)((1ull << 62) - (uint64_t)V * mul_hi(Y, Y));
