@@ -73,6 +73,12 @@ struct Grp {
   }
   __device__ __forceinline__ void sync() const { __syncwarp(mask); }
   __device__ __forceinline__ bool any(bool p) const { return __any_sync(mask, p); }
+  __device__ __forceinline__ uint32_t min_u32(uint32_t v) const { return __reduce_min_sync(mask, v); }
+  // group-relative ballot
+  __device__ __forceinline__ unsigned ballot(bool p) const {
+    const unsigned m = __ballot_sync(mask, p) & mask;
+    return GW == 32 ? m : m >> (__ffs(mask) - 1);
+  }
   // group-relative index of the first lane where p holds, or -1
   __device__ __forceinline__ int first(bool p) const {
     const unsigned m = __ballot_sync(mask, p) & mask;
@@ -89,35 +95,50 @@ __device__ __forceinline__ bool node_less(const Node& a, const Node& b) {
   return key_less(a.b, a.tk, a.tie, a.idx, b.b, b.tk, b.tie, b.idx);
 }
 
+// Group-relative lane of the least node: word by word from the top of the key
+// (b, time, tie, idx), each word's minimum by one redux instruction.  The
+// first two words (bucket and the upper half of the time) decide almost
+// always.  A butterfly that moves whole 24-byte nodes takes five steps of six
+// shuffles and a four-word compare; a redux takes 28 cycles where one shuffle
+// takes 42.
 template <int GW>
-__device__ __forceinline__ void grp_min(Node& n, const Grp<GW>& G) {
-#pragma unroll
-  for (int o = GW / 2; o > 0; o >>= 1) {
-    Node m;
-    m.tk = G.shfl_xor(n.tk, o);
-    m.tie = G.shfl_xor(n.tie, o);
-    m.b = G.shfl_xor(n.b, o);
-    m.idx = G.shfl_xor(n.idx, o);
-    if (node_less(m, n)) n = m;
+__device__ __forceinline__ int grp_argmin(const Node& n, const Grp<GW>& G) {
+  const uint32_t mb = G.min_u32(n.b);
+  bool in = n.b == mb;
+  auto next = [&](uint32_t w) {
+    const uint32_t v = in ? w : 0xffffffffu;
+    const uint32_t m = G.min_u32(v);            // every lane of the group takes part
+    in = in && v == m;
+  };
+  next((uint32_t)(n.tk >> 32));
+  unsigned q = G.ballot(in);
+  if (q & (q - 1)) {
+    next((uint32_t)n.tk);
+    next((uint32_t)(n.tie >> 32));
+    next((uint32_t)n.tie);
+    next((uint32_t)n.idx);
+    q = G.ballot(in);
   }
+  return __ffs(q) - 1;
 }
 
-// the minimum of the 32 children of node `par` of level h-1, on every lane
+// this lane's child of node `par` of level h-1 (the least of its 32 / GW
+// children), with the nodes at ia and ib taken from na and nb
 template <int GW>
-__device__ __forceinline__ Node children_min(const SysDev& S, int h, int par, const Grp<GW>& G) {
-  const int ch = (par << 5) + G.lane;
-  Node c = ch < S.lev_cnt[h - 1] ? S.tree[S.lev_off[h - 1] + ch] : empty_node(0x7fffffff);
-  if (GW < 32) {
+__device__ __forceinline__ Node child_node(const SysDev& S, int h, int par, int ia, const Node& na, int ib,
+                                           const Node& nb, const Grp<GW>& G) {
+  const int cnt = S.lev_cnt[h - 1];
+  const Node* __restrict__ T = S.tree + S.lev_off[h - 1];
+  Node c = empty_node(0x7fffffff);
 #pragma unroll
-    for (int k = GW; k < 32; k += GW) {
-      const int c2 = ch + k;
-      if (c2 < S.lev_cnt[h - 1]) {
-        const Node m = S.tree[S.lev_off[h - 1] + c2];
-        if (node_less(m, c)) c = m;
-      }
-    }
+  for (int k = 0; k < 32; k += GW) {
+    const int ch = (par << 5) + k + G.lane;
+    Node m = empty_node(0x7fffffff);
+    if (ch == ia) m = na;
+    else if (ch == ib) m = nb;
+    else if (ch < cnt) m = T[ch];
+    if (GW == 32 || node_less(m, c)) c = m;
   }
-  grp_min(c, G);
   return c;
 }
 
@@ -126,56 +147,79 @@ __device__ __forceinline__ Node ev_node(const Ev& e, int idx) {
   return n;
 }
 
-// recompute the leaf of `leaf` from its events and fix its path to the root
-template <int GW>
-__device__ void leaf_update(const SysDev& S, int leaf, const Grp<GW>& G) {
-  const int lane = G.lane;
+// a leaf's node: the earlier of its events
+__device__ __forceinline__ Node leaf_node(const SysDev& S, int leaf) {
   const int N = S.B.N;
   Node n = empty_node(leaf);
   if (leaf < N) {
-    Ev e0 = S.ev[leaf], e1 = S.ev[N + leaf];
+    const Ev e0 = S.ev[leaf], e1 = S.ev[N + leaf];
     if (e0.st == ST_QUEUED) n = ev_node(e0, leaf);
-    if (e1.st == ST_QUEUED) { Node m = ev_node(e1, leaf); if (node_less(m, n)) n = m; }
+    if (e1.st == ST_QUEUED) { const Node m = ev_node(e1, leaf); if (node_less(m, n)) n = m; }
   } else {
-    Ev e = S.ev[2 * N + (leaf - N)];
+    const Ev e = S.ev[2 * N + (leaf - N)];
     if (e.st == ST_QUEUED) n = ev_node(e, leaf);
   }
-  if (lane == 0) S.tree[leaf] = n;
-  G.sync();
-  int idx = leaf;
-  for (int h = 1; h < S.nlev; h++) {
-    int par = idx >> 5;
-    const Node c = children_min(S, h, par, G);
-    if (lane == 0) S.tree[S.lev_off[h] + par] = c;
-    G.sync();
-    idx = par;
+  return n;
+}
+
+template <int GW>
+__device__ __forceinline__ Node shfl_node(const Node& n, int src, const Grp<GW>& G) {
+  Node r;
+  r.tk = G.shfl(n.tk, src); r.tie = G.shfl(n.tie, src);
+  r.b = G.shfl(n.b, src); r.idx = G.shfl(n.idx, src);
+  return r;
+}
+
+// recompute the leaves la and lb (lb < 0: none) from their events and fix
+// their paths to the root, both paths level by level: a parent they share is
+// reduced once, and a node just changed is carried in registers, so no level
+// waits for the stores of the one below it
+template <int GW>
+__device__ __forceinline__ void leaf_update(const SysDev& S, int la, int lb, const Grp<GW>& G) {
+  const int lane = G.lane;
+  Node na = leaf_node(S, la), nb = na;
+  if (lane == 0) S.tree[la] = na;
+  int ia = la, ib = -1;
+  if (lb >= 0) {
+    nb = leaf_node(S, lb);
+    if (lane == 0) S.tree[lb] = nb;
+    ib = lb;
   }
+#pragma unroll 1
+  for (int h = 1; h < S.nlev; h++) {
+    Node* T = S.tree + S.lev_off[h];
+    const int pa = ia >> 5, pb = ib >> 5;       // pb = -1: one path (left)
+    const Node ca = child_node(S, h, pa, ia, na, ib, nb, G);
+    Node cb = ca;
+    if (pb >= 0 && pb != pa) cb = child_node(S, h, pb, ib, nb, -1, nb, G);
+    int src = grp_argmin(ca, G);
+    if (lane == src) T[pa] = ca;
+    na = shfl_node(ca, src, G);
+    ia = pa;
+    ib = -1;
+    if (pb >= 0 && pb != pa) {
+      src = grp_argmin(cb, G);
+      if (lane == src) T[pb] = cb;
+      nb = shfl_node(cb, src, G);
+      ib = pb;
+    }
+  }
+  G.sync();
 }
 
 // rebuild every level of the tree (after init or the growth stop)
 template <int GW>
 __device__ __noinline__ void tree_rebuild(const SysDev& S, const Grp<GW>& G) {
   const int lane = G.lane;
-  const int N = S.B.N;
-  for (int l = lane; l < S.L; l += GW) {
-    Node n = empty_node(l);
-    if (l < N) {
-      Ev e0 = S.ev[l], e1 = S.ev[N + l];
-      if (e0.st == ST_QUEUED) n = ev_node(e0, l);
-      if (e1.st == ST_QUEUED) { Node m = ev_node(e1, l); if (node_less(m, n)) n = m; }
-    } else {
-      Ev e = S.ev[2 * N + (l - N)];
-      if (e.st == ST_QUEUED) n = ev_node(e, l);
-    }
-    S.tree[l] = n;
-  }
+  for (int l = lane; l < S.L; l += GW) S.tree[l] = leaf_node(S, l);
   G.sync();
 #pragma unroll
   for (int h = 1; h < MAXLEV; h++) {
     if (h >= S.nlev) break;
     for (int par = 0; par < S.lev_cnt[h]; par++) {
-      const Node c = children_min(S, h, par, G);
-      if (lane == 0) S.tree[S.lev_off[h] + par] = c;
+      const Node none = empty_node(0x7fffffff);
+      const Node c = child_node(S, h, par, -1, none, -1, none, G);
+      if (lane == grp_argmin(c, G)) S.tree[S.lev_off[h] + par] = c;
     }
     G.sync();
   }
@@ -273,7 +317,7 @@ __device__ __noinline__ bool do_wrap(const SysDev& S, SysState& R, const Grp<GW>
     schedule(S, R, e, T, j, ca, 0ull, G);
     G.sync();
     int leaf = e < 2 * N ? (e < N ? e : e - N) : N + (e - 2 * N);
-    leaf_update(S, leaf, G);
+    leaf_update(S, leaf, -1, G);
     e = n;
   }
   return e == NIL;
@@ -308,6 +352,27 @@ __device__ __forceinline__ uint64_t cand_key(double d) {
 __device__ __forceinline__ void best_merge(uint64_t& bk, int& bo, int& bp, uint32_t& bc,
                                            uint64_t k, int o, int p, uint32_t c) {
   if (k < bk || (k == bk && o < bo)) { bk = k; bo = o; bp = p; bc = c; }
+}
+
+// group-relative lane of the least (time key, scan order), word by word like
+// grp_argmin; a lane without a candidate has order -1, the largest word, and
+// the least key only when no lane has a candidate
+template <int GW>
+__device__ __forceinline__ int best_lane(uint64_t k, int o, const Grp<GW>& G) {
+  const uint32_t h = (uint32_t)(k >> 32);
+  uint32_t m = G.min_u32(h);
+  bool in = h == m;
+  unsigned q = G.ballot(in);
+  if (q & (q - 1)) {
+    uint32_t v = in ? (uint32_t)k : 0xffffffffu;
+    m = G.min_u32(v);                           // every lane of the group takes part
+    in = in && v == m;
+    v = in ? (uint32_t)o : 0xffffffffu;
+    m = G.min_u32(v);
+    in = in && v == m;
+    q = G.ballot(in);
+  }
+  return __ffs(q) - 1;
 }
 
 // collisionEventNormal / Grow (src/EDMD.c:2829 / 3104) for disks a0 and a1
@@ -443,14 +508,11 @@ __device__ void predict2(const SysDev& S, SysState& R, int a0, int a1, Pred& r0,
     for (int o = GW / 2; o > 0; o >>= 1) tot += G.shfl_xor(tot, o);
   }
   // lexicographic (dt, scan order) minimum over the group
-#pragma unroll
-  for (int o = GW / 2; o > 0; o >>= 1) {
-    uint64_t d = G.shfl_xor(bd0, o); int oo = G.shfl_xor(bo0, o);
-    int pp = G.shfl_xor(bp0, o); uint32_t cc = G.shfl_xor(bc0, o);
-    best_merge(bd0, bo0, bp0, bc0, d, oo, pp, cc);
-    d = G.shfl_xor(bd1, o); oo = G.shfl_xor(bo1, o);
-    pp = G.shfl_xor(bp1, o); cc = G.shfl_xor(bc1, o);
-    best_merge(bd1, bo1, bp1, bc1, d, oo, pp, cc);
+  const int w0 = best_lane(bd0, bo0, G);
+  bd0 = G.shfl(bd0, w0); bo0 = G.shfl(bo0, w0); bp0 = G.shfl(bp0, w0); bc0 = G.shfl(bc0, w0);
+  if (a1 >= 0) {
+    const int w1 = best_lane(bd1, bo1, G);
+    bd1 = G.shfl(bd1, w1); bo1 = G.shfl(bo1, w1); bp1 = G.shfl(bp1, w1); bc1 = G.shfl(bc1, w1);
   }
   if (bo0 < 0) bc0 = S.d[0].coll;   // no partner: partner 0 (src/EDMD.c:2830)
   if (bo1 < 0) bc1 = S.d[0].coll;
@@ -876,11 +938,7 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
     }
     if (se0 >= 0) schedule2(S, R, se0, sT0, sj0, sca0, se1, sT1, sj1, sca1, G);
     G.sync();
-    for (int q = 0; q < 2; q++) {
-      const int lf = q ? lb : la;
-      if (lf < 0) break;
-      leaf_update(S, lf, G);
-    }
+    if (la >= 0) leaf_update(S, la, lb, G);
     if (ovl) { status = oa == OVL_CORRUPT ? EDMD_ERR_BUDGET : EDMD_ERR_OVERLAP; break; }
     if (stop) break;
   }
@@ -1164,27 +1222,15 @@ __global__ void __launch_bounds__(256) k_tree_build(const SysDev* __restrict__ s
   const int s = blockIdx.x;
   if (s >= nsys) return;
   const SysDev& S = sys[s];
-  const int N = S.B.N;
-  for (int l = threadIdx.x; l < S.L; l += blockDim.x) {
-    Node n = empty_node(l);
-    if (l < N) {
-      Ev e0 = S.ev[l], e1 = S.ev[N + l];
-      if (e0.st == ST_QUEUED) n = ev_node(e0, l);
-      if (e1.st == ST_QUEUED) { Node m = ev_node(e1, l); if (node_less(m, n)) n = m; }
-    } else {
-      Ev e = S.ev[2 * N + (l - N)];
-      if (e.st == ST_QUEUED) n = ev_node(e, l);
-    }
-    S.tree[l] = n;
-  }
+  for (int l = threadIdx.x; l < S.L; l += blockDim.x) S.tree[l] = leaf_node(S, l);
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int h = 1; h < S.nlev; h++) {
     for (int par = w; par < S.lev_cnt[h]; par += nw) {
-      const int ch = (par << 5) + lane;
-      Node c = ch < S.lev_cnt[h - 1] ? S.tree[S.lev_off[h - 1] + ch] : empty_node(0x7fffffff);
-      grp_min(c, Grp<32>(threadIdx.x));
-      if (lane == 0) S.tree[S.lev_off[h] + par] = c;
+      const Grp<32> G(threadIdx.x);
+      const Node none = empty_node(0x7fffffff);
+      const Node c = child_node(S, h, par, -1, none, -1, none, G);
+      if (lane == grp_argmin(c, G)) S.tree[S.lev_off[h] + par] = c;
     }
     __syncthreads();
   }
