@@ -42,7 +42,7 @@ cudaError_t lane_run_launch(const SysDev* ds, const RunArgs& A, int threads_per_
 
 namespace {
 
-constexpr int MAXC = 8;          // candidates buffered per cell list per lane
+constexpr int MAXC = 7;          // candidates buffered per cell list per lane (a count of three bits)
 constexpr int WARPS_PER_BLOCK = 4;
 
 // scratch of one lane group (one system)
@@ -51,7 +51,7 @@ struct WarpSmem {
   int32_t comp[2 * 9 * MAXC];    // packed candidates
   int16_t ord[2 * 9 * MAXC];     // their scan order
   long long msum[2];             // last two mass sums of the collision rule (bits) ...
-  double inv[2];                 // ... and 1 / msum, the same division's result
+  double inv[2];                 // ... and (1 / msum) (1 + res), the same operations' result
 };
 
 // A group of GW lanes that runs one system: the whole warp (GW = 32) or one
@@ -147,17 +147,16 @@ __device__ __forceinline__ Node ev_node(const Ev& e, int idx) {
   return n;
 }
 
-// a leaf's node: the earlier of its events
+// a leaf's node: the earlier of its events, with that event's slot
 __device__ __forceinline__ Node leaf_node(const SysDev& S, int leaf) {
   const int N = S.B.N;
-  Node n = empty_node(leaf);
+  const int slot = leaf < N ? leaf : N + leaf;           // disk: crossing slot; special: 2N + (leaf - N)
+  Node n = empty_node(slot);
+  const Ev e0 = S.ev[slot];
+  if (e0.st == ST_QUEUED) n = ev_node(e0, slot);
   if (leaf < N) {
-    const Ev e0 = S.ev[leaf], e1 = S.ev[N + leaf];
-    if (e0.st == ST_QUEUED) n = ev_node(e0, leaf);
-    if (e1.st == ST_QUEUED) { const Node m = ev_node(e1, leaf); if (node_less(m, n)) n = m; }
-  } else {
-    const Ev e = S.ev[2 * N + (leaf - N)];
-    if (e.st == ST_QUEUED) n = ev_node(e, leaf);
+    const Ev e1 = S.ev[N + leaf];
+    if (e1.st == ST_QUEUED) { const Node m = ev_node(e1, N + leaf); if (node_less(m, n)) n = m; }
   }
   return n;
 }
@@ -170,21 +169,16 @@ __device__ __forceinline__ Node shfl_node(const Node& n, int src, const Grp<GW>&
   return r;
 }
 
-// recompute the leaves la and lb (lb < 0: none) from their events and fix
-// their paths to the root, both paths level by level: a parent they share is
-// reduced once, and a node just changed is carried in registers, so no level
-// waits for the stores of the one below it
+// the leaves la and lb (lb < 0: none) become na and nb: fix their paths to
+// the root, both paths level by level.  A parent they share is reduced once,
+// and a node just changed is carried in registers, so no level waits for the
+// stores of the one below it.
 template <int GW>
-__device__ __forceinline__ void leaf_update(const SysDev& S, int la, int lb, const Grp<GW>& G) {
+__device__ __forceinline__ void path_update(const SysDev& S, int la, int lb, Node na, Node nb, const Grp<GW>& G) {
   const int lane = G.lane;
-  Node na = leaf_node(S, la), nb = na;
   if (lane == 0) S.tree[la] = na;
-  int ia = la, ib = -1;
-  if (lb >= 0) {
-    nb = leaf_node(S, lb);
-    if (lane == 0) S.tree[lb] = nb;
-    ib = lb;
-  }
+  if (lane == 1 && lb >= 0) S.tree[lb] = nb;
+  int ia = la, ib = lb;
 #pragma unroll 1
   for (int h = 1; h < S.nlev; h++) {
     Node* T = S.tree + S.lev_off[h];
@@ -205,6 +199,13 @@ __device__ __forceinline__ void leaf_update(const SysDev& S, int la, int lb, con
     }
   }
   G.sync();
+}
+
+// one leaf recomputed from its events
+template <int GW>
+__device__ __forceinline__ void leaf_update(const SysDev& S, int leaf, const Grp<GW>& G) {
+  const Node n = leaf_node(S, leaf);
+  path_update(S, leaf, -1, n, n, G);
 }
 
 // rebuild every level of the tree (after init or the growth stop)
@@ -238,25 +239,32 @@ __device__ __forceinline__ int sched_place(const SysDev& S, const SysState& R, d
   return bucket_offset(dt, B.dtP, S.rdtP);
 }
 
+// queue key and state of an event placed at `place` with insertion counter C;
 // `cls_direct` is 2 for a schedule from an event handler and 0 for the
 // re-add done by a wrap
+__device__ __forceinline__ void sched_key(const SysState& R, uint64_t C, uint64_t cls_direct, int place, Ev& ev) {
+  if (place == -1) {
+    ev.b = (uint32_t)R.k; ev.tie = (cls_direct << 62) | C; ev.st = ST_QUEUED;
+  } else if (place == -2) {
+    ev.b = BINF; ev.tie = C; ev.st = ST_OVF;
+  } else {
+    ev.b = (uint32_t)(R.k + (uint64_t)place); ev.tie = (1ull << 62) | (TIE_MAX - C); ev.st = ST_QUEUED;
+  }
+}
+
 template <int GW>
 __device__ __forceinline__ void sched_insert(const SysDev& S, SysState& R, int e, double T, int32_t j,
                                              uint32_t ca, uint64_t cls_direct, int place, const Grp<GW>& G) {
   const int lane = G.lane;
   Ev ev;
   ev.t = T; ev.j = j; ev.ca = ca;
-  if (place == -1) {
-    ev.b = (uint32_t)R.k; ev.tie = (cls_direct << 62) | R.C; ev.st = ST_QUEUED;
-  } else if (place == -2) {
-    ev.b = BINF; ev.tie = R.C; ev.st = ST_OVF;
+  sched_key(R, R.C, cls_direct, place, ev);
+  if (place == -2) {
     if (lane == 0) {
       S.on[e] = R.ovf; S.op[e] = NIL;
       if (R.ovf != NIL) S.op[R.ovf] = e;
     }
     R.ovf = e;
-  } else {
-    ev.b = (uint32_t)(R.k + (uint64_t)place); ev.tie = (1ull << 62) | (TIE_MAX - R.C); ev.st = ST_QUEUED;
   }
   R.C++;
   if (lane == 0) S.ev[e] = ev;
@@ -267,19 +275,6 @@ template <int GW>
 __device__ void schedule(const SysDev& S, SysState& R, int e, double T, int32_t j, uint32_t ca,
                          uint64_t cls_direct, const Grp<GW>& G) {
   sched_insert(S, R, e, T, j, ca, cls_direct, sched_place(S, R, T), G);
-}
-
-// one or two handler schedules in a row (e0 first; e1 < 0: none): the FP64
-// placement of e0 on even lanes and of e1 on odd lanes in shared
-// instructions, then the insertions
-template <int GW>
-__device__ void schedule2(const SysDev& S, SysState& R, int e0, double T0, int32_t j0, uint32_t ca0,
-                          int e1, double T1, int32_t j1, uint32_t ca1, const Grp<GW>& G) {
-  const int lane = G.lane;
-  const int pl = sched_place(S, R, (lane & 1) && e1 >= 0 ? T1 : T0);
-  const int p0 = G.shfl(pl, 0), p1 = G.shfl(pl, 1);
-  sched_insert(S, R, e0, T0, j0, ca0, 2ull, p0, G);
-  if (e1 >= 0) sched_insert(S, R, e1, T1, j1, ca1, 2ull, p1, G);
 }
 
 // removeEventFromQueue (src/EDMD.c:2209) in key form
@@ -317,7 +312,7 @@ __device__ __noinline__ bool do_wrap(const SysDev& S, SysState& R, const Grp<GW>
     schedule(S, R, e, T, j, ca, 0ull, G);
     G.sync();
     int leaf = e < 2 * N ? (e < N ? e : e - N) : N + (e - 2 * N);
-    leaf_update(S, leaf, -1, G);
+    leaf_update(S, leaf, G);
     e = n;
   }
   return e == NIL;
@@ -325,20 +320,37 @@ __device__ __noinline__ bool do_wrap(const SysDev& S, SysState& R, const Grp<GW>
 
 // ---------------------------------------------------------------- prediction
 
-struct Pred { double dt; int32_t partner; uint32_t ca; };
-constexpr int OVL_CORRUPT = -2;  // overlap marker: a cell list longer than N (EDMD_ERR_BUDGET)
-
 __device__ __forceinline__ void grow_fly(const SysDev& S, Disk& p, int i, double t, bool grow) {
   double dt = t - p.tl;
   free_fly_i(S.B, p, t);
   if (grow) p.rad += dt * S.vr[i];
 }
 
-template <bool ADD>
-__device__ __forceinline__ double pair_time(const SysDev& S, const Disk& A, int a, const Disk& P,
-                                            int p, double t, bool grow, bool* ovl) {
-  if (grow) return coll_time_grow(S.B, A, S.vr[a], P, S.vr[p], t, ovl);
-  return coll_time_normal_i<ADD>(S.B, A, P, t, ovl);
+// Lanes of the event handlers.  The (one or two) disks an event changes are
+// spread over four lane roles, repeated over the group: disk `lane & 1` (the
+// owner, or the partner of a collision) and axis `lane & 2` (x, or y).  Each
+// lane holds its disk's coordinate, velocity and cell along its axis, so the
+// scalar FP64 work of both disks and both axes shares its instructions: an
+// FP64 instruction costs its ~76 issue cycles whatever the lanes it serves.
+struct Own {
+  double p, v, rad, vr;            // coordinate and velocity along the axis; radius, growth rate
+  int c;                           // cell index along the axis
+};
+
+// a collision prediction of the lane's disk: time image, partner, its counter
+struct Next { uint64_t key; int32_t partner; uint32_t ca; };
+constexpr int OVL_CORRUPT = -2;    // overlap marker: a cell list longer than N (EDMD_ERR_BUDGET)
+
+// a disk record's coordinate or velocity along an axis (x, y, vx, vy lead it)
+__device__ __forceinline__ double* axis_pos(Disk* d, bool y) { return &d->x + (y ? 1 : 0); }
+__device__ __forceinline__ double* axis_vel(Disk* d, bool y) { return &d->vx + (y ? 1 : 0); }
+static_assert(offsetof(Disk, y) == offsetof(Disk, x) + 8 && offsetof(Disk, vy) == offsetof(Disk, vx) + 8, "axis layout");
+
+// nearest periodic image of a difference along an axis (PBC src/EDMD.c:5896)
+__device__ __forceinline__ double near_image(double d, double hL, double L) {
+  if (ge_pos(d, hL)) d -= L;
+  else if (lt_neg(d, hL)) d += L;
+  return d;
 }
 
 // candidate times compared as their order-preserving integer images: the
@@ -352,6 +364,61 @@ __device__ __forceinline__ uint64_t cand_key(double d) {
 __device__ __forceinline__ void best_merge(uint64_t& bk, int& bo, int& bp, uint32_t& bc,
                                            uint64_t k, int o, int p, uint32_t c) {
   if (k < bk || (k == bk && o < bo)) { bk = k; bo = o; bp = p; bc = c; }
+}
+
+// collisionTimeNormal (src/EDMD.c:2661-2723) and collisionTimeGrow (2598-2659)
+// of an owner current at t and a candidate P, by the two lanes 2k, 2k + 1: one
+// axis each (p1, v1 of the owner), the sums over the axes by shuffle.  A pair
+// costs 16 FP64 instructions instead of the 24 of one lane, and the
+// candidates of an event (about 6 per disk) still fit one pass of a warp.
+// Same operations and roundings as coll_time_normal_i / coll_time_grow (the
+// sums of two products commute).  Every lane of the group takes part; `act`
+// marks the pairs that count.
+template <int GW, bool ADD>
+__device__ __forceinline__ double pair_time_lanes(const Box& B, const Grp<GW>& G, bool act, double p1, double v1,
+                                                  double rad1, double vr1, const Disk* P, const double* vr2p,
+                                                  double t, bool grow, bool* ovl) {
+  const bool y = G.lane & 1;
+  const double pos = (&P->x)[y ? 1 : 0], vel = (&P->vx)[y ? 1 : 0], rad2 = P->rad;
+  const double lat2 = t - P->tl;
+  const double dv = vel - v1;
+  const double d = near_image((pos + lat2 * vel) - p1, y ? B.hLy : B.hLx, y ? B.Ly : B.Lx);
+  double b = d * dv, v2 = dv * dv, d2 = d * d;
+  b += G.shfl_xor(b, 1);
+  v2 += G.shfl_xor(v2, 1);
+  d2 += G.shfl_xor(d2, 1);
+  if (!grow) {
+    d2 -= contact2<ADD>(B, rad1, rad2);
+    // b b on the y lane, v2 d2 on the x lane
+    const double u = (y ? b : v2) * (y ? b : d2);
+    const double w = G.shfl_xor(u, 1);
+    const double det = (y ? u : w) - (y ? w : u);
+    if (!act || is_pos(b)) return NEVER;
+    if (lt_neg(d2, 0.01)) { *ovl = true; return NEVER; }
+    if (is_neg(det)) return NEVER;
+    return div_rn(-b - sqrt_rn(det), v2);
+  }
+  const double vr2 = *vr2p;
+  const double dvr = vr1 + vr2;
+  const double dr = contact(B, rad1, rad2 + lat2 * vr2);
+  b -= dvr * dr;
+  const double den = v2 - dvr * dvr, gap = d2 - dr * dr;
+  const double det = b * b - den * gap;
+  const bool root = act && !(det < 0);
+  // the two roots on the two lanes: -b - s on x, -b + s on y
+  double r = 0;
+  if (root) {
+    const double s = sqrt_rn(det);
+    r = div_rn(-b + flip(s, !y), den);
+  }
+  const double q = G.shfl_xor(r, 1);
+  const double minus = y ? q : r, plus = y ? r : q;
+  if (!root) return NEVER;
+  if (((minus > 0) && (plus > 0) && (minus < plus)) || ((minus > 0) && (plus < 0))) return minus;
+  else if (((minus > 0) && (plus > 0.000000001) && (plus < minus)) || ((minus < 0) && (plus > 0.000000001)))
+    return plus;
+  if (gap < -0.01) *ovl = true;
+  return NEVER;
 }
 
 // group-relative lane of the least (time key, scan order), word by word like
@@ -376,32 +443,34 @@ __device__ __forceinline__ int best_lane(uint64_t k, int o, const Grp<GW>& G) {
 }
 
 // collisionEventNormal / Grow (src/EDMD.c:2829 / 3104) for disks a0 and a1
-// (a1 may be -1): scan the 3x3 neighbour cells, dy outer and dx inner, list
-// order, keep the first strict minimum.  The (disk, cell) walks are tasks
-// t = 0..8 (a0's cells in scan order) and 9..17 (a1's): task t runs on lane
-// t % GW, a lane with two tasks walks both lists at once.  The candidates are
-// then packed over the group in task order and solved GW at a time.
+// (a1 may be -1), both current at t, whose lane roles hold `own`: scan the
+// 3x3 neighbour cells, dy outer and dx inner, list order, keep the first
+// strict minimum.  The (disk, cell) walks are tasks t = 0..8 (a0's cells in
+// scan order) and 9..17 (a1's): task t runs on lane t % GW, a lane with two
+// tasks walks both lists at once.  The candidates are then packed over the
+// group in task order and solved by two lanes each.
 template <int GW, bool ADD>
-__device__ void predict2(const SysDev& S, SysState& R, int a0, int a1, Pred& r0, Pred& r1,
-                         const Grp<GW>& G, WarpSmem* sm, bool* ovl, int* ovl_a, int* ovl_b) {
+__device__ __forceinline__ Next predict2(const SysDev& S, double t, bool grow, int a0, int a1, const Own& own,
+                                         uint64_t* npair, const Grp<GW>& G, WarpSmem* sm, bool* ovl, int* ovl_a,
+                                         int* ovl_b) {
   const Box& B = S.B;
   const int lane = G.lane;
-  const bool grow = R.grow != 0;
   const double dinit = grow ? 10000000 : NEVER;
   const int ntask = a1 >= 0 ? 18 : 9;
+  const int X0 = G.shfl(own.c, 0), X1 = G.shfl(own.c, 1), Y0 = G.shfl(own.c, 2), Y1 = G.shfl(own.c, 3);
   // the tasks of this lane: t = lane + k GW, k < NT (a warp: one task per
   // lane; 16 lanes: two; 8 lanes: three; 4 lanes: five)
   constexpr int NT = (18 + GW - 1) / GW;
-  auto task_cell = [&](int own, int q) {
-    return pbc_cy(B, S.cy[own] + q / 3 - 1) * B.Nxc + pbc_cx(B, S.cx[own] + q % 3 - 1);
-  };
-  int pt[NT], ct[NT], ot[NT], qt[NT];
+  int pt[NT], ct[NT], ot[NT], qt[NT], hc[NT];
 #pragma unroll
   for (int k = 0; k < NT; k++) {
-    const int t = lane + k * GW;
-    ot[k] = t >= 9 ? a1 : a0;
-    qt[k] = t >= 9 ? t - 9 : t;
-    pt[k] = t < ntask ? S.head[task_cell(ot[k], qt[k])] : NIL;
+    const int u = lane + k * GW;
+    const bool second = u >= 9;
+    ot[k] = second ? a1 : a0;
+    const int q = second ? u - 9 : u;
+    qt[k] = q;
+    hc[k] = pbc_cy(B, (second ? Y1 : Y0) + q / 3 - 1) * B.Nxc + pbc_cx(B, (second ? X1 : X0) + q % 3 - 1);
+    pt[k] = u < ntask ? S.head[hc[k]] : NIL;
     ct[k] = 0;
   }
   bool lcorrupt = false;
@@ -413,8 +482,8 @@ __device__ void predict2(const SysDev& S, SysState& R, int a0, int a1, Pred& r0,
 #pragma unroll
       for (int k = 0; k < NT; k++) {
         if (pt[k] != NIL) {
-          const int t = lane + k * GW;
-          if (pt[k] != ot[k]) { if (ct[k] < MAXC) sm->reg[t * MAXC + ct[k]] = pt[k]; ct[k]++; }
+          const int u = lane + k * GW;
+          if (pt[k] != ot[k]) { if (ct[k] < MAXC) sm->reg[u * MAXC + ct[k]] = pt[k]; ct[k]++; }
           pt[k] = S.d[pt[k]].nxt;
           more |= pt[k] != NIL;
         }
@@ -430,103 +499,115 @@ __device__ void predict2(const SysDev& S, SysState& R, int a0, int a1, Pred& r0,
 #pragma unroll
   for (int k = 0; k < NT; k++) over |= ct[k] > MAXC;
   const bool spill = G.any(over);
-  Disk A0 = S.d[a0];
-  Disk A1 = a1 >= 0 ? S.d[a1] : A0;
   uint64_t bd0 = cand_key(dinit), bd1 = bd0;
   int bo0 = -1, bo1 = -1, bp0 = 0, bp1 = 0;
   uint32_t bc0 = 0, bc1 = 0;
-  bool lovl = false;
+  // of several overlapping pairs the one named is fixed by the order the
+  // candidates have when each takes a lane of its own
+  uint32_t lk = 0xffffffffu;
   int la = -1, lb = -1;
   int tot;
   if (!spill) {
-    // exclusive prefix of the counts in task order: tasks 0..GW-1, then GW..
+    // exclusive prefix of the counts (at most 7) in task order, bit by bit
     int ex[NT];
     int base = 0;
+    const unsigned below = (1u << lane) - 1u;
 #pragma unroll
     for (int k = 0; k < NT; k++) {
-      int in = ct[k];
-#pragma unroll
-      for (int o = 1; o < GW; o <<= 1) {
-        const int u = G.shfl_up(in, o);
-        if (lane >= o) in += u;
-      }
-      ex[k] = base + in - ct[k];
-      base += G.shfl(in, GW - 1);
+      const unsigned c0 = G.ballot(ct[k] & 1), c1 = G.ballot(ct[k] & 2), c2 = G.ballot(ct[k] & 4);
+      ex[k] = base + __popc(c0 & below) + 2 * __popc(c1 & below) + 4 * __popc(c2 & below);
+      base += __popc(c0) + 2 * __popc(c1) + 4 * __popc(c2);
     }
     // a0's candidates are tasks 0..8: their count is the prefix at task 9
     const int tot0 = G.shfl(ex[9 / GW], 9 % GW);
     tot = base;
 #pragma unroll
     for (int k = 0; k < NT; k++) {
-      const int t = lane + k * GW;
+      const int u = lane + k * GW;
       for (int m = 0; m < ct[k]; m++) {
-        sm->comp[ex[k] + m] = sm->reg[t * MAXC + m];
+        sm->comp[ex[k] + m] = sm->reg[u * MAXC + m];
         sm->ord[ex[k] + m] = (int16_t)(qt[k] * MAXC + m);
       }
     }
     G.sync();
-    for (int f = lane; f < tot; f += GW) {
-      int p = sm->comp[f];
-      int o = sm->ord[f];
-      Disk P = S.d[p];
-      bool g1 = f >= tot0;
+    for (int f0 = 0; f0 < tot; f0 += GW / 2) {
+      const int f = f0 + (lane >> 1);
+      const bool act = f < tot;
+      const bool g1 = act && f >= tot0;
+      const int src = (g1 ? 1 : 0) | ((lane & 1) << 1);
+      const double p1 = G.shfl(own.p, src), v1 = G.shfl(own.v, src), rad1 = G.shfl(own.rad, src);
+      const double vr1 = grow ? G.shfl(own.vr, src) : 0.0;
+      const int p = act ? sm->comp[f] : a0;
+      const int o = act ? sm->ord[f] : 0;
+      const Disk* P = S.d + p;
+      const uint32_t pc = P->coll;
       bool ov = false;
-      double d = pair_time<ADD>(S, g1 ? A1 : A0, g1 ? a1 : a0, P, p, R.t, grow, &ov);
-      if (ov) { lovl = true; la = g1 ? a1 : a0; lb = p; }
-      if (g1) best_merge(bd1, bo1, bp1, bc1, cand_key(d), o, p, P.coll);
-      else best_merge(bd0, bo0, bp0, bc0, cand_key(d), o, p, P.coll);
+      const uint64_t kd =
+          cand_key(pair_time_lanes<GW, ADD>(B, G, act, p1, v1, rad1, vr1, P, S.vr + p, t, grow, &ov));
+      if (ov) {
+        const uint32_t k = ((uint32_t)(f % GW) << 16) | (0xffffu - (uint32_t)f);
+        if (k < lk) { lk = k; la = g1 ? a1 : a0; lb = p; }
+      }
+      if (g1) best_merge(bd1, bo1, bp1, bc1, kd, o, p, pc);
+      else if (act) best_merge(bd0, bo0, bp0, bc0, kd, o, p, pc);
     }
     G.sync();
   } else {
-    // a cell list longer than MAXC: every task walks its own list again,
-    // solving as it goes
+    // a cell list longer than MAXC: the lists are walked again, one after the
+    // other, every pair by the first two lanes
     tot = 0;
-#pragma unroll
-    for (int w = 0; w < NT; w++) {
-      const int t = lane + w * GW;
-      if (t >= ntask) continue;
-      const int own = ot[w], q = qt[w];
-      const bool g1 = t >= 9;
-      const Disk& AA = g1 ? A1 : A0;
-      int p = S.head[task_cell(own, q)];
+#pragma unroll 1
+    for (int u = 0; u < ntask; u++) {
+      const bool g1 = u >= 9;
+      const int q = g1 ? u - 9 : u, a = g1 ? a1 : a0;
+      const int src = (g1 ? 1 : 0) | ((lane & 1) << 1);
+      const double p1 = G.shfl(own.p, src), v1 = G.shfl(own.v, src), rad1 = G.shfl(own.rad, src);
+      const double vr1 = grow ? G.shfl(own.vr, src) : 0.0;
+      int p = S.head[pbc_cy(B, (g1 ? Y1 : Y0) + q / 3 - 1) * B.Nxc + pbc_cx(B, (g1 ? X1 : X0) + q % 3 - 1)];
       int k = 0, guard = 0;
       while (p != NIL && guard++ < B.N) {
-        Disk P = S.d[p];
-        if (p != own) {
+        const Disk* P = S.d + p;
+        const int nx = P->nxt;
+        if (p != a) {
           bool ov = false;
-          double d = pair_time<ADD>(S, AA, own, P, p, R.t, grow, &ov);
-          if (ov) { lovl = true; la = own; lb = p; }
-          if (g1) best_merge(bd1, bo1, bp1, bc1, cand_key(d), q * 4096 + k, p, P.coll);
-          else best_merge(bd0, bo0, bp0, bc0, cand_key(d), q * 4096 + k, p, P.coll);
+          const uint64_t kd =
+              cand_key(pair_time_lanes<GW, ADD>(B, G, true, p1, v1, rad1, vr1, P, S.vr + p, t, grow, &ov));
+          if (ov) {
+            const uint32_t w = ((uint32_t)(u % GW) << 16) | (0xffffu - (uint32_t)(u * 2048 + min(k, 2047)));
+            if (w < lk) { lk = w; la = a; lb = p; }
+          }
+          if (g1) best_merge(bd1, bo1, bp1, bc1, kd, q * 4096 + k, p, P->coll);
+          else best_merge(bd0, bo0, bp0, bc0, kd, q * 4096 + k, p, P->coll);
           k++;
         }
-        p = P.nxt;
+        p = nx;
       }
       if (p != NIL) lcorrupt = true;
       tot += k;
     }
-    for (int o = GW / 2; o > 0; o >>= 1) tot += G.shfl_xor(tot, o);
   }
+  *npair += (uint64_t)tot;
   // lexicographic (dt, scan order) minimum over the group
-  const int w0 = best_lane(bd0, bo0, G);
-  bd0 = G.shfl(bd0, w0); bo0 = G.shfl(bo0, w0); bp0 = G.shfl(bp0, w0); bc0 = G.shfl(bc0, w0);
+  Next r;
+  {
+    const int w0 = best_lane(bd0, bo0, G);
+    bd0 = G.shfl(bd0, w0); bo0 = G.shfl(bo0, w0); bp0 = G.shfl(bp0, w0); bc0 = G.shfl(bc0, w0);
+  }
   if (a1 >= 0) {
     const int w1 = best_lane(bd1, bo1, G);
     bd1 = G.shfl(bd1, w1); bo1 = G.shfl(bo1, w1); bp1 = G.shfl(bp1, w1); bc1 = G.shfl(bc1, w1);
+    if (lane & 1) { bd0 = bd1; bo0 = bo1; bp0 = bp1; bc0 = bc1; }
   }
   if (bo0 < 0) bc0 = S.d[0].coll;   // no partner: partner 0 (src/EDMD.c:2830)
-  if (bo1 < 0) bc1 = S.d[0].coll;
-  r0.dt = key_time(bd0); r0.partner = bp0; r0.ca = bc0;
-  r1.dt = key_time(bd1); r1.partner = bp1; r1.ca = bc1;
-  R.npair += (uint64_t)tot;
-  R.npred += (a1 >= 0) ? 2 : 1;
-  const int src = G.first(lovl);
-  if (src >= 0) {
+  r.key = bd0; r.partner = bp0; r.ca = bc0;
+  if (G.any(lk != 0xffffffffu || lcorrupt)) {
+    const uint32_t least = G.min_u32(lk);
+    const int src = G.first(lk == least && lk != 0xffffffffu);
     *ovl = true;
-    *ovl_a = G.shfl(la, src);
-    *ovl_b = G.shfl(lb, src);
+    if (src >= 0) { *ovl_a = G.shfl(la, src); *ovl_b = G.shfl(lb, src); }
+    if (G.any(lcorrupt)) { *ovl_a = OVL_CORRUPT; *ovl_b = a0; }
   }
-  if (G.any(lcorrupt)) { *ovl = true; *ovl_a = OVL_CORRUPT; *ovl_b = a0; }
+  return r;
 }
 
 // ---------------------------------------------------------------- handlers
@@ -641,9 +722,13 @@ __device__ __noinline__ void do_growstop(const SysDev& S, SysState& R, const Grp
     if (lane == 0) S.d[i].coll = c;
     G.sync();
     unqueue(S, R, N + i, G);
-    Pred r0, r1;
-    predict2<GW, ADD>(S, R, i, -1, r0, r1, G, sm, ovl, oa, ob);
-    schedule(S, R, N + i, R.t + r0.dt, r0.partner, r0.ca, 2ull, G);
+    Own own;
+    own.p = *axis_pos(S.d + i, lane & 2); own.v = *axis_vel(S.d + i, lane & 2); own.rad = S.d[i].rad;
+    own.vr = 0;
+    own.c = (lane & 2 ? S.cy : S.cx)[i];
+    R.npred++;
+    const Next r = predict2<GW, ADD>(S, R.t, false, i, -1, own, &R.npair, G, sm, ovl, oa, ob);
+    schedule(S, R, N + i, R.t + key_time(r.key), r.partner, r.ca, 2ull, G);
     unqueue(S, R, i, G);
     int dir;
     Disk p = S.d[i];
@@ -652,23 +737,6 @@ __device__ __noinline__ void do_growstop(const SysDev& S, SysState& R, const Grp
     G.sync();
   }
   tree_rebuild(S, G);
-}
-
-// crossing_time_i with the two divisions on two lanes of the group: the lane
-// with (lane & xmask) == 0 takes the x axis of its disk, its partner lane ^
-// xmask the y axis; both return the disk's crossing
-template <int GW>
-__device__ __forceinline__ double crossing_time_grp(const Box& B, const Disk& p, int cx, int cy, double t,
-                                                    const Grp<GW>& G, int xmask, int* dir) {
-  const bool ydim = (G.lane & xmask) != 0;
-  int d;
-  const double ta = axis_time(B, p, cx, cy, ydim, &d);
-  const double tb = G.shfl_xor(ta, xmask);
-  const int db = G.shfl_xor(d, xmask);
-  const double tx = ydim ? tb : ta, ty = ydim ? ta : tb;
-  const bool ux = lt_i(tx, ty);
-  *dir = ux ? (ydim ? db : d) : (ydim ? d : db);
-  return t + (ux ? tx : ty);
 }
 
 // ---------------------------------------------------------------- run loop
@@ -681,18 +749,31 @@ __device__ __forceinline__ void gather_virial(SysState& R, double ctl, const Grp
   for (int k = 0; k < 4; k++) R.collT[k] = G.shfl(ctl, k);
 }
 
+// The event loop of one system.  One event is one chain of dependent
+// instructions, so its latency is what counts (a single system) and its FP64
+// instructions (a full GPU).  Both disks and both axes share the scalar FP64
+// work (struct Own), the two or four events an event schedules are placed and
+// stored by one lane each, and a changed leaf of the tree is built from those
+// lanes' registers.
 // ADD = false: a context without additive-contact systems (the rule's
 // switch compiled out of the pair solves and the collision rule)
 template <int GW, bool ADD = true>
 __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, const Grp<GW>& G,
                            WarpSmem* sm) {
   const int lane = G.lane;
+  const bool odd = lane & 1, ydim = lane & 2;
   const Box& B = S.B;
   const int N = B.N;
   SysState R = *S.st;
   if (R.status != EDMD_OK) return;
   double ctl = R.collT[lane & 3];      // this lane's virial term, see gather_virial
-  if (lane == 0) { sm->msum[0] = sm->msum[1] = 0; }   // no mass sum is +0
+  const double onepr = 1 + S.res;
+  // (1 + res) / (m_i + m_j) of the last two mass sums: a repeated quotient and
+  // product give the same bits.  2 is first (1 / 2 is exact); no sum is +0
+  if (lane == 0) {
+    sm->msum[0] = 0x4000000000000000ll; sm->inv[0] = 0.5 * onepr;
+    sm->msum[1] = 0; sm->inv[1] = 0;
+  }
   G.sync();
   const int root = S.lev_off[S.nlev - 1];
   int64_t logged = 0, nev = 0;
@@ -719,226 +800,263 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
       break;
     }
     if (status != EDMD_OK) break;
-    int leaf = r.idx, e;
-    if (leaf < N) {
-      Ev e0 = S.ev[leaf];
-      e = (e0.st == ST_QUEUED && e0.b == r.b && time_key(e0.t) == r.tk && e0.tie == r.tie) ? leaf : N + leaf;
-    } else {
-      e = 2 * N + (leaf - N);
-    }
-    Ev E = S.ev[e];
+    const int e = r.idx;
+    const Ev E = S.ev[e];
     if (le_i(A.t_stop, E.t)) { stop = EDMD_STOP_TIME; break; }
-    R.t = E.t;
+    const double t = E.t;
+    R.t = t;
     nev++;
     R.nevents++;
-    if (lane == 0) S.ev[e].st = ST_NONE;
-    G.sync();
     const bool grow = R.grow != 0;
-    int ka = -1, kb = -1, uq = -1;     // disks whose crossing events are scheduled below, event removed
-    int pa = -1, pb = -1;              // disks whose collision events are predicted below
-    int se0 = -1, se1 = -1;            // events inserted below, their times, partners, counters
-    double sT0 = 0, sT1 = 0;
-    int32_t sj0 = 0, sj1 = 0;
-    uint32_t sca0 = 0, sca1 = 0;
-    int la = -1, lb = -1;              // leaves whose tree paths are updated below
-    if (e >= N && e < 2 * N) {
-      // ---------------- collision (doTheCollisionNormal 3542 / Grow 3465)
-      const int i = e - N, j = E.j;
-      Disk di = S.d[i];
-      Disk dj = S.d[j];
-      const bool stale = E.ca != dj.coll;
+    if (e < 2 * N) {
+      const bool coll = e >= N;
+      const int i = coll ? e - N : e, j = coll ? E.j : i;
+      const int my = odd ? j : i;
+      Disk* const D = S.d + my;
+      Own own;
+      own.p = *axis_pos(D, ydim); own.v = *axis_vel(D, ydim); own.rad = D->rad;
+      own.c = (ydim ? S.cy : S.cx)[my];
+      own.vr = grow ? S.vr[my] : 0.0;
+      const double m = D->m;
+      const uint32_t hits = D->coll;
+      // events replaced by this one's, beside the popped one: the crossings of
+      // both disks and the partner's collision, or a crossing disk's collision
+      const int old = coll ? (lane == 0 ? i : lane == 1 ? j : lane == 3 ? N + j : -1) : (lane == 2 ? N + i : -1);
+      const uint32_t old_st = old >= 0 ? S.ev[old].st : ST_NONE;
       {
-        // free flights of i (even lanes) and j (odd lanes) in shared
-        // instructions; j's is used only when the event is not stale
-        const bool odd = lane & 1;
-        Disk M = odd ? dj : di;
-        grow_fly(S, M, odd ? j : i, R.t, grow);
-        di.x = G.shfl(M.x, 0); di.y = G.shfl(M.y, 0);
-        di.tl = G.shfl(M.tl, 0); di.rad = G.shfl(M.rad, 0);
-        dj.x = G.shfl(M.x, 1); dj.y = G.shfl(M.y, 1);
-        dj.tl = G.shfl(M.tl, 1); dj.rad = G.shfl(M.rad, 1);
+        // freeFlyNormal / Grow (src/EDMD.c:4954 / 4992) of the lane's coordinate
+        const double L = ydim ? B.Ly : B.Lx;
+        const double dt = t - D->tl;
+        own.p += dt * own.v;
+        if (is_neg(own.p)) own.p += L;
+        else if (ge_pos(own.p, L)) own.p -= L;
+        if (grow) own.rad += dt * own.vr;
       }
-      if (stale) {
-        if (lane == 0) S.d[i] = di;
-        G.sync();
-        R.nstale++;
-        pa = i;
-      } else {
-        const int ci = S.cy[i] * B.Nxc + S.cx[i];
-        const int cj = S.cy[j] * B.Nxc + S.cx[j];
-        if ((A.flags & EDMD_F_TRACE) && S.trace && (int64_t)R.ntrace < S.trace_cap && lane == 0) {
-          edmd_collision* tr = (edmd_collision*)S.trace + R.ntrace;
-          tr->i = i; tr->j = j; tr->cell_i = ci; tr->cell_j = cj; tr->t = R.t;
+      const bool stale = coll && E.ca != G.shfl(hits, 1);
+      const bool two = coll && !stale;       // a second disk changes
+      if (two) {
+        // ---------------- collision (doTheCollisionNormal 3542 / Grow 3465)
+        if ((A.flags & EDMD_F_TRACE) && S.trace && (int64_t)R.ntrace < S.trace_cap) {
+          const int ci = G.shfl(own.c, 2) * B.Nxc + G.shfl(own.c, 0), cj = G.shfl(own.c, 3) * B.Nxc + G.shfl(own.c, 1);
+          if (lane == 0) {
+            edmd_collision* tr = (edmd_collision*)S.trace + R.ntrace;
+            tr->i = i; tr->j = j; tr->cell_i = ci; tr->cell_j = cj; tr->t = t;
+          }
         }
         R.ntrace++;
         if (!(A.flags & EDMD_F_COUNT_NORMAL) || !grow) logged++;
         R.ncol++;
         R.ncol_total++;
-        di.coll++;
-        dj.coll++;
-        // dx, dy, dvx, dvy on lanes 0..3 (mod 4) in one instruction
-        const int q4 = lane & 3;
-        double dx, dy, dvx, dvy;
-        {
-          const double d4 = (q4 == 0 ? dj.x : q4 == 1 ? dj.y : q4 == 2 ? dj.vx : dj.vy) -
-                            (q4 == 0 ? di.x : q4 == 1 ? di.y : q4 == 2 ? di.vx : di.vy);
-          dx = G.shfl(d4, 0); dy = G.shfl(d4, 1);
-          dvx = G.shfl(d4, 2); dvy = G.shfl(d4, 3);
-        }
+        // j minus i, the same value on both disks' lanes
+        const double po = G.shfl_xor(own.p, 1), vo = G.shfl_xor(own.v, 1);
+        const double mo = G.shfl_xor(m, 1), ro = G.shfl_xor(own.rad, 1);
+        const double d = near_image((odd ? own.p : po) - (odd ? po : own.p), ydim ? B.hLy : B.hLx, ydim ? B.Ly : B.Lx);
+        const double dv = (odd ? own.v : vo) - (odd ? vo : own.v);
+        const double msum = m + mo;
+        const long long mk = __double_as_longlong(msum);
         if (!grow) {   // elastic branch src/EDMD.c:3802-3827
-          // 1/(1+1) and x/4 are exact, so these shortcuts round identically
-          // (== 2.0 and == 4.0 as bit compares, on the integer pipe)
-          // 1 / msum repeats for the few mass pairs of a system: the last two
-          // results are kept (a bit-identical value, without the division)
-          double msum = di.m + dj.m;
-          const long long mk = __double_as_longlong(msum);
-          double invMass;
-          if (mk == 0x4000000000000000ll) invMass = 0.5;
-          else if (mk == sm->msum[0]) invMass = sm->inv[0];
-          else if (mk == sm->msum[1]) invMass = sm->inv[1];
+          double pr = d * dv;
+          pr += G.shfl_xor(pr, 2);
+          double inv;
+          if (mk == sm->msum[0]) inv = sm->inv[0];
+          else if (mk == sm->msum[1]) inv = sm->inv[1];
           else {
-            invMass = div_rn(1.0, msum);
+            inv = div_rn(1.0, msum) * onepr;
             G.sync();
             if (lane == 0) {
               sm->msum[1] = sm->msum[0]; sm->inv[1] = sm->inv[0];
-              sm->msum[0] = mk; sm->inv[0] = invMass;
+              sm->msum[0] = mk; sm->inv[0] = inv;
             }
             G.sync();
           }
-          pbc_i(B, dx, dy);
-          // dx*dvx on even lanes, dy*dvy on odd lanes, then their sum
-          const double pm = ((q4 & 1) ? dy : dx) * ((q4 & 1) ? dvy : dvx);
-          double collKernel = invMass * (1 + S.res) * (G.shfl(pm, 0) + G.shfl(pm, 1));
-          double distSquared = contact2<ADD>(B, di.rad, dj.rad);
-          double f = __double_as_longlong(distSquared) == 0x4010000000000000ll ? collKernel * 0.25
-                                                                                : div_rn(collKernel, distSquared);
-          double ct = di.m * dj.m * f;
-          // collTermX, Y, XY, YX: term lane % 4 on each lane, in shared instructions
+          const double collKernel = inv * pr;
+          // sigma^2 and m_i m_j
+          const double distSquared = contact2<ADD>(B, odd ? ro : own.rad, odd ? own.rad : ro);
+          const double mm = (odd ? mo : m) * (odd ? m : mo);
+          // x/4 is exact, so the shortcut rounds identically
+          const double f = __double_as_longlong(distSquared) == 0x4010000000000000ll
+              ? collKernel * 0.25 : div_rn(collKernel, distSquared);
+          const double od = G.shfl_xor(d, 2);
+          const double dx = ydim ? od : d, dy = ydim ? d : od;
           {
+            // collTermX, Y, XY, YX: term lane % 4 on each lane
             const int q = lane & 3;
+            const double ct = mm * f;
             ctl += ct * ((q & 1) ? dy : dx) * ((q == 0 || q == 3) ? dx : dy);
           }
-          if ((A.flags & EDMD_F_LOG) && S.log && (int64_t)R.nlog < S.log_cap && lane == 0) {
-            edmd_log_entry* lg = (edmd_log_entry*)S.log + R.nlog;
-            lg->i = i; lg->j = j; lg->t = R.t; lg->dx = dx; lg->dy = dy;
-            lg->dvx = dvx; lg->dvy = dvy; lg->f = f;
+          if (A.flags & EDMD_F_LOG) {
+            const double dvo = G.shfl_xor(dv, 2);
+            if (S.log && (int64_t)R.nlog < S.log_cap && lane == 0) {
+              edmd_log_entry* lg = (edmd_log_entry*)S.log + R.nlog;
+              lg->i = i; lg->j = j; lg->t = t; lg->dx = dx; lg->dy = dy;
+              lg->dvx = dv; lg->dvy = dvo; lg->f = f;
+            }
+            R.nlog++;
           }
-          if (A.flags & EDMD_F_LOG) R.nlog++;
-          // lanes 0..3 (mod 4) update i.vx, j.vx, i.vy, j.vy in shared
-          // instructions (v - x computed as v + (-x), the same rounding)
-          {
-            const bool oj = q4 & 1, yax = q4 & 2;
-            const double v = yax ? (oj ? dj.vy : di.vy) : (oj ? dj.vx : di.vx);
-            const double inc = f * (oj ? di.m : dj.m) * (yax ? dy : dx);
-            const double nv = v + flip(inc, oj);
-            di.vx = G.shfl(nv, 0); dj.vx = G.shfl(nv, 1);
-            di.vy = G.shfl(nv, 2); dj.vy = G.shfl(nv, 3);
-          }
-        } else {       // growth rule src/EDMD.c:3479-3520
-          double delta = 0.1 * 0;
-          double res = 0.75 * 0 + 1;
-          double dvr = S.vr[i] + S.vr[j];
-          pbc(B, dx, dy);
-          double dist = sqrt_rn(dx * dx + dy * dy);
-          double dxr = div_rn(dx, dist), dyr = div_rn(dy, dist);
-          double invMass = div_rn(1.0, di.m + dj.m);
-          double collKernel = invMass * (1 + res) * (dxr * dvx + dyr * dvy - dvr);
-          di.vx += collKernel * dj.m * dxr - 2 * dj.m * invMass * delta * dxr;
-          di.vy += collKernel * dj.m * dyr - 2 * dj.m * invMass * delta * dyr;
-          dj.vx -= collKernel * di.m * dxr - 2 * di.m * invMass * delta * dxr;
-          dj.vy -= collKernel * di.m * dyr - 2 * di.m * invMass * delta * dyr;
+          // v_i += f m_j r, v_j -= f m_i r (v - x as v + (-x), the same rounding)
+          own.v += flip(f * mo * d, odd);
+        } else {       // growth rule src/EDMD.c:3479-3520, with its res = 1 and delta = 0
+          const double dvr = own.vr + G.shfl_xor(own.vr, 1);
+          double s2 = d * d;
+          s2 += G.shfl_xor(s2, 2);
+          const double dist = sqrt_rn(s2);
+          const double dr = div_rn(d, dist);
+          double pr = dr * dv;
+          pr += G.shfl_xor(pr, 2);
+          const double inv = mk == 0x4000000000000000ll ? 0.5 : div_rn(1.0, msum);
+          const double collKernel = inv * 2.0 * (pr - dvr);
+          // the rule's second term, 2 m inv delta r, is a zero of r's sign
+          const double delta = 0;
+          own.v += flip(collKernel * mo * dr - 2 * mo * inv * delta * dr, odd);
         }
-        if (lane == 0) { S.d[i] = di; S.d[j] = dj; }
-        G.sync();
-        unqueue(S, R, i, G);
-        unqueue(S, R, j, G);
-        ka = i; kb = j; uq = N + j;
-        pa = i;
-        pb = j;
+        if (lane < 4) {
+          *axis_pos(D, ydim) = own.p;
+          *axis_vel(D, ydim) = own.v;
+          if (!ydim) {
+            D->tl = t;
+            D->coll = hits + 1;
+            if (grow) D->rad = own.rad;
+          }
+        }
+      } else if (stale) {
+        if (lane == 0 || lane == 2) *axis_pos(D, ydim) = own.p;
+        if (lane == 0) {
+          D->tl = t;
+          if (grow) D->rad = own.rad;
+        }
+        R.nstale++;
+      } else {
+        // ---------------- cell crossing (doTheCrossing 2501)
+        R.ncross++;
+        const int from = G.shfl(own.c, 2) * B.Nxc + G.shfl(own.c, 0);
+        int wrap = 0;
+        if (ydim == (E.j >= 3)) {
+          const int n = ydim ? B.Nyc : B.Nxc;
+          if (E.j & 1) { if (own.c - 1 == -1) { own.c = n - 1; wrap = -1; } else own.c -= 1; }
+          else { if (own.c + 1 == n) { own.c = 0; wrap = 1; } else own.c += 1; }
+        }
+        const int to = G.shfl(own.c, 2) * B.Nxc + G.shfl(own.c, 0);
+        if (lane == 0 || lane == 2) {
+          *axis_pos(D, ydim) = own.p;
+          (ydim ? S.cy : S.cx)[i] = own.c;
+          if (wrap) (ydim ? S.crossY : S.crossX)[i] += wrap;
+        }
+        if (lane == 0) {
+          const int pv = S.prv[i], nx = D->nxt;
+          if (pv == NIL) S.head[from] = nx;
+          else S.d[pv].nxt = nx;
+          if (nx != NIL) S.prv[nx] = pv;
+          const int h = S.head[to];
+          S.prv[i] = NIL;
+          D->nxt = h;
+          D->tl = t;
+          if (grow) D->rad = own.rad;
+          S.head[to] = i;
+          if (h != NIL) S.prv[h] = i;
+        }
       }
-    } else if (e < N) {
-      // ---------------- cell crossing (doTheCrossing 2501)
-      const int i = e;
-      R.ncross++;
-      Disk di = S.d[i];
-      grow_fly(S, di, i, R.t, grow);
-      int cx = S.cx[i], cy = S.cy[i];
-      if (lane == 0) {
-        int pv = S.prv[i], nx = di.nxt;
-        if (pv == NIL) S.head[cy * B.Nxc + cx] = nx;
-        else S.d[pv].nxt = nx;
-        if (nx != NIL) S.prv[nx] = pv;
+      // removeEventFromQueue (src/EDMD.c:2209) of the replaced events: every
+      // slot is written again below, so only the overflow list needs work
+      // (lane 0 alone touches its links)
+      unsigned gone = G.ballot(!stale && old_st == ST_OVF);
+      while (gone) {
+        const int q = __ffs(gone) - 1;
+        gone &= gone - 1;
+        const int x = G.shfl(old, q);
+        int first = R.ovf;
+        if (lane == 0) {
+          const int p = S.op[x], n = S.on[x];
+          if (p != NIL) S.on[p] = n;
+          if (n != NIL) S.op[n] = p;
+          if (p == NIL) first = n;
+        }
+        R.ovf = G.shfl(first, 0);
       }
-      int dx = 0, dy = 0;
-      switch (E.j) {
-        case 1: if (cx - 1 == -1) { cx = B.Nxc - 1; dx = -1; } else cx -= 1; break;
-        case 2: if (cx + 1 == B.Nxc) { cx = 0; dx = 1; } else cx += 1; break;
-        case 3: if (cy - 1 == -1) { cy = B.Nyc - 1; dy = -1; } else cy -= 1; break;
-        case 4: if (cy + 1 == B.Nyc) { cy = 0; dy = 1; } else cy += 1; break;
+      // the next crossing (src/EDMD.c:2405-2482): one axis per lane
+      double tc = 0;
+      int dir = 0;
+      if (!stale) {
+        const bool neg = is_neg(own.v);
+        const double a = near_image((neg ? own.c : 1 + own.c) * (ydim ? B.cys : B.cxs) - own.p, ydim ? B.hLy : B.hLx,
+                                    ydim ? B.Ly : B.Lx);
+        const double ta = div_rn(a, own.v);
+        const int da = (ydim ? 3 : 1) + (neg ? 0 : 1);
+        const double tb = G.shfl_xor(ta, 2);
+        const int db = G.shfl_xor(da, 2);
+        const bool ux = lt_i(ydim ? tb : ta, ydim ? ta : tb);
+        tc = ux == ydim ? tb : ta;
+        dir = ux == ydim ? db : da;
       }
       G.sync();
-      if (lane == 0) {
-        int c = cy * B.Nxc + cx;
-        int h = S.head[c];
-        S.cx[i] = cx; S.cy[i] = cy;
-        if (dx) S.crossX[i] += dx;
-        if (dy) S.crossY[i] += dy;
-        S.prv[i] = NIL;
-        di.nxt = h;
-        S.d[i] = di;
-        S.head[c] = i;
-        if (h != NIL) S.prv[h] = i;
+      R.npred += two ? 2 : 1;
+      const Next nx = predict2<GW, ADD>(S, t, grow, i, two ? j : -1, own, &R.npair, G, sm, &ovl, &oa, &ob);
+      // addEventToQueue (src/EDMD.c:2144): lanes 0 and 1 take the crossings of
+      // the two disks, lanes 2 and 3 their collisions; in that order they get
+      // the insertion counters and join the overflow list
+      const unsigned who = stale ? 4u : two ? 15u : 5u;
+      const bool mine = lane < 4 && ((who >> lane) & 1u);
+      Ev ev;
+      ev.t = t + (ydim ? key_time(nx.key) : tc);
+      ev.j = ydim ? nx.partner : dir;
+      ev.ca = ydim ? nx.ca : 0;
+      const int slot = (ydim ? N : 0) + my;
+      const uint64_t C = R.C + __popc(who & ((1u << lane) - 1u));
+      const int place = mine ? sched_place(S, R, ev.t) : 0;
+      sched_key(R, C, 2ull, place, ev);
+      R.C += __popc(who);
+      unsigned over = G.ballot(mine && place == -2);
+      while (over) {
+        const int q = __ffs(over) - 1;
+        over &= over - 1;
+        const int x = G.shfl(slot, q);
+        if (lane == 0) {
+          S.on[x] = R.ovf; S.op[x] = NIL;
+          if (R.ovf != NIL) S.op[R.ovf] = x;
+        }
+        R.ovf = x;
       }
-      G.sync();
-      ka = i; uq = N + i;
-      pa = i;
-    } else if (e == 2 * N + SP_SCREEN) {
-      // ---------------- screenshot (takeAScreenshot 4657): free-fly everything
-      for (int i = lane; i < N; i += GW) {
-        Disk p = S.d[i];
-        grow_fly(S, p, i, R.t, grow);
-        S.d[i] = p;
+      if (mine) S.ev[slot] = ev;
+      else if (stale && lane == 0) ev = S.ev[slot];      // the crossing that stays
+      // the leaves: the earlier of a disk's two events
+      Node n = empty_node(slot);
+      if (ev.st == ST_QUEUED) n = ev_node(ev, slot);
+      {
+        Node o;
+        o.tk = G.shfl_xor(n.tk, 2); o.tie = G.shfl_xor(n.tie, 2);
+        o.b = G.shfl_xor(n.b, 2); o.idx = G.shfl_xor(n.idx, 2);
+        if (node_less(o, n)) n = o;
       }
-      G.sync();
-      se0 = e; sT0 = R.t + S.dtime;
-      la = N + SP_SCREEN;
-      if (A.flags & EDMD_F_STOP_AT_SCREEN) { stop = EDMD_STOP_SCREEN; }
-    } else if (e == 2 * N + SP_THERMO) {
-      gather_virial(R, ctl, G);
-      do_thermo(S, R, G);
-      ctl = R.collT[lane & 3];
-      se0 = e; sT0 = R.t + S.dtimeTh;
-      la = N + SP_THERMO;
+      path_update(S, i, two ? j : -1, shfl_node(n, 0, G), shfl_node(n, 1, G), G);
     } else {
-      do_growstop<GW, ADD>(S, R, G, sm, &ovl, &oa, &ob);
-      if (A.flags & EDMD_F_STOP_AT_GROW) stop = EDMD_STOP_GROW;
+      if (lane == 0) S.ev[e].st = ST_NONE;
+      G.sync();
+      bool again = true;
+      double next = 0;
+      if (e == 2 * N + SP_SCREEN) {
+        // ---------------- screenshot (takeAScreenshot 4657): free-fly everything
+        for (int i = lane; i < N; i += GW) {
+          Disk p = S.d[i];
+          grow_fly(S, p, i, t, grow);
+          S.d[i] = p;
+        }
+        G.sync();
+        next = t + S.dtime;
+        if (A.flags & EDMD_F_STOP_AT_SCREEN) { stop = EDMD_STOP_SCREEN; }
+      } else if (e == 2 * N + SP_THERMO) {
+        gather_virial(R, ctl, G);
+        do_thermo(S, R, G);
+        ctl = R.collT[lane & 3];
+        next = t + S.dtimeTh;
+      } else {
+        do_growstop<GW, ADD>(S, R, G, sm, &ovl, &oa, &ob);
+        if (A.flags & EDMD_F_STOP_AT_GROW) stop = EDMD_STOP_GROW;
+        again = false;
+      }
+      if (again) {
+        schedule(S, R, e, next, 0, 0, 2ull, G);
+        leaf_update(S, N + (e - 2 * N), G);
+      }
     }
-    // the tail shared by the handlers: new crossing events of the one or two
-    // disks that changed (crossingEvent for i, then j; even lanes take i,
-    // odd lanes j), the removal of the collision event they replace, new
-    // collision events (collisionEvent for i, then j), the insertion of the
-    // handler's new events, and the tree paths of the changed leaves
-    if (ka >= 0) {
-      const int k = (lane & 1) && kb >= 0 ? kb : ka;
-      const Disk dk = S.d[k];
-      int dir;
-      const double tc = crossing_time_grp(B, dk, S.cx[k], S.cy[k], R.t, G, 2, &dir);
-      schedule2(S, R, ka, G.shfl(tc, 0), G.shfl(dir, 0), 0,
-                kb, G.shfl(tc, 1), G.shfl(dir, 1), 0, G);
-      unqueue(S, R, uq, G);
-    }
-    if (pa >= 0) {
-      Pred r0, r1;
-      predict2<GW, ADD>(S, R, pa, pb, r0, r1, G, sm, &ovl, &oa, &ob);
-      const double tn = R.t + ((lane & 1) ? r1.dt : r0.dt);
-      se0 = N + pa; sT0 = G.shfl(tn, 0); sj0 = r0.partner; sca0 = r0.ca;
-      if (pb >= 0) { se1 = N + pb; sT1 = G.shfl(tn, 1); sj1 = r1.partner; sca1 = r1.ca; }
-      la = pa;
-      lb = pb;
-    }
-    if (se0 >= 0) schedule2(S, R, se0, sT0, sj0, sca0, se1, sT1, sj1, sca1, G);
-    G.sync();
-    if (la >= 0) leaf_update(S, la, lb, G);
     if (ovl) { status = oa == OVL_CORRUPT ? EDMD_ERR_BUDGET : EDMD_ERR_OVERLAP; break; }
     if (stop) break;
   }
