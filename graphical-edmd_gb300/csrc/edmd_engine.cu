@@ -228,10 +228,26 @@ __device__ __noinline__ void tree_rebuild(const SysDev& S, const Grp<GW>& G) {
 
 // ---------------------------------------------------------------- queue
 
+// the queue's scalar state; out-of-line functions take and return it by value,
+// so that the event loop's copy stays in registers
+struct Queue {
+  double P;                      // paulTime of the current bucket
+  uint64_t C, k, next_wrap;      // insertion counter, current bucket, next overflow wrap
+  int32_t ovf;                   // head of the overflow list
+};
+__device__ __forceinline__ Queue queue_of(const SysState& R) {
+  Queue q;
+  q.P = R.P; q.C = R.C; q.k = R.k; q.next_wrap = R.next_wrap; q.ovf = R.ovf;
+  return q;
+}
+__device__ __forceinline__ void queue_to(SysState& R, const Queue& q) {
+  R.P = q.P; R.C = q.C; R.k = q.k; R.next_wrap = q.next_wrap; R.ovf = q.ovf;
+}
+
 // addEventToQueue (src/EDMD.c:2144) in key form, in two parts: where the
 // event goes (FP64: its offset from paulTime; -1 current bucket, -2
 // overflow, else the bucket offset), and the insertion (integer work).
-__device__ __forceinline__ int sched_place(const SysDev& S, const SysState& R, double T) {
+__device__ __forceinline__ int sched_place(const SysDev& S, const Queue& R, double T) {
   const Box& B = S.B;
   const double dt = T - R.P;
   if (!ge_pos(dt, B.dtP)) return -1;           // dt < dtPaul
@@ -242,7 +258,7 @@ __device__ __forceinline__ int sched_place(const SysDev& S, const SysState& R, d
 // queue key and state of an event placed at `place` with insertion counter C;
 // `cls_direct` is 2 for a schedule from an event handler and 0 for the
 // re-add done by a wrap
-__device__ __forceinline__ void sched_key(const SysState& R, uint64_t C, uint64_t cls_direct, int place, Ev& ev) {
+__device__ __forceinline__ void sched_key(const Queue& R, uint64_t C, uint64_t cls_direct, int place, Ev& ev) {
   if (place == -1) {
     ev.b = (uint32_t)R.k; ev.tie = (cls_direct << 62) | C; ev.st = ST_QUEUED;
   } else if (place == -2) {
@@ -253,7 +269,7 @@ __device__ __forceinline__ void sched_key(const SysState& R, uint64_t C, uint64_
 }
 
 template <int GW>
-__device__ __forceinline__ void sched_insert(const SysDev& S, SysState& R, int e, double T, int32_t j,
+__device__ __forceinline__ void sched_insert(const SysDev& S, Queue& R, int e, double T, int32_t j,
                                              uint32_t ca, uint64_t cls_direct, int place, const Grp<GW>& G) {
   const int lane = G.lane;
   Ev ev;
@@ -272,14 +288,14 @@ __device__ __forceinline__ void sched_insert(const SysDev& S, SysState& R, int e
 }
 
 template <int GW>
-__device__ void schedule(const SysDev& S, SysState& R, int e, double T, int32_t j, uint32_t ca,
+__device__ void schedule(const SysDev& S, Queue& R, int e, double T, int32_t j, uint32_t ca,
                          uint64_t cls_direct, const Grp<GW>& G) {
   sched_insert(S, R, e, T, j, ca, cls_direct, sched_place(S, R, T), G);
 }
 
 // removeEventFromQueue (src/EDMD.c:2209) in key form
 template <int GW>
-__device__ void unqueue(const SysDev& S, SysState& R, int e, const Grp<GW>& G) {
+__device__ void unqueue(const SysDev& S, Queue& R, int e, const Grp<GW>& G) {
   const int lane = G.lane;
   uint32_t st = S.ev[e].st;
   if (st == ST_OVF) {
@@ -296,9 +312,10 @@ __device__ void unqueue(const SysDev& S, SysState& R, int e, const Grp<GW>& G) {
 
 // the overflow bucket is redistributed when the calendar wraps
 // (addNextPaulEvent src/EDMD.c:2287-2300)
-// (false: the list is longer than it can be, i.e. corrupt)
+// (head OVF_CORRUPT: the list is longer than it can be, i.e. corrupt)
+constexpr int32_t OVF_CORRUPT = -2;
 template <int GW>
-__device__ __noinline__ bool do_wrap(const SysDev& S, SysState& R, const Grp<GW>& G) {
+__device__ __noinline__ Queue do_wrap(const SysDev& S, Queue R, Grp<GW> G) {
   const int N = S.B.N;
   int e = R.ovf;
   R.ovf = NIL;
@@ -315,7 +332,9 @@ __device__ __noinline__ bool do_wrap(const SysDev& S, SysState& R, const Grp<GW>
     leaf_update(S, leaf, G);
     e = n;
   }
-  return e == NIL;
+  R.next_wrap += (uint64_t)N;
+  if (e != NIL) R.ovf = OVF_CORRUPT;
+  return R;
 }
 
 // ---------------------------------------------------------------- prediction
@@ -374,10 +393,10 @@ __device__ __forceinline__ void best_merge(uint64_t& bk, int& bo, int& bp, uint3
 // Same operations and roundings as coll_time_normal_i / coll_time_grow (the
 // sums of two products commute).  Every lane of the group takes part; `act`
 // marks the pairs that count.
-template <int GW, bool ADD>
+template <int GW, bool ADD, bool GROW>
 __device__ __forceinline__ double pair_time_lanes(const Box& B, const Grp<GW>& G, bool act, double p1, double v1,
                                                   double rad1, double vr1, const Disk* P, const double* vr2p,
-                                                  double t, bool grow, bool* ovl) {
+                                                  double t, bool* ovl) {
   const bool y = G.lane & 1;
   const double pos = (&P->x)[y ? 1 : 0], vel = (&P->vx)[y ? 1 : 0], rad2 = P->rad;
   const double lat2 = t - P->tl;
@@ -387,7 +406,7 @@ __device__ __forceinline__ double pair_time_lanes(const Box& B, const Grp<GW>& G
   b += G.shfl_xor(b, 1);
   v2 += G.shfl_xor(v2, 1);
   d2 += G.shfl_xor(d2, 1);
-  if (!grow) {
+  if constexpr (!GROW) {
     d2 -= contact2<ADD>(B, rad1, rad2);
     // b b on the y lane, v2 d2 on the x lane
     const double u = (y ? b : v2) * (y ? b : d2);
@@ -397,7 +416,7 @@ __device__ __forceinline__ double pair_time_lanes(const Box& B, const Grp<GW>& G
     if (lt_neg(d2, 0.01)) { *ovl = true; return NEVER; }
     if (is_neg(det)) return NEVER;
     return div_rn(-b - sqrt_rn(det), v2);
-  }
+  } else {
   const double vr2 = *vr2p;
   const double dvr = vr1 + vr2;
   const double dr = contact(B, rad1, rad2 + lat2 * vr2);
@@ -419,6 +438,7 @@ __device__ __forceinline__ double pair_time_lanes(const Box& B, const Grp<GW>& G
     return plus;
   if (gap < -0.01) *ovl = true;
   return NEVER;
+  }
 }
 
 // group-relative lane of the least (time key, scan order), word by word like
@@ -449,13 +469,13 @@ __device__ __forceinline__ int best_lane(uint64_t k, int o, const Grp<GW>& G) {
 // scan order) and 9..17 (a1's): task t runs on lane t % GW, a lane with two
 // tasks walks both lists at once.  The candidates are then packed over the
 // group in task order and solved by two lanes each.
-template <int GW, bool ADD>
-__device__ __forceinline__ Next predict2(const SysDev& S, double t, bool grow, int a0, int a1, const Own& own,
+template <int GW, bool ADD, bool GROW>
+__device__ __forceinline__ Next predict2(const SysDev& S, double t, int a0, int a1, const Own& own,
                                          uint64_t* npair, const Grp<GW>& G, WarpSmem* sm, bool* ovl, int* ovl_a,
                                          int* ovl_b) {
   const Box& B = S.B;
   const int lane = G.lane;
-  const double dinit = grow ? 10000000 : NEVER;
+  const double dinit = GROW ? 10000000 : NEVER;
   const int ntask = a1 >= 0 ? 18 : 9;
   const int X0 = G.shfl(own.c, 0), X1 = G.shfl(own.c, 1), Y0 = G.shfl(own.c, 2), Y1 = G.shfl(own.c, 3);
   // the tasks of this lane: t = lane + k GW, k < NT (a warp: one task per
@@ -536,14 +556,14 @@ __device__ __forceinline__ Next predict2(const SysDev& S, double t, bool grow, i
       const bool g1 = act && f >= tot0;
       const int src = (g1 ? 1 : 0) | ((lane & 1) << 1);
       const double p1 = G.shfl(own.p, src), v1 = G.shfl(own.v, src), rad1 = G.shfl(own.rad, src);
-      const double vr1 = grow ? G.shfl(own.vr, src) : 0.0;
+      const double vr1 = GROW ? G.shfl(own.vr, src) : 0.0;
       const int p = act ? sm->comp[f] : a0;
       const int o = act ? sm->ord[f] : 0;
       const Disk* P = S.d + p;
       const uint32_t pc = P->coll;
       bool ov = false;
       const uint64_t kd =
-          cand_key(pair_time_lanes<GW, ADD>(B, G, act, p1, v1, rad1, vr1, P, S.vr + p, t, grow, &ov));
+          cand_key(pair_time_lanes<GW, ADD, GROW>(B, G, act, p1, v1, rad1, vr1, P, S.vr + p, t, &ov));
       if (ov) {
         const uint32_t k = ((uint32_t)(f % GW) << 16) | (0xffffu - (uint32_t)f);
         if (k < lk) { lk = k; la = g1 ? a1 : a0; lb = p; }
@@ -562,7 +582,7 @@ __device__ __forceinline__ Next predict2(const SysDev& S, double t, bool grow, i
       const int q = g1 ? u - 9 : u, a = g1 ? a1 : a0;
       const int src = (g1 ? 1 : 0) | ((lane & 1) << 1);
       const double p1 = G.shfl(own.p, src), v1 = G.shfl(own.v, src), rad1 = G.shfl(own.rad, src);
-      const double vr1 = grow ? G.shfl(own.vr, src) : 0.0;
+      const double vr1 = GROW ? G.shfl(own.vr, src) : 0.0;
       int p = S.head[pbc_cy(B, (g1 ? Y1 : Y0) + q / 3 - 1) * B.Nxc + pbc_cx(B, (g1 ? X1 : X0) + q % 3 - 1)];
       int k = 0, guard = 0;
       while (p != NIL && guard++ < B.N) {
@@ -571,7 +591,7 @@ __device__ __forceinline__ Next predict2(const SysDev& S, double t, bool grow, i
         if (p != a) {
           bool ov = false;
           const uint64_t kd =
-              cand_key(pair_time_lanes<GW, ADD>(B, G, true, p1, v1, rad1, vr1, P, S.vr + p, t, grow, &ov));
+              cand_key(pair_time_lanes<GW, ADD, GROW>(B, G, true, p1, v1, rad1, vr1, P, S.vr + p, t, &ov));
           if (ov) {
             const uint32_t w = ((uint32_t)(u % GW) << 16) | (0xffffu - (uint32_t)(u * 2048 + min(k, 2047)));
             if (w < lk) { lk = w; la = a; lb = p; }
@@ -645,7 +665,7 @@ __device__ __noinline__ void physical_q(const SysDev& S, const Grp<GW>& G, doubl
 
 // takeAThermo + saveThermo (src/EDMD.c:4679, 5232-5697) with Nthermo = 1
 template <int GW>
-__device__ __noinline__ void do_thermo(const SysDev& S, SysState& R, const Grp<GW>& G) {
+__device__ void do_thermo(const SysDev& S, SysState& R, const Grp<GW>& G) {
   const int lane = G.lane;
   const int N = S.B.N;
   double E, px, py;
@@ -685,7 +705,7 @@ __device__ __noinline__ void do_thermo(const SysDev& S, SysState& R, const Grp<G
 
 // stopGrow (src/EDMD.c:4740-4800)
 template <int GW, bool ADD>
-__device__ __noinline__ void do_growstop(const SysDev& S, SysState& R, const Grp<GW>& G, WarpSmem* sm,
+__device__ void do_growstop(const SysDev& S, SysState& R, const Grp<GW>& G, WarpSmem* sm,
                             bool* ovl, int* oa, int* ob) {
   const int lane = G.lane;
   const int N = S.B.N;
@@ -717,56 +737,81 @@ __device__ __noinline__ void do_growstop(const SysDev& S, SysState& R, const Grp
     S.d[i] = p;
   }
   G.sync();
+  Queue Q = queue_of(R);
   for (int i = 0; i < N; i++) {
     uint32_t c = S.d[i].coll + 1;
     if (lane == 0) S.d[i].coll = c;
     G.sync();
-    unqueue(S, R, N + i, G);
+    unqueue(S, Q, N + i, G);
     Own own;
     own.p = *axis_pos(S.d + i, lane & 2); own.v = *axis_vel(S.d + i, lane & 2); own.rad = S.d[i].rad;
     own.vr = 0;
     own.c = (lane & 2 ? S.cy : S.cx)[i];
     R.npred++;
-    const Next r = predict2<GW, ADD>(S, R.t, false, i, -1, own, &R.npair, G, sm, ovl, oa, ob);
-    schedule(S, R, N + i, R.t + key_time(r.key), r.partner, r.ca, 2ull, G);
-    unqueue(S, R, i, G);
+    const Next r = predict2<GW, ADD, false>(S, R.t, i, -1, own, &R.npair, G, sm, ovl, oa, ob);
+    schedule(S, Q, N + i, R.t + key_time(r.key), r.partner, r.ca, 2ull, G);
+    unqueue(S, Q, i, G);
     int dir;
     Disk p = S.d[i];
     double tc = crossing_time_i(S.B, p, S.cx[i], S.cy[i], R.t, &dir);
-    schedule(S, R, i, tc, dir, 0, 2ull, G);
+    schedule(S, Q, i, tc, dir, 0, 2ull, G);
     G.sync();
   }
+  queue_to(R, Q);
   tree_rebuild(S, G);
 }
 
 // ---------------------------------------------------------------- run loop
 
-// the four virial sums live on lanes 0..3 (lane l accumulates term l % 4)
-// during the event loop; every lane gets all four back here
+// what ends a stretch of disk events
+enum { END_STOP, END_SPECIAL };
+
+// A product per quad of lanes in one FP64 instruction: quad 0 (lanes 0..3 of
+// every 16) takes a b, quad 1 c d, quad 2 e f, and every lane gets the last two
+// back.  Groups too narrow for that multiply in turn.
 template <int GW>
-__device__ __forceinline__ void gather_virial(SysState& R, double ctl, const Grp<GW>& G) {
-#pragma unroll
-  for (int k = 0; k < 4; k++) R.collT[k] = G.shfl(ctl, k);
+__device__ __forceinline__ double quad_products(const Grp<GW>& G, double a, double b, double c, double d, double e,
+                                                double f, double* cd, double* ef) {
+  if constexpr (GW >= 16) {
+    const int q = (G.lane >> 2) & 3;
+    const double r = (q == 0 ? a : q == 1 ? c : e) * (q == 0 ? b : q == 1 ? d : f);
+    *cd = G.shfl(r, 4);
+    *ef = G.shfl(r, 8);
+    return r;
+  } else {
+    *cd = c * d;
+    *ef = e * f;
+    return a * b;
+  }
 }
 
-// The event loop of one system.  One event is one chain of dependent
-// instructions, so its latency is what counts (a single system) and its FP64
-// instructions (a full GPU).  Both disks and both axes share the scalar FP64
-// work (struct Own), the two or four events an event schedules are placed and
-// stored by one lane each, and a changed leaf of the tree is built from those
-// lanes' registers.
+// A stretch of disk events of one system: until a stop, or a special event
+// (screenshot, thermo, growth stop), which is taken off the queue and left in
+// *special.  One event is one chain of dependent instructions, so its latency
+// is what counts (a single system), and its FP64 instructions and code size (a
+// full GPU).  Both disks and both axes share the scalar FP64 work (struct
+// Own), the two or four events an event schedules are placed and stored by one
+// lane each, a changed leaf of the tree is built from those lanes' registers,
+// and the scalar state is held in registers: the growth phase has its own copy
+// of the loop, and everything rare is left to serve_special.
 // ADD = false: a context without additive-contact systems (the rule's
 // switch compiled out of the pair solves and the collision rule)
-template <int GW, bool ADD = true>
-__device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, const Grp<GW>& G,
-                           WarpSmem* sm) {
+template <int GW, bool ADD, bool GROW>
+__device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int64_t max_coll, const Grp<GW>& G,
+                                          WarpSmem* sm, int64_t& logged, int64_t& nev, int* special) {
+  constexpr bool QUADS = GW >= 16;
   const int lane = G.lane;
   const bool odd = lane & 1, ydim = lane & 2;
+  const bool quad1 = ((lane >> 2) & 3) == 1;
   const Box& B = S.B;
   const int N = B.N;
-  SysState R = *S.st;
-  if (R.status != EDMD_OK) return;
-  double ctl = R.collT[lane & 3];      // this lane's virial term, see gather_virial
+  SysState* const st = S.st;
+  double t = st->t;
+  Queue Q = queue_of(*st);
+  // the four virial sums: lane l accumulates term l % 4 (the lanes of quad 1
+  // count, or of the only quad)
+  double ctl = st->collT[lane & 3];
+  const double tmax = S.tmax;
   const double onepr = 1 + S.res;
   // (1 + res) / (m_i + m_j) of the last two mass sums: a repeated quotient and
   // product give the same bits.  2 is first (1 / 2 is exact); no sum is +0
@@ -776,39 +821,43 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
   }
   G.sync();
   const int root = S.lev_off[S.nlev - 1];
-  int64_t logged = 0, nev = 0;
-  int stop = 0, status = EDMD_OK;
+  uint64_t ncoll = 0, nstale = 0, npair = 0, nlog = st->nlog;
+  const uint64_t ntrace0 = st->ntrace;
+  const int64_t nev0 = nev;
+  int stop = 0, status = EDMD_OK, end = END_STOP;
   bool ovl = false;
   int oa = -1, ob = -1;
   for (;;) {
-    if (!le_i(R.t, S.tmax)) { stop = EDMD_STOP_TMAX; break; }
+    if (!le_i(t, tmax)) { stop = EDMD_STOP_TMAX; break; }
     if (logged >= max_coll) { stop = EDMD_STOP_COLL; break; }
     if (nev >= A.max_events) { status = EDMD_ERR_BUDGET; break; }
     Node r;
     int guard = 0;
     for (;;) {
       r = S.tree[root];
-      if (r.b == BINF || (uint64_t)r.b >= R.next_wrap) {
-        if (r.b == BINF && R.ovf == NIL) { status = EDMD_ERR_BUDGET; break; }
-        while (R.k < R.next_wrap) { R.P += B.dtP; R.k++; }
-        if (!do_wrap(S, R, G)) { status = EDMD_ERR_BUDGET; break; }
-        R.next_wrap += (uint64_t)N;
+      if (r.b == BINF || (uint64_t)r.b >= Q.next_wrap) {
+        if (r.b == BINF && Q.ovf == NIL) { status = EDMD_ERR_BUDGET; break; }
+        while (Q.k < Q.next_wrap) { Q.P += B.dtP; Q.k++; }
+        Q = do_wrap(S, Q, G);
+        if (Q.ovf == OVF_CORRUPT) { Q.ovf = NIL; status = EDMD_ERR_BUDGET; break; }
         if (++guard > (1 << 20)) { status = EDMD_ERR_BUDGET; break; }
         continue;
       }
-      while (R.k < (uint64_t)r.b) { R.P += B.dtP; R.k++; }
+      while (Q.k < (uint64_t)r.b) { Q.P += B.dtP; Q.k++; }
       break;
     }
     if (status != EDMD_OK) break;
     const int e = r.idx;
     const Ev E = S.ev[e];
     if (le_i(A.t_stop, E.t)) { stop = EDMD_STOP_TIME; break; }
-    const double t = E.t;
-    R.t = t;
+    t = E.t;
     nev++;
-    R.nevents++;
-    const bool grow = R.grow != 0;
-    if (e < 2 * N) {
+    if (e >= 2 * N) {
+      *special = e;
+      end = END_SPECIAL;
+      break;
+    }
+    {
       const bool coll = e >= N;
       const int i = coll ? e - N : e, j = coll ? E.j : i;
       const int my = odd ? j : i;
@@ -816,7 +865,7 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
       Own own;
       own.p = *axis_pos(D, ydim); own.v = *axis_vel(D, ydim); own.rad = D->rad;
       own.c = (ydim ? S.cy : S.cx)[my];
-      own.vr = grow ? S.vr[my] : 0.0;
+      own.vr = GROW ? S.vr[my] : 0.0;
       const double m = D->m;
       const uint32_t hits = D->coll;
       // events replaced by this one's, beside the popped one: the crossings of
@@ -830,23 +879,21 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
         own.p += dt * own.v;
         if (is_neg(own.p)) own.p += L;
         else if (ge_pos(own.p, L)) own.p -= L;
-        if (grow) own.rad += dt * own.vr;
+        if (GROW) own.rad += dt * own.vr;
       }
       const bool stale = coll && E.ca != G.shfl(hits, 1);
       const bool two = coll && !stale;       // a second disk changes
       if (two) {
         // ---------------- collision (doTheCollisionNormal 3542 / Grow 3465)
-        if ((A.flags & EDMD_F_TRACE) && S.trace && (int64_t)R.ntrace < S.trace_cap) {
+        if ((A.flags & EDMD_F_TRACE) && S.trace && (int64_t)(ntrace0 + ncoll) < S.trace_cap) {
           const int ci = G.shfl(own.c, 2) * B.Nxc + G.shfl(own.c, 0), cj = G.shfl(own.c, 3) * B.Nxc + G.shfl(own.c, 1);
           if (lane == 0) {
-            edmd_collision* tr = (edmd_collision*)S.trace + R.ntrace;
+            edmd_collision* tr = (edmd_collision*)S.trace + (ntrace0 + ncoll);
             tr->i = i; tr->j = j; tr->cell_i = ci; tr->cell_j = cj; tr->t = t;
           }
         }
-        R.ntrace++;
-        if (!(A.flags & EDMD_F_COUNT_NORMAL) || !grow) logged++;
-        R.ncol++;
-        R.ncol_total++;
+        ncoll++;
+        if (!GROW || !(A.flags & EDMD_F_COUNT_NORMAL)) logged++;
         // j minus i, the same value on both disks' lanes
         const double po = G.shfl_xor(own.p, 1), vo = G.shfl_xor(own.v, 1);
         const double mo = G.shfl_xor(m, 1), ro = G.shfl_xor(own.rad, 1);
@@ -854,9 +901,17 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
         const double dv = (odd ? own.v : vo) - (odd ? vo : own.v);
         const double msum = m + mo;
         const long long mk = __double_as_longlong(msum);
-        if (!grow) {   // elastic branch src/EDMD.c:3802-3827
-          double pr = d * dv;
-          pr += G.shfl_xor(pr, 2);
+        if constexpr (!GROW) {   // elastic branch src/EDMD.c:3802-3827
+          // (r . v), sigma^2 and m_i m_j
+          double distSquared, mm, pr;
+          if (ADD && B.additive) {
+            const double s = own.rad + ro;
+            pr = quad_products(G, d, dv, s, s, m, mo, &distSquared, &mm);
+          } else {
+            pr = quad_products(G, d, dv, times4(own.rad), ro, m, mo, &distSquared, &mm);
+          }
+          if constexpr (QUADS) pr = G.shfl(pr, 0) + G.shfl(pr, 2);
+          else pr += G.shfl_xor(pr, 2);
           double inv;
           if (mk == sm->msum[0]) inv = sm->inv[0];
           else if (mk == sm->msum[1]) inv = sm->inv[1];
@@ -870,31 +925,35 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
             G.sync();
           }
           const double collKernel = inv * pr;
-          // sigma^2 and m_i m_j
-          const double distSquared = contact2<ADD>(B, odd ? ro : own.rad, odd ? own.rad : ro);
-          const double mm = (odd ? mo : m) * (odd ? m : mo);
           // x/4 is exact, so the shortcut rounds identically
           const double f = __double_as_longlong(distSquared) == 0x4010000000000000ll
               ? collKernel * 0.25 : div_rn(collKernel, distSquared);
           const double od = G.shfl_xor(d, 2);
           const double dx = ydim ? od : d, dy = ydim ? d : od;
-          {
-            // collTermX, Y, XY, YX: term lane % 4 on each lane
-            const int q = lane & 3;
-            const double ct = mm * f;
-            ctl += ct * ((q & 1) ? dy : dx) * ((q == 0 || q == 3) ? dx : dy);
-          }
           if (A.flags & EDMD_F_LOG) {
             const double dvo = G.shfl_xor(dv, 2);
-            if (S.log && (int64_t)R.nlog < S.log_cap && lane == 0) {
-              edmd_log_entry* lg = (edmd_log_entry*)S.log + R.nlog;
+            if (S.log && (int64_t)nlog < S.log_cap && lane == 0) {
+              edmd_log_entry* lg = (edmd_log_entry*)S.log + nlog;
               lg->i = i; lg->j = j; lg->t = t; lg->dx = dx; lg->dy = dy;
               lg->dvx = dv; lg->dvy = dvo; lg->f = f;
             }
-            R.nlog++;
+            nlog++;
           }
-          // v_i += f m_j r, v_j -= f m_i r (v - x as v + (-x), the same rounding)
-          own.v += flip(f * mo * d, odd);
+          // v_i += f m_j r, v_j -= f m_i r (v - x as v + (-x), the same rounding),
+          // and collTermX, Y, XY, YX: term lane % 4, m_i m_j f r_a r_b, beside
+          // it on quad 1
+          const double ra = odd ? dy : dx, rb = ydim == odd ? dx : dy;
+          if constexpr (QUADS) {
+            const double w1 = f * (quad1 ? mm : mo);
+            const double w2 = w1 * (quad1 ? ra : d);
+            const double w3 = w2 * rb;
+            const double s = (quad1 ? ctl : own.v) + (quad1 ? w3 : flip(w2, odd));
+            if (quad1) ctl = s;
+            else own.v = s;
+          } else {
+            ctl += mm * f * ra * rb;
+            own.v += flip(f * mo * d, odd);
+          }
         } else {       // growth rule src/EDMD.c:3479-3520, with its res = 1 and delta = 0
           const double dvr = own.vr + G.shfl_xor(own.vr, 1);
           double s2 = d * d;
@@ -915,19 +974,18 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
           if (!ydim) {
             D->tl = t;
             D->coll = hits + 1;
-            if (grow) D->rad = own.rad;
+            if (GROW) D->rad = own.rad;
           }
         }
       } else if (stale) {
         if (lane == 0 || lane == 2) *axis_pos(D, ydim) = own.p;
         if (lane == 0) {
           D->tl = t;
-          if (grow) D->rad = own.rad;
+          if (GROW) D->rad = own.rad;
         }
-        R.nstale++;
+        nstale++;
       } else {
         // ---------------- cell crossing (doTheCrossing 2501)
-        R.ncross++;
         const int from = G.shfl(own.c, 2) * B.Nxc + G.shfl(own.c, 0);
         int wrap = 0;
         if (ydim == (E.j >= 3)) {
@@ -950,7 +1008,7 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
           S.prv[i] = NIL;
           D->nxt = h;
           D->tl = t;
-          if (grow) D->rad = own.rad;
+          if (GROW) D->rad = own.rad;
           S.head[to] = i;
           if (h != NIL) S.prv[h] = i;
         }
@@ -963,14 +1021,14 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
         const int q = __ffs(gone) - 1;
         gone &= gone - 1;
         const int x = G.shfl(old, q);
-        int first = R.ovf;
+        int first = Q.ovf;
         if (lane == 0) {
           const int p = S.op[x], n = S.on[x];
           if (p != NIL) S.on[p] = n;
           if (n != NIL) S.op[n] = p;
           if (p == NIL) first = n;
         }
-        R.ovf = G.shfl(first, 0);
+        Q.ovf = G.shfl(first, 0);
       }
       // the next crossing (src/EDMD.c:2405-2482): one axis per lane
       double tc = 0;
@@ -988,8 +1046,7 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
         dir = ux == ydim ? db : da;
       }
       G.sync();
-      R.npred += two ? 2 : 1;
-      const Next nx = predict2<GW, ADD>(S, t, grow, i, two ? j : -1, own, &R.npair, G, sm, &ovl, &oa, &ob);
+      const Next nx = predict2<GW, ADD, GROW>(S, t, i, two ? j : -1, own, &npair, G, sm, &ovl, &oa, &ob);
       // addEventToQueue (src/EDMD.c:2144): lanes 0 and 1 take the crossings of
       // the two disks, lanes 2 and 3 their collisions; in that order they get
       // the insertion counters and join the overflow list
@@ -1000,20 +1057,20 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
       ev.j = ydim ? nx.partner : dir;
       ev.ca = ydim ? nx.ca : 0;
       const int slot = (ydim ? N : 0) + my;
-      const uint64_t C = R.C + __popc(who & ((1u << lane) - 1u));
-      const int place = mine ? sched_place(S, R, ev.t) : 0;
-      sched_key(R, C, 2ull, place, ev);
-      R.C += __popc(who);
+      const uint64_t C = Q.C + __popc(who & ((1u << lane) - 1u));
+      const int place = mine ? sched_place(S, Q, ev.t) : 0;
+      sched_key(Q, C, 2ull, place, ev);
+      Q.C += __popc(who);
       unsigned over = G.ballot(mine && place == -2);
       while (over) {
         const int q = __ffs(over) - 1;
         over &= over - 1;
         const int x = G.shfl(slot, q);
         if (lane == 0) {
-          S.on[x] = R.ovf; S.op[x] = NIL;
-          if (R.ovf != NIL) S.op[R.ovf] = x;
+          S.on[x] = Q.ovf; S.op[x] = NIL;
+          if (Q.ovf != NIL) S.op[Q.ovf] = x;
         }
-        R.ovf = x;
+        Q.ovf = x;
       }
       if (mine) S.ev[slot] = ev;
       else if (stale && lane == 0) ev = S.ev[slot];      // the crossing that stays
@@ -1027,45 +1084,88 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
         if (node_less(o, n)) n = o;
       }
       path_update(S, i, two ? j : -1, shfl_node(n, 0, G), shfl_node(n, 1, G), G);
-    } else {
-      if (lane == 0) S.ev[e].st = ST_NONE;
-      G.sync();
-      bool again = true;
-      double next = 0;
-      if (e == 2 * N + SP_SCREEN) {
-        // ---------------- screenshot (takeAScreenshot 4657): free-fly everything
-        for (int i = lane; i < N; i += GW) {
-          Disk p = S.d[i];
-          grow_fly(S, p, i, t, grow);
-          S.d[i] = p;
-        }
-        G.sync();
-        next = t + S.dtime;
-        if (A.flags & EDMD_F_STOP_AT_SCREEN) { stop = EDMD_STOP_SCREEN; }
-      } else if (e == 2 * N + SP_THERMO) {
-        gather_virial(R, ctl, G);
-        do_thermo(S, R, G);
-        ctl = R.collT[lane & 3];
-        next = t + S.dtimeTh;
-      } else {
-        do_growstop<GW, ADD>(S, R, G, sm, &ovl, &oa, &ob);
-        if (A.flags & EDMD_F_STOP_AT_GROW) stop = EDMD_STOP_GROW;
-        again = false;
-      }
-      if (again) {
-        schedule(S, R, e, next, 0, 0, 2ull, G);
-        leaf_update(S, N + (e - 2 * N), G);
-      }
     }
     if (ovl) { status = oa == OVL_CORRUPT ? EDMD_ERR_BUDGET : EDMD_ERR_OVERLAP; break; }
-    if (stop) break;
   }
-  gather_virial(R, ctl, G);
+  const double vir = QUADS ? G.shfl(ctl, 4 | (lane & 3)) : ctl;
+  if (lane < 4) st->collT[lane] = vir;
+  if (lane == 0) {
+    const uint64_t n = (uint64_t)(nev - nev0) - (end == END_SPECIAL ? 1 : 0);   // disk events
+    const uint64_t cross = n - ncoll - nstale;
+    st->t = t;
+    queue_to(*st, Q);
+    st->ncol += ncoll; st->ncol_total += ncoll; st->ntrace = ntrace0 + ncoll;
+    st->ncross += cross; st->nstale += nstale;
+    st->npair += npair; st->npred += 2 * ncoll + cross + nstale;
+    st->nevents += (uint64_t)(nev - nev0);
+    st->nlog = nlog;
+    st->stop_reason = stop;
+    st->status = status;
+    if (ovl) { st->err_a = oa; st->err_b = ob; }
+  }
+  G.sync();
+  return end;
+}
+
+// a special event e just popped, on the system's state in memory; false when
+// the run ends with it
+template <int GW, bool ADD>
+__device__ __noinline__ bool serve_special(const SysDev& S, uint32_t flags, int e, Grp<GW> G, WarpSmem* sm) {
+  const int lane = G.lane;
+  const int N = S.B.N;
+  SysState R = *S.st;
+  const bool grow = R.grow != 0;
+  int stop = 0, oa = -1, ob = -1;
+  bool ovl = false;
+  if (lane == 0) S.ev[e].st = ST_NONE;
+  G.sync();
+  if (e == 2 * N + SP_GROW) {
+    do_growstop<GW, ADD>(S, R, G, sm, &ovl, &oa, &ob);
+    if (flags & EDMD_F_STOP_AT_GROW) stop = EDMD_STOP_GROW;
+  } else {
+    double next;
+    if (e == 2 * N + SP_SCREEN) {
+      // ---------------- screenshot (takeAScreenshot 4657): free-fly everything
+      for (int i = lane; i < N; i += GW) {
+        Disk p = S.d[i];
+        grow_fly(S, p, i, R.t, grow);
+        S.d[i] = p;
+      }
+      G.sync();
+      next = R.t + S.dtime;
+      if (flags & EDMD_F_STOP_AT_SCREEN) stop = EDMD_STOP_SCREEN;
+    } else {
+      do_thermo(S, R, G);
+      next = R.t + S.dtimeTh;
+    }
+    Queue Q = queue_of(R);
+    schedule(S, Q, e, next, 0, 0, 2ull, G);
+    queue_to(R, Q);
+    leaf_update(S, e - N, G);
+  }
+  if (ovl) {
+    R.status = oa == OVL_CORRUPT ? EDMD_ERR_BUDGET : EDMD_ERR_OVERLAP;
+    R.err_a = oa; R.err_b = ob;
+  }
   R.stop_reason = stop;
-  R.status = status;
-  if (ovl) { R.err_a = oa; R.err_b = ob; }
+  G.sync();
   if (lane == 0) *S.st = R;
   G.sync();
+  return !ovl && !stop;
+}
+
+// the event loop of one system
+template <int GW, bool ADD = true>
+__device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, const Grp<GW>& G,
+                           WarpSmem* sm) {
+  if (S.st->status != EDMD_OK) return;
+  int64_t logged = 0, nev = 0;
+  for (;;) {
+    int special = 0, end;
+    if (S.st->grow) end = run_events<GW, ADD, true>(S, A, max_coll, G, sm, logged, nev, &special);
+    else end = run_events<GW, ADD, false>(S, A, max_coll, G, sm, logged, nev, &special);
+    if (end != END_SPECIAL || !serve_special<GW, ADD>(S, A.flags, special, G, sm)) break;
+  }
 }
 
 // Persistent launch: lane groups (GW lanes, one system each) pull systems
