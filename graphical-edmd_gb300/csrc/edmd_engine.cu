@@ -1171,8 +1171,9 @@ __device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, 
 // Persistent launch: lane groups (GW lanes, one system each) pull systems
 // from a counter, in A.order, and record each system's run time
 // (globaltimer) for the next call's order.
-template <int GW, bool ADD = true>
-__global__ void __launch_bounds__(32 * WARPS_PER_BLOCK, 4)
+// MINB: blocks of four warps per SM the registers allow for (run_shape).
+template <int GW, bool ADD, int MINB>
+__global__ void __launch_bounds__(32 * WARPS_PER_BLOCK, MINB)
 k_run(const SysDev* __restrict__ sys, RunArgs A) {
   __shared__ WarpSmem smem[WARPS_PER_BLOCK * (32 / GW)];
   const Grp<GW> G(threadIdx.x);
@@ -1192,6 +1193,27 @@ k_run(const SysDev* __restrict__ sys, RunArgs A) {
       A.cost[s] = c > 0xffffffffull ? 0xffffffffu : (uint32_t)c;
     }
   }
+}
+
+// How nsys systems are run with gw lanes each: kernel and warps per block.
+// Measured with 32 lanes (203 disks alone / 192 growth starts / 1824 < 2600
+// mixed systems, ms; every build has the same event loop):
+//   3 blocks per SM, 168 registers: 1.41 / 15.2 / 36
+//   4 blocks, 128 registers:        1.45 / 15.5 / 40.5 (2432 warps, a second wave)
+//   5 blocks, 102 registers:        1.50 / 16.4 / 30.2 (3040 warps)
+//   6 blocks, 85 registers:         1.58 / 17.6 / 32.2
+// so systems that all find a warp at three blocks per SM run there, without
+// spills, and larger batches at five.  Few enough for one warp in each SM
+// sub-partition, they are spread over the SMs in one-warp blocks.
+using RunKernel = void (*)(const SysDev*, RunArgs);
+struct RunShape { RunKernel kernel; int warps; };
+RunShape run_shape(int gw, bool additive, int nsys, int nsm) {
+  if (gw == 4) return {k_run<4, true, 4>, WARPS_PER_BLOCK};
+  if (gw == 8) return {k_run<8, true, 4>, WARPS_PER_BLOCK};
+  if (gw == 16) return {k_run<16, true, 4>, WARPS_PER_BLOCK};
+  if (nsys <= 3 * WARPS_PER_BLOCK * nsm)
+    return {additive ? k_run<32, true, 3> : k_run<32, false, 3>, nsys <= 4 * nsm ? 1 : WARPS_PER_BLOCK};
+  return {additive ? k_run<32, true, 5> : k_run<32, false, 5>, WARPS_PER_BLOCK};
 }
 
 // ---------------------------------------------------------------- shared-memory kernel
@@ -1768,7 +1790,7 @@ extern "C" int edmd_load_state(edmd_ctx* ctx, const double* x, const double* y, 
 // stream (longest first by the previous call's run times, as without the
 // flag); both start after e0 and the context's stream waits for the second
 // one before e1.
-static int advance_smem_split(edmd_ctx* ctx, RunArgs A, int kgrid_max, int nsm) {
+static int advance_smem_split(edmd_ctx* ctx, RunArgs A, int nsm) {
   int dev = 0, optin = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -1818,11 +1840,11 @@ static int advance_smem_split(edmd_ctx* ctx, RunArgs A, int kgrid_max, int nsm) 
     RunArgs B = A;
     B.nsys = (int32_t)rest.size();
     B.order = ctx->order;
-    const int per_block = WARPS_PER_BLOCK;
-    int grid = ((int)rest.size() + per_block - 1) / per_block;
-    if (grid > kgrid_max) grid = kgrid_max;
-    if (ctx->any_additive) k_run<32><<<grid, 32 * WARPS_PER_BLOCK, 0, ctx->stream>>>(ctx->ds, B);
-    else k_run<32, false><<<grid, 32 * WARPS_PER_BLOCK, 0, ctx->stream>>>(ctx->ds, B);
+    const RunShape shape = run_shape(32, ctx->any_additive, (int)rest.size(), nsm);
+    int per_sm = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shape.kernel, 32 * shape.warps, 0));
+    const int grid = std::max(1, std::min(((int)rest.size() + shape.warps - 1) / shape.warps, per_sm * nsm));
+    shape.kernel<<<grid, 32 * shape.warps, 0, ctx->stream>>>(ctx->ds, B);
     CK(cudaGetLastError());
     ctx->last_launches++;
   }
@@ -1851,18 +1873,13 @@ extern "C" int edmd_advance(edmd_ctx* ctx, int64_t max_coll, double t_stop, uint
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     int per_sm = 0;
     const int gw = g_group;                     // lanes per system: 4, 8, 16 or 32
-    const int per_block = WARPS_PER_BLOCK * (32 / gw);
-    if (gw == 4) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<4>, 32 * WARPS_PER_BLOCK, 0));
-    else if (gw == 8) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<8>, 32 * WARPS_PER_BLOCK, 0));
-    else if (gw == 16) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<16>, 32 * WARPS_PER_BLOCK, 0));
-    else CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<32>, 32 * WARPS_PER_BLOCK, 0));
+    const RunShape shape = run_shape(gw, ctx->any_additive, ctx->nsys, nsm);
+    const int per_block = shape.warps * (32 / gw);
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shape.kernel, 32 * shape.warps, 0));
     int want = (ctx->nsys + per_block - 1) / per_block;
     int grid = per_sm * nsm;
     if (grid > want) grid = want;
     if (grid < 1) grid = 1;
-    // more systems than resident warps: with one item per system the last
-    // wave runs on part of the GPU; chunks of the collision budget let the
-    // warps share the remaining work evenly (same events, same results)
     const int64_t resident = (int64_t)grid * per_block;
     if (ctx->nsys > resident) {
       // more systems than resident warps: the systems that took longest in
@@ -1881,16 +1898,12 @@ extern "C" int edmd_advance(edmd_ctx* ctx, int64_t max_coll, double t_stop, uint
     }
     ctx->last_launches = 0;
     if ((flags & EDMD_F_SMEM) && gw == 32) {
-      int rc = advance_smem_split(ctx, A, per_sm * nsm, nsm);
+      int rc = advance_smem_split(ctx, A, nsm);
       if (rc) return rc;
     } else {
     ctx->last_launches = 1;
     CK(cudaEventRecord(ctx->e0, ctx->stream));
-    if (gw == 4) k_run<4><<<grid, 32 * WARPS_PER_BLOCK, 0, ctx->stream>>>(ctx->ds, A);
-    else if (gw == 8) k_run<8><<<grid, 32 * WARPS_PER_BLOCK, 0, ctx->stream>>>(ctx->ds, A);
-    else if (gw == 16) k_run<16><<<grid, 32 * WARPS_PER_BLOCK, 0, ctx->stream>>>(ctx->ds, A);
-    else if (ctx->any_additive) k_run<32><<<grid, 32 * WARPS_PER_BLOCK, 0, ctx->stream>>>(ctx->ds, A);
-    else k_run<32, false><<<grid, 32 * WARPS_PER_BLOCK, 0, ctx->stream>>>(ctx->ds, A);
+    shape.kernel<<<grid, 32 * shape.warps, 0, ctx->stream>>>(ctx->ds, A);
     }
   }
   CK(cudaGetLastError());
@@ -2239,8 +2252,8 @@ extern "C" int edmd_run_noalloc(const edmd_system_desc* desc, double* x, double*
   k_tree_build<<<1, 256, 0, st>>>(dsys, 1);
   if (cudaMemsetAsync(work, 0, sizeof(int32_t), st) != cudaSuccess)
     return noalloc_fail(EDMD_ERR_CUDA, "edmd_run_noalloc: memset failed");
-  if (B.additive) k_run<32><<<1, 32 * WARPS_PER_BLOCK, 0, st>>>(dsys, A);
-  else k_run<32, false><<<1, 32 * WARPS_PER_BLOCK, 0, st>>>(dsys, A);
+  const RunShape shape = run_shape(32, B.additive != 0, 1, 1);
+  shape.kernel<<<1, 32 * shape.warps, 0, st>>>(dsys, A);
   k_sync<<<1, 256, 0, st>>>(dsys, 1);
   k_noalloc_out<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(dsys, x, y, vx, vy);
   cudaError_t ce = cudaGetLastError();
