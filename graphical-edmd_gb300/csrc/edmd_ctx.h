@@ -29,6 +29,8 @@ struct edmd_ctx {
   std::vector<edmd_system_desc> desc;
   std::vector<int64_t> disk_off, cell_off;
   SysDev* ds = nullptr;
+  int64_t* doff = nullptr;          // first disk of each system
+  unsigned long long* bad = nullptr;  // first bad disk of a staged state
   // device arrays shared by all systems (each system owns a slice)
   Disk* d = nullptr; double* vr = nullptr;
   int32_t *cx = nullptr, *cy = nullptr, *prv = nullptr, *crossX = nullptr, *crossY = nullptr;

@@ -27,8 +27,6 @@
 #include <cstring>
 #include <string>
 #include <algorithm>
-#include <memory>
-#include <thread>
 #include <vector>
 
 using namespace edmd;
@@ -1385,8 +1383,8 @@ __global__ void k_init_events(const SysDev* __restrict__ sys) {
   }
 }
 
-// link the initial overflow bucket in LIFO order and finish the scalar state;
-// one block per system.  The reference pushes the initial events in the order
+// link the initial overflow bucket in LIFO order and finish the scalar state.
+// The reference pushes the initial events in the order
 // thermo, [growth stop], screenshot, then crossing i and collision i for
 // i = 0..N-1 (eventListInit, src/EDMD.c:1935-2019); an overflow event's `on`
 // link is the previous overflow event in that order and `op` the next one, so
@@ -1402,19 +1400,52 @@ __device__ __forceinline__ int init_slot(int p, int N, bool grow) {
   return (k & 1) ? N + (k >> 1) : (k >> 1);
 }
 
-__global__ void __launch_bounds__(256) k_init_finish(const SysDev* __restrict__ sys, int nsys) {
-  const int s = blockIdx.x;
-  if (s >= nsys) return;
-  const SysDev& S = sys[s];
+// The running maximum goes chunk by chunk: k_init_last leaves each chunk's
+// last overflow position in the tree's array (built after it), k_init_finish
+// takes the nearest one before its chunk.  One block walked a whole system
+// before: 4x10^6 disks took 31,000 block steps.
+constexpr int INIT_CHUNK = 4096;
+
+__global__ void __launch_bounds__(256) k_init_last(const SysDev* __restrict__ sys) {
+  const SysDev& S = sys[blockIdx.y];
   const int N = S.B.N;
   const bool grow = S.st->grow != 0;
-  const int P = (grow ? 3 : 2) + 2 * N;
+  const int P = (grow ? 3 : 2) + 2 * N, p0 = blockIdx.x * INIT_CHUNK;
+  if (p0 >= P) return;
+  int last = -1;
+  for (int p = p0 + threadIdx.x; p < min(P, p0 + INIT_CHUNK); p += 256)
+    if (S.ev[init_slot(p, N, grow)].st == ST_OVF) last = p;
+  __shared__ int m[8];
+  last = __reduce_max_sync(FULL, last);
+  if ((threadIdx.x & 31) == 0) m[threadIdx.x >> 5] = last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) last = max(last, m[w]);
+    ((int*)S.tree)[blockIdx.x] = last;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_init_finish(const SysDev* __restrict__ sys) {
+  const SysDev& S = sys[blockIdx.y];
+  const int N = S.B.N;
+  const bool grow = S.st->grow != 0;
+  const int P = (grow ? 3 : 2) + 2 * N, p0 = blockIdx.x * INIT_CHUNK;
+  if (p0 >= P) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int* last_of = (const int*)S.tree;
   __shared__ int wmax[8];
   __shared__ int carry;
-  if (threadIdx.x == 0) carry = -1;
+  // the last overflow position before this chunk
+  if (w == 0) {
+    int before = -1;
+    for (int c = blockIdx.x - 1; c >= 0 && before < 0; c -= 32) {
+      const int l = c - lane >= 0 ? last_of[c - lane] : -1;
+      before = __reduce_max_sync(FULL, l);
+    }
+    if (lane == 0) carry = before;
+  }
   __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int base = 0; base < P; base += blockDim.x) {
+  for (int base = p0; base < min(P, p0 + INIT_CHUNK); base += blockDim.x) {
     const int p = base + threadIdx.x;
     const int e = p < P ? init_slot(p, N, grow) : -1;
     const bool ovf = e >= 0 && S.ev[e].st == ST_OVF;
@@ -1445,7 +1476,7 @@ __global__ void __launch_bounds__(256) k_init_finish(const SysDev* __restrict__ 
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && p0 + INIT_CHUNK >= P) {         // the system's last chunk
     SysState& R = *S.st;
     R.ovf = carry >= 0 ? init_slot(carry, N, grow) : NIL;
     if (R.ovf != NIL) S.op[R.ovf] = NIL;
@@ -1456,37 +1487,139 @@ __global__ void __launch_bounds__(256) k_init_finish(const SysDev* __restrict__ 
   }
 }
 
-// one block per system: the leaves in parallel, then one level at a time
-// with a warp per parent node
-__global__ void __launch_bounds__(256) k_tree_build(const SysDev* __restrict__ sys, int nsys) {
-  const int s = blockIdx.x;
-  if (s >= nsys) return;
-  const SysDev& S = sys[s];
-  for (int l = threadIdx.x; l < S.L; l += blockDim.x) S.tree[l] = leaf_node(S, l);
+// levels 0, 1 and 2 of the tree, 1024 leaves per block: a warp's leaves are
+// one parent's children, a block's parents another's
+__global__ void __launch_bounds__(1024) k_tree_leaves(const SysDev* __restrict__ sys) {
+  const SysDev& S = sys[blockIdx.y];
+  const int l = blockIdx.x * 1024 + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (blockIdx.x * 1024 >= S.L) return;
+  const Grp<32> G(threadIdx.x);
+  __shared__ Node up[32];
+  Node n = empty_node(0x7fffffff);
+  if (l < S.L) S.tree[l] = n = leaf_node(S, l);
+  const int src = grp_argmin(n, G);
+  if (lane == src) {
+    up[w] = n;
+    if ((l >> 5) < S.lev_cnt[1]) S.tree[S.lev_off[1] + (l >> 5)] = n;     // a system has at least two leaves
+  }
+  if (S.nlev < 3) return;
   __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int h = 1; h < S.nlev; h++) {
+  if (w == 0) {
+    const Node m = up[lane];
+    if (lane == grp_argmin(m, G)) S.tree[S.lev_off[2] + blockIdx.x] = m;
+  }
+}
+
+// the levels above, for systems of more than 1024 leaves: one block per
+// system, a warp per parent, level by level
+__global__ void __launch_bounds__(256) k_tree_build(const SysDev* __restrict__ sys) {
+  const SysDev& S = sys[blockIdx.x];
+  const Grp<32> G(threadIdx.x);
+  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int h = 3; h < S.nlev; h++) {
     for (int par = w; par < S.lev_cnt[h]; par += nw) {
-      const Grp<32> G(threadIdx.x);
       const Node none = empty_node(0x7fffffff);
       const Node c = child_node(S, h, par, -1, none, -1, none, G);
-      if (lane == grp_argmin(c, G)) S.tree[S.lev_off[h] + par] = c;
+      if (G.lane == grp_argmin(c, G)) S.tree[S.lev_off[h] + par] = c;
     }
     __syncthreads();
   }
 }
 
-__global__ void k_sync(const SysDev* __restrict__ sys, int nsys) {
-  int s = blockIdx.x;
-  if (s >= nsys) return;
-  const SysDev& S = sys[s];
-  const double t = S.st->t;
-  const bool grow = S.st->grow != 0;
-  for (int i = threadIdx.x; i < S.B.N; i += blockDim.x) {
-    Disk p = S.d[i];
-    grow_fly(S, p, i, t, grow);
-    S.d[i] = p;
+// event set, overflow list and (warp engine) tree of nsys systems of at most
+// maxN disks whose disks and cell lists are in place
+cudaError_t init_queues(const SysDev* sys, int nsys, int maxN, bool tree, cudaStream_t st) {
+  k_init_events<<<dim3((maxN + 1 + 127) / 128, nsys), 128, 0, st>>>(sys);
+  const dim3 g((3 + 2 * maxN + INIT_CHUNK - 1) / INIT_CHUNK, nsys);
+  k_init_last<<<g, 256, 0, st>>>(sys);
+  k_init_finish<<<g, 256, 0, st>>>(sys);
+  if (tree) {
+    k_tree_leaves<<<dim3((maxN + NSPECIAL + 1023) / 1024, nsys), 1024, 0, st>>>(sys);
+    if (maxN + NSPECIAL > 1024) k_tree_build<<<nsys, 256, 0, st>>>(sys);
   }
+  return cudaGetLastError();
+}
+
+// freeFly of every disk to its system's time: blocks of 256 disks
+__global__ void __launch_bounds__(256) k_sync(const SysDev* __restrict__ sys) {
+  const SysDev& S = sys[blockIdx.y];
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= S.B.N) return;
+  Disk p = S.d[i];
+  grow_fly(S, p, i, S.st->t, S.st->grow != 0);
+  S.d[i] = p;
+}
+
+// ---- a system's disks and cell lists from host arrays
+
+// a disk the engine cannot take: its position (after the periodic wrap of a
+// restart), then its radius
+__host__ __device__ __forceinline__ void wrap_restart(double& x, double& y, double Lx, double Ly) {
+  if (x < 0) x += Lx; else if (x >= Lx) x -= Lx;     // PBCpostX/Y (src/EDMD.c:1405-1406)
+  if (y < 0) y += Ly; else if (y >= Ly) y -= Ly;
+}
+// 0: good, 1: position outside the box, 2: radius not zero or normal positive
+__host__ __device__ __forceinline__ int bad_disk(double x, double y, double rad, double Lx, double Ly, bool restart) {
+  if (restart) wrap_restart(x, y, Lx, Ly);
+  if (!(x >= 0 && x < Lx && y >= 0 && y < Ly)) return 1;
+  return radius_ok(rad) ? 0 : 2;
+}
+
+// SoA staging arrays (x y vx vy rad m of all disks, `total` each) of the
+// systems; doff[s]: first disk of system s
+__global__ void k_check(const SysDev* __restrict__ sys, const int64_t* __restrict__ doff,
+                        const double* __restrict__ in, int64_t total, bool restart, unsigned long long* bad) {
+  const SysDev& S = sys[blockIdx.y];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= S.B.N) return;
+  const int64_t g = doff[blockIdx.y] + i;
+  const int b = bad_disk(in[g], in[total + g], in[4 * total + g], S.B.Lx, S.B.Ly, restart);
+  if (b) atomicMin(bad, 2ull * (unsigned long long)g + (unsigned long long)(b - 1));
+}
+
+// records and cells (src/EDMD.c:1906 cellListInit); each disk also joins a
+// chain of its cell, in any order, through the overflow links (not yet in use)
+__global__ void k_stage(const SysDev* __restrict__ sys, const int64_t* __restrict__ doff,
+                        const double* __restrict__ in, int64_t total, bool restart) {
+  const SysDev& S = sys[blockIdx.y];
+  const Box& B = S.B;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= B.N) return;
+  const int64_t g = doff[blockIdx.y] + i;
+  Disk q;
+  q.x = in[g]; q.y = in[total + g]; q.vx = in[2 * total + g]; q.vy = in[3 * total + g];
+  q.rad = in[4 * total + g]; q.m = in[5 * total + g];
+  if (restart) wrap_restart(q.x, q.y, B.Lx, B.Ly);
+  q.tl = 0; q.nxt = NIL; q.coll = 0;
+  int X = (int)(q.x * B.cxf), Y = (int)(q.y * B.cyf);
+  if (X >= B.Nxc) X = B.Nxc - 1;
+  if (Y >= B.Nyc) Y = B.Nyc - 1;
+  S.d[i] = q;
+  S.cx[i] = X; S.cy[i] = Y;
+  S.crossX[i] = 0; S.crossY[i] = 0;
+  S.on[i] = atomicExch(&S.head[Y * B.Nxc + X], i);
+}
+
+// the reference pushes disks onto their cells' lists in index order (addToCell
+// src/EDMD.c:2053, push-front), so a list runs from the largest index down:
+// each disk finds its neighbours in that order on its cell's chain
+__global__ void k_links(const SysDev* __restrict__ sys) {
+  const SysDev& S = sys[blockIdx.y];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= S.B.N) return;
+  int below = NIL, above = NIL;
+  for (int j = S.head[S.cy[i] * S.B.Nxc + S.cx[i]]; j != NIL; j = S.on[j]) {
+    if (j < i && j > below) below = j;
+    if (j > i && (above == NIL || j < above)) above = j;
+  }
+  S.d[i].nxt = below;
+  S.prv[i] = above;
+}
+
+__global__ void k_heads(const SysDev* __restrict__ sys) {
+  const SysDev& S = sys[blockIdx.y];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < S.B.N && S.prv[i] == NIL) S.head[S.cy[i] * S.B.Nxc + S.cx[i]] = i;
 }
 
 // disk records of every system -> concatenated SoA staging (x y vx vy rad m)
@@ -1538,31 +1671,12 @@ extern "C" int edmd_device_info(char* name, int32_t cap, int32_t* sm_count) {
 
 
 
-// host threads for staging n disks: one below 2^16 disks, else up to 16
-static int staging_threads(int64_t n) {
-  if (n < ((int64_t)1 << 16)) return 1;
-  const unsigned hc = std::thread::hardware_concurrency();
-  return (int)std::max(1u, std::min(hc, 16u));
-}
-
-// run f(0) .. f(n-1), on n threads where they can be had (inline otherwise)
-template <class F>
-static void run_threads(int n, F&& f) {
-  std::vector<std::thread> pool;
-  for (int k = 1; k < n; k++) {
-    try {
-      pool.emplace_back(f, k);
-    } catch (...) {
-      f(k);
-    }
-  }
-  f(0);
-  for (auto& th : pool) th.join();
-}
-
-// (Re)initialise every system from host arrays: the cell lists are built on
-// the host in index order (cellListInit src/EDMD.c:1906 -> addToCell 2053,
-// push-front), the event set on the device (eventListInit 1935).
+// (Re)initialise every system from host arrays: the arrays go to the device
+// as they are, the records, the cell lists in index order (cellListInit
+// src/EDMD.c:1906 -> addToCell 2053, push-front) and the event set
+// (eventListInit 1935) are made there.  Measured on 4x10^6 disks: 83 ms with
+// records and lists made on 16 host threads and the overflow list and tree
+// walked by one block; on 10^6 disks 18.9 ms.
 // first_screen/first_thermo/t_growstop per system come from `desc` unless
 // `restart`, which follows the -l load path: normal phase, firstScreen 1,
 // firstThermo 1000 (src/EDMD.c:244-247; eventListInit 1958 skips the growth
@@ -1573,64 +1687,39 @@ static int stage_all(edmd_ctx* ctx, const double* x, const double* y, const doub
   ctx->round_dirty = false;
   const int64_t TN = ctx->total_N;
   const int nsys = ctx->nsys;
-  // every field of every staged record is written below
-  std::unique_ptr<Disk[]> hd(new Disk[TN]);
-  std::unique_ptr<int32_t[]> hcx(new int32_t[TN]), hcy(new int32_t[TN]), hprv(new int32_t[TN]);
-  std::vector<int32_t> hhead(ctx->total_C, NIL);
-  std::vector<SysState> hst(nsys);
-  const int nth = staging_threads(TN);
-  // records and cells, disk by disk, in contiguous slices of the concatenated
-  // disks; each slice stops at its first bad disk, so the smallest of those is
-  // the first bad disk in index order (2 g: position, 2 g + 1: radius)
-  std::vector<int64_t> bad(nth, INT64_MAX);
-  run_threads(nth, [&](int k) {
-    const int64_t lo = TN * k / nth, hi = TN * (k + 1) / nth;
-    int s = (int)(std::upper_bound(ctx->disk_off.begin(), ctx->disk_off.end(), lo) - ctx->disk_off.begin()) - 1;
-    for (int64_t g = lo; g < hi; g++) {
-      while (s + 1 < nsys && g >= ctx->disk_off[s + 1]) s++;
-      const Box& B = ctx->hs[s].B;
-      const edmd_system_desc& D = ctx->desc[s];
-      double px = x[g], py = y[g];
-      if (restart) {                     // PBCpostX/Y on loaded positions (src/EDMD.c:1405-1406)
-        if (px < 0) px += D.Lx; else if (px >= D.Lx) px -= D.Lx;
-        if (py < 0) py += D.Ly; else if (py >= D.Ly) py -= D.Ly;
-      }
-      if (!(px >= 0 && px < D.Lx && py >= 0 && py < D.Ly)) { bad[k] = 2 * g; return; }
-      if (!radius_ok(rad[g])) { bad[k] = 2 * g + 1; return; }
-      Disk& q = hd[g];
-      q.x = px; q.y = py; q.vx = vx[g]; q.vy = vy[g]; q.tl = 0; q.rad = rad[g]; q.m = m[g];
-      q.coll = 0;
-      int X = (int)(q.x * B.cxf), Y = (int)(q.y * B.cyf);
-      if (X >= B.Nxc) X = B.Nxc - 1;
-      if (Y >= B.Nyc) Y = B.Nyc - 1;
-      hcx[g] = X; hcy[g] = Y;
-    }
-  });
-  const int64_t first_bad = *std::min_element(bad.begin(), bad.end());
-  if (first_bad != INT64_MAX) {
-    const int64_t g = first_bad / 2;
+  cudaStream_t sm = ctx->stream;
+  if (!ctx->stage) CK(dalloc(&ctx->stage, 6 * TN));
+  const double* const in[6] = {x, y, vx, vy, rad, m};
+  const dim3 gd((ctx->maxN + 255) / 256, nsys);
+  // the first bad disk in index order (2 g: position, 2 g + 1: radius), found
+  // before any state changes: a small context on the host, without waiting
+  // for the device
+  unsigned long long first_bad = ~0ull;
+  const bool on_device = TN >= ((int64_t)1 << 14);
+  if (!on_device)
+    for (int s = 0; s < nsys && first_bad == ~0ull; s++)
+      for (int64_t g = ctx->disk_off[s]; g < ctx->disk_off[s] + ctx->desc[s].N; g++)
+        if (const int b = bad_disk(x[g], y[g], rad[g], ctx->desc[s].Lx, ctx->desc[s].Ly, restart)) {
+          first_bad = 2ull * g + (b - 1);
+          break;
+        }
+  if (first_bad == ~0ull)
+    for (int k = 0; k < 6; k++)
+      CK(cudaMemcpyAsync(ctx->stage + k * TN, in[k], TN * 8, cudaMemcpyHostToDevice, sm));
+  if (on_device) {
+    CK(cudaMemcpyAsync(ctx->bad, &first_bad, 8, cudaMemcpyHostToDevice, sm));
+    k_check<<<gd, 256, 0, sm>>>(ctx->ds, ctx->doff, ctx->stage, TN, restart, ctx->bad);
+    CK(cudaGetLastError());
+    CK(sync_copy(ctx, &first_bad, ctx->bad, 8, cudaMemcpyDeviceToHost));
+  }
+  if (first_bad != ~0ull) {
+    const int64_t g = (int64_t)(first_bad / 2);
     const int s = (int)(std::upper_bound(ctx->disk_off.begin(), ctx->disk_off.end(), g) - ctx->disk_off.begin()) - 1;
     return set_err(ctx, EDMD_ERR_ARG, std::string(first_bad % 2 ? "radius not zero or normal positive"
                                                                   : "position outside the box") +
                                           " (system " + std::to_string(s) + ")");
   }
-  // cell lists, system by system: push-front in index order (cellListInit
-  // src/EDMD.c:1906 -> addToCell 2053)
-  run_threads(std::min(nth, nsys), [&](int k) {
-    for (int s = k; s < nsys; s += std::min(nth, nsys)) {
-      const Box& B = ctx->hs[s].B;
-      const int64_t o = ctx->disk_off[s];
-      int32_t* head = hhead.data() + ctx->cell_off[s];
-      for (int64_t i = 0; i < B.N; i++) {
-        const int64_t g = o + i;
-        const int c = hcy[g] * B.Nxc + hcx[g];
-        hprv[g] = NIL;
-        hd[g].nxt = head[c];
-        head[c] = (int32_t)i;
-        if (hd[g].nxt != NIL) hprv[o + hd[g].nxt] = (int32_t)i;
-      }
-    }
-  });
+  std::vector<SysState> hst(nsys);
   for (int s = 0; s < nsys; s++) {
     const SysDev& S = ctx->hs[s];
     const Box& B = S.B;
@@ -1644,24 +1733,16 @@ static int stage_all(edmd_ctx* ctx, const double* x, const double* y, const doub
     st.collT[0] = st.grow ? D.t_growstop : -1;
     st.collT[1] = fs;
   }
-  cudaStream_t sm = ctx->stream;
-  CK(cudaMemcpyAsync(ctx->st, hst.data(), ctx->nsys * sizeof(SysState), cudaMemcpyHostToDevice, sm));
-  CK(cudaMemcpyAsync(ctx->d, hd.get(), TN * sizeof(Disk), cudaMemcpyHostToDevice, sm));
+  CK(cudaMemcpyAsync(ctx->st, hst.data(), nsys * sizeof(SysState), cudaMemcpyHostToDevice, sm));
   if (vr && !restart) CK(cudaMemcpyAsync(ctx->vr, vr, TN * 8, cudaMemcpyHostToDevice, sm));
   else if (!vr && !restart) CK(cudaMemsetAsync(ctx->vr, 0, TN * 8, sm));
-  CK(cudaMemcpyAsync(ctx->cx, hcx.get(), TN * 4, cudaMemcpyHostToDevice, sm));
-  CK(cudaMemcpyAsync(ctx->cy, hcy.get(), TN * 4, cudaMemcpyHostToDevice, sm));
-  CK(cudaMemcpyAsync(ctx->prv, hprv.get(), TN * 4, cudaMemcpyHostToDevice, sm));
-  CK(cudaMemsetAsync(ctx->crossX, 0, TN * 4, sm));
-  CK(cudaMemsetAsync(ctx->crossY, 0, TN * 4, sm));
-  CK(cudaMemcpyAsync(ctx->head, hhead.data(), ctx->total_C * 4, cudaMemcpyHostToDevice, sm));
-  dim3 g((ctx->maxN + 1 + 127) / 128, ctx->nsys);
-  k_init_events<<<g, 128, 0, sm>>>(ctx->ds);
-  k_init_finish<<<ctx->nsys, 256, 0, sm>>>(ctx->ds, ctx->nsys);
-  if (ctx->engine == EDMD_ENGINE_LANE) CK(lane_build(ctx->ds, ctx->nsys, sm));
-  else k_tree_build<<<ctx->nsys, 256, 0, sm>>>(ctx->ds, ctx->nsys);
+  CK(cudaMemsetAsync(ctx->head, 0xff, ctx->total_C * 4, sm));      // NIL
+  k_stage<<<gd, 256, 0, sm>>>(ctx->ds, ctx->doff, ctx->stage, TN, restart);
+  k_links<<<gd, 256, 0, sm>>>(ctx->ds);
+  k_heads<<<gd, 256, 0, sm>>>(ctx->ds);
   CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(sm));   // host staging vectors go out of scope
+  CK(init_queues(ctx->ds, nsys, ctx->maxN, ctx->engine != EDMD_ENGINE_LANE, sm));
+  if (ctx->engine == EDMD_ENGINE_LANE) CK(lane_build(ctx->ds, nsys, sm));
   return report_status(ctx, "initial configuration");
 }
 
@@ -1751,6 +1832,8 @@ extern "C" int edmd_create(int32_t nsys, const edmd_system_desc* desc, const dou
   CK(dalloc(&ctx->cost, nsys));
   CK(cudaMemsetAsync(ctx->cost, 0, nsys * sizeof(uint32_t), ctx->stream));
   CK(dalloc(&ctx->ds, nsys));
+  CK(dalloc(&ctx->doff, nsys));
+  CK(dalloc(&ctx->bad, 1));
   if (ctx->engine == EDMD_ENGINE_LANE) {
     CK(dalloc(&ctx->cal, (size_t)TN * CAL_SUB * CAL_LINE));
     CK(dalloc(&ctx->mask, (size_t)TN));
@@ -1776,6 +1859,7 @@ extern "C" int edmd_create(int32_t nsys, const edmd_system_desc* desc, const dou
     }
   }
   CK(cudaMemcpyAsync(ctx->ds, ctx->hs.data(), nsys * sizeof(SysDev), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->doff, ctx->disk_off.data(), nsys * 8, cudaMemcpyHostToDevice, ctx->stream));
   return stage_all(ctx, x, y, vx, vy, rad, m, vr, false);
 }
 
@@ -1916,7 +2000,7 @@ extern "C" int edmd_advance(edmd_ctx* ctx, int64_t max_coll, double t_stop, uint
 
 extern "C" int edmd_sync(edmd_ctx* ctx) {
   if (!ctx) return EDMD_ERR_ARG;
-  k_sync<<<ctx->nsys, 256, 0, ctx->stream>>>(ctx->ds, ctx->nsys);
+  k_sync<<<dim3((ctx->maxN + 255) / 256, ctx->nsys), 256, 0, ctx->stream>>>(ctx->ds);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->stream));
   return EDMD_OK;
@@ -2043,7 +2127,7 @@ extern "C" int edmd_destroy(edmd_ctx* ctx) {
   round_free(ctx);
   void* ptrs[] = {ctx->d, ctx->vr, ctx->cx, ctx->cy, ctx->prv, ctx->crossX, ctx->crossY, ctx->head,
                   ctx->ev, ctx->on, ctx->op, ctx->tree, ctx->st, ctx->trace, ctx->rows, ctx->stage,
-                  ctx->work, ctx->order, ctx->cost, ctx->ds, ctx->cal, ctx->mask};
+                  ctx->work, ctx->order, ctx->cost, ctx->ds, ctx->doff, ctx->bad, ctx->cal, ctx->mask};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (void* p : ctx->ckpt)
@@ -2247,14 +2331,13 @@ extern "C" int edmd_run_noalloc(const edmd_system_desc* desc, double* x, double*
   A.nsys = 1; A.work = work; A.order = nullptr; A.cost = nullptr;
   k_noalloc_put<<<1, 1, 0, st>>>(S, dsys);
   k_noalloc_stage<<<1, 32, 0, st>>>(dsys, x, y, vx, vy, rad, m, D.first_screen, D.first_thermo);
-  k_init_events<<<dim3((unsigned)((N + 1 + 127) / 128), 1), 128, 0, st>>>(dsys);
-  k_init_finish<<<1, 256, 0, st>>>(dsys, 1);
-  k_tree_build<<<1, 256, 0, st>>>(dsys, 1);
+  if (cudaError_t qe = init_queues(dsys, 1, N, true, st); qe != cudaSuccess)
+    return noalloc_fail(EDMD_ERR_CUDA, cudaGetErrorString(qe));
   if (cudaMemsetAsync(work, 0, sizeof(int32_t), st) != cudaSuccess)
     return noalloc_fail(EDMD_ERR_CUDA, "edmd_run_noalloc: memset failed");
   const RunShape shape = run_shape(32, B.additive != 0, 1, 1);
   shape.kernel<<<1, 32 * shape.warps, 0, st>>>(dsys, A);
-  k_sync<<<1, 256, 0, st>>>(dsys, 1);
+  k_sync<<<dim3((N + 255) / 256, 1), 256, 0, st>>>(dsys);
   k_noalloc_out<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(dsys, x, y, vx, vy);
   cudaError_t ce = cudaGetLastError();
   if (ce != cudaSuccess) return noalloc_fail(EDMD_ERR_CUDA, cudaGetErrorString(ce));
