@@ -2,7 +2,9 @@
 // (internal; the public interface is include/edmd_gpu.h).
 #pragma once
 #include <cstddef>
+#include <algorithm>
 #include <string>
+#include <thread>
 #include <vector>
 #include <cuda_runtime.h>
 #include "edmd_device.cuh"
@@ -144,6 +146,52 @@ static inline cudaError_t sync_copy2d(edmd_ctx* c, void* dst, size_t dp, const v
 static inline cudaError_t sync_set(edmd_ctx* c, void* dst, int v, size_t n) {
   cudaError_t e = cudaMemsetAsync(dst, v, n, c->stream);
   return e != cudaSuccess ? e : cudaStreamSynchronize(c->stream);
+}
+
+// host threads for a job of n small pieces: one below `least`, else up to 16
+static inline int host_threads(int64_t n, int64_t least) {
+  if (n < least) return 1;
+  const unsigned hc = std::thread::hardware_concurrency();
+  return (int)std::max<int64_t>(1, std::min<int64_t>(std::min(hc, 16u), n));
+}
+
+// run f(0) .. f(n-1), on n threads where they can be had (inline otherwise)
+template <class F>
+static inline void run_threads(int n, F&& f) {
+  std::vector<std::thread> pool;
+  for (int k = 1; k < n; k++) {
+    try {
+      pool.emplace_back(f, k);
+    } catch (...) {
+      f(k);
+    }
+  }
+  f(0);
+  for (auto& th : pool) th.join();
+}
+
+// Make the pages of host buffers resident before a device copy writes them:
+// into fresh pageable memory the copy engine faults page by page (192 MB into
+// new arrays took 160 ms; 4.5 ms into resident ones), host threads do not.
+// Every byte keeps its value.
+static inline void make_resident(double* const* bufs, int nbufs, int64_t bytes) {
+  constexpr int64_t PAGE = 4096;
+  const int64_t pages = (bytes + PAGE - 1) / PAGE;
+  const int nth = host_threads(pages * nbufs, 256);
+  run_threads(nth, [&](int k) {
+    for (int b = 0; b < nbufs; b++) {
+      if (!bufs[b]) continue;
+      volatile char* p = (volatile char*)bufs[b];
+      for (int64_t g = pages * k / nth; g < pages * (k + 1) / nth; g++) {
+        const char v = p[g * PAGE];
+        p[g * PAGE] = v;
+      }
+      if (k == nth - 1 && bytes > 0) {
+        const char v = p[bytes - 1];
+        p[bytes - 1] = v;
+      }
+    }
+  });
 }
 
 template <class T>

@@ -2037,6 +2037,7 @@ extern "C" int edmd_get_states(edmd_ctx* ctx, double* x, double* y, double* vx, 
   k_gather<<<(unsigned)((TN + 255) / 256), 256, 0, ctx->stream>>>(ctx->d, TN, ctx->stage);
   CK(cudaGetLastError());
   double* outs[6] = {x, y, vx, vy, rad, m};
+  make_resident(outs, 6, TN * 8);
   for (int k = 0; k < 6; k++)
     if (outs[k]) CK(cudaMemcpyAsync(outs[k], ctx->stage + k * TN, TN * 8, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));

@@ -17,8 +17,10 @@
 // The adjoint applies the transpose of the same map backwards over the log.
 #include "edmd_ctx.h"
 
+#include <atomic>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <random>
 
 namespace {
@@ -849,17 +851,25 @@ extern "C" int edmd_tangent_run_batch(edmd_ctx* ctx, int32_t K, int64_t n_coll, 
   const unsigned gs = (unsigned)((nsys + 127) / 128);
   // system s starts from the vectors edmd_tangent_run draws from seed + s
   // (drawn on the host before the timed part of the call)
-  std::vector<double> h((size_t)4 * TN * K);
-  for (int s = 0; s < nsys; s++) {
-    std::mt19937_64 g(seed + (uint64_t)s);
-    std::normal_distribution<double> nd(0.0, 1.0);
-    double* hs = h.data() + (size_t)4 * ctx->disk_off[s] * K;
-    for (size_t e = 0; e < (size_t)4 * ctx->hs[s].B.N * K; e++) hs[e] = nd(g);
+  // systems are drawn on host threads, each from its own generator (128 systems
+  // of 448 disks, 16 vectors: 40 ms on one thread)
+  const size_t nh = (size_t)4 * TN * K;
+  std::unique_ptr<double[]> h(new double[nh]);
+  {
+    std::atomic<int> next{0};
+    run_threads(std::min(nsys, host_threads((int64_t)nh, 1 << 14)), [&](int) {
+      for (int s = next++; s < nsys; s = next++) {
+        std::mt19937_64 g(seed + (uint64_t)s);
+        std::normal_distribution<double> nd(0.0, 1.0);
+        double* hs = h.get() + (size_t)4 * ctx->disk_off[s] * K;
+        for (size_t e = 0; e < (size_t)4 * ctx->hs[s].B.N * K; e++) hs[e] = nd(g);
+      }
+    });
   }
   CK(call_begin(ctx));
   std::vector<double> t0(nsys), t1(nsys);
   if ((rc = sys_times(ctx, t0.data()))) return rc;
-  CK(cudaMemcpyAsync(T, h.data(), h.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(T, h.get(), nh * 8, cudaMemcpyHostToDevice, ctx->stream));
   k_fill_sys_time<<<(unsigned)((TN + 255) / 256), 256, 0, ctx->stream>>>(ctx->ds, bi.dsys, TN, tl);
   CK(cudaMemsetAsync(logdiag, 0, (size_t)nsys * K * sizeof(double), ctx->stream));
   CK(cudaMemsetAsync(fail, 0, nsys * sizeof(int), ctx->stream));

@@ -58,6 +58,8 @@ class Counters(C.Structure):
                 ("stop_reason", C.c_int32), ("nscreen", C.c_uint64)]
 
 
+COUNTERS_DTYPE = np.dtype(Counters)
+
 # every symbol the public headers declare, in declaration order
 EXPORTS = [
     "edmd_create", "edmd_load_state", "edmd_advance", "edmd_advance_rounds", "edmd_sync",
@@ -323,9 +325,9 @@ class Engine:
         return out
 
     def all_counters(self):
-        arr = (Counters * self.n)()
-        self._ck(self._L.edmd_get_all_counters(self.h, C.cast(arr, C.c_void_p)))
-        return {k: np.array([getattr(c, k) for c in arr]) for k, _ in Counters._fields_}
+        arr = np.zeros(self.n, COUNTERS_DTYPE)
+        self._ck(self._L.edmd_get_all_counters(self.h, _ptr(arr)))
+        return {k: arr[k].astype(np.float64 if k == "t" else np.int64) for k in COUNTERS_DTYPE.names}
 
     # ---- differentiation
     def checkpoint_save(self, slot):
