@@ -19,7 +19,7 @@
 // each tree level is fixed by one coalesced 32-wide load and a warp butterfly.
 // Collision prediction packs the candidates of the 3x3 neighbour cells of the
 // (up to two) disks that changed into the lanes of the warp.
-#include "edmd_device.cuh"
+#include "edmd_lanes.cuh"
 #include "../../include/edmd_gpu.h"
 
 #include <cstdio>
@@ -40,49 +40,14 @@ cudaError_t lane_run_launch(const SysDev* ds, const RunArgs& A, int threads_per_
 
 namespace {
 
-constexpr int MAXC = 7;          // candidates buffered per cell list per lane (a count of three bits)
 constexpr int WARPS_PER_BLOCK = 4;
 
 // scratch of one lane group (one system)
-struct WarpSmem {
-  int32_t reg[2 * 9 * MAXC];     // walk buffers, one per (disk, cell) task
-  int32_t comp[2 * 9 * MAXC];    // packed candidates
-  int16_t ord[2 * 9 * MAXC];     // their scan order
+struct WarpSmem : LaneScratch {
   long long msum[2];             // last two mass sums of the collision rule (bits) ...
   double inv[2];                 // ... and (1 / msum) (1 + res), the same operations' result
 };
 
-// A group of GW lanes that runs one system: the whole warp (GW = 32) or one
-// half of it (GW = 16, two systems per warp).  Every collective of the event
-// loop goes through the group's mask and width, so the two halves of a warp
-// are independent and may diverge.
-template <int GW>
-struct Grp {
-  int lane;                      // 0 .. GW-1
-  unsigned mask;                 // the group's lanes within the warp
-  __device__ __forceinline__ explicit Grp(int tid)
-      : lane(tid & (GW - 1)), mask(GW == 32 ? 0xffffffffu : (((1u << GW) - 1u) << ((tid & 31) & ~(GW - 1)))) {}
-  template <class T> __device__ __forceinline__ T shfl(T v, int src) const { return __shfl_sync(mask, v, src, GW); }
-  template <class T> __device__ __forceinline__ T shfl_xor(T v, int o) const {
-    return __shfl_xor_sync(mask, v, o, GW);
-  }
-  template <class T> __device__ __forceinline__ T shfl_up(T v, int o) const {
-    return __shfl_up_sync(mask, v, o, GW);
-  }
-  __device__ __forceinline__ void sync() const { __syncwarp(mask); }
-  __device__ __forceinline__ bool any(bool p) const { return __any_sync(mask, p); }
-  __device__ __forceinline__ uint32_t min_u32(uint32_t v) const { return __reduce_min_sync(mask, v); }
-  // group-relative ballot
-  __device__ __forceinline__ unsigned ballot(bool p) const {
-    const unsigned m = __ballot_sync(mask, p) & mask;
-    return GW == 32 ? m : m >> (__ffs(mask) - 1);
-  }
-  // group-relative index of the first lane where p holds, or -1
-  __device__ __forceinline__ int first(bool p) const {
-    const unsigned m = __ballot_sync(mask, p) & mask;
-    return m ? ((__ffs(m) - 1) & (GW - 1)) : -1;
-  }
-};
 
 __device__ __forceinline__ Node empty_node(int idx) {
   Node n; n.tk = ~0ull; n.tie = ~0ull; n.b = BINF; n.idx = idx;
@@ -343,291 +308,6 @@ __device__ __forceinline__ void grow_fly(const SysDev& S, Disk& p, int i, double
   if (grow) p.rad += dt * S.vr[i];
 }
 
-// Lanes of the event handlers.  The (one or two) disks an event changes are
-// spread over four lane roles, repeated over the group: disk `lane & 1` (the
-// owner, or the partner of a collision) and axis `lane & 2` (x, or y).  Each
-// lane holds its disk's coordinate, velocity and cell along its axis, so the
-// scalar FP64 work of both disks and both axes shares its instructions: an
-// FP64 instruction costs its ~76 issue cycles whatever the lanes it serves.
-struct Own {
-  double p, v, rad, vr;            // coordinate and velocity along the axis; radius, growth rate
-  int c;                           // cell index along the axis
-};
-
-// a collision prediction of the lane's disk: time image, partner, its counter
-struct Next { uint64_t key; int32_t partner; uint32_t ca; };
-constexpr int OVL_CORRUPT = -2;    // overlap marker: a cell list longer than N (EDMD_ERR_BUDGET)
-
-// a disk record's coordinate or velocity along an axis (x, y, vx, vy lead it)
-__device__ __forceinline__ double* axis_pos(Disk* d, bool y) { return &d->x + (y ? 1 : 0); }
-__device__ __forceinline__ double* axis_vel(Disk* d, bool y) { return &d->vx + (y ? 1 : 0); }
-static_assert(offsetof(Disk, y) == offsetof(Disk, x) + 8 && offsetof(Disk, vy) == offsetof(Disk, vx) + 8, "axis layout");
-
-// nearest periodic image of a difference along an axis (PBC src/EDMD.c:5896)
-__device__ __forceinline__ double near_image(double d, double hL, double L) {
-  if (ge_pos(d, hL)) d -= L;
-  else if (lt_neg(d, hL)) d += L;
-  return d;
-}
-
-// candidate times compared as their order-preserving integer images: the
-// same order as FP64 '<' (both zeros share one image; a NaN, which '<' never
-// selects, maps above every number), on the integer pipe
-__device__ __forceinline__ uint64_t cand_key(double d) {
-  const uint64_t u = (uint64_t)__double_as_longlong(d);
-  return (u & 0x7fffffffffffffffull) > 0x7ff0000000000000ull ? ~0ull : time_key(d);
-}
-
-__device__ __forceinline__ void best_merge(uint64_t& bk, int& bo, int& bp, uint32_t& bc,
-                                           uint64_t k, int o, int p, uint32_t c) {
-  if (k < bk || (k == bk && o < bo)) { bk = k; bo = o; bp = p; bc = c; }
-}
-
-// collisionTimeNormal (src/EDMD.c:2661-2723) and collisionTimeGrow (2598-2659)
-// of an owner current at t and a candidate P, by the two lanes 2k, 2k + 1: one
-// axis each (p1, v1 of the owner), the sums over the axes by shuffle.  A pair
-// costs 16 FP64 instructions instead of the 24 of one lane, and the
-// candidates of an event (about 6 per disk) still fit one pass of a warp.
-// Same operations and roundings as coll_time_normal_i / coll_time_grow (the
-// sums of two products commute).  Every lane of the group takes part; `act`
-// marks the pairs that count.
-template <int GW, bool ADD, bool GROW>
-__device__ __forceinline__ double pair_time_lanes(const Box& B, const Grp<GW>& G, bool act, double p1, double v1,
-                                                  double rad1, double vr1, const Disk* P, const double* vr2p,
-                                                  double t, bool* ovl) {
-  const bool y = G.lane & 1;
-  const double pos = (&P->x)[y ? 1 : 0], vel = (&P->vx)[y ? 1 : 0], rad2 = P->rad;
-  const double lat2 = t - P->tl;
-  const double dv = vel - v1;
-  const double d = near_image((pos + lat2 * vel) - p1, y ? B.hLy : B.hLx, y ? B.Ly : B.Lx);
-  double b = d * dv, v2 = dv * dv, d2 = d * d;
-  b += G.shfl_xor(b, 1);
-  v2 += G.shfl_xor(v2, 1);
-  d2 += G.shfl_xor(d2, 1);
-  if constexpr (!GROW) {
-    d2 -= contact2<ADD>(B, rad1, rad2);
-    // b b on the y lane, v2 d2 on the x lane
-    const double u = (y ? b : v2) * (y ? b : d2);
-    const double w = G.shfl_xor(u, 1);
-    const double det = (y ? u : w) - (y ? w : u);
-    if (!act || is_pos(b)) return NEVER;
-    if (lt_neg(d2, 0.01)) { *ovl = true; return NEVER; }
-    if (is_neg(det)) return NEVER;
-    return div_rn(-b - sqrt_rn(det), v2);
-  } else {
-  const double vr2 = *vr2p;
-  const double dvr = vr1 + vr2;
-  const double dr = contact(B, rad1, rad2 + lat2 * vr2);
-  b -= dvr * dr;
-  const double den = v2 - dvr * dvr, gap = d2 - dr * dr;
-  const double det = b * b - den * gap;
-  const bool root = act && !(det < 0);
-  // the two roots on the two lanes: -b - s on x, -b + s on y
-  double r = 0;
-  if (root) {
-    const double s = sqrt_rn(det);
-    r = div_rn(-b + flip(s, !y), den);
-  }
-  const double q = G.shfl_xor(r, 1);
-  const double minus = y ? q : r, plus = y ? r : q;
-  if (!root) return NEVER;
-  if (((minus > 0) && (plus > 0) && (minus < plus)) || ((minus > 0) && (plus < 0))) return minus;
-  else if (((minus > 0) && (plus > 0.000000001) && (plus < minus)) || ((minus < 0) && (plus > 0.000000001)))
-    return plus;
-  if (gap < -0.01) *ovl = true;
-  return NEVER;
-  }
-}
-
-// group-relative lane of the least (time key, scan order), word by word like
-// grp_argmin; a lane without a candidate has order -1, the largest word, and
-// the least key only when no lane has a candidate
-template <int GW>
-__device__ __forceinline__ int best_lane(uint64_t k, int o, const Grp<GW>& G) {
-  const uint32_t h = (uint32_t)(k >> 32);
-  uint32_t m = G.min_u32(h);
-  bool in = h == m;
-  unsigned q = G.ballot(in);
-  if (q & (q - 1)) {
-    uint32_t v = in ? (uint32_t)k : 0xffffffffu;
-    m = G.min_u32(v);                           // every lane of the group takes part
-    in = in && v == m;
-    v = in ? (uint32_t)o : 0xffffffffu;
-    m = G.min_u32(v);
-    in = in && v == m;
-    q = G.ballot(in);
-  }
-  return __ffs(q) - 1;
-}
-
-// collisionEventNormal / Grow (src/EDMD.c:2829 / 3104) for disks a0 and a1
-// (a1 may be -1), both current at t, whose lane roles hold `own`: scan the
-// 3x3 neighbour cells, dy outer and dx inner, list order, keep the first
-// strict minimum.  The (disk, cell) walks are tasks t = 0..8 (a0's cells in
-// scan order) and 9..17 (a1's): task t runs on lane t % GW, a lane with two
-// tasks walks both lists at once.  The candidates are then packed over the
-// group in task order and solved by two lanes each.
-template <int GW, bool ADD, bool GROW>
-__device__ __forceinline__ Next predict2(const SysDev& S, double t, int a0, int a1, const Own& own,
-                                         uint64_t* npair, const Grp<GW>& G, WarpSmem* sm, bool* ovl, int* ovl_a,
-                                         int* ovl_b) {
-  const Box& B = S.B;
-  const int lane = G.lane;
-  const double dinit = GROW ? 10000000 : NEVER;
-  const int ntask = a1 >= 0 ? 18 : 9;
-  const int X0 = G.shfl(own.c, 0), X1 = G.shfl(own.c, 1), Y0 = G.shfl(own.c, 2), Y1 = G.shfl(own.c, 3);
-  // the tasks of this lane: t = lane + k GW, k < NT (a warp: one task per
-  // lane; 16 lanes: two; 8 lanes: three; 4 lanes: five)
-  constexpr int NT = (18 + GW - 1) / GW;
-  int pt[NT], ct[NT], ot[NT], qt[NT], hc[NT];
-#pragma unroll
-  for (int k = 0; k < NT; k++) {
-    const int u = lane + k * GW;
-    const bool second = u >= 9;
-    ot[k] = second ? a1 : a0;
-    const int q = second ? u - 9 : u;
-    qt[k] = q;
-    hc[k] = pbc_cy(B, (second ? Y1 : Y0) + q / 3 - 1) * B.Nxc + pbc_cx(B, (second ? X1 : X0) + q % 3 - 1);
-    pt[k] = u < ntask ? S.head[hc[k]] : NIL;
-    ct[k] = 0;
-  }
-  bool lcorrupt = false;
-  {
-    int guard = 0;                   // the lists hold N disks in all
-    bool more = true;
-    while (more && guard++ < 2 * B.N) {
-      more = false;
-#pragma unroll
-      for (int k = 0; k < NT; k++) {
-        if (pt[k] != NIL) {
-          const int u = lane + k * GW;
-          if (pt[k] != ot[k]) { if (ct[k] < MAXC) sm->reg[u * MAXC + ct[k]] = pt[k]; ct[k]++; }
-          pt[k] = S.d[pt[k]].nxt;
-          more |= pt[k] != NIL;
-        }
-      }
-    }
-    // a list longer than N is corrupt: reported like an overlap, with the
-    // marker OVL_CORRUPT in place of the first disk (EDMD_ERR_BUDGET)
-#pragma unroll
-    for (int k = 0; k < NT; k++)
-      if (pt[k] != NIL) lcorrupt = true;
-  }
-  bool over = false;
-#pragma unroll
-  for (int k = 0; k < NT; k++) over |= ct[k] > MAXC;
-  const bool spill = G.any(over);
-  uint64_t bd0 = cand_key(dinit), bd1 = bd0;
-  int bo0 = -1, bo1 = -1, bp0 = 0, bp1 = 0;
-  uint32_t bc0 = 0, bc1 = 0;
-  // of several overlapping pairs the one named is fixed by the order the
-  // candidates have when each takes a lane of its own
-  uint32_t lk = 0xffffffffu;
-  int la = -1, lb = -1;
-  int tot;
-  if (!spill) {
-    // exclusive prefix of the counts (at most 7) in task order, bit by bit
-    int ex[NT];
-    int base = 0;
-    const unsigned below = (1u << lane) - 1u;
-#pragma unroll
-    for (int k = 0; k < NT; k++) {
-      const unsigned c0 = G.ballot(ct[k] & 1), c1 = G.ballot(ct[k] & 2), c2 = G.ballot(ct[k] & 4);
-      ex[k] = base + __popc(c0 & below) + 2 * __popc(c1 & below) + 4 * __popc(c2 & below);
-      base += __popc(c0) + 2 * __popc(c1) + 4 * __popc(c2);
-    }
-    // a0's candidates are tasks 0..8: their count is the prefix at task 9
-    const int tot0 = G.shfl(ex[9 / GW], 9 % GW);
-    tot = base;
-#pragma unroll
-    for (int k = 0; k < NT; k++) {
-      const int u = lane + k * GW;
-      for (int m = 0; m < ct[k]; m++) {
-        sm->comp[ex[k] + m] = sm->reg[u * MAXC + m];
-        sm->ord[ex[k] + m] = (int16_t)(qt[k] * MAXC + m);
-      }
-    }
-    G.sync();
-    for (int f0 = 0; f0 < tot; f0 += GW / 2) {
-      const int f = f0 + (lane >> 1);
-      const bool act = f < tot;
-      const bool g1 = act && f >= tot0;
-      const int src = (g1 ? 1 : 0) | ((lane & 1) << 1);
-      const double p1 = G.shfl(own.p, src), v1 = G.shfl(own.v, src), rad1 = G.shfl(own.rad, src);
-      const double vr1 = GROW ? G.shfl(own.vr, src) : 0.0;
-      const int p = act ? sm->comp[f] : a0;
-      const int o = act ? sm->ord[f] : 0;
-      const Disk* P = S.d + p;
-      const uint32_t pc = P->coll;
-      bool ov = false;
-      const uint64_t kd =
-          cand_key(pair_time_lanes<GW, ADD, GROW>(B, G, act, p1, v1, rad1, vr1, P, S.vr + p, t, &ov));
-      if (ov) {
-        const uint32_t k = ((uint32_t)(f % GW) << 16) | (0xffffu - (uint32_t)f);
-        if (k < lk) { lk = k; la = g1 ? a1 : a0; lb = p; }
-      }
-      if (g1) best_merge(bd1, bo1, bp1, bc1, kd, o, p, pc);
-      else if (act) best_merge(bd0, bo0, bp0, bc0, kd, o, p, pc);
-    }
-    G.sync();
-  } else {
-    // a cell list longer than MAXC: the lists are walked again, one after the
-    // other, every pair by the first two lanes
-    tot = 0;
-#pragma unroll 1
-    for (int u = 0; u < ntask; u++) {
-      const bool g1 = u >= 9;
-      const int q = g1 ? u - 9 : u, a = g1 ? a1 : a0;
-      const int src = (g1 ? 1 : 0) | ((lane & 1) << 1);
-      const double p1 = G.shfl(own.p, src), v1 = G.shfl(own.v, src), rad1 = G.shfl(own.rad, src);
-      const double vr1 = GROW ? G.shfl(own.vr, src) : 0.0;
-      int p = S.head[pbc_cy(B, (g1 ? Y1 : Y0) + q / 3 - 1) * B.Nxc + pbc_cx(B, (g1 ? X1 : X0) + q % 3 - 1)];
-      int k = 0, guard = 0;
-      while (p != NIL && guard++ < B.N) {
-        const Disk* P = S.d + p;
-        const int nx = P->nxt;
-        if (p != a) {
-          bool ov = false;
-          const uint64_t kd =
-              cand_key(pair_time_lanes<GW, ADD, GROW>(B, G, true, p1, v1, rad1, vr1, P, S.vr + p, t, &ov));
-          if (ov) {
-            const uint32_t w = ((uint32_t)(u % GW) << 16) | (0xffffu - (uint32_t)(u * 2048 + min(k, 2047)));
-            if (w < lk) { lk = w; la = a; lb = p; }
-          }
-          if (g1) best_merge(bd1, bo1, bp1, bc1, kd, q * 4096 + k, p, P->coll);
-          else best_merge(bd0, bo0, bp0, bc0, kd, q * 4096 + k, p, P->coll);
-          k++;
-        }
-        p = nx;
-      }
-      if (p != NIL) lcorrupt = true;
-      tot += k;
-    }
-  }
-  *npair += (uint64_t)tot;
-  // lexicographic (dt, scan order) minimum over the group
-  Next r;
-  {
-    const int w0 = best_lane(bd0, bo0, G);
-    bd0 = G.shfl(bd0, w0); bo0 = G.shfl(bo0, w0); bp0 = G.shfl(bp0, w0); bc0 = G.shfl(bc0, w0);
-  }
-  if (a1 >= 0) {
-    const int w1 = best_lane(bd1, bo1, G);
-    bd1 = G.shfl(bd1, w1); bo1 = G.shfl(bo1, w1); bp1 = G.shfl(bp1, w1); bc1 = G.shfl(bc1, w1);
-    if (lane & 1) { bd0 = bd1; bo0 = bo1; bp0 = bp1; bc0 = bc1; }
-  }
-  if (bo0 < 0) bc0 = S.d[0].coll;   // no partner: partner 0 (src/EDMD.c:2830)
-  r.key = bd0; r.partner = bp0; r.ca = bc0;
-  if (G.any(lk != 0xffffffffu || lcorrupt)) {
-    const uint32_t least = G.min_u32(lk);
-    const int src = G.first(lk == least && lk != 0xffffffffu);
-    *ovl = true;
-    if (src >= 0) { *ovl_a = G.shfl(la, src); *ovl_b = G.shfl(lb, src); }
-    if (G.any(lcorrupt)) { *ovl_a = OVL_CORRUPT; *ovl_b = a0; }
-  }
-  return r;
-}
-
 // ---------------------------------------------------------------- handlers
 
 
@@ -746,7 +426,7 @@ __device__ void do_growstop(const SysDev& S, SysState& R, const Grp<GW>& G, Warp
     own.vr = 0;
     own.c = (lane & 2 ? S.cy : S.cx)[i];
     R.npred++;
-    const Next r = predict2<GW, ADD, false>(S, R.t, i, -1, own, &R.npair, G, sm, ovl, oa, ob);
+    const Next r = predict2<GW, ADD, false, GW>(S, R.t, i, -1, own, &R.npair, G, sm, ovl, oa, ob, [](int) {});
     schedule(S, Q, N + i, R.t + key_time(r.key), r.partner, r.ca, 2ull, G);
     unqueue(S, Q, i, G);
     int dir;
@@ -764,25 +444,6 @@ __device__ void do_growstop(const SysDev& S, SysState& R, const Grp<GW>& G, Warp
 // what ends a stretch of disk events
 enum { END_STOP, END_SPECIAL };
 
-// A product per quad of lanes in one FP64 instruction: quad 0 (lanes 0..3 of
-// every 16) takes a b, quad 1 c d, quad 2 e f, and every lane gets the last two
-// back.  Groups too narrow for that multiply in turn.
-template <int GW>
-__device__ __forceinline__ double quad_products(const Grp<GW>& G, double a, double b, double c, double d, double e,
-                                                double f, double* cd, double* ef) {
-  if constexpr (GW >= 16) {
-    const int q = (G.lane >> 2) & 3;
-    const double r = (q == 0 ? a : q == 1 ? c : e) * (q == 0 ? b : q == 1 ? d : f);
-    *cd = G.shfl(r, 4);
-    *ef = G.shfl(r, 8);
-    return r;
-  } else {
-    *cd = c * d;
-    *ef = e * f;
-    return a * b;
-  }
-}
-
 // A stretch of disk events of one system: until a stop, or a special event
 // (screenshot, thermo, growth stop), which is taken off the queue and left in
 // *special.  One event is one chain of dependent instructions, so its latency
@@ -797,17 +458,14 @@ __device__ __forceinline__ double quad_products(const Grp<GW>& G, double a, doub
 template <int GW, bool ADD, bool GROW>
 __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int64_t max_coll, const Grp<GW>& G,
                                           WarpSmem* sm, int64_t& logged, int64_t& nev, int* special) {
-  constexpr bool QUADS = GW >= 16;
   const int lane = G.lane;
   const bool odd = lane & 1, ydim = lane & 2;
-  const bool quad1 = ((lane >> 2) & 3) == 1;
   const Box& B = S.B;
   const int N = B.N;
   SysState* const st = S.st;
   double t = st->t;
   Queue Q = queue_of(*st);
-  // the four virial sums: lane l accumulates term l % 4 (the lanes of quad 1
-  // count, or of the only quad)
+  // the four virial sums: lane l accumulates term l % 4 (see elastic_lanes)
   double ctl = st->collT[lane & 3];
   const double tmax = S.tmax;
   const double onepr = 1 + S.res;
@@ -892,24 +550,11 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
         }
         ncoll++;
         if (!GROW || !(A.flags & EDMD_F_COUNT_NORMAL)) logged++;
-        // j minus i, the same value on both disks' lanes
-        const double po = G.shfl_xor(own.p, 1), vo = G.shfl_xor(own.v, 1);
-        const double mo = G.shfl_xor(m, 1), ro = G.shfl_xor(own.rad, 1);
-        const double d = near_image((odd ? own.p : po) - (odd ? po : own.p), ydim ? B.hLy : B.hLx, ydim ? B.Ly : B.Lx);
-        const double dv = (odd ? own.v : vo) - (odd ? vo : own.v);
+        const Meet c = meet_lanes(B, G, own, m);
+        const double d = c.d, dv = c.dv, mo = c.mo;
         const double msum = m + mo;
         const long long mk = __double_as_longlong(msum);
         if constexpr (!GROW) {   // elastic branch src/EDMD.c:3802-3827
-          // (r . v), sigma^2 and m_i m_j
-          double distSquared, mm, pr;
-          if (ADD && B.additive) {
-            const double s = own.rad + ro;
-            pr = quad_products(G, d, dv, s, s, m, mo, &distSquared, &mm);
-          } else {
-            pr = quad_products(G, d, dv, times4(own.rad), ro, m, mo, &distSquared, &mm);
-          }
-          if constexpr (QUADS) pr = G.shfl(pr, 0) + G.shfl(pr, 2);
-          else pr += G.shfl_xor(pr, 2);
           double inv;
           if (mk == sm->msum[0]) inv = sm->inv[0];
           else if (mk == sm->msum[1]) inv = sm->inv[1];
@@ -922,12 +567,8 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
             }
             G.sync();
           }
-          const double collKernel = inv * pr;
-          // x/4 is exact, so the shortcut rounds identically
-          const double f = __double_as_longlong(distSquared) == 0x4010000000000000ll
-              ? collKernel * 0.25 : div_rn(collKernel, distSquared);
-          const double od = G.shfl_xor(d, 2);
-          const double dx = ydim ? od : d, dy = ydim ? d : od;
+          double dx, dy;
+          const double f = elastic_lanes<GW, ADD>(B, G, own, m, c, inv, ctl, &dx, &dy);
           if (A.flags & EDMD_F_LOG) {
             const double dvo = G.shfl_xor(dv, 2);
             if (S.log && (int64_t)nlog < S.log_cap && lane == 0) {
@@ -936,21 +577,6 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
               lg->dvx = dv; lg->dvy = dvo; lg->f = f;
             }
             nlog++;
-          }
-          // v_i += f m_j r, v_j -= f m_i r (v - x as v + (-x), the same rounding),
-          // and collTermX, Y, XY, YX: term lane % 4, m_i m_j f r_a r_b, beside
-          // it on quad 1
-          const double ra = odd ? dy : dx, rb = ydim == odd ? dx : dy;
-          if constexpr (QUADS) {
-            const double w1 = f * (quad1 ? mm : mo);
-            const double w2 = w1 * (quad1 ? ra : d);
-            const double w3 = w2 * rb;
-            const double s = (quad1 ? ctl : own.v) + (quad1 ? w3 : flip(w2, odd));
-            if (quad1) ctl = s;
-            else own.v = s;
-          } else {
-            ctl += mm * f * ra * rb;
-            own.v += flip(f * mo * d, odd);
           }
         } else {       // growth rule src/EDMD.c:3479-3520, with its res = 1 and delta = 0
           const double dvr = own.vr + G.shfl_xor(own.vr, 1);
@@ -1044,7 +670,7 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
         dir = ux == ydim ? db : da;
       }
       G.sync();
-      const Next nx = predict2<GW, ADD, GROW>(S, t, i, two ? j : -1, own, &npair, G, sm, &ovl, &oa, &ob);
+      const Next nx = predict2<GW, ADD, GROW, GW>(S, t, i, two ? j : -1, own, &npair, G, sm, &ovl, &oa, &ob, [](int) {});
       // addEventToQueue (src/EDMD.c:2144): lanes 0 and 1 take the crossings of
       // the two disks, lanes 2 and 3 their collisions; in that order they get
       // the insertion counters and join the overflow list
@@ -1085,7 +711,7 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
     }
     if (ovl) { status = oa == OVL_CORRUPT ? EDMD_ERR_BUDGET : EDMD_ERR_OVERLAP; break; }
   }
-  const double vir = QUADS ? G.shfl(ctl, 4 | (lane & 3)) : ctl;
+  const double vir = G.shfl(ctl, virial_lane<GW>(lane & 3));
   if (lane < 4) st->collT[lane] = vir;
   if (lane == 0) {
     const uint64_t n = (uint64_t)(nev - nev0) - (end == END_SPECIAL ? 1 : 0);   // disk events

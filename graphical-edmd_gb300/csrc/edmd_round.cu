@@ -44,6 +44,7 @@
 #include <cstdint>
 #include <cstring>
 #include "edmd_ctx.h"
+#include "edmd_lanes.cuh"
 
 namespace {
 
@@ -55,18 +56,15 @@ constexpr int TX = 16, TY = 32;       // selection tile (cells): 2.1 cells loade
                                       // measured against 32x16, 32x8 and 64x8 (best by ~1%)
 constexpr int RTILE = 12;             // largest window radius of the tile kernel
 constexpr int MAXDIRTY = 8;           // cells whose minimum one event can change
-constexpr int MAXC = 8;               // candidates buffered per cell list per lane
 constexpr int OB_CORRUPT = -2;        // overlap partner marker: a cell list longer than N (EDMD_ERR_BUDGET)
 // tie ranks of collision events (the top byte of an event id, see event_id):
 // inherited mutual pairs are 1 (pops first) and 2, events this engine makes
 // are R_NEW, or R_FIRST when the serial queue would pop them before the
 // inherited event of equal time they tie with (new_rank)
 constexpr uint8_t R_FIRST = 0, R_NEW = 3;
-constexpr int WPB = 1;                // warps per block of the processing kernel (measured best:
-                                      // one-warp blocks, 20 per SM, 96 registers)
 constexpr int NSTRIPE = 32;           // copies of each system's counters
 // counters of the round engine, per system and stripe (u64 slots)
-enum { C_CT0, C_CT1, C_CT2, C_CT3, C_NCOL, C_NCROSS, C_NSTALE, C_NPAIR, C_NPRED, C_NEV, C_NSCREEN, C_TLAST, NCNT };
+enum { C_CT0, C_CT1, C_CT2, C_CT3, C_NCOL, C_NCROSS, C_NSTALE, C_NPAIR, C_NSCREEN, C_TLAST, NCNT };
 
 struct RoundArgs {
   int32_t nsys;
@@ -290,7 +288,7 @@ __global__ void k_prep(const SysDev* __restrict__ sys, RoundArgs A) {
   }
   const double ep = S.st->t;
   if (i == 0) A.epoch[s] = ep;
-  shadow_write(A, g, B, S.d[i], S.cx[i], S.cy[i], ep);
+  if (A.flags & EDMD_F_SCREEN) shadow_write(A, g, B, S.d[i], S.cx[i], S.cy[i], ep);
   uint64_t key;
   int c1, c2;
   const int slot = attribution(S, i, &key, &c1, &c2);
@@ -501,185 +499,19 @@ __device__ bool stamp_write(const RoundArgs& A, int64_t base, int c, uint64_t cl
   return bad;
 }
 
-// collisionEventNormal (src/EDMD.c:2829-2905) for disks a0 and a1 (a1 may be
-// -1), each current at time t, by one warp: lanes 0..8 walk a0's 3x3 cells and
-// lanes 16..24 a1's (dy outer, dx inner), the candidates are packed over the
-// warp and each lane solves a share of the pairs; the result is the first
-// strict minimum below NEVER in the reference's scan order (lexicographic
-// (time, scan position)); with none the partner stays 0 and collActual is
-// disk 0's counter.
+// a prediction by one thread (predict_thread)
 struct Pred {
   double dt;
   int partner;
   uint32_t ca;
   int pcell;     // partner's cell, or the owner's when there is none
 };
-struct WarpScratch {
-  int32_t reg[32 * MAXC];
-  int32_t comp[2 * 9 * MAXC];
-  int16_t ord[2 * 9 * MAXC];
-};
-
-__device__ __forceinline__ void merge(double& bd, uint64_t& bk, int& bo, int& bp, uint32_t& bc,
-                                      double d, uint64_t kd, int o, int p, uint32_t c) {
-  if (kd < bk || (kd == bk && o < bo)) { bd = d; bk = kd; bo = o; bp = p; bc = c; }
-}
-
-__device__ void predict_warp(const SysDev& S, int a0, const Disk& A0, int X0, int Y0, int a1,
-                             const Disk& A1, int X1, int Y1, double t, Pred& r0, Pred& r1,
-                             WarpScratch* W, int lane, unsigned long long* npair, bool* ovl, int* oa,
-                             int* ob) {
-  const Box& B = S.B;
-  const int grp = lane >> 4, q = lane & 15;
-  const int a = grp ? a1 : a0;
-  const int X = grp ? X1 : X0, Y = grp ? Y1 : Y0;
-  int cnt = 0;
-  bool lcorrupt = false;
-  int32_t* reg = W->reg + lane * MAXC;
-  if (a >= 0 && q < 9) {
-    int p = S.head[pbc_cy(B, Y + q / 3 - 1) * B.Nxc + pbc_cx(B, X + q % 3 - 1)];
-    int guard = 0;                   // a list is never longer than N
-    while (p != NIL && guard++ < B.N) {
-      if (p != a) {
-        if (cnt < MAXC) reg[cnt] = p;
-        cnt++;
-      }
-      p = S.d[p].nxt;
-    }
-    if (p != NIL) { lcorrupt = true; }   // a list longer than N is corrupt
-  }
-  const bool spill = __any_sync(FULLM, cnt > MAXC);
-  const uint64_t knever = time_key(NEVER);
-  double bd0 = NEVER, bd1 = NEVER;
-  uint64_t bk0 = knever, bk1 = knever;
-  int bo0 = -1, bo1 = -1, bp0 = 0, bp1 = 0;
-  uint32_t bc0 = 0, bc1 = 0;
-  bool lovl = false;
-  int la = -1, lb = -1;               // the predicting disk and the partner that overlaps it
-  unsigned long long tot;
-  if (!spill) {
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 16; o <<= 1) {
-      const int v = __shfl_up_sync(FULLM, incl, o, 16);
-      if (q >= o) incl += v;
-    }
-    const int excl = incl - cnt;
-    const int tot0 = __shfl_sync(FULLM, incl, 15), tot1 = __shfl_sync(FULLM, incl, 31);
-    const int bse = grp ? tot0 : 0;
-    for (int k = 0; k < cnt; k++) {
-      W->comp[bse + excl + k] = reg[k];
-      W->ord[bse + excl + k] = (int16_t)(q * MAXC + k);
-    }
-    __syncwarp();
-    tot = (unsigned long long)(tot0 + tot1);
-    for (int f = lane; f < tot0 + tot1; f += 32) {
-      const int p = W->comp[f];
-      const int o = W->ord[f];
-      const Disk P = S.d[p];
-      const bool g1 = f >= tot0;
-      bool ov = false;
-      const double d = coll_time_normal_i(B, g1 ? A1 : A0, P, t, &ov);
-      if (ov) { lovl = true; la = g1 ? a1 : a0; lb = p; }
-      const uint64_t kd = time_key(d);
-      if (g1) merge(bd1, bk1, bo1, bp1, bc1, d, kd, o, p, P.coll);
-      else merge(bd0, bk0, bo0, bp0, bc0, d, kd, o, p, P.coll);
-    }
-    __syncwarp();
-  } else {
-    // a list longer than MAXC: every lane walks and solves its own list
-    unsigned long long mine = 0;
-    if (a >= 0 && q < 9) {
-      const Disk& AA = grp ? A1 : A0;
-      int p = S.head[pbc_cy(B, Y + q / 3 - 1) * B.Nxc + pbc_cx(B, X + q % 3 - 1)];
-      int k = 0, guard = 0;
-      while (p != NIL && guard++ < B.N) {
-        const Disk P = S.d[p];
-        if (p != a) {
-          bool ov = false;
-          const double d = coll_time_normal_i(B, AA, P, t, &ov);
-          if (ov) { lovl = true; la = a; lb = p; }
-          const uint64_t kd = time_key(d);
-          if (grp) merge(bd1, bk1, bo1, bp1, bc1, d, kd, q * (1 << 20) + k, p, P.coll);
-          else merge(bd0, bk0, bo0, bp0, bc0, d, kd, q * (1 << 20) + k, p, P.coll);
-          k++;
-          mine++;
-        }
-        p = P.nxt;
-      }
-      if (p != NIL) lcorrupt = true;
-    }
-    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(FULLM, mine, o);
-    tot = mine;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    double d = __shfl_xor_sync(FULLM, bd0, o);
-    uint64_t kd = __shfl_xor_sync(FULLM, bk0, o);
-    int oo = __shfl_xor_sync(FULLM, bo0, o), pp = __shfl_xor_sync(FULLM, bp0, o);
-    uint32_t cc = __shfl_xor_sync(FULLM, bc0, o);
-    merge(bd0, bk0, bo0, bp0, bc0, d, kd, oo, pp, cc);
-    d = __shfl_xor_sync(FULLM, bd1, o);
-    kd = __shfl_xor_sync(FULLM, bk1, o);
-    oo = __shfl_xor_sync(FULLM, bo1, o);
-    pp = __shfl_xor_sync(FULLM, bp1, o);
-    cc = __shfl_xor_sync(FULLM, bc1, o);
-    merge(bd1, bk1, bo1, bp1, bc1, d, kd, oo, pp, cc);
-  }
-  const int div = spill ? (1 << 20) : MAXC;
-  r0.dt = bd0; r0.partner = bp0; r0.ca = bo0 < 0 ? S.d[0].coll : bc0;
-  {
-    const int qq = bo0 < 0 ? 4 : bo0 / div;
-    r0.pcell = pbc_cy(B, Y0 + qq / 3 - 1) * B.Nxc + pbc_cx(B, X0 + qq % 3 - 1);
-  }
-  if (a1 >= 0) {
-    r1.dt = bd1; r1.partner = bp1; r1.ca = bo1 < 0 ? S.d[0].coll : bc1;
-    const int qq = bo1 < 0 ? 4 : bo1 / div;
-    r1.pcell = pbc_cy(B, Y1 + qq / 3 - 1) * B.Nxc + pbc_cx(B, X1 + qq % 3 - 1);
-  }
-  *npair += tot;
-  const unsigned m = __ballot_sync(FULLM, lovl);
-  if (m) {
-    *ovl = true;
-    *oa = __shfl_sync(FULLM, la, __ffs(m) - 1);
-    *ob = __shfl_sync(FULLM, lb, __ffs(m) - 1);
-  }
-  if (__any_sync(FULLM, lcorrupt)) { *ovl = true; *oa = a0; *ob = OB_CORRUPT; }
-}
 
 __device__ __forceinline__ void set_event(const SysDev& S, int slot, double t, int j, uint32_t ca,
                                           uint32_t pcell, uint64_t clock) {
   Ev e;
   e.t = t; e.tie = kmax(time_key(t), clock); e.b = pcell; e.j = j; e.ca = ca; e.st = ST_QUEUED;
   S.ev[slot] = e;
-}
-
-// new attribution of disk i (global index g); its cells join the dirty list
-__device__ __forceinline__ void reattribute(const SysDev& S, const RoundArgs& A, int i, int64_t g,
-                                            int64_t base, int32_t* dc, int* nd) {
-  uint64_t key;
-  int c1, c2;
-  const int slot = attribution(S, i, &key, &c1, &c2);
-  A.dkey[g] = key;
-  A.dpk[g] = event_id(A, g, slot, S.B.N);
-  A.fc[2 * g] = c1;
-  A.fc[2 * g + 1] = c2;
-  dc[(*nd)++] = (int32_t)(base + c1);
-  if (c2 != c1) dc[(*nd)++] = (int32_t)(base + c2);
-}
-
-// read stamps of the 3x3 cells around c by lanes l0..l0+8 (warp-wide result)
-__device__ __forceinline__ bool stamp_read_warp(const Box& B, const RoundArgs& A, int64_t base, int c,
-                                                uint64_t clk, int lane, int l0) {
-  bool bad = false;
-  const int q = lane - l0;
-  if (q >= 0 && q < 9) {
-    const int x = c % B.Nxc, y = c / B.Nxc;
-    const int64_t gc = base + pbc_cy(B, y + q / 3 - 1) * B.Nxc + pbc_cx(B, x + q % 3 - 1);
-    if (A.lw[gc] > clk) bad = true;
-    if (A.lr[gc] < clk) atomicMax((unsigned long long*)&A.lr[gc], (unsigned long long)clk);
-  }
-  return __any_sync(FULLM, bad);
 }
 
 __device__ __forceinline__ void cnt_add(const RoundArgs& A, int s, int stripe, int k, unsigned long long v) {
@@ -689,211 +521,198 @@ __device__ __forceinline__ void cnt_addf(const RoundArgs& A, int s, int stripe, 
   atomicAdd((double*)&A.cnt[((int64_t)s * NSTRIPE + stripe) * NCNT + k], v);
 }
 
-__device__ __forceinline__ Disk shfl_disk(const Disk& v, int src) {
-  Disk r;
-  r.x = __shfl_sync(FULLM, v.x, src);
-  r.y = __shfl_sync(FULLM, v.y, src);
-  r.vx = __shfl_sync(FULLM, v.vx, src);
-  r.vy = __shfl_sync(FULLM, v.vy, src);
-  r.tl = __shfl_sync(FULLM, v.tl, src);
-  r.rad = __shfl_sync(FULLM, v.rad, src);
-  r.m = __shfl_sync(FULLM, v.m, src);
-  r.nxt = __shfl_sync(FULLM, v.nxt, src);
-  r.coll = __shfl_sync(FULLM, v.coll, src);
-  return r;
-}
-
-// outcome of one processed event (lane 0 holds everything but `ct`, which
-// lane q < 4 holds for virial term q)
+// outcome of one processed event, the same on all lanes of its group but for
+// `dc` (lanes 0..7: one cell each whose minimum can have changed, or -1) and
+// `ct` (lane virial_lane(k): virial term k)
 struct EvResult {
-  int32_t dc[MAXDIRTY];              // cells whose minimum can have changed
-  int nd;
-  unsigned long long npair, npred, ncol, ncross, nstale, nscreen;
+  int32_t dc;
+  bool ncol, ncross, nstale;
+  uint64_t npair;
   double ct;
   uint64_t key;
   bool bad, ovl;
   int a, ob;
 };
 
-// one selected event g of system s processed by one warp: doTheCollisionNormal
-// (src/EDMD.c:3542, elastic rule 3802-3827), its stale branch (3553-3556) or
-// doTheCrossing (2501).  The scalar work is repeated by every lane (same
-// values), stores are made by lane 0, predictions are shared by the warp.
-__device__ void process_event_warp(const SysDev& S, const RoundArgs& A, int s, int64_t g, WarpScratch* W,
-                                   int lane, EvResult& res) {
-    const Box& B = S.B;
-    const int N = B.N;
-    const int64_t base = A.coff[s], dbase = A.doff[s];
-    const int a = (int)(g - dbase);
-    uint64_t key;
-    const int slot = next_slot(S, a, &key);
-    const Ev E = S.ev[slot];
-    const double t = E.t;
-    const uint64_t clk = E.tie;        // serial pop clock of this event
-    int32_t dc[MAXDIRTY];
-    int nd = 0;
-    dc[nd++] = (int32_t)(base + A.fc[2 * g]);
-    if (A.fc[2 * g + 1] != A.fc[2 * g]) dc[nd++] = (int32_t)(base + A.fc[2 * g + 1]);
-    Disk Da = S.d[a];
-    const int ax = S.cx[a], ay = S.cy[a];
-    const int ca = cell_of(B, ax, ay);
-    unsigned long long npair = 0, npred = 0, ncol = 0, ncross = 0, nstale = 0;
-    double ct[1] = {0};
-    bool ovl = false, bad = false;
-    int ob = -1;
-    // what the shared tail does, set by the handler: the second disk of a
-    // collision, the cells of the disks, the cells stamped as written and
-    // the centres of the 3x3 blocks stamped as read, new crossing events
-    int b = -1;
-    int64_t gb = -1;
-    int pax = ax, pay = ay, pbx = ax, pby = ay;
-    int wc1 = -1, rc0 = ca, rc1 = -1;
-    bool cross = false;
-    Disk Db = Da;
-    if (slot >= N) {
-      Db = S.d[E.j];
-      if (E.ca != Db.coll) {
-        free_fly_i(B, Da, t);
-        __syncwarp();
-        if (lane == 0) {
-          S.d[a] = Da;
-          shadow_write(A, g, B, Da, ax, ay, A.epoch[s]);
-        }
-        nstale = 1;
-      } else {
-        b = E.j;
-        gb = dbase + b;
-        dc[nd++] = (int32_t)(base + A.fc[2 * gb]);
-        if (A.fc[2 * gb + 1] != A.fc[2 * gb]) dc[nd++] = (int32_t)(base + A.fc[2 * gb + 1]);
-        const int bx = S.cx[b], by = S.cy[b];
-        const int cb = cell_of(B, bx, by);
-        // even lanes advance a, odd lanes b: the per-disk FP64 work of the
-        // two disks shares its instructions
-        const bool odd = lane & 1;
-        Disk M = odd ? Db : Da;
-        free_fly_i(B, M, t);
-        M.coll++;
-        Da = shfl_disk(M, 0);
-        Db = shfl_disk(M, 1);
-        double dx = Db.x - Da.x, dy = Db.y - Da.y;
-        const double dvx = Db.vx - Da.vx, dvy = Db.vy - Da.vy;
-        const double msum = Da.m + Db.m;
-        const double invMass = __double_as_longlong(msum) == 0x4000000000000000ll ? 0.5 : div_rn(1.0, msum);
-        pbc_i(B, dx, dy);
-        const double collKernel = invMass * (1 + S.res) * (dx * dvx + dy * dvy);
-        const double distSquared = contact2(B, Da.rad, Db.rad);
-        const double f = __double_as_longlong(distSquared) == 0x4010000000000000ll
-            ? collKernel * 0.25 : div_rn(collKernel, distSquared);
-        const double cf = Da.m * Db.m * f;
-        // virial term q on lane q: collTermX, Y, XY, YX
-        {
-          const double u = (lane == 1 || lane == 3) ? dy : dx;
-          const double w = (lane == 0 || lane == 3) ? dx : dy;
-          ct[0] = cf * u * w;
-        }
-        // v - x as v + (-x) (the same rounding): no divergent branch
-        {
-          const double fm = f * (odd ? Da.m : Db.m);
-          M.vx = M.vx + flip(fm * dx, odd);
-          M.vy = M.vy + flip(fm * dy, odd);
-        }
-        Da.vx = __shfl_sync(FULLM, M.vx, 0);
-        Da.vy = __shfl_sync(FULLM, M.vy, 0);
-        Db.vx = __shfl_sync(FULLM, M.vx, 1);
-        Db.vy = __shfl_sync(FULLM, M.vy, 1);
-        __syncwarp();
-        if (lane == 0) {
-          S.d[a] = Da;
-          S.d[b] = Db;
-          shadow_write(A, g, B, Da, ax, ay, A.epoch[s]);
-          shadow_write(A, gb, B, Db, bx, by, A.epoch[s]);
-          if ((A.flags & EDMD_F_TRACE) && S.trace) {
-            const unsigned long long k = atomicAdd((unsigned long long*)&S.st->ntrace, 1ull);
-            if ((int64_t)k < S.trace_cap) {
-              edmd_collision* tr = (edmd_collision*)S.trace + k;
-              tr->i = a; tr->j = b; tr->cell_i = ca; tr->cell_j = cb; tr->t = t;
-            }
-          }
-        }
-        pbx = bx; pby = by;
-        wc1 = cb; rc1 = cb;
-        cross = true;
-        ncol = 1;
+// One selected event g of system s processed by a group of GW lanes:
+// doTheCollisionNormal (src/EDMD.c:3542, elastic rule 3802-3827), its stale
+// branch (3553-3556) or doTheCrossing (2501).  The lanes hold the roles of
+// edmd_lanes.cuh, so an event's scalar FP64 work (and, with GW = 8, that of the
+// four events of a warp) shares its instructions; `on` is false in a group
+// without an event, which follows along on event g without storing anything.
+template <int GW>
+__device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& A, int s, int64_t g, bool on,
+                                              LaneScratch* W, const Grp<GW>& G, EvResult& res) {
+  const Box& B = S.B;
+  const int N = B.N, gl = G.lane;
+  const bool odd = gl & 1, ydim = gl & 2;
+  const int64_t base = A.coff[s], dbase = A.doff[s];
+  const int a = (int)(g - dbase);
+  const Ev ec = S.ev[a], ek = S.ev[N + a];
+  const uint64_t kc = (ec.st & 3u) ? time_key(ec.t) : KINF, kk = (ek.st & 3u) ? time_key(ek.t) : KINF;
+  const bool coll = kk < kc;                 // the crossing wins an exact tie (next_slot)
+  res.key = coll ? kk : kc;
+  const double t = coll ? ek.t : ec.t;
+  const uint64_t clk = coll ? ek.tie : ec.tie;          // serial pop clock of this event
+  const int j = coll ? ek.j : a, my = odd ? j : a;
+  const int64_t gm = dbase + my;
+  Disk* const D = S.d + my;
+  Own own;
+  own.p = *axis_pos(D, ydim); own.v = *axis_vel(D, ydim); own.rad = D->rad; own.vr = 0;
+  own.c = (ydim ? S.cy : S.cx)[my];
+  const double m = D->m;
+  const uint32_t hits = D->coll;
+  const int32_t fold = A.fc[2 * gm + (ydim ? 1 : 0)];   // cells the disk's old event was attributed to
+  {
+    const double L = ydim ? B.Ly : B.Lx;
+    own.p += (t - D->tl) * own.v;
+    if (is_neg(own.p)) own.p += L;
+    else if (ge_pos(own.p, L)) own.p -= L;
+  }
+  const uint32_t hits_j = G.shfl(hits, 1);
+  const bool stale = coll && ek.ca != hits_j, two = coll && !stale, cross = !coll;
+  const int ca = cell_of(B, G.shfl(own.c, 0), G.shfl(own.c, 2));
+  const int cb = cell_of(B, G.shfl(own.c, 1), G.shfl(own.c, 3));
+  int wc1 = two ? cb : -1;                   // the second cell stamped as written
+  res.ct = 0;
+  if (two) {
+    const Meet c = meet_lanes(B, G, own, m);
+    const double msum = m + c.mo;
+    const double inv = (__double_as_longlong(msum) == 0x4000000000000000ll ? 0.5 : div_rn(1.0, msum)) * (1 + S.res);
+    double dx, dy;
+    elastic_lanes<GW, true>(B, G, own, m, c, inv, res.ct, &dx, &dy);
+    if (on && gl < 4) {
+      *axis_pos(D, ydim) = own.p;
+      *axis_vel(D, ydim) = own.v;
+      if (!ydim) {
+        D->tl = t;
+        D->coll = hits + 1;
       }
-    } else {
-      free_fly_i(B, Da, t);
-      int cx = ax, cy = ay;
-      int wrapx = 0, wrapy = 0;
-      switch (E.j) {
-        case 1: if (cx - 1 == -1) { cx = B.Nxc - 1; wrapx = -1; } else cx -= 1; break;
-        case 2: if (cx + 1 == B.Nxc) { cx = 0; wrapx = 1; } else cx += 1; break;
-        case 3: if (cy - 1 == -1) { cy = B.Nyc - 1; wrapy = -1; } else cy -= 1; break;
-        default: if (cy + 1 == B.Nyc) { cy = 0; wrapy = 1; } else cy += 1; break;
+    }
+    if (on && (A.flags & EDMD_F_TRACE) && S.trace && gl == 0) {
+      const unsigned long long k = atomicAdd((unsigned long long*)&S.st->ntrace, 1ull);
+      if ((int64_t)k < S.trace_cap) {
+        edmd_collision* tr = (edmd_collision*)S.trace + k;
+        tr->i = a; tr->j = j; tr->cell_i = ca; tr->cell_j = cb; tr->t = t;
       }
-      const int c = cell_of(B, cx, cy);
-      __syncwarp();
-      if (lane == 0) {
-        // unlink from the old cell, relink at the head of the new one
-        const int pv = S.prv[a], nx = Da.nxt;
-        if (pv == NIL) S.head[ca] = nx;
-        else S.d[pv].nxt = nx;
-        if (nx != NIL) S.prv[nx] = pv;
-        if (wrapx) S.crossX[a] += wrapx;
-        if (wrapy) S.crossY[a] += wrapy;
-        const int h = S.head[c];
-        S.cx[a] = cx;
-        S.cy[a] = cy;
-        S.prv[a] = NIL;
-        Da.nxt = h;
-        S.d[a] = Da;
-        shadow_write(A, g, B, Da, cx, cy, A.epoch[s]);
-        S.head[c] = a;
-        if (h != NIL) S.prv[h] = a;
+    }
+  } else {
+    int wrap = 0;
+    if (cross && ydim == (ec.j >= 3)) {
+      const int n = ydim ? B.Nyc : B.Nxc;
+      if (ec.j & 1) { if (own.c - 1 == -1) { own.c = n - 1; wrap = -1; } else own.c -= 1; }
+      else { if (own.c + 1 == n) { own.c = 0; wrap = 1; } else own.c += 1; }
+    }
+    const int to = cell_of(B, G.shfl(own.c, 0), G.shfl(own.c, 2));
+    if (cross) wc1 = to;
+    if (on && (gl == 0 || gl == 2)) {
+      *axis_pos(D, ydim) = own.p;
+      if (cross) {
+        (ydim ? S.cy : S.cx)[a] = own.c;
+        if (wrap) (ydim ? S.crossY : S.crossX)[a] += wrap;
       }
-      pax = cx; pay = cy;
-      wc1 = c; rc0 = c;
-      cross = true;
-      ncross = 1;
+      if (!ydim) D->tl = t;
     }
-    // ---- the tail shared by the three handlers: causality stamps, new
-    // crossing events (a on even lanes, b on odd ones), new collision events
-    // (collisionEvent for a, then b), the event records and attribution
-    bad |= lane == 0 && (stamp_write(A, base, ca, clk) | (wc1 >= 0 && stamp_write(A, base, wc1, clk)));
-    bad |= stamp_read_warp(B, A, base, rc0, clk, lane, 0);
-    if (rc1 >= 0) bad |= stamp_read_warp(B, A, base, rc1, clk, lane, 16);
-    __syncwarp();
-    double ctc = 0;
-    int cdir = 0;
-    if (cross) {
-      const bool od = (lane & 1) && b >= 0;
-      ctc = crossing_time_lanes(B, od ? Db : Da, od ? pbx : pax, od ? pby : pay, t, lane, 2, &cdir);
+    if (on && cross && gl == 0) {
+      // unlink from the old cell, relink at the head of the new one
+      const int pv = S.prv[a], nx = D->nxt;
+      if (pv == NIL) S.head[ca] = nx;
+      else S.d[pv].nxt = nx;
+      if (nx != NIL) S.prv[nx] = pv;
+      const int h = S.head[to];
+      S.prv[a] = NIL;
+      D->nxt = h;
+      S.head[to] = a;
+      if (h != NIL) S.prv[h] = a;
     }
-    Pred p0, p1;
-    int oa = a;
-    predict_warp(S, a, Da, pax, pay, b, Db, pbx, pby, t, p0, p1, W, lane, &npair, &ovl, &oa, &ob);
-    npred = b >= 0 ? 2 : 1;
-    const double tca = __shfl_sync(FULLM, ctc, 0), tcb = __shfl_sync(FULLM, ctc, 1);
-    const int dira = __shfl_sync(FULLM, cdir, 0), dirb = __shfl_sync(FULLM, cdir, 1);
-    if (lane == 0) {
-      if (cross) set_event(S, a, tca, dira, 0, 0, clk);
-      if (b >= 0) set_event(S, b, tcb, dirb, 0, 0, clk);
-      const uint8_t rka = new_rank(S, A, dbase, a, b, t + p0.dt, p0.partner, clk);
-      const uint8_t rkb = b >= 0 ? new_rank(S, A, dbase, b, a, t + p1.dt, p1.partner, clk) : R_NEW;
-      set_event(S, N + a, t + p0.dt, p0.partner, p0.ca, p0.pcell, clk);
-      if (b >= 0) set_event(S, N + b, t + p1.dt, p1.partner, p1.ca, p1.pcell, clk);
-      A.drank[g] = rka;
-      if (b >= 0) A.drank[gb] = rkb;
-      reattribute(S, A, a, g, base, dc, &nd);
-      if (b >= 0) reattribute(S, A, b, gb, base, dc, &nd);
+  }
+  // causality stamps of the written cells
+  bool bad = false;
+  if (on && gl == 0) bad = stamp_write(A, base, ca, clk);
+  if (on && gl == 1 && wc1 >= 0) bad = stamp_write(A, base, wc1, clk);
+  // the next crossing (src/EDMD.c:2405-2482): one axis per lane
+  double tc = 0;
+  int dir = 0;
+  {
+    const bool neg = is_neg(own.v);
+    const double w = near_image((neg ? own.c : 1 + own.c) * (ydim ? B.cys : B.cxs) - own.p, ydim ? B.hLy : B.hLx,
+                                ydim ? B.Ly : B.Lx);
+    const double ta = stale ? 0.0 : div_rn(w, own.v);
+    const int da = (ydim ? 3 : 1) + (neg ? 0 : 1);
+    const double tb = G.shfl_xor(ta, 2);
+    const int db = G.shfl_xor(da, 2);
+    const bool ux = lt_i(ydim ? tb : ta, ydim ? ta : tb);
+    tc = ux == ydim ? tb : ta;
+    dir = ux == ydim ? db : da;
+  }
+  __syncwarp();
+  res.npair = 0;
+  res.ovl = false;
+  res.a = a;
+  res.ob = -1;
+  const Next nx = predict2<GW, true, false, 32>(S, t, a, two ? j : -1, own, &res.npair, G, W, &res.ovl, &res.a,
+                                                &res.ob, [&](int cell) {
+    // stamps of the cells read
+    const int64_t gc = base + cell;
+    if (!on) return;
+    if (A.lw[gc] > clk) bad = true;
+    if (A.lr[gc] < clk) atomicMax((unsigned long long*)&A.lr[gc], (unsigned long long)clk);
+  });
+  if (res.ovl && res.a == OVL_CORRUPT) { res.a = a; res.ob = OB_CORRUPT; }
+  // event records: lanes 0 and 1 take the crossings, lanes 2 and 3 the
+  // collisions of the two disks
+  const unsigned who = stale ? 4u : two ? 15u : 5u;
+  const bool mine = gl < 4 && ((who >> gl) & 1u);
+  const int X = G.shfl(own.c, odd ? 1 : 0), Y = G.shfl(own.c, odd ? 3 : 2);
+  const int pcell = pbc_cy(B, Y + nx.q / 3 - 1) * B.Nxc + pbc_cx(B, X + nx.q % 3 - 1);
+  Ev ev;
+  ev.t = t + (ydim ? key_time(nx.key) : tc);
+  ev.tie = kmax(time_key(ev.t), clk);
+  ev.b = ydim ? (uint32_t)pcell : 0;
+  ev.j = ydim ? nx.partner : dir;
+  ev.ca = ydim ? nx.ca : 0;
+  ev.st = ST_QUEUED;
+  if (on && mine) S.ev[(ydim ? N : 0) + my] = ev;
+  uint8_t rank = 0;
+  if (on && mine && ydim) {
+    rank = new_rank(S, A, dbase, my, odd ? a : two ? j : -1, ev.t, nx.partner, clk);
+    A.drank[gm] = rank;
+  }
+  // attribution of the changed disks: their earlier event and its cells
+  uint64_t key = time_key(ev.t);
+  int way = dir;
+  if (stale && !ydim) { key = kc; way = ec.j; }         // the crossing that stays
+  const uint64_t other = G.shfl_xor(key, 2);
+  const uint64_t keyc = ydim ? other : key, keyk = ydim ? key : other;
+  const bool hit = keyk < keyc;
+  const int wayc = G.shfl(way, odd ? 1 : 0), rk = G.shfl((int)rank, odd ? 3 : 2);
+  const int own_cell = cell_of(B, X, Y);
+  const int c2 = hit ? pcell : target_cell(B, X, Y, wayc);
+  const bool changed = on && (!odd || two);
+  if (changed && gl < 4) {
+    if (!ydim) {
+      A.dkey[gm] = hit ? keyk : keyc;
+      A.dpk[gm] = (hit ? rk << 24 : 0) | (int32_t)gm;
     }
-    for (int k = 0; k < MAXDIRTY; k++) res.dc[k] = dc[k];
-    res.nd = nd;
-    res.npair = npair; res.npred = npred; res.ncol = ncol; res.ncross = ncross; res.nstale = nstale;
-    res.nscreen = 0;
-    res.ct = ct[0];
-    res.key = key;
-    res.bad = bad; res.ovl = ovl;
-    res.a = oa; res.ob = ob;
+    A.fc[2 * gm + (ydim ? 1 : 0)] = ydim ? c2 : own_cell;
+  }
+  // cells whose minimum can have changed: the old and the new attributions
+  // (the new ones from lanes 0..3: the virial's lanes hold no new velocity)
+  const int cnew = G.shfl(ydim ? c2 : own_cell, gl & 3);
+  int32_t dc = -1;
+  if (changed && gl < 8) dc = (int32_t)base + (gl < 4 ? fold : cnew);
+#pragma unroll
+  for (int k = 0; k < 7; k++) {              // the first of equal ones stays
+    const int32_t o = G.shfl(dc, k);
+    if (gl > k && o == dc) dc = -1;
+  }
+  res.dc = dc;
+  res.ncol = two; res.ncross = cross; res.nstale = stale;
+  res.bad = G.any(bad);
+  if (A.flags & EDMD_F_SCREEN) {             // the FP32 shadows serve the thread path's screen only
+    G.sync();
+    if (changed && gl < 2) shadow_write(A, gm, B, S.d[my], S.cx[my], S.cy[my], A.epoch[s]);
+  }
 }
 
 // ---- one thread per event (rounds with many selected events): the lanes of
@@ -976,9 +795,18 @@ __device__ bool stamp_read_thread(const Box& B, const RoundArgs& A, int64_t base
   return bad;
 }
 
-// one selected event by one thread: the handlers of process_event_warp with
+// one selected event by one thread: the handlers of process_event with
 // the same arithmetic; all four virial terms end in r.ct4
-__device__ void process_event_thread(const SysDev& S, const RoundArgs& A, int s, int64_t g, EvResult& res,
+struct ThreadResult {
+  int32_t dc[MAXDIRTY];              // cells whose minimum can have changed
+  int nd;
+  unsigned long long npair, npred, ncol, ncross, nstale, nscreen;
+  uint64_t key;
+  bool bad, ovl;
+  int a, ob;
+};
+
+__device__ void process_event_thread(const SysDev& S, const RoundArgs& A, int s, int64_t g, ThreadResult& res,
                                      double* ct4) {
   const Box& B = S.B;
   const int N = B.N;
@@ -999,7 +827,7 @@ __device__ void process_event_thread(const SysDev& S, const RoundArgs& A, int s,
   ct4[0] = ct4[1] = ct4[2] = ct4[3] = 0;
   res.ovl = res.bad = false;
   res.ob = -1;
-  // what the shared tail does, set by the handler (see process_event_warp)
+  // what the shared tail does, set by the handler (see process_event)
   int b = -1;
   int64_t gb = -1;
   int pax = ax, pay = ay, pbx = ax, pby = ay;
@@ -1011,7 +839,7 @@ __device__ void process_event_thread(const SysDev& S, const RoundArgs& A, int s,
     free_fly_i(B, Da, t);
     if (E.ca != Db.coll) {
       S.d[a] = Da;
-      shadow_write(A, g, B, Da, ax, ay, A.epoch[s]);
+      if (A.flags & EDMD_F_SCREEN) shadow_write(A, g, B, Da, ax, ay, A.epoch[s]);
       res.nstale = 1;
     } else {
       b = E.j;
@@ -1043,8 +871,10 @@ __device__ void process_event_thread(const SysDev& S, const RoundArgs& A, int s,
       Db.vy -= f * Da.m * dy;
       S.d[a] = Da;
       S.d[b] = Db;
-      shadow_write(A, g, B, Da, ax, ay, A.epoch[s]);
-      shadow_write(A, gb, B, Db, bx, by, A.epoch[s]);
+      if (A.flags & EDMD_F_SCREEN) {
+        shadow_write(A, g, B, Da, ax, ay, A.epoch[s]);
+        shadow_write(A, gb, B, Db, bx, by, A.epoch[s]);
+      }
       if ((A.flags & EDMD_F_TRACE) && S.trace) {
         const unsigned long long k = atomicAdd((unsigned long long*)&S.st->ntrace, 1ull);
         if ((int64_t)k < S.trace_cap) {
@@ -1077,7 +907,7 @@ __device__ void process_event_thread(const SysDev& S, const RoundArgs& A, int s,
     S.prv[a] = NIL;
     Da.nxt = h;
     S.d[a] = Da;
-    shadow_write(A, g, B, Da, cx, cy, A.epoch[s]);
+    if (A.flags & EDMD_F_SCREEN) shadow_write(A, g, B, Da, cx, cy, A.epoch[s]);
     S.head[c] = a;
     if (h != NIL) S.prv[h] = a;
     pax = cx; pay = cy;
@@ -1173,7 +1003,7 @@ __global__ void __launch_bounds__(32, 16) k_process_thread(const SysDev* __restr
     const int n = w + lane;
     const bool valid = n < nsafe;
     int s = -1;
-    EvResult r;
+    ThreadResult r;
     double ct4[4] = {0, 0, 0, 0};
     r.nd = 0; r.npair = r.npred = r.ncol = r.ncross = r.nstale = r.nscreen = 0; r.key = 0;
     r.bad = r.ovl = false; r.a = r.ob = -1;
@@ -1196,7 +1026,7 @@ __global__ void __launch_bounds__(32, 16) k_process_thread(const SysDev* __restr
     const double c2 = group_sum(m, ct4[2]), c3 = group_sum(m, ct4[3]);
     const unsigned long long ncol = group_sum_u(m, r.ncol), ncross = group_sum_u(m, r.ncross);
     const unsigned long long nstale = group_sum_u(m, r.nstale), npair = group_sum_u(m, r.npair);
-    const unsigned long long npred = group_sum_u(m, r.npred), nscr = group_sum_u(m, r.nscreen);
+    const unsigned long long nscr = group_sum_u(m, r.nscreen);
     const uint64_t kmx = group_max(m, r.key);
     if (leader && s >= 0) {
       if (ncol) {
@@ -1209,8 +1039,6 @@ __global__ void __launch_bounds__(32, 16) k_process_thread(const SysDev* __restr
       cnt_add(A, s, stripe, C_NCROSS, ncross);
       cnt_add(A, s, stripe, C_NSTALE, nstale);
       cnt_add(A, s, stripe, C_NPAIR, npair);
-      cnt_add(A, s, stripe, C_NPRED, npred);
-      cnt_add(A, s, stripe, C_NEV, (unsigned long long)__popc(m));
       cnt_add(A, s, stripe, C_NSCREEN, nscr);
       atomicMax((unsigned long long*)&A.cnt[((int64_t)s * NSTRIPE + stripe) * NCNT + C_TLAST],
                 (unsigned long long)kmx);
@@ -1218,42 +1046,47 @@ __global__ void __launch_bounds__(32, 16) k_process_thread(const SysDev* __restr
   }
 }
 
-// the selected events of a round, one warp each; per-system counters go to
-// one of NSTRIPE stripes to spread the atomics
-__global__ void __launch_bounds__(32 * WPB, 20) k_process(const SysDev* __restrict__ sys, RoundArgs A) {
-  __shared__ WarpScratch scr[WPB];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  WarpScratch* W = &scr[wid];
+// The selected events of a round, GW lanes each: a warp an event (GW = 32), or
+// four events a warp.  Per-system counters go to one of NSTRIPE stripes to
+// spread the atomics.
+template <int GW, int MINB>
+__global__ void __launch_bounds__(32, MINB) k_process(const SysDev* __restrict__ sys, RoundArgs A) {
+  constexpr int PER = 32 / GW;
+  __shared__ LaneScratch scr[PER];
+  const int lane = threadIdx.x & 31;
+  const Grp<GW> G(lane);
+  LaneScratch* W = &scr[lane / GW];
   const int nsafe = *A.nsafe;
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicMax(A.maxsafe, nsafe);
   if (A.thread_kernel && nsafe >= A.thr_min) return;   // k_process_thread takes the round
-  const int gw = blockIdx.x * WPB + wid, nw = gridDim.x * WPB;
-  const int stripe = gw & (NSTRIPE - 1);
-  // one resident wave: each warp takes the event at its own index, then the
+  const int stripe = blockIdx.x & (NSTRIPE - 1);
+  const int wave = gridDim.x * PER;
+  // one resident wave: each warp takes the events at its own index, then the
   // warps that finish first take the rest from a counter (a grid of one
   // block per event would mostly launch blocks that find nothing to do)
-  for (int n = gw; n < nsafe; n = next_chunk(A, lane, nw, 1, nsafe)) {
-    const int64_t g = A.safe[n];
+  for (int w = blockIdx.x * PER; w < nsafe; w = next_chunk(A, lane, wave, PER, nsafe)) {
+    const int n = w + lane / GW;
+    const bool on = n < nsafe;
+    const int64_t g = A.safe[on ? n : w];
     const int s = A.dsys[g];
     EvResult r;
-    process_event_warp(sys[s], A, s, g, W, lane, r);
-    if (r.ncol && lane < 4) cnt_addf(A, s, stripe, C_CT0 + lane, r.ct);
-    if (lane == 0) {
-      for (int k = 0; k < MAXDIRTY; k++) A.dcell[(int64_t)n * MAXDIRTY + k] = k < r.nd ? r.dc[k] : -1;
-      cnt_add(A, s, stripe, C_NCOL, r.ncol);
-      cnt_add(A, s, stripe, C_NCROSS, r.ncross);
-      cnt_add(A, s, stripe, C_NSTALE, r.nstale);
-      cnt_add(A, s, stripe, C_NPAIR, r.npair);
-      cnt_add(A, s, stripe, C_NPRED, r.npred);
-      cnt_add(A, s, stripe, C_NEV, 1ull);
-      atomicMax((unsigned long long*)&A.cnt[((int64_t)s * NSTRIPE + stripe) * NCNT + C_TLAST],
-                (unsigned long long)r.key);
-      if (r.bad) atomicAdd(A.violations, 1ull);
-      if (r.ovl) {
-        SysState* R = sys[s].st;
-        R->err_a = r.a;
-        R->err_b = r.ob;
-        R->status = r.ob == OB_CORRUPT ? EDMD_ERR_BUDGET : EDMD_ERR_OVERLAP;
+    process_event<GW>(sys[s], A, s, g, on, W, G, r);
+    if (on) {
+      if (r.ncol && G.lane >= virial_lane<GW>(0) && G.lane < virial_lane<GW>(0) + 4)
+        cnt_addf(A, s, stripe, C_CT0 + (G.lane & 3), r.ct);
+      if (G.lane < MAXDIRTY) A.dcell[(int64_t)n * MAXDIRTY + G.lane] = r.dc;
+      if (G.lane == 0) {
+        cnt_add(A, s, stripe, r.ncol ? C_NCOL : r.ncross ? C_NCROSS : C_NSTALE, 1ull);
+        cnt_add(A, s, stripe, C_NPAIR, r.npair);
+        atomicMax((unsigned long long*)&A.cnt[((int64_t)s * NSTRIPE + stripe) * NCNT + C_TLAST],
+                  (unsigned long long)r.key);
+        if (r.bad) atomicAdd(A.violations, 1ull);
+        if (r.ovl) {
+          SysState* R = sys[s].st;
+          R->err_a = r.a;
+          R->err_b = r.ob;
+          R->status = r.ob == OB_CORRUPT ? EDMD_ERR_BUDGET : EDMD_ERR_OVERLAP;
+        }
       }
     }
     __syncwarp();
@@ -1369,7 +1202,7 @@ constexpr int BWPB = 4;              // warps per system block
 
 __global__ void __launch_bounds__(32 * BWPB, 4) k_block_rounds(const SysDev* __restrict__ sys, RoundArgs A,
                                                             int32_t* __restrict__ work, int64_t max_rounds) {
-  __shared__ WarpScratch scr[BWPB];
+  __shared__ LaneScratch scr[BWPB];
   __shared__ int32_t evl[BMAXEV];
   __shared__ int32_t dl[BMAXEV * MAXDIRTY];
   __shared__ int nev, ndl, s_sh, go, stop;
@@ -1434,7 +1267,7 @@ __global__ void __launch_bounds__(32 * BWPB, 4) k_block_rounds(const SysDev* __r
             Disk p = S.d[i];
             free_fly_i(B, p, tbar);
             S.d[i] = p;
-            shadow_write(A, dbase + i, B, p, S.cx[i], S.cy[i], A.epoch[s]);
+            if (A.flags & EDMD_F_SCREEN) shadow_write(A, dbase + i, B, p, S.cx[i], S.cy[i], A.epoch[s]);
           }
           __syncthreads();
           if (tid == 0) {
@@ -1447,16 +1280,15 @@ __global__ void __launch_bounds__(32 * BWPB, 4) k_block_rounds(const SysDev* __r
       }
       for (int e = wid; e < n; e += BWPB) {
         EvResult r;
-        process_event_warp(S, A, s, evl[e], &scr[wid], lane, r);
-        if (r.ncol && lane < 4) atomicAdd(&c_ct[lane], r.ct);
+        process_event<32>(S, A, s, evl[e], true, &scr[wid], Grp<32>(lane), r);
+        if (r.ncol && lane >= virial_lane<32>(0) && lane < virial_lane<32>(0) + 4) atomicAdd(&c_ct[lane & 3], r.ct);
+        if (lane < MAXDIRTY && r.dc >= 0) dl[atomicAdd(&ndl, 1)] = r.dc;
         if (lane == 0) {
-          const int q = atomicAdd(&ndl, r.nd);
-          for (int k = 0; k < r.nd; k++) dl[q + k] = r.dc[k];
-          atomicAdd(&c_ncol, r.ncol);
-          atomicAdd(&c_ncross, r.ncross);
-          atomicAdd(&c_nstale, r.nstale);
-          atomicAdd(&c_npair, r.npair);
-          atomicAdd(&c_npred, r.npred);
+          atomicAdd(&c_ncol, (unsigned long long)r.ncol);
+          atomicAdd(&c_ncross, (unsigned long long)r.ncross);
+          atomicAdd(&c_nstale, (unsigned long long)r.nstale);
+          atomicAdd(&c_npair, (unsigned long long)r.npair);
+          atomicAdd(&c_npred, r.ncol ? 2ull : 1ull);
           atomicAdd(&c_nev, 1ull);
           atomicMax((unsigned long long*)&tlast, (unsigned long long)r.key);
           if (r.bad) atomicAdd(A.violations, 1ull);
@@ -1550,7 +1382,7 @@ __device__ void barrier_systems(const SysDev* __restrict__ sys, const RoundArgs&
         S.d[i].x = p.x;
         S.d[i].y = p.y;
         S.d[i].tl = p.tl;
-        shadow_write(A, A.doff[s] + i, S.B, p, S.cx[i], S.cy[i], A.epoch[s]);
+        if (A.flags & EDMD_F_SCREEN) shadow_write(A, A.doff[s] + i, S.B, p, S.cx[i], S.cy[i], A.epoch[s]);
       }
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -1601,8 +1433,8 @@ __global__ void k_round_finish(const SysDev* __restrict__ sys, RoundArgs A) {
   R->ncross += v[C_NCROSS];
   R->nstale += v[C_NSTALE];
   R->npair += v[C_NPAIR];
-  R->npred += v[C_NPRED];
-  R->nevents += v[C_NEV];
+  R->npred += 2 * v[C_NCOL] + v[C_NCROSS] + v[C_NSTALE];
+  R->nevents += v[C_NCOL] + v[C_NCROSS] + v[C_NSTALE];
   R->nscreen += v[C_NSCREEN];
   if (tl != 0) {
     const double t = key_time(tl);
@@ -1711,7 +1543,7 @@ cudaError_t enqueue_round(edmd_ctx* ctx, const RoundBufs* R, const RoundArgs& A0
   }
   // one resident wave of each event kernel: one-warp blocks, 20 per SM (k_process)
   // and 16 per SM (k_process_thread), measured best
-  k_process<<<nsm * 20 / WPB, 32 * WPB, 0, st>>>(ctx->ds, A);
+  k_process<32, 20><<<nsm * 20, 32, 0, st>>>(ctx->ds, A);
   if (with_thread) k_process_thread<<<nsm * 16, 32, 0, st>>>(ctx->ds, A);
   k_recompute_barrier<<<nsm * 8, 256, 0, st>>>(ctx->ds, A, ctx->nsys < nsm * 8 ? ctx->nsys : nsm * 8);
   return cudaGetLastError();
