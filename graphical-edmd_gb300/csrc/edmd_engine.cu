@@ -426,7 +426,7 @@ __device__ void do_growstop(const SysDev& S, SysState& R, const Grp<GW>& G, Warp
     own.vr = 0;
     own.c = (lane & 2 ? S.cy : S.cx)[i];
     R.npred++;
-    const Next r = predict2<GW, ADD, false, GW>(S, R.t, i, -1, own, &R.npair, G, sm, ovl, oa, ob, [](int) {});
+    const Next r = predict2<GW, ADD, false, GW>(S, R.t, i, -1, own, &R.npair, G, sm, ovl, oa, ob, [](int) {}, [](int) { return 0; });
     schedule(S, Q, N + i, R.t + key_time(r.key), r.partner, r.ca, 2ull, G);
     unqueue(S, Q, i, G);
     int dir;
@@ -670,7 +670,7 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
         dir = ux == ydim ? db : da;
       }
       G.sync();
-      const Next nx = predict2<GW, ADD, GROW, GW>(S, t, i, two ? j : -1, own, &npair, G, sm, &ovl, &oa, &ob, [](int) {});
+      const Next nx = predict2<GW, ADD, GROW, GW>(S, t, i, two ? j : -1, own, &npair, G, sm, &ovl, &oa, &ob, [](int) {}, [](int) { return 0; });
       // addEventToQueue (src/EDMD.c:2144): lanes 0 and 1 take the crossings of
       // the two disks, lanes 2 and 3 their collisions; in that order they get
       // the insertion counters and join the overflow list

@@ -60,9 +60,9 @@ struct Own {
 };
 
 // a collision prediction of the lane's disk: time image, partner, its counter,
-// and the scan position (0..8) of the cell the partner was found in (4, the
-// disk's own, when there is none)
-struct Next { uint64_t key; int32_t partner; uint32_t ca; int q; };
+// the scan position (0..8) of the cell the partner was found in (4, the disk's
+// own, when there is none), and the partner's tag (3 when there is none)
+struct Next { uint64_t key; int32_t partner; uint32_t ca; int q, tag; };
 constexpr int OVL_CORRUPT = -2;    // overlap marker: a cell list longer than N (EDMD_ERR_BUDGET)
 
 // a disk record's coordinate or velocity along an axis (x, y, vx, vy lead it)
@@ -174,15 +174,17 @@ __device__ __forceinline__ int best_lane(uint64_t k, int o, const Grp<GW>& G) {
 // scan order) and 9..17 (a1's): task t runs on lane t % GW, a lane with two
 // tasks walks both lists at once.  The candidates are then packed over the
 // group in task order and solved by two lanes each.
-// `on_cell(cell)` is called for every cell scanned, by the lane that walks it.
+// `on_cell(cell)` is called for every cell scanned, by the lane that walks it;
+// `tag_of(p)` gives 0..3 for a candidate, loaded beside its record.
 // ORD: lanes the naming order of overlapping pairs refers to.
-template <int GW, bool ADD, bool GROW, int ORD, class F>
+template <int GW, bool ADD, bool GROW, int ORD, class F, class T>
 __device__ __forceinline__ Next predict2(const SysDev& S, double t, int a0, int a1, const Own& own,
                                          uint64_t* npair, const Grp<GW>& G, LaneScratch* sm, bool* ovl, int* ovl_a,
-                                         int* ovl_b, F&& on_cell) {
+                                         int* ovl_b, F&& on_cell, T&& tag_of) {
   const Box& B = S.B;
   const int lane = G.lane;
   const double dinit = GROW ? 10000000 : NEVER;
+  const uint32_t coll0 = S.d[0].coll;
   const int ntask = a1 >= 0 ? 18 : 9;
   const int X0 = G.shfl(own.c, 0), X1 = G.shfl(own.c, 1), Y0 = G.shfl(own.c, 2), Y1 = G.shfl(own.c, 3);
   // the tasks of this lane: t = lane + k GW, k < NT (a warp: one task per
@@ -266,7 +268,7 @@ __device__ __forceinline__ Next predict2(const SysDev& S, double t, int a0, int 
       const double p1 = G.shfl(own.p, src), v1 = G.shfl(own.v, src), rad1 = G.shfl(own.rad, src);
       const double vr1 = GROW ? G.shfl(own.vr, src) : 0.0;
       const int p = act ? sm->comp[f] : a0;
-      const int o = act ? sm->ord[f] : 0;
+      const int o = act ? (int)sm->ord[f] << 2 | tag_of(p) : 0;
       const Disk* P = S.d + p;
       const uint32_t pc = P->coll;
       bool ov = false;
@@ -304,8 +306,8 @@ __device__ __forceinline__ Next predict2(const SysDev& S, double t, int a0, int 
             const uint32_t w = ((uint32_t)(u % ORD) << 16) | (0xffffu - (uint32_t)(u * 2048 + min(k, 2047)));
             if (w < lk) { lk = w; la = a; lb = p; }
           }
-          if (g1) best_merge(bd1, bo1, bp1, bc1, kd, q * (1 << 20) + k, p, P->coll);
-          else best_merge(bd0, bo0, bp0, bc0, kd, q * (1 << 20) + k, p, P->coll);
+          if (g1) best_merge(bd1, bo1, bp1, bc1, kd, (q * (1 << 20) + k) << 2 | tag_of(p), p, P->coll);
+          else best_merge(bd0, bo0, bp0, bc0, kd, (q * (1 << 20) + k) << 2 | tag_of(p), p, P->coll);
           k++;
         }
         p = nx;
@@ -326,9 +328,10 @@ __device__ __forceinline__ Next predict2(const SysDev& S, double t, int a0, int 
     bd1 = G.shfl(bd1, w1); bo1 = G.shfl(bo1, w1); bp1 = G.shfl(bp1, w1); bc1 = G.shfl(bc1, w1);
     if (lane & 1) { bd0 = bd1; bo0 = bo1; bp0 = bp1; bc0 = bc1; }
   }
-  if (bo0 < 0) bc0 = S.d[0].coll;   // no partner: partner 0 (src/EDMD.c:2830)
+  if (bo0 < 0) bc0 = coll0;         // no partner: partner 0 (src/EDMD.c:2830)
   r.key = bd0; r.partner = bp0; r.ca = bc0;
-  r.q = bo0 < 0 ? 4 : spill ? bo0 >> 20 : bo0 / MAXC;
+  r.q = bo0 < 0 ? 4 : spill ? bo0 >> 22 : (bo0 >> 2) / MAXC;
+  r.tag = bo0 & 3;
   if (G.any(lk != 0xffffffffu || lcorrupt)) {
     const uint32_t least = G.min_u32(lk);
     const int src = G.first(lk == least && lk != 0xffffffffu);

@@ -66,6 +66,17 @@ constexpr int NSTRIPE = 32;           // copies of each system's counters
 // counters of the round engine, per system and stripe (u64 slots)
 enum { C_CT0, C_CT1, C_CT2, C_CT3, C_NCOL, C_NCROSS, C_NSTALE, C_NPAIR, C_NSCREEN, C_TLAST, NCNT };
 
+// What the cell minima are made of, in one 32-byte sector per disk: the minima
+// of a round's dirty cells are found by walking ~11 disks around each, which
+// took four sectors a disk with the fields in arrays of their own.
+struct __align__(32) Att {
+  uint64_t key;                  // time key of the disk's next event (KINF: none)
+  int32_t id;                    // its id: serial tie rank << 24 | disk
+  int32_t c1, c2;                // its footprint cells (local)
+  int32_t nxt;                   // copy of the disk's list link (Disk::nxt)
+  int32_t pad[2];
+};
+
 struct RoundArgs {
   int32_t nsys;
   int32_t radius;
@@ -76,12 +87,10 @@ struct RoundArgs {
   const int32_t* dsys;           // system of each disk
   const int64_t* doff;           // disk offset of each system
   const int64_t* coff;           // cell offset of each system
-  uint64_t* dkey;                // time key of each disk's next event (KINF: none)
-  int32_t* dpk;                  // its id: serial tie rank << 24 | disk
+  Att* att;                      // each disk's next event, its cells and its list link
   uint8_t* drank;                // tie rank of each disk's collision event (R_FIRST .. R_NEW)
   uint32_t* ikb;                 // serial queue key (bucket, tie) of each disk's collision event
   uint64_t* iktie;               // as inherited from a serial engine (k_rank)
-  int32_t* fc;                   // its two footprint cells (local), 2 per disk
   uint64_t* cmt; int32_t* cmi;   // attributed minimum (key, id) per cell
   uint64_t* lw; uint64_t* lr;    // causality stamps per cell
   int32_t* safe; int32_t* nsafe; // selected events of the round
@@ -105,7 +114,24 @@ struct RoundArgs {
   const int32_t* tx0;
   const int32_t* ty0;
   unsigned long long* violations;
+  SysDev one;                    // the system of a one-system context, so that its fields are kernel constants
 };
+
+// system s, its first disk and cell.  A one-system context (ONE) has them in
+// the kernel's parameters: every L2 access an event waits for in turn costs
+// 0.3-0.4 us, and a descriptor in memory adds three to its chain.
+template <bool ONE>
+__device__ __forceinline__ const SysDev& sys_of(const SysDev* sys, const RoundArgs& A, int s) {
+  if constexpr (ONE) return A.one;
+  else return sys[s];
+}
+template <bool ONE>
+__device__ __forceinline__ int sys_index(const RoundArgs& A, int64_t g) { return ONE ? 0 : A.dsys[g]; }
+template <bool ONE>
+__device__ __forceinline__ int64_t first_disk(const RoundArgs& A, int s) { return ONE ? 0 : A.doff[s]; }
+template <bool ONE>
+__device__ __forceinline__ int64_t first_cell(const RoundArgs& A, int s) { return ONE ? 0 : A.coff[s]; }
+
 
 __device__ __forceinline__ bool pair_less(uint64_t t1, int32_t i1, uint64_t t2, int32_t i2) {
   return t1 < t2 || (t1 == t2 && i1 < i2);
@@ -249,16 +275,15 @@ __device__ bool new_before_inherited(const SysDev& S, double tn, uint64_t clk, u
 }
 
 // tie rank of the new collision event of disk d (time tn, partner p) made by
-// an event of pop clock clk whose other disk is `other`: R_FIRST when it ties
+// an event of pop clock clk whose other disk is `other`, rp being p's rank: R_FIRST when it ties
 // exactly with p's still inherited event for the mutual pair and the serial
 // queue pops it first (a tie of a stale inherited event, such as stopGrow
 // leaves, with a valid new one decides the trajectory), else R_NEW
 __device__ __forceinline__ uint8_t new_rank(const SysDev& S, const RoundArgs& A, int64_t dbase, int d, int other,
-                                            double tn, int p, uint64_t clk) {
+                                            double tn, int p, int rp, uint64_t clk) {
   if (p == d || p == other) return R_NEW;
-  const int64_t gp = dbase + p;
-  const uint8_t rp = A.drank[gp];
   if (rp == R_NEW || rp == R_FIRST) return R_NEW;
+  const int64_t gp = dbase + p;
   const Ev X = S.ev[S.B.N + p];
   if (!(X.st & 3u) || X.j != d || __double_as_longlong(X.t) != __double_as_longlong(tn)) return R_NEW;
   return new_before_inherited(S, tn, clk, A.ikb[gp], A.iktie[gp]) ? R_FIRST : R_NEW;
@@ -292,10 +317,10 @@ __global__ void k_prep(const SysDev* __restrict__ sys, RoundArgs A) {
   uint64_t key;
   int c1, c2;
   const int slot = attribution(S, i, &key, &c1, &c2);
-  A.dkey[g] = key;
-  A.dpk[g] = event_id(A, g, slot, N);
-  A.fc[2 * g] = c1;
-  A.fc[2 * g + 1] = c2;
+  Att at;
+  at.key = key; at.id = event_id(A, g, slot, N); at.c1 = c1; at.c2 = c2; at.nxt = S.d[i].nxt;
+  at.pad[0] = at.pad[1] = 0;
+  A.att[g] = at;
   if (key != KINF) {
     atomicMin((unsigned long long*)&A.cmt[A.coff[s] + c1], (unsigned long long)key);
     if (c2 != c1) atomicMin((unsigned long long*)&A.cmt[A.coff[s] + c2], (unsigned long long)key);
@@ -305,11 +330,12 @@ __global__ void k_prep(const SysDev* __restrict__ sys, RoundArgs A) {
 __global__ void k_prep_owner(RoundArgs A) {
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= A.TN) return;
-  const uint64_t key = A.dkey[g];
+  const Att at = A.att[g];
+  const uint64_t key = at.key;
   if (key == KINF) return;
   const int64_t base = A.coff[A.dsys[g]];
-  const int64_t a = base + A.fc[2 * g], b = base + A.fc[2 * g + 1];
-  const int32_t id = A.dpk[g];
+  const int64_t a = base + at.c1, b = base + at.c2;
+  const int32_t id = at.id;
   if (A.cmt[a] == key) atomicMin(&A.cmi[a], id);
   if (b != a && A.cmt[b] == key) atomicMin(&A.cmi[b], id);
 }
@@ -392,26 +418,31 @@ struct SelGeom {
   static constexpr size_t bytes = (size_t)(CH * CW + CH * HW + NVB * SB * HW) * sizeof(kid_t);
 };
 
-// Window minima of one tile in shared memory and selection of its events;
-// the window radius R is a compile-time constant (3..12).
-template <int R>
-__global__ void __launch_bounds__(TX * TY, 4) k_select(const SysDev* __restrict__ sys, RoundArgs A) {
+// Window minima of tiles in shared memory and selection of their events into
+// A.safe, counted in *nsafe; the window radius R is a compile-time constant
+// (3..12).  By a block of TX x TY threads, on every gridDim-th tile.
+template <int R, bool ONE>
+__device__ __forceinline__ void select_tiles(const SysDev* __restrict__ sys, const RoundArgs& A, kid_t* sel_smem,
+                                             int32_t* nsafe) {
   using G = SelGeom<R>;
   constexpr int H = G::H, W = G::W, SB = G::SB, HW = G::HW, CW = G::CW, CH = G::CH;
-  extern __shared__ kid_t sel_smem[];
-  // the round's count of running systems is rebuilt by k_barrier
-  if (blockIdx.x == 0 && threadIdx.x == 0) *A.active = 0;
   kid_t* ck = sel_smem;                // CH x CW
   kid_t* hk = ck + CH * CW;            // CH x HW
   kid_t* wk = hk + CH * HW;            // NVB*SB x HW
   for (int t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
-  const int s = A.tsys[t];
+  const int s = ONE ? 0 : A.tsys[t];
   const uint64_t lim = A.lim[s];
   if (lim == 0) continue;             // the system has stopped: nothing to select
-  const Box& B = sys[s].B;
+  const Box& B = sys_of<ONE>(sys, A, s).B;
   const int Nxc = B.Nxc, Nyc = B.Nyc;
-  const int x0 = A.tx0[t], y0 = A.ty0[t];
-  const int64_t base = A.coff[s];
+  int x0, y0;
+  if constexpr (ONE) {                 // row by row, as the tile list is made
+    const int row = (Nxc + TX - 1) / TX;
+    x0 = t % row * TX; y0 = t / row * TY;
+  } else {
+    x0 = A.tx0[t]; y0 = A.ty0[t];
+  }
+  const int64_t base = first_cell<ONE>(A, s);
   if (x0 >= H && x0 - H + CW <= Nxc && y0 >= H && y0 - H + CH <= Nyc) {
     // a tile away from the periodic edges: no wrap
     const int64_t c0 = base + (int64_t)(y0 - H) * Nxc + (x0 - H);
@@ -462,8 +493,8 @@ __global__ void __launch_bounds__(TX * TY, 4) k_select(const SysDev* __restrict_
     const int w = (iy + 1) * HW + ix + 1;
     if (k < lim && wk[w] == v) {
       const int c = cy * Nxc + cx;
-      if (A.fc[2 * (int64_t)g] == c) {
-        const int c2 = A.fc[2 * (int64_t)g + 1];
+      if (A.att[g].c1 == c) {
+        const int c2 = A.att[g].c2;
         if (c2 == c) {
           sel = true;
         } else {
@@ -482,13 +513,21 @@ __global__ void __launch_bounds__(TX * TY, 4) k_select(const SysDev* __restrict_
     const int lane = threadIdx.x & 31;
     const int lead = __ffs(m) - 1;
     int pos = 0;
-    if (lane == lead) pos = atomicAdd(A.nsafe, __popc(m));
+    if (lane == lead) pos = atomicAdd(nsafe, __popc(m));
     pos = __shfl_sync(FULLM, pos, lead);
     if (sel) A.safe[pos + __popc(m & ((1u << lane) - 1))] = g;
     if (lane == lead) A.selflag[s] = 1;
   }
   __syncthreads();
   }
+}
+
+template <int R, bool ONE>
+__global__ void __launch_bounds__(TX * TY, 4) k_select(const SysDev* __restrict__ sys, const __grid_constant__ RoundArgs A) {
+  extern __shared__ kid_t sel_smem[];
+  // the round's count of running systems is rebuilt by the barrier
+  if (blockIdx.x == 0 && threadIdx.x == 0) *A.active = 0;
+  select_tiles<R, ONE>(sys, A, sel_smem, A.nsafe);
 }
 
 // causality stamp of a write of local cell c
@@ -540,13 +579,13 @@ struct EvResult {
 // edmd_lanes.cuh, so an event's scalar FP64 work (and, with GW = 8, that of the
 // four events of a warp) shares its instructions; `on` is false in a group
 // without an event, which follows along on event g without storing anything.
-template <int GW>
+template <int GW, bool ONE>
 __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& A, int s, int64_t g, bool on,
                                               LaneScratch* W, const Grp<GW>& G, EvResult& res) {
   const Box& B = S.B;
   const int N = B.N, gl = G.lane;
   const bool odd = gl & 1, ydim = gl & 2;
-  const int64_t base = A.coff[s], dbase = A.doff[s];
+  const int64_t base = first_cell<ONE>(A, s), dbase = first_disk<ONE>(A, s);
   const int a = (int)(g - dbase);
   const Ev ec = S.ev[a], ek = S.ev[N + a];
   const uint64_t kc = (ec.st & 3u) ? time_key(ec.t) : KINF, kk = (ek.st & 3u) ? time_key(ek.t) : KINF;
@@ -562,7 +601,7 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
   own.c = (ydim ? S.cy : S.cx)[my];
   const double m = D->m;
   const uint32_t hits = D->coll;
-  const int32_t fold = A.fc[2 * gm + (ydim ? 1 : 0)];   // cells the disk's old event was attributed to
+  const int32_t fold = (&A.att[gm].c1)[ydim ? 1 : 0];   // cells the disk's old event was attributed to
   {
     const double L = ydim ? B.Ly : B.Lx;
     own.p += (t - D->tl) * own.v;
@@ -617,19 +656,26 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
       // unlink from the old cell, relink at the head of the new one
       const int pv = S.prv[a], nx = D->nxt;
       if (pv == NIL) S.head[ca] = nx;
-      else S.d[pv].nxt = nx;
+      else { S.d[pv].nxt = nx; A.att[dbase + pv].nxt = nx; }
       if (nx != NIL) S.prv[nx] = pv;
       const int h = S.head[to];
       S.prv[a] = NIL;
       D->nxt = h;
+      A.att[gm].nxt = h;
       S.head[to] = a;
       if (h != NIL) S.prv[h] = a;
     }
   }
-  // causality stamps of the written cells
-  bool bad = false;
-  if (on && gl == 0) bad = stamp_write(A, base, ca, clk);
-  if (on && gl == 1 && wc1 >= 0) bad = stamp_write(A, base, wc1, clk);
+  // causality stamps of the written cells; what was there is compared at the
+  // end, so that nothing waits for it
+  uint64_t lw_old = 0, lr_old = 0;
+  {
+    const int c = gl == 0 ? ca : wc1;
+    if (on && gl < 2 && c >= 0) {
+      lr_old = A.lr[base + c];
+      lw_old = atomicMax((unsigned long long*)&A.lw[base + c], (unsigned long long)clk);
+    }
+  }
   // the next crossing (src/EDMD.c:2405-2482): one axis per lane
   double tc = 0;
   int dir = 0;
@@ -646,6 +692,8 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
     dir = ux == ydim ? db : da;
   }
   __syncwarp();
+  uint64_t lw_seen[(18 + GW - 1) / GW] = {};
+  int seen = 0;
   res.npair = 0;
   res.ovl = false;
   res.a = a;
@@ -653,11 +701,10 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
   const Next nx = predict2<GW, true, false, 32>(S, t, a, two ? j : -1, own, &res.npair, G, W, &res.ovl, &res.a,
                                                 &res.ob, [&](int cell) {
     // stamps of the cells read
-    const int64_t gc = base + cell;
     if (!on) return;
-    if (A.lw[gc] > clk) bad = true;
-    if (A.lr[gc] < clk) atomicMax((unsigned long long*)&A.lr[gc], (unsigned long long)clk);
-  });
+    lw_seen[seen++] = A.lw[base + cell];
+    atomicMax((unsigned long long*)&A.lr[base + cell], (unsigned long long)clk);
+  }, [&](int p) { return (int)A.drank[dbase + p]; });
   if (res.ovl && res.a == OVL_CORRUPT) { res.a = a; res.ob = OB_CORRUPT; }
   // event records: lanes 0 and 1 take the crossings, lanes 2 and 3 the
   // collisions of the two disks
@@ -675,7 +722,7 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
   if (on && mine) S.ev[(ydim ? N : 0) + my] = ev;
   uint8_t rank = 0;
   if (on && mine && ydim) {
-    rank = new_rank(S, A, dbase, my, odd ? a : two ? j : -1, ev.t, nx.partner, clk);
+    rank = new_rank(S, A, dbase, my, odd ? a : two ? j : -1, ev.t, nx.partner, nx.tag, clk);
     A.drank[gm] = rank;
   }
   // attribution of the changed disks: their earlier event and its cells
@@ -690,11 +737,14 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
   const int c2 = hit ? pcell : target_cell(B, X, Y, wayc);
   const bool changed = on && (!odd || two);
   if (changed && gl < 4) {
+    Att* const at = A.att + gm;
     if (!ydim) {
-      A.dkey[gm] = hit ? keyk : keyc;
-      A.dpk[gm] = (hit ? rk << 24 : 0) | (int32_t)gm;
+      at->key = hit ? keyk : keyc;
+      at->id = (hit ? rk << 24 : 0) | (int32_t)gm;
+      at->c1 = own_cell;
+    } else {
+      at->c2 = c2;
     }
-    A.fc[2 * gm + (ydim ? 1 : 0)] = ydim ? c2 : own_cell;
   }
   // cells whose minimum can have changed: the old and the new attributions
   // (the new ones from lanes 0..3: the virial's lanes hold no new velocity)
@@ -708,6 +758,9 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
   }
   res.dc = dc;
   res.ncol = two; res.ncross = cross; res.nstale = stale;
+  bool bad = lw_old > clk || lr_old > clk;
+#pragma unroll
+  for (int k = 0; k < (18 + GW - 1) / GW; k++) bad |= lw_seen[k] > clk;
   res.bad = G.any(bad);
   if (A.flags & EDMD_F_SCREEN) {             // the FP32 shadows serve the thread path's screen only
     G.sync();
@@ -818,8 +871,8 @@ __device__ void process_event_thread(const SysDev& S, const RoundArgs& A, int s,
   const double t = E.t;
   const uint64_t clk = E.tie;
   int nd = 0;
-  res.dc[nd++] = (int32_t)(base + A.fc[2 * g]);
-  if (A.fc[2 * g + 1] != A.fc[2 * g]) res.dc[nd++] = (int32_t)(base + A.fc[2 * g + 1]);
+  res.dc[nd++] = (int32_t)(base + A.att[g].c1);
+  if (A.att[g].c2 != A.att[g].c1) res.dc[nd++] = (int32_t)(base + A.att[g].c2);
   Disk Da = S.d[a];
   const int ax = S.cx[a], ay = S.cy[a];
   const int ca = cell_of(B, ax, ay);
@@ -844,8 +897,8 @@ __device__ void process_event_thread(const SysDev& S, const RoundArgs& A, int s,
     } else {
       b = E.j;
       gb = dbase + b;
-      res.dc[nd++] = (int32_t)(base + A.fc[2 * gb]);
-      if (A.fc[2 * gb + 1] != A.fc[2 * gb]) res.dc[nd++] = (int32_t)(base + A.fc[2 * gb + 1]);
+      res.dc[nd++] = (int32_t)(base + A.att[gb].c1);
+      if (A.att[gb].c2 != A.att[gb].c1) res.dc[nd++] = (int32_t)(base + A.att[gb].c2);
       const int bx = S.cx[b], by = S.cy[b];
       const int cb = cell_of(B, bx, by);
       free_fly_i(B, Db, t);
@@ -892,7 +945,7 @@ __device__ void process_event_thread(const SysDev& S, const RoundArgs& A, int s,
     int cx = ax, cy = ay;
     const int pv = S.prv[a], nx = Da.nxt;
     if (pv == NIL) S.head[ca] = nx;
-    else S.d[pv].nxt = nx;
+    else { S.d[pv].nxt = nx; A.att[dbase + pv].nxt = nx; }
     if (nx != NIL) S.prv[nx] = pv;
     switch (E.j) {
       case 1: if (cx - 1 == -1) { cx = B.Nxc - 1; S.crossX[a] -= 1; } else cx -= 1; break;
@@ -906,6 +959,7 @@ __device__ void process_event_thread(const SysDev& S, const RoundArgs& A, int s,
     S.cy[a] = cy;
     S.prv[a] = NIL;
     Da.nxt = h;
+    A.att[g].nxt = h;
     S.d[a] = Da;
     if (A.flags & EDMD_F_SCREEN) shadow_write(A, g, B, Da, cx, cy, A.epoch[s]);
     S.head[c] = a;
@@ -937,12 +991,12 @@ __device__ void process_event_thread(const SysDev& S, const RoundArgs& A, int s,
     const bool had = res.ovl;
     const Pred pr = predict_thread(S, A, s, d, Dd, X, Y, t, &res.npair, &res.nscreen, &res.ovl, &res.ob);
     if (res.ovl && !had) res.a = d;        // the disk whose prediction met the overlap
-    const uint8_t rk = new_rank(S, A, dbase, d, q ? a : b, t + pr.dt, pr.partner, clk);
+    const uint8_t rk = new_rank(S, A, dbase, d, q ? a : b, t + pr.dt, pr.partner, A.drank[dbase + pr.partner], clk);
     set_event(S, N + d, t + pr.dt, pr.partner, pr.ca, pr.pcell, clk);
     A.drank[gd] = rk;
     uint64_t k2; int c1, c2;
     const int sl = attribution(S, d, &k2, &c1, &c2);
-    A.dkey[gd] = k2; A.dpk[gd] = event_id(A, gd, sl, N); A.fc[2 * gd] = c1; A.fc[2 * gd + 1] = c2;
+    A.att[gd].key = k2; A.att[gd].id = event_id(A, gd, sl, N); A.att[gd].c1 = c1; A.att[gd].c2 = c2;
     res.dc[nd++] = (int32_t)(base + c1);
     if (c2 != c1) res.dc[nd++] = (int32_t)(base + c2);
   }
@@ -1046,11 +1100,61 @@ __global__ void __launch_bounds__(32, 16) k_process_thread(const SysDev* __restr
   }
 }
 
+// minimum (key, id) of the events on list q of the 3x3 block around local
+// cell c that are attributed to c (the walk of recompute_cell for one list)
+__device__ __forceinline__ void list_min(const SysDev& S, const RoundArgs& A, int64_t dbase, int c, int q,
+                                         uint64_t& bk, int32_t& bi) {
+  const Box& B = S.B;
+  const int x = c % B.Nxc, y = c / B.Nxc;
+  int p = S.head[pbc_cy(B, y + q / 3 - 1) * B.Nxc + pbc_cx(B, x + q % 3 - 1)];
+  int guard = 0;
+  while (p != NIL && guard++ < B.N) {
+    const Att at = A.att[dbase + p];
+    if (at.key != KINF && (at.c1 == c || at.c2 == c) && pair_less(at.key, at.id, bk, bi)) {
+      bk = at.key;
+      bi = at.id;
+    }
+    p = at.nxt;
+  }
+}
+
+// the selected events w .. w + 32 / GW - 1 by the groups of a warp: the event,
+// its system's counters (one of NSTRIPE stripes, to spread the atomics), its
+// dirty cells, its errors
+template <int GW, bool ONE>
+__device__ __forceinline__ void run_event(const SysDev* __restrict__ sys, const RoundArgs& A, int w, int nsafe,
+                                          int stripe, LaneScratch* W, const Grp<GW>& G) {
+  const int n = w + (threadIdx.x & 31) / GW;
+  const bool on = n < nsafe;
+  const int64_t g = A.safe[on ? n : w];
+  const int s = sys_index<ONE>(A, g);
+  const SysDev& S = sys_of<ONE>(sys, A, s);
+  EvResult r;
+  process_event<GW, ONE>(S, A, s, g, on, W, G, r);
+  if (on) {
+    if (r.ncol && G.lane >= virial_lane<GW>(0) && G.lane < virial_lane<GW>(0) + 4)
+      cnt_addf(A, s, stripe, C_CT0 + (G.lane & 3), r.ct);
+    if (G.lane < MAXDIRTY) A.dcell[(int64_t)n * MAXDIRTY + G.lane] = r.dc;
+    if (G.lane == 0) {
+      cnt_add(A, s, stripe, r.ncol ? C_NCOL : r.ncross ? C_NCROSS : C_NSTALE, 1ull);
+      cnt_add(A, s, stripe, C_NPAIR, r.npair);
+      atomicMax((unsigned long long*)&A.cnt[((int64_t)s * NSTRIPE + stripe) * NCNT + C_TLAST],
+                (unsigned long long)r.key);
+      if (r.bad) atomicAdd(A.violations, 1ull);
+      if (r.ovl) {
+        SysState* R = S.st;
+        R->err_a = r.a;
+        R->err_b = r.ob;
+        R->status = r.ob == OB_CORRUPT ? EDMD_ERR_BUDGET : EDMD_ERR_OVERLAP;
+      }
+    }
+  }
+}
+
 // The selected events of a round, GW lanes each: a warp an event (GW = 32), or
-// four events a warp.  Per-system counters go to one of NSTRIPE stripes to
-// spread the atomics.
-template <int GW, int MINB>
-__global__ void __launch_bounds__(32, MINB) k_process(const SysDev* __restrict__ sys, RoundArgs A) {
+// four events a warp.
+template <int GW, int MINB, bool ONE>
+__global__ void __launch_bounds__(32, MINB) k_process(const SysDev* __restrict__ sys, const __grid_constant__ RoundArgs A) {
   constexpr int PER = 32 / GW;
   __shared__ LaneScratch scr[PER];
   const int lane = threadIdx.x & 31;
@@ -1065,30 +1169,7 @@ __global__ void __launch_bounds__(32, MINB) k_process(const SysDev* __restrict__
   // warps that finish first take the rest from a counter (a grid of one
   // block per event would mostly launch blocks that find nothing to do)
   for (int w = blockIdx.x * PER; w < nsafe; w = next_chunk(A, lane, wave, PER, nsafe)) {
-    const int n = w + lane / GW;
-    const bool on = n < nsafe;
-    const int64_t g = A.safe[on ? n : w];
-    const int s = A.dsys[g];
-    EvResult r;
-    process_event<GW>(sys[s], A, s, g, on, W, G, r);
-    if (on) {
-      if (r.ncol && G.lane >= virial_lane<GW>(0) && G.lane < virial_lane<GW>(0) + 4)
-        cnt_addf(A, s, stripe, C_CT0 + (G.lane & 3), r.ct);
-      if (G.lane < MAXDIRTY) A.dcell[(int64_t)n * MAXDIRTY + G.lane] = r.dc;
-      if (G.lane == 0) {
-        cnt_add(A, s, stripe, r.ncol ? C_NCOL : r.ncross ? C_NCROSS : C_NSTALE, 1ull);
-        cnt_add(A, s, stripe, C_NPAIR, r.npair);
-        atomicMax((unsigned long long*)&A.cnt[((int64_t)s * NSTRIPE + stripe) * NCNT + C_TLAST],
-                  (unsigned long long)r.key);
-        if (r.bad) atomicAdd(A.violations, 1ull);
-        if (r.ovl) {
-          SysState* R = sys[s].st;
-          R->err_a = r.a;
-          R->err_b = r.ob;
-          R->status = r.ob == OB_CORRUPT ? EDMD_ERR_BUDGET : EDMD_ERR_OVERLAP;
-        }
-      }
-    }
+    run_event<GW, ONE>(sys, A, w, nsafe, stripe, W, G);
     __syncwarp();
   }
 }
@@ -1106,13 +1187,12 @@ __device__ void recompute_cell(const SysDev& S, const RoundArgs& A, int64_t base
     int p = S.head[pbc_cy(B, y + lane / 3 - 1) * B.Nxc + pbc_cx(B, x + lane % 3 - 1)];
     int guard = 0;
     while (p != NIL && guard++ < B.N) {
-      const int64_t g = dbase + p;
-      const uint64_t k = A.dkey[g];
-      if (k != KINF && (A.fc[2 * g] == c || A.fc[2 * g + 1] == c) && pair_less(k, A.dpk[g], bk, bi)) {
-        bk = k;
-        bi = A.dpk[g];
+      const Att at = A.att[dbase + p];
+      if (at.key != KINF && (at.c1 == c || at.c2 == c) && pair_less(at.key, at.id, bk, bi)) {
+        bk = at.key;
+        bi = at.id;
       }
-      p = S.d[p].nxt;
+      p = at.nxt;
     }
   }
   for (int o = 16; o > 0; o >>= 1) {
@@ -1126,31 +1206,13 @@ __device__ void recompute_cell(const SysDev& S, const RoundArgs& A, int64_t base
   }
 }
 
-// minimum (key, id) of the events on list q of the 3x3 block around local
-// cell c that are attributed to c (the walk of recompute_cell for one list)
-__device__ __forceinline__ void list_min(const SysDev& S, const RoundArgs& A, int64_t dbase, int c, int q,
-                                         uint64_t& bk, int32_t& bi) {
-  const Box& B = S.B;
-  const int x = c % B.Nxc, y = c / B.Nxc;
-  int p = S.head[pbc_cy(B, y + q / 3 - 1) * B.Nxc + pbc_cx(B, x + q % 3 - 1)];
-  int guard = 0;
-  while (p != NIL && guard++ < B.N) {
-    const int64_t g = dbase + p;
-    const uint64_t k = A.dkey[g];
-    if (k != KINF && (A.fc[2 * g] == c || A.fc[2 * g + 1] == c) && pair_less(k, A.dpk[g], bk, bi)) {
-      bk = k;
-      bi = A.dpk[g];
-    }
-    p = S.d[p].nxt;
-  }
-}
-
 // the cells whose minimum the selected events can have changed: four cells
 // per warp, one 8-lane group each (lane q walks list q of the 3x3 block,
 // lane 0 also list 8), the same minima as recompute_cell
-__device__ void recompute_cells(const SysDev* __restrict__ sys, const RoundArgs& A) {
+template <bool ONE>
+__device__ __forceinline__ void recompute_cells(const SysDev* __restrict__ sys, const RoundArgs& A, int nsafe) {
   const int lane = threadIdx.x & 31, grp = lane >> 3, q = lane & 7;
-  const int64_t total = (int64_t)(*A.nsafe) * MAXDIRTY;
+  const int64_t total = (int64_t)nsafe * MAXDIRTY;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 4 < total; w += nwarps) {
     const int64_t item = w * 4 + grp;
@@ -1158,10 +1220,10 @@ __device__ void recompute_cells(const SysDev* __restrict__ sys, const RoundArgs&
     uint64_t bk = KINF;
     int32_t bi = IINF;
     if (gc >= 0) {
-      const int s = A.dsys[A.safe[item / MAXDIRTY]];
-      const SysDev& S = sys[s];
-      const int c = (int)(gc - A.coff[s]);
-      const int64_t dbase = A.doff[s];
+      const int s = ONE ? 0 : A.dsys[A.safe[item / MAXDIRTY]];
+      const SysDev& S = sys_of<ONE>(sys, A, s);
+      const int c = (int)(gc - first_cell<ONE>(A, s));
+      const int64_t dbase = first_disk<ONE>(A, s);
       list_min(S, A, dbase, c, q, bk, bi);
       if (q == 0) list_min(S, A, dbase, c, 8, bk, bi);
     }
@@ -1243,9 +1305,9 @@ __global__ void __launch_bounds__(32 * BWPB, 4) k_block_rounds(const SysDev* __r
         if (k >= lim) continue;
         const int32_t id = A.cmi[base + c];
         const int64_t g = id & GMASK;
-        if (A.fc[2 * g] != c) continue;                 // decided at the owner's cell
+        if (A.att[g].c1 != c) continue;                 // decided at the owner's cell
         if (!window_min(A, base, B.Nxc, B.Nyc, c, k, id, A.radius)) continue;
-        const int c2 = A.fc[2 * g + 1];
+        const int c2 = A.att[g].c2;
         if (c2 != c && !window_min(A, base, B.Nxc, B.Nyc, c2, k, id, A.radius)) continue;
         const int q = atomicAdd(&nev, 1);
         if (q < BMAXEV) evl[q] = (int32_t)g;          // the rest waits for the next round
@@ -1280,7 +1342,7 @@ __global__ void __launch_bounds__(32 * BWPB, 4) k_block_rounds(const SysDev* __r
       }
       for (int e = wid; e < n; e += BWPB) {
         EvResult r;
-        process_event<32>(S, A, s, evl[e], true, &scr[wid], Grp<32>(lane), r);
+        process_event<32, false>(S, A, s, evl[e], true, &scr[wid], Grp<32>(lane), r);
         if (r.ncol && lane >= virial_lane<32>(0) && lane < virial_lane<32>(0) + 4) atomicAdd(&c_ct[lane & 3], r.ct);
         if (lane < MAXDIRTY && r.dc >= 0) dl[atomicAdd(&ndl, 1)] = r.dc;
         if (lane == 0) {
@@ -1336,11 +1398,14 @@ __global__ void __launch_bounds__(32 * BWPB, 4) k_block_rounds(const SysDev* __r
 // run); a system with nothing eligible left before its screenshot time
 // free-flies every disk to it (takeAScreenshot, src/EDMD.c:4657-4661) and
 // reschedules it; then the eligibility bound of the next round
-__device__ void barrier_systems(const SysDev* __restrict__ sys, const RoundArgs& A, int first, int stride) {
+template <bool ONE>
+__device__ __forceinline__ void barrier_systems(const SysDev* __restrict__ sys, const RoundArgs& A, int first, int stride) {
   __shared__ int go;
   for (int s = first; s < A.nsys; s += stride) {
-    if (A.lim[s] == 0) continue;      // stopped for the rest of the call
-    const SysDev& S = sys[s];
+    const bool stopped = A.lim[s] == 0;   // for the rest of the call
+    __syncthreads();                  // thread 0 writes lim below
+    if (stopped) continue;
+    const SysDev& S = sys_of<ONE>(sys, A, s);
     const int N = S.B.N;
     bool run = false;
     if (threadIdx.x < 32) {
@@ -1382,7 +1447,7 @@ __device__ void barrier_systems(const SysDev* __restrict__ sys, const RoundArgs&
         S.d[i].x = p.x;
         S.d[i].y = p.y;
         S.d[i].tl = p.tl;
-        if (A.flags & EDMD_F_SCREEN) shadow_write(A, A.doff[s] + i, S.B, p, S.cx[i], S.cy[i], A.epoch[s]);
+        if (A.flags & EDMD_F_SCREEN) shadow_write(A, first_disk<ONE>(A, s) + i, S.B, p, S.cx[i], S.cy[i], A.epoch[s]);
       }
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -1400,15 +1465,19 @@ __device__ void barrier_systems(const SysDev* __restrict__ sys, const RoundArgs&
 // two are independent: the barrier reads the round's counters and writes
 // each system's limits and, when it passes a screenshot, the disks'
 // positions; the recompute reads event keys, footprints and list links.
-__global__ void __launch_bounds__(256) k_recompute_barrier(const SysDev* __restrict__ sys, RoundArgs A,
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_recompute_barrier(const SysDev* __restrict__ sys, const __grid_constant__ RoundArgs A,
                                                           int nbar) {
   // the next round's selection count starts empty (this round's is still read)
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *A.nsafe_next = 0;
     *A.pnext = 0;                    // the event kernels of this round are done with it
   }
-  if ((int)blockIdx.x < nbar) barrier_systems(sys, A, blockIdx.x, nbar);
-  recompute_cells(sys, A);
+  // the barriers go to the last blocks, the cells from the first ones on, so
+  // that in a round of few events no block does both
+  const int last = gridDim.x - 1 - blockIdx.x;
+  if (last < nbar) barrier_systems<ONE>(sys, A, last, nbar);
+  recompute_cells<ONE>(sys, A, *A.nsafe);
 }
 
 // fold the call's counters into each system's state; its time is the last
@@ -1452,14 +1521,15 @@ __global__ void k_round_setup(const int64_t* __restrict__ doff, const SysDev* __
 }
 
 struct RoundBufs {
-  int32_t *dsys = nullptr, *fc = nullptr, *cmi = nullptr, *safe = nullptr, *nsafe = nullptr;
-  int32_t *dcell = nullptr, *selflag = nullptr, *active = nullptr, *dpk = nullptr, *work = nullptr;
+  Att* att = nullptr;
+  int32_t *dsys = nullptr, *cmi = nullptr, *safe = nullptr, *nsafe = nullptr;
+  int32_t *dcell = nullptr, *selflag = nullptr, *active = nullptr, *work = nullptr;
   uint8_t *drank = nullptr, *drank_bak = nullptr;
   uint32_t* ikb = nullptr;
   uint64_t* iktie = nullptr;
   int32_t *tsys = nullptr, *tx0 = nullptr, *ty0 = nullptr;
   int64_t *doff = nullptr, *coff = nullptr;
-  uint64_t *dkey = nullptr, *cmt = nullptr, *lw = nullptr, *lr = nullptr;
+  uint64_t *cmt = nullptr, *lw = nullptr, *lr = nullptr;
   uint64_t *lim = nullptr, *target = nullptr, *freeze = nullptr, *tlast = nullptr, *cnt = nullptr;
   float4* shp = nullptr;
   float* sht = nullptr;
@@ -1487,7 +1557,7 @@ int round_init(edmd_ctx* ctx) {
   }
   R->ntiles = (int64_t)tsys.size();
   if (TN > GMASK) return set_err(ctx, EDMD_ERR_CAPACITY, "the round engine supports up to 2^24 disks per context");
-  CK(dalloc(&R->dsys, TN)); CK(dalloc(&R->fc, 2 * TN)); CK(dalloc(&R->dkey, TN)); CK(dalloc(&R->dpk, TN));
+  CK(dalloc(&R->dsys, TN)); CK(dalloc(&R->att, TN));
   CK(dalloc(&R->drank, TN)); CK(dalloc(&R->drank_bak, TN));
   CK(dalloc(&R->ikb, TN)); CK(dalloc(&R->iktie, TN));
   CK(dalloc(&R->cmi, TC)); CK(dalloc(&R->cmt, TC)); CK(dalloc(&R->lw, TC)); CK(dalloc(&R->lr, TC));
@@ -1507,16 +1577,12 @@ int round_init(edmd_ctx* ctx) {
   CK(sync_set(ctx, R->selflag, 0, ctx->nsys * 4));
   // selection tiles of wide windows need more than the default 48 KB of
   // dynamic shared memory
-  CK(cudaFuncSetAttribute(k_select<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SelGeom<3>::bytes));
-  CK(cudaFuncSetAttribute(k_select<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SelGeom<4>::bytes));
-  CK(cudaFuncSetAttribute(k_select<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SelGeom<5>::bytes));
-  CK(cudaFuncSetAttribute(k_select<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SelGeom<6>::bytes));
-  CK(cudaFuncSetAttribute(k_select<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SelGeom<7>::bytes));
-  CK(cudaFuncSetAttribute(k_select<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SelGeom<8>::bytes));
-  CK(cudaFuncSetAttribute(k_select<9>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SelGeom<9>::bytes));
-  CK(cudaFuncSetAttribute(k_select<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SelGeom<10>::bytes));
-  CK(cudaFuncSetAttribute(k_select<11>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SelGeom<11>::bytes));
-  CK(cudaFuncSetAttribute(k_select<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SelGeom<12>::bytes));
+#define SEL_SMEM(R) \
+  CK(cudaFuncSetAttribute(k_select<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SelGeom<R>::bytes)); \
+  CK(cudaFuncSetAttribute(k_select<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SelGeom<R>::bytes));
+  SEL_SMEM(3) SEL_SMEM(4) SEL_SMEM(5) SEL_SMEM(6) SEL_SMEM(7)
+  SEL_SMEM(8) SEL_SMEM(9) SEL_SMEM(10) SEL_SMEM(11) SEL_SMEM(12)
+#undef SEL_SMEM
   k_round_setup<<<dim3(64, ctx->nsys), 256, 0, ctx->stream>>>(R->doff, ctx->ds, R->dsys);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->stream));
@@ -1532,10 +1598,14 @@ cudaError_t enqueue_round(edmd_ctx* ctx, const RoundBufs* R, const RoundArgs& A0
   A.nsafe = R->nsafe + (k & 1);
   A.nsafe_next = R->nsafe + ((k + 1) & 1);
   A.thread_kernel = with_thread ? 1 : 0;
+  const bool one = ctx->nsys == 1;
   const unsigned tgrid = (unsigned)(R->ntiles < nsm * 8 ? R->ntiles : nsm * 8);
   switch (A.radius) {
 #define SEL_CASE(R) \
-    case R: k_select<R><<<tgrid, TX * TY, SelGeom<R>::bytes, st>>>(ctx->ds, A); break;
+    case R: \
+      if (one) k_select<R, true><<<tgrid, TX * TY, SelGeom<R>::bytes, st>>>(ctx->ds, A); \
+      else k_select<R, false><<<tgrid, TX * TY, SelGeom<R>::bytes, st>>>(ctx->ds, A); \
+      break;
     SEL_CASE(3) SEL_CASE(4) SEL_CASE(5) SEL_CASE(6) SEL_CASE(7)
     SEL_CASE(8) SEL_CASE(9) SEL_CASE(10) SEL_CASE(11) SEL_CASE(12)
 #undef SEL_CASE
@@ -1543,9 +1613,12 @@ cudaError_t enqueue_round(edmd_ctx* ctx, const RoundBufs* R, const RoundArgs& A0
   }
   // one resident wave of each event kernel: one-warp blocks, 20 per SM (k_process)
   // and 16 per SM (k_process_thread), measured best
-  k_process<32, 20><<<nsm * 20, 32, 0, st>>>(ctx->ds, A);
+  if (one) k_process<32, 20, true><<<nsm * 20, 32, 0, st>>>(ctx->ds, A);
+  else k_process<32, 20, false><<<nsm * 20, 32, 0, st>>>(ctx->ds, A);
   if (with_thread) k_process_thread<<<nsm * 16, 32, 0, st>>>(ctx->ds, A);
-  k_recompute_barrier<<<nsm * 8, 256, 0, st>>>(ctx->ds, A, ctx->nsys < nsm * 8 ? ctx->nsys : nsm * 8);
+  const int nbar = ctx->nsys < nsm * 8 ? ctx->nsys : nsm * 8;
+  if (one) k_recompute_barrier<true><<<nsm * 8, 256, 0, st>>>(ctx->ds, A, nbar);
+  else k_recompute_barrier<false><<<nsm * 8, 256, 0, st>>>(ctx->ds, A, nbar);
   return cudaGetLastError();
 }
 
@@ -1554,9 +1627,9 @@ cudaError_t enqueue_round(edmd_ctx* ctx, const RoundBufs* R, const RoundArgs& A0
 void round_free(edmd_ctx* ctx) {
   RoundBufs* R = (RoundBufs*)ctx->round;
   if (!R) return;
-  void* p[] = {R->dsys, R->fc, R->cmi, R->safe, R->nsafe, R->dcell, R->selflag, R->active,
-               R->tsys, R->tx0, R->ty0, R->doff, R->coff, R->dkey, R->cmt, R->lw, R->lr,
-               R->lim, R->target, R->freeze, R->tlast, R->cnt, R->viol, R->dpk, R->drank,
+  void* p[] = {R->dsys, R->att, R->cmi, R->safe, R->nsafe, R->dcell, R->selflag, R->active,
+               R->tsys, R->tx0, R->ty0, R->doff, R->coff, R->cmt, R->lw, R->lr,
+               R->lim, R->target, R->freeze, R->tlast, R->cnt, R->viol, R->drank,
                R->drank_bak, R->ikb, R->iktie, R->work, R->shp, R->sht, R->epoch};
   for (void* q : p)
     if (q) cudaFree(q);
@@ -1581,6 +1654,7 @@ static int run_rounds(edmd_ctx* ctx, const std::vector<uint64_t>& tgt, double t_
   CK(cudaMemsetAsync(R->cmt, 0xff, TC * 8, st));
   CK(cudaMemsetAsync(R->cmi, 0x7f, TC * 4, st));
   RoundArgs A;
+  A.one = ctx->hs[0];
   A.nsys = ctx->nsys; A.radius = radius; A.TN = TN; A.flags = flags; A.ntiles = (int32_t)R->ntiles;
   {
     // the order-preserving integer image of t_stop (time_key on the host)
@@ -1590,7 +1664,7 @@ static int run_rounds(edmd_ctx* ctx, const std::vector<uint64_t>& tgt, double t_
     A.tstop_key = (u >> 63) ? ~u : (u | 0x8000000000000000ull);
   }
   A.dsys = R->dsys; A.doff = R->doff; A.coff = R->coff;
-  A.dkey = R->dkey; A.dpk = R->dpk; A.drank = R->drank; A.ikb = R->ikb; A.iktie = R->iktie; A.fc = R->fc; A.cmt = R->cmt; A.cmi = R->cmi; A.lw = R->lw; A.lr = R->lr;
+  A.att = R->att; A.drank = R->drank; A.ikb = R->ikb; A.iktie = R->iktie; A.cmt = R->cmt; A.cmi = R->cmi; A.lw = R->lw; A.lr = R->lr;
   A.safe = R->safe; A.nsafe = R->nsafe; A.dcell = R->dcell; A.selflag = R->selflag;
   A.pnext = R->nsafe + 2;
   A.active = R->active; A.lim = R->lim; A.target = R->target; A.freeze = R->freeze;
@@ -1604,7 +1678,7 @@ static int run_rounds(edmd_ctx* ctx, const std::vector<uint64_t>& tgt, double t_
   // 2.1e7; 4*10^6 disks, 22k events a round: thread 3.2e7, warp 2.9e7)
   A.thr_min = (flags & EDMD_F_ROUND_THREAD) ? 0
             : (flags & EDMD_F_ROUND_WARP) ? INT32_MAX
-            : (TN / ctx->nsys <= 65536 ? 4096 : 16384);
+            : ctx->nsys > 1 ? (TN / ctx->nsys <= 65536 ? 4096 : 16384) : (flags & EDMD_F_SCREEN) ? 16384 : INT32_MAX;
   A.tlast = R->tlast; A.cnt = R->cnt; A.shp = R->shp; A.sht = R->sht; A.epoch = R->epoch; A.tsys = R->tsys; A.tx0 = R->tx0; A.ty0 = R->ty0; A.violations = R->viol;
   const unsigned gd = (unsigned)((TN + 255) / 256);
   // the serial queue keys are still in the event records only when the
