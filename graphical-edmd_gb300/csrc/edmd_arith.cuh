@@ -1,5 +1,6 @@
-// edmd_arith.cuh -- correctly rounded FP64 division and square root on the
-// integer pipe, bit for bit the IEEE results of `a / b` and `sqrt(x)`.
+// edmd_arith.cuh -- exact FP64 arithmetic on the integer pipe: correctly rounded
+// division and square root, bit for bit the IEEE results of `a / b` and
+// `sqrt(x)`, and the event calendar's repeated additions in closed form.
 //
 // GB300 issues one FP64 warp instruction per ~76 cycles and SM sub-partition
 // (dependent latency ~38), and the compiler's FP64 division and square root
@@ -143,6 +144,32 @@ EDMD_HD double sqrt_normal(double x, bool* other, int seed_ulps = 0) {
   if (r <= -(int64_t)S) S--;                         // v < (S - 1/2)^2
   const uint32_t eo = (ex + 1023u - (odd ? 1u : 0u)) >> 1;
   return bits_f64(((uint64_t)(eo - 1) << 52) + S);
+}
+
+// The serial loop's calendar walk: while P + d <= tc, P becomes fl(P + d) and k
+// counts, for at most 2^24 steps.  Inside a binade of P every step but the
+// first adds the same multiple of its ulp (d rounds the same way each time,
+// and a tie leaves P even), so the steps up to tc or to the binade's end are
+// taken at once, as integers: ~20 divisions instead of tc / d additions
+// (140,000 for 10^6 disks at t = 0.7, 2.7 ms of a round that held such an event).
+EDMD_HD void walk_calendar(double d, double tc, double& P, uint64_t& k) {
+  int64_t left = 1 << 24;
+  while (left > 0 && P + d <= tc) {
+    const uint64_t p0 = f64_bits(P);
+    P += d; k++; left--;
+    if (left == 0 || !(P + d <= tc)) return;
+    const uint64_t p1 = f64_bits(P), p2 = f64_bits(P + d), e = p1 >> 52;
+    if (p0 >> 52 != e || p2 >> 52 != e || (p1 >> 63) || e == 0) continue;
+    const uint64_t step = p2 - p1, tb = f64_bits(tc), end = (e + 1) << 52;
+    uint64_t n = (uint64_t)left;
+    if (step) {
+      const uint64_t room = ((tb < end ? tb : end - 1) - p1) / step;
+      if (room < n) n = room;
+    }
+    P = bits_f64(p1 + n * step);
+    k += n;
+    left -= (int64_t)n;
+  }
 }
 
 #ifdef __CUDACC__

@@ -257,10 +257,9 @@ __global__ void k_rank(const SysDev* __restrict__ sys, RoundArgs A) {
 __device__ bool new_before_inherited(const SysDev& S, double tn, uint64_t clk, uint32_t bx, uint64_t tiex) {
   const Box& B = S.B;
   const SysState& R = *S.st;
-  const double tc = key_time(clk);
   uint64_t k = R.k;
   double P = R.P;
-  for (int guard = 0; guard < (1 << 24) && P + B.dtP <= tc; guard++) { P += B.dtP; k++; }
+  walk_calendar(B.dtP, key_time(clk), P, k);
   const double dt = tn - P;
   const bool ovf_new = dt >= B.dtPN;
   if (bx == BINF) return ovf_new;

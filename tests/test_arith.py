@@ -83,3 +83,33 @@ def test_quotients_and_roots_equal_ieee_bit_for_bit(lib, ulps):
         s = np.sqrt(x)
     assert np.array_equal(got[own].view(np.uint64), s[own].view(np.uint64))
     assert np.array_equal(own, normal(x) & (x > 0))
+
+
+WALK = r"""
+#include "edmd_arith.cuh"
+extern "C" void walk_both(double d, double tc, double* P, unsigned long* k) {
+  uint64_t n = k[1];
+  for (int i = 0; i < (1 << 24) && P[0] + d <= tc; i++) { P[0] += d; k[0]++; }
+  edmd::walk_calendar(d, tc, P[1], n);
+  k[1] = n;
+}
+"""
+
+
+def test_calendar_walk_equals_repeated_additions(tmp_path):
+    (tmp_path / "w.cpp").write_text(WALK)
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-fPIC", "-shared", "-o", str(tmp_path / "w.so"), str(tmp_path / "w.cpp"),
+                    "-I" + os.path.join(ROOT, "graphical-edmd_gb300", "csrc")], check=True)
+    w = ctypes.CDLL(str(tmp_path / "w.so"))
+    rng = np.random.default_rng(5)
+    for n in range(600):
+        N = int(rng.integers(2, 3000 if n % 3 else 2000000))
+        d = 5.0 / N if n % 7 else np.ldexp(1.0 + rng.integers(0, 4), -int(rng.integers(0, 30)))      # widths that tie too
+        P0 = 0.0 if n % 2 else float(np.add.accumulate(np.full(int(rng.integers(1, 50000)), d))[-1])
+        if n % 11 == 0:
+            P0 = np.ldexp(1.0 + rng.random(), int(rng.integers(-10, 50)))                            # steps below half an ulp among them
+        tc = P0 + rng.random() * d * (100000 if n % 5 == 0 else 3000) if n % 13 else P0 - 1.0
+        P = np.array([P0, P0])
+        k = np.array([7, 7], np.uint64)
+        w.walk_both(ctypes.c_double(d), ctypes.c_double(tc), p(P), p(k))
+        assert P[0] == P[1] and k[0] == k[1], (d, tc, P0)
