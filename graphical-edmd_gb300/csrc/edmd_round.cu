@@ -66,6 +66,13 @@ constexpr int NSTRIPE = 32;           // copies of each system's counters
 // counters of the round engine, per system and stripe (u64 slots)
 enum { C_CT0, C_CT1, C_CT2, C_CT3, C_NCOL, C_NCROSS, C_NSTALE, C_NPAIR, C_NSCREEN, C_TLAST, NCNT };
 
+// The selection compares times as 32-bit numbers, (key - base) >> shift clamped
+// to 32 bits: the order of the times, coarse to about 2^-26 of a time unit, for
+// 32 time units (early in a run more) around the system's last event.  Equal numbers (rare: the
+// events around a cell are ~10^-3 apart) are told apart by the exact (key, id)
+// of the cells concerned, so the selected events are those of the exact order.
+struct SelScale { uint64_t base; int32_t shift, pad; };
+
 // What the cell minima are made of, in one 32-byte sector per disk: the minima
 // of a round's dirty cells are found by walking ~11 disks around each, which
 // took four sectors a disk with the fields in arrays of their own.
@@ -100,6 +107,7 @@ struct RoundArgs {
   int32_t* selflag;              // some event of the system was selected
   int32_t* active;               // systems still running after the round
   uint64_t* lim;                 // per-system bound on eligible keys for the round
+  SelScale* scale;               // per-system scale of the selection's 32-bit times (sel_time)
   const uint64_t* target;        // per-system ncol at which the budget is met
   uint64_t* freeze;              // per-system key bound once the budget is met
   uint64_t* tlast;               // per-system largest screenshot key passed
@@ -339,6 +347,24 @@ __global__ void k_prep_owner(RoundArgs A) {
   if (b != a && A.cmt[b] == key) atomicMin(&A.cmi[b], id);
 }
 
+constexpr uint32_t SEL_NONE = 0xffffffffu;
+// the scale around the key of the system's last event
+__device__ __forceinline__ SelScale sel_scale(uint64_t last) {
+  const int e = (int)((last >> 52) & 0x7ff) - 1023;
+  SelScale c;
+  c.shift = e > 26 ? 0 : e < -5 ? 31 : 26 - e;
+  const uint64_t zero = 1ull << 63, back = (uint64_t)1 << (31 + c.shift);
+  c.base = last > zero + back ? last - back : zero;
+  c.pad = 0;
+  return c;
+}
+__device__ __forceinline__ uint32_t sel_time(uint64_t k, const SelScale& c) {
+  const uint64_t d = k - c.base;
+  const uint32_t hi = (uint32_t)(d >> 32);
+  const uint32_t q = __funnelshift_r((uint32_t)d, hi, c.shift);
+  return k == KINF ? SEL_NONE : k < c.base ? 0u : (hi >> c.shift) || q == SEL_NONE ? 0xfffffffeu : q;
+}
+
 // eligibility bound of every system for the next round
 __device__ __forceinline__ uint64_t system_limit(const SysDev& S, const RoundArgs& A, int s) {
   if (S.st->status != EDMD_OK) return 0;
@@ -350,7 +376,9 @@ __device__ __forceinline__ uint64_t system_limit(const SysDev& S, const RoundArg
 
 __global__ void k_limits(const SysDev* __restrict__ sys, RoundArgs A) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < A.nsys) A.lim[s] = system_limit(sys[s], A, s);
+  if (s >= A.nsys) return;
+  A.lim[s] = system_limit(sys[s], A, s);
+  A.scale[s] = sel_scale(time_key(sys[s].st->t));
 }
 
 // ---------------------------------------------------------------- per round
@@ -364,38 +392,31 @@ __device__ __forceinline__ int wrapi(int v, int n) {
   return v < 0 ? v + n : v;
 }
 
-// (time key, event id) as one 96-bit value in a 128-bit word: the unsigned
-// order of the word is the lexicographic order pair_less uses (ids are
-// non-negative), so a window minimum is one compare-and-select per element
-typedef unsigned __int128 kid_t;
-__device__ __forceinline__ kid_t kid(uint64_t k, int32_t id) { return ((kid_t)k << 32) | (uint32_t)id; }
-__device__ __forceinline__ kid_t kid_min(kid_t a, kid_t b) { return b < a ? b : a; }
-
 // Window minima of S consecutive positions: out[k] = min(a[k .. k+W-1]).
 // The W-S+1 middle elements are common to all S windows; each window adds a
 // suffix of the left part and a prefix of the right part (a van Herk /
 // Gil-Werman block): W + 2S - 4 compares instead of S (W - 1).
 template <int S, int W>
-__device__ __forceinline__ void block_window_min(const kid_t (&a)[S + W - 1], kid_t (&out)[S]) {
+__device__ __forceinline__ void block_window_min(const uint32_t (&a)[S + W - 1], uint32_t (&out)[S]) {
   static_assert(W >= S, "window narrower than the block");
-  kid_t c = a[S - 1];
+  uint32_t c = a[S - 1];
 #pragma unroll
-  for (int j = S; j < W; j++) c = kid_min(c, a[j]);
+  for (int j = S; j < W; j++) c = min(c, a[j]);
   if constexpr (S == 1) {
     out[0] = c;
     return;
   }
-  kid_t rp[S];
+  uint32_t rp[S];
   rp[0] = c;
 #pragma unroll
-  for (int k = 1; k < S; k++) rp[k] = kid_min(rp[k - 1], a[W + k - 1]);
+  for (int k = 1; k < S; k++) rp[k] = min(rp[k - 1], a[W + k - 1]);
   out[S - 1] = rp[S - 1];
   if constexpr (S > 1) {
-    kid_t ls = a[S - 2];
+    uint32_t ls = a[S - 2];
 #pragma unroll
     for (int k = S - 2; k >= 0; k--) {
-      if (k < S - 2) ls = kid_min(ls, a[k]);
-      out[k] = kid_min(ls, rp[k]);
+      if (k < S - 2) ls = min(ls, a[k]);
+      out[k] = min(ls, rp[k]);
     }
   }
 }
@@ -405,8 +426,6 @@ __device__ __forceinline__ void block_window_min(const kid_t (&a)[S + W - 1], ki
 // of SB outputs reads in range; the padding's outputs are never used)
 template <int R>
 struct SelGeom {
-  // two outputs per thread: measured best of 1, 2 and 4 (fewer compares per
-  // output against idle threads at the tile's barriers)
   static constexpr int H = R + 1, W = 2 * R + 1, SB = 2;
   static constexpr int HW = TX + 2;                    // outputs per row: columns -1..TX
   static constexpr int NHB = (HW + SB - 1) / SB;
@@ -414,24 +433,24 @@ struct SelGeom {
   static constexpr int VR = TY + 2;                    // outputs per column: rows -1..TY
   static constexpr int NVB = (VR + SB - 1) / SB;
   static constexpr int CH = NVB * SB + W - 1;          // rows of cell and horizontal minima
-  static constexpr size_t bytes = (size_t)(CH * CW + CH * HW + NVB * SB * HW) * sizeof(kid_t);
+  static constexpr int words = CH * CW + CH * HW + NVB * SB * HW;
 };
 
 // Window minima of tiles in shared memory and selection of their events into
 // A.safe, counted in *nsafe; the window radius R is a compile-time constant
 // (3..12).  By a block of TX x TY threads, on every gridDim-th tile.
 template <int R, bool ONE>
-__device__ __forceinline__ void select_tiles(const SysDev* __restrict__ sys, const RoundArgs& A, kid_t* sel_smem,
+__device__ __forceinline__ void select_tiles(const SysDev* __restrict__ sys, const RoundArgs& A, uint32_t* smem,
                                              int32_t* nsafe) {
   using G = SelGeom<R>;
   constexpr int H = G::H, W = G::W, SB = G::SB, HW = G::HW, CW = G::CW, CH = G::CH;
-  kid_t* ck = sel_smem;                // CH x CW
-  kid_t* hk = ck + CH * CW;            // CH x HW
-  kid_t* wk = hk + CH * HW;            // NVB*SB x HW
+  uint32_t* ck = smem;                 // CH x CW
+  uint32_t* hk = ck + CH * CW;         // CH x HW
+  uint32_t* wk = hk + CH * HW;         // NVB*SB x HW
   for (int t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
   const int s = ONE ? 0 : A.tsys[t];
   const uint64_t lim = A.lim[s];
-  if (lim == 0) continue;             // the system has stopped: nothing to select
+  const SelScale scale = A.scale[s];
   const Box& B = sys_of<ONE>(sys, A, s).B;
   const int Nxc = B.Nxc, Nyc = B.Nyc;
   int x0, y0;
@@ -442,26 +461,35 @@ __device__ __forceinline__ void select_tiles(const SysDev* __restrict__ sys, con
     x0 = A.tx0[t]; y0 = A.ty0[t];
   }
   const int64_t base = first_cell<ONE>(A, s);
+  const int ix = threadIdx.x % TX, iy = threadIdx.x / TX, lane = threadIdx.x & 31;
+  const int cx = x0 + ix, cy = y0 + iy;
+  // the thread's own cell, exact, on its way beside the tile
+  uint64_t k = KINF;
+  int32_t id = 0;
+  if (cx < Nxc && cy < Nyc) {
+    k = A.cmt[base + cy * Nxc + cx];
+    id = A.cmi[base + cy * Nxc + cx];
+  }
   if (x0 >= H && x0 - H + CW <= Nxc && y0 >= H && y0 - H + CH <= Nyc) {
     // a tile away from the periodic edges: no wrap
-    const int64_t c0 = base + (int64_t)(y0 - H) * Nxc + (x0 - H);
-    for (int q = threadIdx.x; q < CW * CH; q += blockDim.x) {
+    const uint64_t* __restrict__ c0 = A.cmt + base + (int64_t)(y0 - H) * Nxc + (x0 - H);
+#pragma unroll 3
+    for (int q = threadIdx.x; q < CW * CH; q += TX * TY) {
       const int lx = q % CW, ly = q / CW;
-      const int64_t c = c0 + (int64_t)ly * Nxc + lx;
-      ck[q] = kid(A.cmt[c], A.cmi[c]);
+      ck[q] = sel_time(c0[(int64_t)ly * Nxc + lx], scale);
     }
   } else {
-    for (int q = threadIdx.x; q < CW * CH; q += blockDim.x) {
+    for (int q = threadIdx.x; q < CW * CH; q += TX * TY) {
       const int lx = q % CW, ly = q / CW;
       const int gx = wrapi(x0 + lx - H, Nxc), gy = wrapi(y0 + ly - H, Nyc);
-      const int64_t c = base + (int64_t)gy * Nxc + gx;
-      ck[q] = kid(A.cmt[c], A.cmi[c]);
+      ck[q] = sel_time(A.cmt[base + (int64_t)gy * Nxc + gx], scale);
     }
   }
+  if (lim == 0) continue;             // the system has stopped: nothing to select
   __syncthreads();
-  for (int q = threadIdx.x; q < CH * G::NHB; q += blockDim.x) {
+  for (int q = threadIdx.x; q < CH * G::NHB; q += TX * TY) {
     const int ly = q / G::NHB, hx0 = (q % G::NHB) * SB;
-    kid_t a[SB + W - 1], o[SB];
+    uint32_t a[SB + W - 1], o[SB];
 #pragma unroll
     for (int j = 0; j < SB + W - 1; j++) a[j] = ck[ly * CW + hx0 + j];
     block_window_min<SB, W>(a, o);
@@ -470,9 +498,9 @@ __device__ __forceinline__ void select_tiles(const SysDev* __restrict__ sys, con
       if (hx0 + k < HW) hk[ly * HW + hx0 + k] = o[k];
   }
   __syncthreads();
-  for (int q = threadIdx.x; q < HW * G::NVB; q += blockDim.x) {
+  for (int q = threadIdx.x; q < HW * G::NVB; q += TX * TY) {
     const int wx = q % HW, wy0 = (q / HW) * SB;
-    kid_t a[SB + W - 1], o[SB];
+    uint32_t a[SB + W - 1], o[SB];
 #pragma unroll
     for (int j = 0; j < SB + W - 1; j++) a[j] = hk[(wy0 + j) * HW + wx];
     block_window_min<SB, W>(a, o);
@@ -480,41 +508,58 @@ __device__ __forceinline__ void select_tiles(const SysDev* __restrict__ sys, con
     for (int k = 0; k < SB; k++) wk[(wy0 + k) * HW + wx] = o[k];
   }
   __syncthreads();
-  const int ix = threadIdx.x % TX, iy = threadIdx.x / TX;
-  const int cx = x0 + ix, cy = y0 + iy;
   bool sel = false;
-  int32_t g = 0;
-  if (cx < Nxc && cy < Nyc) {
-    const kid_t v = ck[(iy + H) * CW + ix + H];
-    const uint64_t k = (uint64_t)(v >> 32);
-    const int32_t id = (int32_t)(uint32_t)v;
-    g = id & GMASK;
-    const int w = (iy + 1) * HW + ix + 1;
-    if (k < lim && wk[w] == v) {
-      const int c = cy * Nxc + cx;
-      if (A.att[g].c1 == c) {
-        const int c2 = A.att[g].c2;
-        if (c2 == c) {
-          sel = true;
-        } else {
-          int dx = c2 % Nxc - cx, dy = c2 / Nxc - cy;
-          if (dx > 1) dx -= Nxc;
-          if (dx < -1) dx += Nxc;
-          if (dy > 1) dy -= Nyc;
-          if (dy < -1) dy += Nyc;
-          if (dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1) sel = wk[(iy + 1 + dy) * HW + ix + 1 + dx] == v;
-        }
+  int dx = 0, dy = 0;
+  const uint32_t v = ck[(iy + H) * CW + ix + H];
+  if (k < lim && wk[(iy + 1) * HW + ix + 1] == v) {
+    // the least of its window, to the coarse order
+    const int c = cy * Nxc + cx;
+    const Att* at = A.att + (id & GMASK);
+    if (at->c1 == c) {
+      const int c2 = at->c2;
+      if (c2 == c) {
+        sel = true;
+      } else {
+        dx = c2 % Nxc - cx; dy = c2 / Nxc - cy;
+        if (dx > 1) dx -= Nxc;
+        if (dx < -1) dx += Nxc;
+        if (dy > 1) dy -= Nyc;
+        if (dy < -1) dy += Nyc;
+        if (dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1) sel = wk[(iy + 1 + dy) * HW + ix + 1 + dx] == v;
       }
     }
   }
+  // exact order against the cells of both windows with the same coarse time,
+  // one candidate of the warp at a time
+  for (unsigned m = __ballot_sync(FULLM, sel); m; m &= m - 1) {
+    const int src = __ffs(m) - 1;
+    const int sx = __shfl_sync(FULLM, ix, src), sy = __shfl_sync(FULLM, iy, src);
+    const int sdx = __shfl_sync(FULLM, dx, src), sdy = __shfl_sync(FULLM, dy, src);
+    const uint32_t sv = __shfl_sync(FULLM, v, src);
+    const uint64_t sk = __shfl_sync(FULLM, k, src);
+    const int32_t sid = __shfl_sync(FULLM, id, src);
+    // the windows' bounding box
+    const int bx = sdx < 0 ? sdx : 0, by = sdy < 0 ? sdy : 0;
+    const int bw = W + (sdx ? 1 : 0), bh = W + (sdy ? 1 : 0);
+    bool less = false;
+    for (int q = lane; q < bw * bh; q += 32) {
+      const int ox = q % bw - R + bx, oy = q / bw - R + by;   // from the owner's cell
+      if (ck[(sy + H + oy) * CW + sx + H + ox] != sv) continue;
+      const bool in1 = ox >= -R && ox <= R && oy >= -R && oy <= R;
+      const bool in2 = ox - sdx >= -R && ox - sdx <= R && oy - sdy >= -R && oy - sdy <= R;
+      if (!(in1 || in2) || (ox == 0 && oy == 0)) continue;
+      const int64_t c = base + (int64_t)wrapi(y0 + sy + oy, Nyc) * Nxc + wrapi(x0 + sx + ox, Nxc);
+      less |= pair_less(A.cmt[c], A.cmi[c], sk, sid);
+    }
+    if (__any_sync(FULLM, less) && lane == src) sel = false;
+  }
   const unsigned m = __ballot_sync(FULLM, sel);
   if (m) {
-    const int lane = threadIdx.x & 31;
     const int lead = __ffs(m) - 1;
     int pos = 0;
     if (lane == lead) pos = atomicAdd(nsafe, __popc(m));
     pos = __shfl_sync(FULLM, pos, lead);
-    if (sel) A.safe[pos + __popc(m & ((1u << lane) - 1))] = g;
+    if (sel) A.safe[pos + __popc(m & ((1u << lane) - 1))] = id & GMASK;
     if (lane == lead) A.selflag[s] = 1;
   }
   __syncthreads();
@@ -523,7 +568,7 @@ __device__ __forceinline__ void select_tiles(const SysDev* __restrict__ sys, con
 
 template <int R, bool ONE>
 __global__ void __launch_bounds__(TX * TY, 4) k_select(const SysDev* __restrict__ sys, const __grid_constant__ RoundArgs A) {
-  extern __shared__ kid_t sel_smem[];
+  __shared__ uint32_t sel_smem[SelGeom<R>::words];
   // the round's count of running systems is rebuilt by the barrier
   if (blockIdx.x == 0 && threadIdx.x == 0) *A.active = 0;
   select_tiles<R, ONE>(sys, A, sel_smem, A.nsafe);
@@ -1425,6 +1470,7 @@ __device__ __forceinline__ void barrier_systems(const SysDev* __restrict__ sys, 
           fz = kmax(tl, A.tlast[s]) + 1;
           A.freeze[s] = fz;
         }
+        if (tl) A.scale[s] = sel_scale(tl);
         const uint64_t lim = A.tstop_key < fz ? A.tstop_key : fz;
         const int selected = A.selflag[s];
         go = (ok && !selected && time_key(S.ev[2 * N + SP_SCREEN].t) < lim) ? 1 : 0;
@@ -1529,6 +1575,7 @@ struct RoundBufs {
   int32_t *tsys = nullptr, *tx0 = nullptr, *ty0 = nullptr;
   int64_t *doff = nullptr, *coff = nullptr;
   uint64_t *cmt = nullptr, *lw = nullptr, *lr = nullptr;
+  SelScale* scale = nullptr;
   uint64_t *lim = nullptr, *target = nullptr, *freeze = nullptr, *tlast = nullptr, *cnt = nullptr;
   float4* shp = nullptr;
   float* sht = nullptr;
@@ -1564,7 +1611,7 @@ int round_init(edmd_ctx* ctx) {
   CK(dalloc(&R->selflag, ctx->nsys)); CK(dalloc(&R->active, 2)); CK(dalloc(&R->work, 1));
   CK(dalloc(&R->doff, ctx->nsys)); CK(dalloc(&R->coff, ctx->nsys));
   CK(dalloc(&R->lim, ctx->nsys)); CK(dalloc(&R->target, ctx->nsys)); CK(dalloc(&R->freeze, ctx->nsys));
-  CK(dalloc(&R->tlast, ctx->nsys)); CK(dalloc(&R->viol, 1));
+  CK(dalloc(&R->scale, ctx->nsys)); CK(dalloc(&R->tlast, ctx->nsys)); CK(dalloc(&R->viol, 1));
   CK(dalloc(&R->cnt, (int64_t)ctx->nsys * NSTRIPE * NCNT));
   CK(dalloc(&R->shp, TN)); CK(dalloc(&R->sht, TN)); CK(dalloc(&R->epoch, ctx->nsys));
   CK(dalloc(&R->tsys, R->ntiles)); CK(dalloc(&R->tx0, R->ntiles)); CK(dalloc(&R->ty0, R->ntiles));
@@ -1574,14 +1621,6 @@ int round_init(edmd_ctx* ctx) {
   CK(sync_copy(ctx, R->tx0, tx0.data(), R->ntiles * 4, cudaMemcpyHostToDevice));
   CK(sync_copy(ctx, R->ty0, ty0.data(), R->ntiles * 4, cudaMemcpyHostToDevice));
   CK(sync_set(ctx, R->selflag, 0, ctx->nsys * 4));
-  // selection tiles of wide windows need more than the default 48 KB of
-  // dynamic shared memory
-#define SEL_SMEM(R) \
-  CK(cudaFuncSetAttribute(k_select<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SelGeom<R>::bytes)); \
-  CK(cudaFuncSetAttribute(k_select<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SelGeom<R>::bytes));
-  SEL_SMEM(3) SEL_SMEM(4) SEL_SMEM(5) SEL_SMEM(6) SEL_SMEM(7)
-  SEL_SMEM(8) SEL_SMEM(9) SEL_SMEM(10) SEL_SMEM(11) SEL_SMEM(12)
-#undef SEL_SMEM
   k_round_setup<<<dim3(64, ctx->nsys), 256, 0, ctx->stream>>>(R->doff, ctx->ds, R->dsys);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->stream));
@@ -1602,8 +1641,8 @@ cudaError_t enqueue_round(edmd_ctx* ctx, const RoundBufs* R, const RoundArgs& A0
   switch (A.radius) {
 #define SEL_CASE(R) \
     case R: \
-      if (one) k_select<R, true><<<tgrid, TX * TY, SelGeom<R>::bytes, st>>>(ctx->ds, A); \
-      else k_select<R, false><<<tgrid, TX * TY, SelGeom<R>::bytes, st>>>(ctx->ds, A); \
+      if (one) k_select<R, true><<<tgrid, TX * TY, 0, st>>>(ctx->ds, A); \
+      else k_select<R, false><<<tgrid, TX * TY, 0, st>>>(ctx->ds, A); \
       break;
     SEL_CASE(3) SEL_CASE(4) SEL_CASE(5) SEL_CASE(6) SEL_CASE(7)
     SEL_CASE(8) SEL_CASE(9) SEL_CASE(10) SEL_CASE(11) SEL_CASE(12)
@@ -1628,7 +1667,7 @@ void round_free(edmd_ctx* ctx) {
   if (!R) return;
   void* p[] = {R->dsys, R->att, R->cmi, R->safe, R->nsafe, R->dcell, R->selflag, R->active,
                R->tsys, R->tx0, R->ty0, R->doff, R->coff, R->cmt, R->lw, R->lr,
-               R->lim, R->target, R->freeze, R->tlast, R->cnt, R->viol, R->drank,
+               R->lim, R->target, R->freeze, R->tlast, R->cnt, R->viol, R->scale, R->drank,
                R->drank_bak, R->ikb, R->iktie, R->work, R->shp, R->sht, R->epoch};
   for (void* q : p)
     if (q) cudaFree(q);
@@ -1666,7 +1705,7 @@ static int run_rounds(edmd_ctx* ctx, const std::vector<uint64_t>& tgt, double t_
   A.att = R->att; A.drank = R->drank; A.ikb = R->ikb; A.iktie = R->iktie; A.cmt = R->cmt; A.cmi = R->cmi; A.lw = R->lw; A.lr = R->lr;
   A.safe = R->safe; A.nsafe = R->nsafe; A.dcell = R->dcell; A.selflag = R->selflag;
   A.pnext = R->nsafe + 2;
-  A.active = R->active; A.lim = R->lim; A.target = R->target; A.freeze = R->freeze;
+  A.active = R->active; A.lim = R->lim; A.scale = R->scale; A.target = R->target; A.freeze = R->freeze;
   A.maxsafe = R->active + 1; A.thread_kernel = 1;
   // one thread per event needs enough events to keep every SM busy with one
   // lane each: the cells of small systems stay in L2, so 4096 events do; the
