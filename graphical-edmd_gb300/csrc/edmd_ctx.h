@@ -59,6 +59,8 @@ struct edmd_ctx {
   bool round_dirty = false;         // queue order lost: set by the round engine, cleared by a restage
   bool any_additive = false;        // some system uses additive contact (EDMD_CONTACT_ADDITIVE)
   std::vector<char> ckpt_dirty;     // round_dirty of each checkpoint
+  char* pin = nullptr;              // two page-locked buffers of host_copies, and their events
+  cudaEvent_t pin_ev[2] = {nullptr, nullptr};
   std::string err;
 };
 
@@ -170,29 +172,16 @@ static inline void run_threads(int n, F&& f) {
   for (auto& th : pool) th.join();
 }
 
-// Make the pages of host buffers resident before a device copy writes them:
-// into fresh pageable memory the copy engine faults page by page (192 MB into
-// new arrays took 160 ms; 4.5 ms into resident ones), host threads do not.
-// Every byte keeps its value.
-static inline void make_resident(double* const* bufs, int nbufs, int64_t bytes) {
-  constexpr int64_t PAGE = 4096;
-  const int64_t pages = (bytes + PAGE - 1) / PAGE;
-  const int nth = host_threads(pages * nbufs, 256);
-  run_threads(nth, [&](int k) {
-    for (int b = 0; b < nbufs; b++) {
-      if (!bufs[b]) continue;
-      volatile char* p = (volatile char*)bufs[b];
-      for (int64_t g = pages * k / nth; g < pages * (k + 1) / nth; g++) {
-        const char v = p[g * PAGE];
-        p[g * PAGE] = v;
-      }
-      if (k == nth - 1 && bytes > 0) {
-        const char v = p[bytes - 1];
-        p[bytes - 1] = v;
-      }
-    }
-  });
-}
+// One array between pageable host memory and the device.
+struct HostCopy { void* host; void* dev; int64_t bytes; };
+
+// Copies in order on the context's stream, complete on return.  Pageable memory
+// that the device has not touched yet is translated for it page by page (192 MB
+// into new arrays: 72 ms, whether the host has touched them or not; 2 ms into
+// arrays a copy has used before), so large copies go through two page-locked
+// buffers: one moves over the link while host threads move the other.
+// Page-locked host arrays and small ones are copied directly.
+cudaError_t host_copies(edmd_ctx* ctx, const std::vector<HostCopy>& list, bool to_device);
 
 template <class T>
 static inline cudaError_t dalloc(T** p, size_t n) { return cudaMalloc((void**)p, (n ? n : 1) * sizeof(T)); }

@@ -869,7 +869,7 @@ extern "C" int edmd_tangent_run_batch(edmd_ctx* ctx, int32_t K, int64_t n_coll, 
   CK(call_begin(ctx));
   std::vector<double> t0(nsys), t1(nsys);
   if ((rc = sys_times(ctx, t0.data()))) return rc;
-  CK(cudaMemcpyAsync(T, h.get(), nh * 8, cudaMemcpyHostToDevice, ctx->stream));
+  CK(host_copies(ctx, {{h.get(), T, (int64_t)nh * 8}}, true));
   k_fill_sys_time<<<(unsigned)((TN + 255) / 256), 256, 0, ctx->stream>>>(ctx->ds, bi.dsys, TN, tl);
   CK(cudaMemsetAsync(logdiag, 0, (size_t)nsys * K * sizeof(double), ctx->stream));
   CK(cudaMemsetAsync(fail, 0, nsys * sizeof(int), ctx->stream));
