@@ -43,17 +43,18 @@ struct edmd_ctx {
   edmd_collision* trace = nullptr;
   double* rows = nullptr;
   double* stage = nullptr;          // SoA gather buffer (6 x total_N)
-  int32_t* work = nullptr;
-  int32_t* order = nullptr;      // warp engine: order the systems are taken in
-  uint32_t* cost = nullptr;      // warp engine: each system's run time in the last call
-  std::vector<int32_t> order_h;
+  int32_t* order = nullptr;         // warp engine: system of each place (shared-memory split)
+  int32_t* waiting = nullptr;       // warp engine: see RunArgs, made when a call first needs them
+  unsigned* ticket = nullptr;
+  RunProgress* progress = nullptr;
   edmd_log_entry* logbuf = nullptr; // per-system collision-geometry logs
   int64_t log_cap = 0;
   std::vector<void*> ckpt;          // device snapshots of the whole engine state
   std::vector<size_t> ckpt_parts;   // bytes of each array in a snapshot
   uint16_t* cal = nullptr;          // calendars of the thread-per-system engine
   uint16_t* mask = nullptr;
-  int engine = 0;                   // EDMD_ENGINE_WARP or EDMD_ENGINE_LANE
+  int engine = 0;                   // EDMD_ENGINE_WARP or EDMD_ENGINE_LANE, as reported
+  bool calendar = false;            // events run by the thread-per-system loop on its calendars
   int64_t total_C = 0;
   void* round = nullptr;            // buffers of the round-parallel engine (edmd_round.cu)
   bool round_dirty = false;         // queue order lost: set by the round engine, cleared by a restage

@@ -116,15 +116,22 @@ struct SysDev {
 constexpr int CAL_SUB = 16;    // sub-buckets per calendar bucket (ordered by time)
 constexpr int CAL_LINE = 32;   // u16 per sub-bucket line: count, 29 ids, spill-list head
 
+// how far a system is in a call
+struct RunProgress { int64_t logged, nev; };
+
 struct RunArgs {
   int64_t max_coll;
   double t_stop;
   uint32_t flags;
   int64_t max_events;
   int32_t nsys;
-  int32_t* work;               // persistent work counter (warp engine)
-  const int32_t* order;        // warp engine: systems in the order they are taken (null: 0, 1, ...)
-  uint32_t* cost;              // warp engine: each system's run time in this call (units of 1.024 us)
+  // warp engine: system of each place (null: 0, 1, ...), and what a call with
+  // more systems than lane groups needs to pass them around (see k_run)
+  const int32_t* order;
+  int32_t* waiting;            // places without a group (-1: a hole), nwait slots
+  int32_t nwait, nrun;         // slots; groups
+  unsigned* ticket;            // [0] next slot, [1] places waiting
+  RunProgress* progress;       // per place
 };
 
 // ---------------------------------------------------------------- arithmetic

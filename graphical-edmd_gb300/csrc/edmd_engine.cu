@@ -443,7 +443,7 @@ __device__ void do_growstop(const SysDev& S, SysState& R, const Grp<GW>& G, Warp
 // ---------------------------------------------------------------- run loop
 
 // what ends a stretch of disk events
-enum { END_STOP, END_SPECIAL };
+enum { END_STOP, END_SPECIAL, END_SHARE };
 
 // A stretch of disk events of one system: until a stop, or a special event
 // (screenshot, thermo, growth stop), which is taken off the queue and left in
@@ -458,7 +458,7 @@ enum { END_STOP, END_SPECIAL };
 // switch compiled out of the pair solves and the collision rule)
 template <int GW, bool ADD, bool GROW>
 __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int64_t max_coll, const Grp<GW>& G,
-                                          WarpSmem* sm, int64_t& logged, int64_t& nev, int* special) {
+                                          WarpSmem* sm, int64_t& logged, int64_t& nev, int64_t share_end, int* special) {
   const int lane = G.lane;
   const bool odd = lane & 1, ydim = lane & 2;
   const Box& B = S.B;
@@ -487,7 +487,11 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
   for (;;) {
     if (!le_i(t, tmax)) { stop = EDMD_STOP_TMAX; break; }
     if (logged >= max_coll) { stop = EDMD_STOP_COLL; break; }
-    if (nev >= A.max_events) { status = EDMD_ERR_BUDGET; break; }
+    if (nev >= share_end) {
+      if (nev >= A.max_events) status = EDMD_ERR_BUDGET;
+      else end = END_SHARE;
+      break;
+    }
     Node r;
     int guard = 0;
     for (;;) {
@@ -779,23 +783,83 @@ __device__ __noinline__ bool serve_special(const SysDev& S, uint32_t flags, int 
   return !ovl && !stop;
 }
 
-// the event loop of one system
+// the event loop of one system, at most `share` events of it; true when the
+// call is done with the system
 template <int GW, bool ADD = true>
-__device__ void run_system(const SysDev& S, const RunArgs& A, int64_t max_coll, const Grp<GW>& G,
-                           WarpSmem* sm) {
-  if (S.st->status != EDMD_OK) return;
-  int64_t logged = 0, nev = 0;
+__device__ bool run_system(const SysDev& S, const RunArgs& A, const Grp<GW>& G, WarpSmem* sm, RunProgress& pr,
+                           int64_t share) {
+  if (S.st->status != EDMD_OK) return true;
+  const int64_t share_end = A.max_events - pr.nev > share ? pr.nev + share : A.max_events;
   for (;;) {
     int special = 0, end;
-    if (S.st->grow) end = run_events<GW, ADD, true>(S, A, max_coll, G, sm, logged, nev, &special);
-    else end = run_events<GW, ADD, false>(S, A, max_coll, G, sm, logged, nev, &special);
-    if (end != END_SPECIAL || !serve_special<GW, ADD>(S, A.flags, special, G, sm)) break;
+    if (S.st->grow) end = run_events<GW, ADD, true>(S, A, A.max_coll, G, sm, pr.logged, pr.nev, share_end, &special);
+    else end = run_events<GW, ADD, false>(S, A, A.max_coll, G, sm, pr.logged, pr.nev, share_end, &special);
+    if (end == END_SHARE) return false;
+    if (end != END_SPECIAL || !serve_special<GW, ADD>(S, A.flags, special, G, sm)) return true;
   }
 }
 
-// Persistent launch: lane groups (GW lanes, one system each) pull systems
-// from a counter, in A.order, and record each system's run time
-// (globaltimer) for the next call's order.
+// Events a system runs before it makes room for a waiting one, ~5 ms: measured
+// on 3100 mixed systems x 1200 collisions 1.18e8 coll/s with 64 and 256, 1.05e8
+// with 1024 (too coarse at the end of the launch).  A call of at most 256
+// collisions takes a system whole: 16384 systems of 96 disks x 150 collisions
+// (257 events each) 16.1 ms against 18.2 ms cut at 256.
+__device__ __forceinline__ int64_t share_of(int64_t max_coll) { return max_coll <= 256 ? 1024 : 256; }
+
+// The place whose system a lane group runs next, -1 when there is none.  A
+// group leaves its own place `mine` (-1: its system is done) in the waiting slot
+// that the ticket names and takes what waited there; slots are only exchanged
+// whole, so no group ever waits for another.  ticket[1] counts the waiting
+// places and is never below their number: raised before a place goes into a
+// slot, lowered after one came out.  The last group to finish looks through
+// slots that no one fills any more, so no place is left behind.
+template <int GW>
+__device__ __noinline__ int next_place(const RunArgs& A, int mine, Grp<GW> G) {
+  const unsigned nw = (unsigned)A.nwait;
+  int got = -1;
+  unsigned at = 0;
+  if (G.lane == 0) {
+    __threadfence();                                  // the system's state before its place
+    at = atomicAdd(&A.ticket[0], 1u) % nw;
+    if (mine >= 0) {
+      atomicAdd(&A.ticket[1], 1u);
+      got = atomicExch(&A.waiting[at], mine);
+      if (got < 0) got = atomicExch(&A.waiting[at], -1);   // a hole: back out (or take what came in since)
+      if (got >= 0) atomicAdd(&A.ticket[1], ~0u);
+    }
+  }
+  got = G.shfl(got, 0);
+  at = (unsigned)G.shfl((int)at, 0);
+  // nothing yet (this system is done, or another group took it from the hole):
+  // any waiting place from the ticket's slot on
+  for (unsigned k = 0; k < nw && got < 0; k += GW) {
+    int left = 0;
+    if (G.lane == 0) left = (int)atomicAdd(&A.ticket[1], 0u);
+    if (G.shfl(left, 0) <= 0) break;
+    const unsigned q = (at + k + G.lane) % nw;
+    unsigned here = G.ballot(k + G.lane < nw && *(volatile int32_t*)&A.waiting[q] >= 0);
+    while (here && got < 0) {
+      const int l = __ffs(here) - 1;
+      here &= here - 1;
+      int v = -1;
+      if (G.lane == l) {
+        v = atomicExch(&A.waiting[q], -1);
+        if (v >= 0) atomicAdd(&A.ticket[1], ~0u);
+      }
+      got = G.shfl(v, l);
+    }
+  }
+  __threadfence();                                    // and the place before the system's state
+  G.sync();
+  return got;
+}
+
+// Lane groups (GW lanes, one system each), all resident.  With more systems
+// than groups the others wait, and after every share of events a group changes
+// its system for a waiting one: the systems advance together and the launch
+// ends with all groups busy.  Whole systems, longest first by the last call's
+// times, left the last ones to a nearly empty GPU: 4096 systems of 256-1024
+// disks 9.5e7 coll/s, 1.2e8 in turns.
 // MINB: blocks of four warps per SM the registers allow for (run_shape).
 template <int GW, bool ADD, int MINB>
 __global__ void __launch_bounds__(32 * WARPS_PER_BLOCK, MINB)
@@ -803,21 +867,25 @@ k_run(const SysDev* __restrict__ sys, RunArgs A) {
   __shared__ WarpSmem smem[WARPS_PER_BLOCK * (32 / GW)];
   const Grp<GW> G(threadIdx.x);
   WarpSmem* sm = &smem[threadIdx.x / GW];
-  for (;;) {
-    int it = 0;
-    if (G.lane == 0) it = atomicAdd(A.work, 1);
-    it = G.shfl(it, 0);
-    if (it >= A.nsys) break;
-    const int s = A.order ? A.order[it] : it;
-    unsigned long long t0 = 0, t1 = 0;
-    if (A.cost) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-    run_system<GW, ADD>(sys[s], A, A.max_coll, G, sm);
-    if (A.cost && G.lane == 0) {
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-      const unsigned long long c = (t1 - t0) >> 10;
-      A.cost[s] = c > 0xffffffffull ? 0xffffffffu : (uint32_t)c;
-    }
+  int p = (int)((blockIdx.x * blockDim.x + threadIdx.x) / GW);
+  if (p >= A.nrun) return;
+  while (p >= 0) {
+    const int s = A.order ? A.order[p] : p;
+    RunProgress pr{0, 0};
+    if (A.nwait) pr = A.progress[p];
+    const bool done = run_system<GW, ADD>(sys[s], A, G, sm, pr, A.nwait ? share_of(A.max_coll) : A.max_events);
+    if (!A.nwait) break;
+    if (G.lane == 0) A.progress[p] = pr;
+    G.sync();
+    p = next_place(A, done ? -1 : p, G);
   }
+}
+
+__global__ void k_waiting(RunArgs A) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < A.nwait) A.waiting[k] = A.nrun + k;
+  if (k < A.nrun + A.nwait) A.progress[k] = RunProgress{0, 0};
+  if (k == 0) { A.ticket[0] = 0; A.ticket[1] = (unsigned)A.nwait; }
 }
 
 // How nsys systems are run with gw lanes each: kernel and warps per block.
@@ -842,17 +910,6 @@ RunShape run_shape(int gw, bool additive, int nsys, int nsm) {
 }
 
 // ---------------------------------------------------------------- shared-memory kernel
-
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ void record_cost(const RunArgs& A, int s, unsigned long long t0) {
-  const unsigned long long c = (global_ns() - t0) >> 10;
-  A.cost[s] = c > 0xffffffffull ? 0xffffffffu : (uint32_t)c;
-}
 
 // where one system's engine state sits in a block's dynamic shared memory:
 // disk records, event slots, tree, cell coordinates and links, cell heads and
@@ -905,7 +962,6 @@ __global__ void __launch_bounds__(32) k_run_smem(const SysDev* __restrict__ sys,
     it = G.shfl(it, 0);
     if (it >= nlist) break;
     const int s = list[it];
-    const unsigned long long t0 = A.cost ? global_ns() : 0;
     const SysDev& S = sys[s];
     const SmemLayout Y = smem_layout(S);
     const size_t N = (size_t)S.B.N, E = 2 * N + NSPECIAL, C = (size_t)S.B.Nxc * S.B.Nyc;
@@ -925,7 +981,8 @@ __global__ void __launch_bounds__(32) k_run_smem(const SysDev* __restrict__ sys,
     warp_copy(L.head, S.head, C * 4, lane);
     warp_copy(L.on, S.on, E * 4, lane); warp_copy(L.op, S.op, E * 4, lane);
     G.sync();
-    run_system(L, A, A.max_coll, G, &wsm);
+    RunProgress pr{0, 0};
+    run_system(L, A, G, &wsm, pr, A.max_events);
     G.sync();
     warp_copy(S.d, L.d, N * sizeof(Disk), lane);
     warp_copy(S.ev, L.ev, E * sizeof(Ev), lane);
@@ -936,7 +993,6 @@ __global__ void __launch_bounds__(32) k_run_smem(const SysDev* __restrict__ sys,
     warp_copy(S.head, L.head, C * 4, lane);
     warp_copy(S.on, L.on, E * 4, lane); warp_copy(S.op, L.op, E * 4, lane);
     G.sync();
-    if (A.cost && lane == 0) record_cost(A, s, t0);
   }
 }
 
@@ -1473,8 +1529,8 @@ static int stage_all(edmd_ctx* ctx, const double* x, const double* y, const doub
   k_links<<<gd, 256, 0, sm>>>(ctx->ds);
   k_heads<<<gd, 256, 0, sm>>>(ctx->ds);
   CK(cudaGetLastError());
-  CK(init_queues(ctx->ds, nsys, ctx->maxN, ctx->engine != EDMD_ENGINE_LANE, sm));
-  if (ctx->engine == EDMD_ENGINE_LANE) CK(lane_build(ctx->ds, nsys, sm));
+  CK(init_queues(ctx->ds, nsys, ctx->maxN, !ctx->calendar, sm));
+  if (ctx->calendar) CK(lane_build(ctx->ds, nsys, sm));
   return report_status(ctx, "initial configuration");
 }
 
@@ -1534,16 +1590,17 @@ extern "C" int edmd_create(int32_t nsys, const edmd_system_desc* desc, const dou
   ctx->total_N = TN; ctx->total_C = TC;
   ctx->engine = g_engine;
   if (ctx->engine == EDMD_ENGINE_AUTO) {
-    // One thread per system issues each FP64 instruction for up to 32
-    // systems, but needs enough systems to hide its dependent loads: measured
-    // on GB300 (Hex starts at phi 0.55, 2000 collisions a call), the lane
-    // engine runs 2.9e7 / 5.2e7 / 9.3e7 / 1.6e8 coll/s at 4096 / 8192 /
-    // 16384 / 32768 systems of 256 disks against 7.5e7 / 7.5e7 / 8.4e7 /
-    // 8.5e7 for one warp per system (16384 systems of 1024 disks: 9.4e7
-    // against 7.6e7).  Its calendar costs ~2 KB per disk.
+    // Contexts of many small systems count as EDMD_ENGINE_LANE, but run the
+    // warp engine's event loop: measured on GB300 (300 collisions a call) it
+    // gives 1.65e8 / 1.55e8 / 1.31e8 coll/s on 16384 systems of 96 / 256 /
+    // 1024 disks against 1.10e8 / 1.07e8 / 1.00e8 for one thread per system,
+    // 1.75e8 against 1.62e8 on 32768 of 96 and 1.77e8 against 1.54e8 on 60000;
+    // and the thread loop's calendars cost 2 KB per disk.
     const bool many = nsys >= 16384 && 2 * (int64_t)ctx->maxN + NSPECIAL <= 65535 &&
                       TN * (int64_t)(CAL_SUB * CAL_LINE * 2 + 2) <= ((int64_t)32 << 30);
     ctx->engine = many ? EDMD_ENGINE_LANE : EDMD_ENGINE_WARP;
+  } else {
+    ctx->calendar = ctx->engine == EDMD_ENGINE_LANE;
   }
   if (ctx->engine == EDMD_ENGINE_LANE && 2 * (int64_t)ctx->maxN + NSPECIAL > 65535)
     return set_err(ctx, EDMD_ERR_ARG, "thread-per-system engine supports N <= 32766");
@@ -1559,14 +1616,11 @@ extern "C" int edmd_create(int32_t nsys, const edmd_system_desc* desc, const dou
   CK(dalloc(&ctx->st, nsys));
   CK(dalloc(&ctx->trace, (size_t)nsys * trace_cap));
   CK(dalloc(&ctx->rows, (size_t)nsys * rows_cap * 9));
-  CK(dalloc(&ctx->work, 1));
   CK(dalloc(&ctx->order, nsys));
-  CK(dalloc(&ctx->cost, nsys));
-  CK(cudaMemsetAsync(ctx->cost, 0, nsys * sizeof(uint32_t), ctx->stream));
   CK(dalloc(&ctx->ds, nsys));
   CK(dalloc(&ctx->doff, nsys));
   CK(dalloc(&ctx->bad, 1));
-  if (ctx->engine == EDMD_ENGINE_LANE) {
+  if (ctx->calendar) {
     CK(dalloc(&ctx->cal, (size_t)TN * CAL_SUB * CAL_LINE));
     CK(dalloc(&ctx->mask, (size_t)TN));
   }
@@ -1584,7 +1638,7 @@ extern "C" int edmd_create(int32_t nsys, const edmd_system_desc* desc, const dou
     S.trace_cap = trace_cap;
     S.rows = ctx->rows + (size_t)s * rows_cap * 9;
     S.rows_cap = rows_cap;
-    if (ctx->engine == EDMD_ENGINE_LANE) {
+    if (ctx->calendar) {
       S.cal = ctx->cal + (size_t)o * CAL_SUB * CAL_LINE;
       S.mask = ctx->mask + o;
       S.invw = CAL_SUB / S.B.dtP;
@@ -1603,16 +1657,37 @@ extern "C" int edmd_load_state(edmd_ctx* ctx, const double* x, const double* y, 
 
 // EDMD_F_SMEM: the systems whose engine state fits one block's shared memory
 // go to k_run_smem on a second stream, the others to k_run on the context's
-// stream (longest first by the previous call's run times, as without the
-// flag); both start after e0 and the context's stream waits for the second
+// stream; both start after e0 and the context's stream waits for the second
 // one before e1.
+// k_run on `nsys` places on the context's stream, with the tables of waiting
+// systems when they exceed the resident lane groups
+static int run_launch(edmd_ctx* ctx, RunArgs A, int nsys, int gw, int nsm) {
+  const RunShape shape = run_shape(gw, ctx->any_additive, nsys, nsm);
+  const int per_block = shape.warps * (32 / gw);
+  int per_sm = 0;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shape.kernel, 32 * shape.warps, 0));
+  const int grid = std::max(1, std::min(per_sm * nsm, (nsys + per_block - 1) / per_block));
+  A.nrun = std::min(nsys, grid * per_block);
+  A.nwait = nsys - A.nrun;
+  if (A.nwait) {
+    if (!ctx->waiting) {
+      CK(dalloc(&ctx->waiting, ctx->nsys)); CK(dalloc(&ctx->ticket, 2)); CK(dalloc(&ctx->progress, ctx->nsys));
+    }
+    A.waiting = ctx->waiting; A.ticket = ctx->ticket; A.progress = ctx->progress;
+    k_waiting<<<(nsys + 255) / 256, 256, 0, ctx->stream>>>(A);
+    ctx->last_launches++;
+  }
+  shape.kernel<<<grid, 32 * shape.warps, 0, ctx->stream>>>(ctx->ds, A);
+  CK(cudaGetLastError());
+  ctx->last_launches++;
+  return EDMD_OK;
+}
+
 static int advance_smem_split(edmd_ctx* ctx, RunArgs A, int nsm) {
   int dev = 0, optin = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const size_t limit = (size_t)optin - sizeof(WarpSmem) - 1024;
-  std::vector<uint32_t> cost(ctx->nsys);
-  CK(sync_copy(ctx, cost.data(), ctx->cost, ctx->nsys * sizeof(uint32_t), cudaMemcpyDeviceToHost));
   std::vector<int32_t> fit, rest;
   size_t need = 0;
   for (int s = 0; s < ctx->nsys; s++) {
@@ -1620,11 +1695,6 @@ static int advance_smem_split(edmd_ctx* ctx, RunArgs A, int nsm) {
     if (b <= limit) { fit.push_back(s); need = b > need ? b : need; }
     else rest.push_back(s);
   }
-  auto longest_first = [&](std::vector<int32_t>& v) {
-    std::stable_sort(v.begin(), v.end(), [&](int32_t a, int32_t b) { return cost[a] > cost[b]; });
-  };
-  longest_first(fit);
-  longest_first(rest);
   if (!ctx->smem_list) {
     CK(dalloc(&ctx->smem_list, ctx->nsys));
     CK(dalloc(&ctx->smem_work, 1));
@@ -1654,15 +1724,9 @@ static int advance_smem_split(edmd_ctx* ctx, RunArgs A, int nsm) {
   }
   if (!rest.empty()) {
     RunArgs B = A;
-    B.nsys = (int32_t)rest.size();
     B.order = ctx->order;
-    const RunShape shape = run_shape(32, ctx->any_additive, (int)rest.size(), nsm);
-    int per_sm = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shape.kernel, 32 * shape.warps, 0));
-    const int grid = std::max(1, std::min(((int)rest.size() + shape.warps - 1) / shape.warps, per_sm * nsm));
-    shape.kernel<<<grid, 32 * shape.warps, 0, ctx->stream>>>(ctx->ds, B);
-    CK(cudaGetLastError());
-    ctx->last_launches++;
+    const int rc = run_launch(ctx, B, (int)rest.size(), 32, nsm);
+    if (rc) return rc;
   }
   if (!fit.empty()) CK(cudaStreamWaitEvent(ctx->stream, ctx->e2, 0));
   return EDMD_OK;
@@ -1676,51 +1740,27 @@ extern "C" int edmd_advance(edmd_ctx* ctx, int64_t max_coll, double t_stop, uint
     return set_err(ctx, EDMD_ERR_ARG, "advanced by the round engine: reload the state with edmd_load_state");
   RunArgs A;
   A.max_coll = max_coll; A.t_stop = t_stop; A.flags = flags; A.max_events = max_events;
-  A.nsys = ctx->nsys; A.work = ctx->work;
-  A.order = nullptr; A.cost = ctx->cost;
-  if (ctx->engine == EDMD_ENGINE_LANE) {
+  A.nsys = ctx->nsys;
+  A.order = nullptr; A.waiting = nullptr; A.ticket = nullptr; A.progress = nullptr;
+  A.nwait = 0; A.nrun = ctx->nsys;
+  ctx->last_launches = 0;
+  if (ctx->calendar) {
     CK(cudaEventRecord(ctx->e0, ctx->stream));
     CK(lane_run_launch(ctx->ds, A, g_lane_threads, ctx->stream));
     ctx->last_launches = 1;
   } else {
-    CK(cudaMemsetAsync(ctx->work, 0, sizeof(int32_t), ctx->stream));
     int dev = 0, nsm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    int per_sm = 0;
-    const int gw = g_group;                     // lanes per system: 4, 8, 16 or 32
-    const RunShape shape = run_shape(gw, ctx->any_additive, ctx->nsys, nsm);
-    const int per_block = shape.warps * (32 / gw);
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shape.kernel, 32 * shape.warps, 0));
-    int want = (ctx->nsys + per_block - 1) / per_block;
-    int grid = per_sm * nsm;
-    if (grid > want) grid = want;
-    if (grid < 1) grid = 1;
-    const int64_t resident = (int64_t)grid * per_block;
-    if (ctx->nsys > resident) {
-      // more systems than resident warps: the systems that took longest in
-      // the previous call start first (longest processing time first), so the
-      // last wave holds the short ones and the launch ends with fewer idle
-      // warps; ties keep index order, and the first call runs in index order
-      std::vector<uint32_t> cost(ctx->nsys);
-      CK(sync_copy(ctx, cost.data(), ctx->cost, ctx->nsys * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-      std::vector<int32_t>& ord = ctx->order_h;
-      ord.resize(ctx->nsys);
-      for (int s = 0; s < ctx->nsys; s++) ord[s] = s;
-      std::stable_sort(ord.begin(), ord.end(), [&](int32_t a, int32_t b) { return cost[a] > cost[b]; });
-      CK(cudaMemcpyAsync(ctx->order, ord.data(), ctx->nsys * sizeof(int32_t), cudaMemcpyHostToDevice,
-                         ctx->stream));
-      A.order = ctx->order;
-    }
-    ctx->last_launches = 0;
-    if ((flags & EDMD_F_SMEM) && gw == 32) {
-      int rc = advance_smem_split(ctx, A, nsm);
-      if (rc) return rc;
+    const int gw = ctx->engine == EDMD_ENGINE_LANE ? 32 : g_group;     // lanes per system: 4, 8, 16 or 32
+    int rc;
+    if ((flags & EDMD_F_SMEM) && gw == 32 && ctx->engine == EDMD_ENGINE_WARP) {
+      rc = advance_smem_split(ctx, A, nsm);
     } else {
-    ctx->last_launches = 1;
-    CK(cudaEventRecord(ctx->e0, ctx->stream));
-    shape.kernel<<<grid, 32 * shape.warps, 0, ctx->stream>>>(ctx->ds, A);
+      CK(cudaEventRecord(ctx->e0, ctx->stream));
+      rc = run_launch(ctx, A, ctx->nsys, gw, nsm);
     }
+    if (rc) return rc;
   }
   CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->e1, ctx->stream));
@@ -1860,7 +1900,7 @@ extern "C" int edmd_destroy(edmd_ctx* ctx) {
   round_free(ctx);
   void* ptrs[] = {ctx->d, ctx->vr, ctx->cx, ctx->cy, ctx->prv, ctx->crossX, ctx->crossY, ctx->head,
                   ctx->ev, ctx->on, ctx->op, ctx->tree, ctx->st, ctx->trace, ctx->rows, ctx->stage,
-                  ctx->work, ctx->order, ctx->cost, ctx->ds, ctx->doff, ctx->bad, ctx->cal, ctx->mask};
+                  ctx->order, ctx->waiting, ctx->ticket, ctx->progress, ctx->ds, ctx->doff, ctx->bad, ctx->cal, ctx->mask};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (void* p : ctx->ckpt)
@@ -2064,13 +2104,12 @@ extern "C" int edmd_run_noalloc(const edmd_system_desc* desc, double* x, double*
   const int64_t per_coll = max_coll > cap / NOALLOC_EVENTS_PER_COLL ? cap : max_coll * NOALLOC_EVENTS_PER_COLL;
   const int64_t budget = std::min(cap, per_coll + (int64_t)N * NOALLOC_EVENTS_PER_DISK + NOALLOC_EVENTS_BASE);
   A.max_coll = max_coll; A.t_stop = t_stop; A.flags = 0; A.max_events = budget;
-  A.nsys = 1; A.work = work; A.order = nullptr; A.cost = nullptr;
+  A.nsys = 1; A.order = nullptr; A.waiting = nullptr; A.ticket = nullptr; A.progress = nullptr;
+  A.nwait = 0; A.nrun = 1;
   k_noalloc_put<<<1, 1, 0, st>>>(S, dsys);
   k_noalloc_stage<<<1, 32, 0, st>>>(dsys, x, y, vx, vy, rad, m, D.first_screen, D.first_thermo);
   if (cudaError_t qe = init_queues(dsys, 1, N, true, st); qe != cudaSuccess)
     return noalloc_fail(EDMD_ERR_CUDA, cudaGetErrorString(qe));
-  if (cudaMemsetAsync(work, 0, sizeof(int32_t), st) != cudaSuccess)
-    return noalloc_fail(EDMD_ERR_CUDA, "edmd_run_noalloc: memset failed");
   const RunShape shape = run_shape(32, B.additive != 0, 1, 1);
   shape.kernel<<<1, 32 * shape.warps, 0, st>>>(dsys, A);
   k_sync<<<dim3((N + 255) / 256, 1), 256, 0, st>>>(dsys);

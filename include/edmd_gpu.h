@@ -46,10 +46,11 @@ extern "C" {
 #define EDMD_STOP_GROW      5   /* stopped right after the growth stop        */
 
 /* engines (edmd_set_engine) */
-#define EDMD_ENGINE_AUTO    0   /* the thread-per-system engine for contexts of at
-                                   least 16384 systems of N <= 32766 (faster there),
-                                   else the warp engine; the differentiation calls
-                                   need EDMD_ENGINE_WARP */
+#define EDMD_ENGINE_AUTO    0   /* EDMD_ENGINE_LANE for contexts of at least 16384
+                                   systems of N <= 32766, else EDMD_ENGINE_WARP; both
+                                   then run the warp engine's event loop, the faster
+                                   one at every size measured.  The differentiation
+                                   calls need EDMD_ENGINE_WARP */
 #define EDMD_ENGINE_WARP    1   /* one warp per system: single large systems  */
 #define EDMD_ENGINE_LANE    2   /* one thread per system: large batches, N <= 32766 */
 
