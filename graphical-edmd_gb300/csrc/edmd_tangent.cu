@@ -27,47 +27,87 @@ namespace {
 
 // ---------------------------------------------------------------- tangent kernels
 
+// A collision of the log with what its maps need beside it, 32 at a time in
+// shared memory: the masses and the quotient come for all 32 in one pass, so
+// the chain from collision to collision waits for none of them.
+struct Coll {
+  double t, dx, dy, dvx, dvy, f, mi, mj, rv, frv;
+  int32_t i, j;
+};
+__device__ __forceinline__ Coll coll_of(const edmd_log_entry& L, const Disk* __restrict__ d) {
+  Coll c;
+  c.i = L.i; c.j = L.j; c.t = L.t;
+  c.dx = L.dx; c.dy = L.dy; c.dvx = L.dvx; c.dvy = L.dvy; c.f = L.f;
+  c.mi = d[L.i].m; c.mj = d[L.j].m;
+  c.rv = L.dx * L.dvx + L.dy * L.dvy;
+  c.frv = div_rn(L.f, c.rv);
+  return c;
+}
+
 // T is row-major [4N][K]: row 4i+c holds component c (dx, dy, dvx, dvy) of disk
 // i for the K tangent vectors, so lane k of a warp reads one coalesced row.
+// One warp, bound by the chain from collision to collision: the rows of the
+// next collision are loaded while this one is computed, unless they share a
+// disk.  1024 disks, 32 vectors: 3.1 -> 1.2 us a collision.
 __device__ __forceinline__ void tangent_apply_warp(const edmd_log_entry* __restrict__ log, int64_t M,
-                                                   const Disk* __restrict__ d, double* __restrict__ T,
-                                                   double* __restrict__ tl, int K, int k) {
-  for (int64_t n = 0; n < M; n++) {
-    const edmd_log_entry L = log[n];
-    const int i = L.i, j = L.j;
-    const double mi = d[i].m, mj = d[j].m;
-    const double ti = tl[i], tj = tl[j];
-    double* Ri = T + (size_t)4 * i * K;
-    double* Rj = T + (size_t)4 * j * K;
-    if (k < K) {
-      double xi = Ri[k], yi = Ri[K + k], vxi = Ri[2 * K + k], vyi = Ri[3 * K + k];
-      double xj = Rj[k], yj = Rj[K + k], vxj = Rj[2 * K + k], vyj = Rj[3 * K + k];
-      // free flight to the collision
-      xi += vxi * (L.t - ti); yi += vyi * (L.t - ti);
-      xj += vxj * (L.t - tj); yj += vyj * (L.t - tj);
-      const double rv = L.dx * L.dvx + L.dy * L.dvy;
-      const double drx = xj - xi, dry = yj - yi, dvx = vxj - vxi, dvy = vyj - vyi;
-      const double dtc = -(L.dx * drx + L.dy * dry) / rv;
-      const double rcx = drx + L.dvx * dtc, rcy = dry + L.dvy * dtc;
-      const double df = (L.f / rv) * (L.dvx * rcx + L.dvy * rcy + L.dx * dvx + L.dy * dvy);
-      const double wx = df * L.dx + L.f * rcx, wy = df * L.dy + L.f * rcy;
-      const double Dvix = L.f * mj * L.dx, Dviy = L.f * mj * L.dy;
-      const double Dvjx = -L.f * mi * L.dx, Dvjy = -L.f * mi * L.dy;
-      Ri[k] = xi - Dvix * dtc;       Ri[K + k] = yi - Dviy * dtc;
-      Rj[k] = xj - Dvjx * dtc;       Rj[K + k] = yj - Dvjy * dtc;
-      Ri[2 * K + k] = vxi + mj * wx; Ri[3 * K + k] = vyi + mj * wy;
-      Rj[2 * K + k] = vxj - mi * wx; Rj[3 * K + k] = vyj - mi * wy;
+                                                   const Disk* __restrict__ d, double* T, double* tl, int K, int k,
+                                                   Coll* tile) {
+  const bool on = k < K;
+  double xi = 0, yi = 0, vxi = 0, vyi = 0, xj = 0, yj = 0, vxj = 0, vyj = 0, ti = 0, tj = 0;
+  auto load = [&](int i, double& x, double& y, double& vx, double& vy, double& t) {
+    const double* R = T + (size_t)4 * i * K + k;
+    if (on) { x = R[0]; y = R[K]; vx = R[2 * K]; vy = R[3 * K]; }
+    t = tl[i];
+  };
+  for (int64_t n0 = 0; n0 < M; n0 += 32) {
+    __syncwarp();
+    if (n0 + k < M) tile[k] = coll_of(log[n0 + k], d);
+    __syncwarp();
+    const int cnt = (int)(M - n0 < 32 ? M - n0 : 32);
+    load(tile[0].i, xi, yi, vxi, vyi, ti);
+    load(tile[0].j, xj, yj, vxj, vyj, tj);
+    for (int n = 0; n < cnt; n++) {
+      const Coll& L = tile[n];
+      const int i = L.i, j = L.j;
+      const int ni = n + 1 < cnt ? tile[n + 1].i : -1, nj = n + 1 < cnt ? tile[n + 1].j : -1;
+      const bool si = ni == i || ni == j, sj = nj == i || nj == j;      // written below
+      double axi = 0, ayi = 0, avxi = 0, avyi = 0, axj = 0, ayj = 0, avxj = 0, avyj = 0, ati = 0, atj = 0;
+      if (ni >= 0 && !si) load(ni, axi, ayi, avxi, avyi, ati);
+      if (nj >= 0 && !sj) load(nj, axj, ayj, avxj, avyj, atj);
+      {
+        double* Ri = T + (size_t)4 * i * K + k;
+        double* Rj = T + (size_t)4 * j * K + k;
+        // free flight to the collision
+        xi += vxi * (L.t - ti); yi += vyi * (L.t - ti);
+        xj += vxj * (L.t - tj); yj += vyj * (L.t - tj);
+        const double drx = xj - xi, dry = yj - yi, dvx = vxj - vxi, dvy = vyj - vyi;
+        const double dtc = div_rn(-(L.dx * drx + L.dy * dry), L.rv);
+        const double rcx = drx + L.dvx * dtc, rcy = dry + L.dvy * dtc;
+        const double df = L.frv * (L.dvx * rcx + L.dvy * rcy + L.dx * dvx + L.dy * dvy);
+        const double wx = df * L.dx + L.f * rcx, wy = df * L.dy + L.f * rcy;
+        const double Dvix = L.f * L.mj * L.dx, Dviy = L.f * L.mj * L.dy;
+        const double Dvjx = -L.f * L.mi * L.dx, Dvjy = -L.f * L.mi * L.dy;
+        if (on) {
+          Ri[0] = xi - Dvix * dtc;           Ri[K] = yi - Dviy * dtc;
+          Rj[0] = xj - Dvjx * dtc;           Rj[K] = yj - Dvjy * dtc;
+          Ri[2 * K] = vxi + L.mj * wx;       Ri[3 * K] = vyi + L.mj * wy;
+          Rj[2 * K] = vxj - L.mi * wx;       Rj[3 * K] = vyj - L.mi * wy;
+        }
+      }
+      if (k == 0) { tl[i] = L.t; tl[j] = L.t; }
+      __syncwarp();
+      if (si) load(ni, axi, ayi, avxi, avyi, ati);
+      if (sj) load(nj, axj, ayj, avxj, avyj, atj);
+      xi = axi; yi = ayi; vxi = avxi; vyi = avyi; ti = ati;
+      xj = axj; yj = ayj; vxj = avxj; vyj = avyj; tj = atj;
     }
-    __syncwarp();
-    if (k == 0) { tl[i] = L.t; tl[j] = L.t; }
-    __syncwarp();
   }
 }
 
-__global__ void k_tangent_apply(const edmd_log_entry* __restrict__ log, int64_t M,
-                                const Disk* __restrict__ d, double* __restrict__ T,
-                                double* __restrict__ tl, int K) {
-  tangent_apply_warp(log, M, d, T, tl, K, threadIdx.x);
+__global__ void __launch_bounds__(32) k_tangent_apply(const edmd_log_entry* __restrict__ log, int64_t M,
+                                                      const Disk* __restrict__ d, double* T, double* tl, int K) {
+  __shared__ Coll tile[32];
+  tangent_apply_warp(log, M, d, T, tl, K, threadIdx.x, tile);
 }
 
 // value of row e at the common time tq (virtual free flight, T itself unchanged)
@@ -153,76 +193,98 @@ __global__ void __launch_bounds__(32) k_chol(const double* __restrict__ G, int K
   chol_warp(G, K, Rinv, logdiag, accumulate, fail, M, Q, threadIdx.x);
 }
 
-// T <- T' Rinv at the common time tq (every disk's tangent clock set to tq)
-__device__ __forceinline__ void apply_rinv_disk(double* __restrict__ T, double* __restrict__ tl, int i, int K,
-                                                double tq, const double* __restrict__ Rinv) {
-  double row[4][32];
-  for (int c = 0; c < 4; c++)
-    for (int k = 0; k < K; k++) row[c][k] = row_at(T, tl, 4 * i + c, k, K, tq);
-  for (int c = 0; c < 4; c++)
-    for (int k = 0; k < K; k++) {
-      double s = 0;
-      for (int l = 0; l <= k; l++) s += row[c][l] * Rinv[l * K + k];
-      T[(size_t)(4 * i + c) * K + k] = s;
-    }
-  tl[i] = tq;
+// T <- T' Rinv at the common time tq (every disk's tangent clock set to tq), one
+// thread per row: its K values in registers (KM: their number rounded up), Rinv
+// from shared memory, column k the sum over l <= k in order.  FP64 issue bounds
+// it, so the lanes are 32 rows and the sums stop at the triangle.  (One thread
+// per disk kept 128 values in local memory, and 1024 disks gave eight blocks:
+// 200 us a pass, 22 so.)
+constexpr int RINV_THREADS = 128;               // rows per block: whole disks to a warp
+template <int KM>
+__device__ __forceinline__ void apply_rinv_rows(double* T, double* tl, int N, int e, int K, double tq,
+                                                const double* __restrict__ Rinv) {
+  __shared__ double Rs[KM][KM];
+  for (int q = threadIdx.x; q < KM * KM; q += RINV_THREADS)
+    Rs[q / KM][q % KM] = q / KM < K && q % KM < K ? Rinv[(q / KM) * K + q % KM] : 0.0;
+  __syncthreads();
+  const bool on = e < 4 * N;
+  double v[KM];
+#pragma unroll
+  for (int k = 0; k < KM; k++) v[k] = on && k < K ? row_at(T, tl, e, k, K, tq) : 0.0;
+  __syncwarp();                                 // the disk's rows are read
+#pragma unroll
+  for (int k = 0; k < KM; k++) {
+    double s = 0;
+#pragma unroll
+    for (int l = 0; l <= k; l++) s += v[l] * Rs[l][k];
+    if (on && k < K) T[(size_t)e * K + k] = s;
+  }
+  if (on && (e & 3) == 0) tl[e >> 2] = tq;
 }
 
-__global__ void k_apply_rinv(double* __restrict__ T, double* __restrict__ tl, int N, int K,
-                             const double* __restrict__ tqp, const double* __restrict__ Rinv) {
-  const double tq = *tqp;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  apply_rinv_disk(T, tl, i, K, tq, Rinv);
+template <int KM>
+__global__ void __launch_bounds__(RINV_THREADS) k_apply_rinv(double* T, double* tl, int N, int K,
+                                                             const double* __restrict__ tqp,
+                                                             const double* __restrict__ Rinv) {
+  apply_rinv_rows<KM>(T, tl, N, blockIdx.x * RINV_THREADS + threadIdx.x, K, *tqp, Rinv);
 }
 
 // ---------------------------------------------------------------- adjoint kernels
 
-// one thread: sweep a segment of the log backwards, applying the transpose of
-// the collision map and of the free flights between collisions.
-// A is [N][4]: (g_x, g_y, g_vx, g_vy) of each disk at its time ta[i].
-__device__ void adjoint_segment(const edmd_log_entry* __restrict__ log, int64_t M,
-                                const Disk* __restrict__ d, double* __restrict__ A,
-                                double* __restrict__ ta) {
-  for (int64_t n = M - 1; n >= 0; n--) {
-    const edmd_log_entry L = log[n];
-    const int i = L.i, j = L.j;
-    const double mi = d[i].m, mj = d[j].m;
-    double* ai = A + 4 * (size_t)i;
-    double* aj = A + 4 * (size_t)j;
-    // transpose of the free flights from the collision to each disk's adjoint time
-    double gxi = ai[0], gyi = ai[1], gvxi = ai[2] + ai[0] * (ta[i] - L.t), gvyi = ai[3] + ai[1] * (ta[i] - L.t);
-    double gxj = aj[0], gyj = aj[1], gvxj = aj[2] + aj[0] * (ta[j] - L.t), gvyj = aj[3] + aj[1] * (ta[j] - L.t);
-    const double rv = L.dx * L.dvx + L.dy * L.dvy;
-    const double Dvix = L.f * mj * L.dx, Dviy = L.f * mj * L.dy;
-    const double Dvjx = -L.f * mi * L.dx, Dvjy = -L.f * mi * L.dy;
-    // w enters dv_i' with +m_j and dv_j' with -m_i
-    const double gwx = mj * gvxi - mi * gvxj, gwy = mj * gvyi - mi * gvyj;
-    // dt_c enters the positions through -Dv dt_c
-    double gdt = -(Dvix * gxi + Dviy * gyi) - (Dvjx * gxj + Dvjy * gyj);
-    // w = df r + f drc
-    const double gdf = L.dx * gwx + L.dy * gwy;
-    double grcx = L.f * gwx, grcy = L.f * gwy;
-    // df = (f/rv) (v . drc + r . dv_ij)
-    const double s = (L.f / rv) * gdf;
-    grcx += s * L.dvx; grcy += s * L.dvy;
-    const double gdvx = s * L.dx, gdvy = s * L.dy;
-    // drc = dr_ij + v dt_c
-    gdt += L.dvx * grcx + L.dvy * grcy;
-    // dt_c = -(r . dr_ij)/rv
-    const double grx = grcx - (gdt / rv) * L.dx, gry = grcy - (gdt / rv) * L.dy;
-    // dr_ij = dr_j - dr_i, dv_ij = dv_j - dv_i
-    ai[0] = gxi - grx; ai[1] = gyi - gry; ai[2] = gvxi - gdvx; ai[3] = gvyi - gdvy;
-    aj[0] = gxj + grx; aj[1] = gyj + gry; aj[2] = gvxj + gdvx; aj[3] = gvyj + gdvy;
-    ta[i] = L.t; ta[j] = L.t;
+// One warp sweeps a log backwards, applying the transpose of the collision map
+// and of the free flights between collisions.  A is [N][4]: (g_x, g_y, g_vx,
+// g_vy) of each disk at its time ta[i].  Lanes hold the disk `lane & 1` and the
+// axis `lane & 2` of a collision, so its chain of FP64 operations is one axis
+// of one disk; masses and quotients come 32 collisions at a time.  (One thread
+// per system: 3.5 us a collision; so 0.9.)
+__device__ __forceinline__ void adjoint_warp(const edmd_log_entry* __restrict__ log, int64_t M,
+                                             const Disk* __restrict__ d, double* A, double* ta, int lane, Coll* tile) {
+  const bool odd = lane & 1, y = lane & 2;
+  auto over_axes = [](double v) { return v + __shfl_xor_sync(0xffffffffu, v, 2); };
+  for (int64_t n1 = M; n1 > 0; n1 -= 32) {
+    const int cnt = (int)(n1 < 32 ? n1 : 32);
+    __syncwarp();
+    if (lane < cnt) tile[lane] = coll_of(log[n1 - 1 - lane], d);
+    __syncwarp();
+    for (int n = 0; n < cnt; n++) {
+      const Coll& L = tile[n];
+      const int me = odd ? L.j : L.i;
+      const double r = y ? L.dy : L.dx, v = y ? L.dvy : L.dvx, mo = odd ? L.mi : L.mj;
+      double* a = A + 4 * (size_t)me + (y ? 1 : 0);
+      const double g = a[0];
+      // transpose of the free flight from the collision to the disk's adjoint time
+      const double gv = a[2] + g * (ta[me] - L.t);
+      // w enters dv_i' with +m_j and dv_j' with -m_i
+      const double pw = mo * gv, po = __shfl_xor_sync(0xffffffffu, pw, 1);
+      const double gw = odd ? po - pw : pw - po;
+      // dt_c enters the positions through -Dv dt_c
+      const double D = (odd ? -L.f : L.f) * mo * r;
+      const double q = over_axes(D * g), qo = __shfl_xor_sync(0xffffffffu, q, 1);
+      double gdt = -(odd ? qo : q) - (odd ? q : qo);
+      // w = df r + f drc, df = (f/rv) (v . drc + r . dv_ij)
+      const double gdf = over_axes(r * gw);
+      const double s = L.frv * gdf;
+      const double grc = L.f * gw + s * v;
+      const double gdv = s * r;
+      // drc = dr_ij + v dt_c, dt_c = -(r . dr_ij)/rv
+      gdt += over_axes(v * grc);
+      const double gr = grc - div_rn(gdt, L.rv) * r;
+      // dr_ij = dr_j - dr_i, dv_ij = dv_j - dv_i
+      __syncwarp();
+      if (lane < 4) {
+        a[0] = g + flip(gr, !odd);
+        a[2] = gv + flip(gdv, !odd);
+        if (!y) ta[me] = L.t;
+      }
+      __syncwarp();
+    }
   }
 }
 
-__global__ void k_adjoint_segment(const edmd_log_entry* __restrict__ log, int64_t M,
-                                  const Disk* __restrict__ d, double* __restrict__ A,
-                                  double* __restrict__ ta) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  adjoint_segment(log, M, d, A, ta);
+__global__ void __launch_bounds__(32) k_adjoint(const edmd_log_entry* __restrict__ log, int64_t M,
+                                                const Disk* __restrict__ d, double* A, double* ta) {
+  __shared__ Coll tile[32];
+  adjoint_warp(log, M, d, A, ta, threadIdx.x, tile);
 }
 
 // every disk's adjoint brought back to t0 (transpose of the first free flight)
@@ -257,21 +319,31 @@ __global__ void k_fill_sys_time(const SysDev* __restrict__ sys, const int32_t* _
   if (g < TN) tl[g] = sys[dsys[g]].st->t;
 }
 
-// one warp per system: the tangent map over the system's collision log
-__global__ void k_tangent_apply_b(const SysDev* __restrict__ sys, const int64_t* __restrict__ doff,
-                                  double* __restrict__ T, double* __restrict__ tl, int K) {
+// one warp per system: the tangent map over its collisions logged from entry
+// `from` to the chunk's end, nend[s]
+__global__ void __launch_bounds__(32) k_tangent_apply_b(const SysDev* __restrict__ sys, const int64_t* __restrict__ doff,
+                                                        double* T, double* tl, int K, int64_t from,
+                                                        const uint64_t* __restrict__ nend) {
+  __shared__ Coll tile[32];
   const SysDev& S = sys[blockIdx.x];
-  int64_t M = (int64_t)S.st->nlog;
-  if (M > S.log_cap) M = S.log_cap;
+  int64_t end = (int64_t)nend[blockIdx.x];
+  if (end > S.log_cap) end = S.log_cap;
   const int64_t o = doff[blockIdx.x];
-  tangent_apply_warp((const edmd_log_entry*)S.log, M, S.d, T + (size_t)4 * o * K, tl + o, K, threadIdx.x);
+  tangent_apply_warp((const edmd_log_entry*)S.log + from, end - from, S.d, T + (size_t)4 * o * K, tl + o, K, threadIdx.x,
+                     tile);
 }
 
-// one block of 32 x 32 threads per system: its Gram matrix at its current
-// time, rows taken 32 at a time in index order (deterministic)
-__global__ void k_gram_b(const SysDev* __restrict__ sys, const int64_t* __restrict__ doff,
-                         const double* __restrict__ T, const double* __restrict__ tl, int K,
-                         const double* __restrict__ tqs, double* __restrict__ G) {
+constexpr int GRAM_WARPS = 17;                  // warps of the 528 pairs of 32 columns
+constexpr int GRAM_LOADS = 8;                   // elements of 32 rows a thread fetches: at least 4 K threads a block
+
+// The Gram matrix of each system at its time tqs[s], one pair (k <= l) of
+// columns per lane, the K (K + 1) / 2 pairs spread over the warps of gridDim.y
+// blocks (deterministic: every pair sums its rows in index order).  FP64 issue
+// bounds it: a warp per column left half its lanes idle and issued 32 columns'
+// instructions for 16 (128 systems of 448 disks, 16 vectors: 665 us).
+__global__ void __launch_bounds__(GRAM_WARPS * 32)
+k_gram_b(const SysDev* __restrict__ sys, const int64_t* __restrict__ doff, const double* __restrict__ T,
+         const double* __restrict__ tl, int K, const double* __restrict__ tqs, double* __restrict__ G) {
   __shared__ double rows[32][33];
   const SysDev& S = sys[blockIdx.x];
   const int N = S.B.N;
@@ -279,17 +351,44 @@ __global__ void k_gram_b(const SysDev* __restrict__ sys, const int64_t* __restri
   const int64_t o = doff[blockIdx.x];
   const double* Ts = T + (size_t)4 * o * K;
   const double* tls = tl + o;
-  const int k = threadIdx.x & 31, l = threadIdx.x >> 5;
+  const int p = blockIdx.y * blockDim.x + threadIdx.x, pairs = K * (K + 1) / 2;
+  // pair p: l from the triangular root, k = p - l (l + 1) / 2
+  int l = 0;
+  while (l < K && (l + 1) * (l + 2) / 2 <= p) l++;
+  const int k = p - l * (l + 1) / 2;
+  const bool on = p < pairs;
   double acc = 0;
+  // the next 32 rows are on their way while this thread's pair is summed: up
+  // to GRAM_LOADS elements a thread, as (value, velocity row, time) still to be
+  // flown to tq
+  double x[GRAM_LOADS], v[GRAM_LOADS], t[GRAM_LOADS];
+  auto fetch = [&](int e0) {
+#pragma unroll
+    for (int u = 0; u < GRAM_LOADS; u++) {
+      const int q = threadIdx.x + u * blockDim.x, e = e0 + q / K, c = q % K;
+      x[u] = v[u] = 0;
+      t[u] = tq;
+      if (q < 32 * K && e < 4 * N) {
+        x[u] = Ts[(size_t)e * K + c];
+        if ((e & 3) < 2) { v[u] = Ts[(size_t)(e + 2) * K + c]; t[u] = tls[e >> 2]; }
+      }
+    }
+  };
+  fetch(0);
   for (int e0 = 0; e0 < 4 * N; e0 += 32) {
-    const int e = e0 + l;
-    rows[l][k] = (e < 4 * N && k < K) ? row_at(Ts, tls, e, k, K, tq) : 0.0;
+#pragma unroll
+    for (int u = 0; u < GRAM_LOADS; u++) {
+      const int q = threadIdx.x + u * blockDim.x, r = q / K;
+      if (q < 32 * K) rows[r][q % K] = (r & 3) < 2 ? x[u] + v[u] * (tq - t[u]) : x[u];
+    }
     __syncthreads();
-    if (k <= l && l < K)                            // the upper triangle; G is symmetric
+    fetch(e0 + 32);
+    if (on)
+#pragma unroll 8
       for (int r = 0; r < 32; r++) acc += rows[r][k] * rows[r][l];
     __syncthreads();
   }
-  if (k <= l && l < K) {
+  if (on) {
     G[(size_t)blockIdx.x * K * K + k * K + l] = acc;
     G[(size_t)blockIdx.x * K * K + l * K + k] = acc;
   }
@@ -306,25 +405,27 @@ __global__ void __launch_bounds__(32) k_chol_b(const double* __restrict__ G, int
             M, Q, threadIdx.x);
 }
 
-__global__ void k_apply_rinv_b(const int64_t* __restrict__ doff, const int32_t* __restrict__ dsys, int64_t TN,
-                               double* __restrict__ T, double* __restrict__ tl, int K,
-                               const double* __restrict__ tqs, const double* __restrict__ Rinv) {
-  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= TN) return;
-  const int s = dsys[g];
+template <int KM>
+__global__ void __launch_bounds__(RINV_THREADS) k_apply_rinv_b(const SysDev* __restrict__ sys,
+                                                               const int64_t* __restrict__ doff, double* T, double* tl,
+                                                               int K, const double* __restrict__ tqs,
+                                                               const double* __restrict__ Rinv) {
+  const int s = blockIdx.y, N = sys[s].B.N;
+  if ((int)blockIdx.x * RINV_THREADS >= 4 * N) return;
   const int64_t o = doff[s];
-  apply_rinv_disk(T + (size_t)4 * o * K, tl + o, (int)(g - o), K, tqs[s], Rinv + (size_t)s * K * K);
+  apply_rinv_rows<KM>(T + (size_t)4 * o * K, tl + o, N, blockIdx.x * RINV_THREADS + threadIdx.x, K, tqs[s],
+                      Rinv + (size_t)s * K * K);
 }
 
-// one thread per system: the transposed map backwards over its segment log
-__global__ void k_adjoint_segment_b(const SysDev* __restrict__ sys, const int64_t* __restrict__ doff, int nsys,
-                                    double* __restrict__ A, double* __restrict__ ta) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsys) return;
-  const SysDev& S = sys[s];
+// one warp per system: the transposed map backwards over its log
+__global__ void __launch_bounds__(32) k_adjoint_b(const SysDev* __restrict__ sys, const int64_t* __restrict__ doff,
+                                                  double* A, double* ta) {
+  __shared__ Coll tile[32];
+  const SysDev& S = sys[blockIdx.x];
   int64_t M = (int64_t)S.st->nlog;
   if (M > S.log_cap) M = S.log_cap;
-  adjoint_segment((const edmd_log_entry*)S.log, M, S.d, A + 4 * (size_t)doff[s], ta + doff[s]);
+  adjoint_warp((const edmd_log_entry*)S.log, M, S.d, A + 4 * (size_t)doff[blockIdx.x], ta + doff[blockIdx.x], threadIdx.x,
+               tile);
 }
 
 // every disk's position flown (virtually) to its system's current time
@@ -404,9 +505,29 @@ __global__ void k_adjoint_finish_b(const int32_t* __restrict__ dsys, int64_t TN,
   A[4 * g + 3] += A[4 * g + 1] * (ta[g] - t);
 }
 
-__global__ void k_sys_times(const SysDev* __restrict__ sys, int nsys, double* __restrict__ t) {
+__global__ void k_sys_times(const SysDev* __restrict__ sys, int nsys, double* __restrict__ t,
+                            uint64_t* __restrict__ nend) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < nsys) t[s] = sys[s].st->t;
+  if (s >= nsys) return;
+  t[s] = sys[s].st->t;
+  if (nend) nend[s] = sys[s].st->nlog;
+}
+
+// a chunk logged from entry `from` on moves to the front of each log, where
+// edmd_get_log reads it
+__global__ void k_log_front(const SysDev* __restrict__ sys, int64_t from) {
+  const SysDev& S = sys[blockIdx.x];
+  edmd_log_entry* log = (edmd_log_entry*)S.log;
+  const int64_t end = (int64_t)S.st->nlog < S.log_cap ? (int64_t)S.st->nlog : S.log_cap;
+  for (int64_t e = from + threadIdx.x; e < end; e += blockDim.x) log[e - from] = log[e];
+  __syncthreads();
+  if (threadIdx.x == 0) S.st->nlog -= (uint64_t)from;
+}
+
+// every system's log written from entry n (or its saved length) on
+__global__ void k_set_log(const SysDev* __restrict__ sys, int nsys, uint64_t n, const uint64_t* __restrict__ saved) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s < nsys) sys[s].st->nlog = saved ? saved[s] : n;
 }
 
 // positions of one system flown (virtually) to time t, without touching the state
@@ -435,6 +556,8 @@ extern "C" int edmd_set_log_capacity(edmd_ctx* ctx, int64_t cap) {
   if (cap > ctx->log_cap) {
     if (ctx->logbuf) cudaFree(ctx->logbuf);
     ctx->logbuf = nullptr;
+    ctx->log_cap = 0;
+    for (SysDev& S : ctx->hs) { S.log = nullptr; S.log_cap = 0; }
     CK(dalloc(&ctx->logbuf, (size_t)ctx->nsys * cap));
     ctx->log_cap = cap;
   }
@@ -447,7 +570,8 @@ extern "C" int edmd_set_log_capacity(edmd_ctx* ctx, int64_t cap) {
 
 extern "C" int edmd_clear_log(edmd_ctx* ctx) {
   if (!ctx) return EDMD_ERR_ARG;
-  for (int s = 0; s < ctx->nsys; s++) CK(cudaMemsetAsync(&ctx->st[s].nlog, 0, 8, ctx->stream));
+  k_set_log<<<(ctx->nsys + 127) / 128, 128, 0, ctx->stream>>>(ctx->ds, ctx->nsys, 0, nullptr);
+  CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->stream));
   return EDMD_OK;
 }
@@ -529,18 +653,75 @@ static int current_time(edmd_ctx* ctx, int s, double* t) {
   return EDMD_OK;
 }
 
-// one advance of every system, logging collision geometry; returns the log length of `s`
-static int advance_logged(edmd_ctx* ctx, int s, int64_t ncoll, int64_t* nlog) {
-  int rc = edmd_clear_log(ctx);
+// one advance of every system, logging collision geometry from entry `from` on,
+// at most `room` entries a system; *longest: the longest log, or that of system
+// s >= 0
+static int advance_logged(edmd_ctx* ctx, int64_t ncoll, int64_t from, int64_t room, int s, int64_t* longest) {
+  k_set_log<<<(ctx->nsys + 127) / 128, 128, 0, ctx->stream>>>(ctx->ds, ctx->nsys, (uint64_t)from, nullptr);
+  CK(cudaGetLastError());
+  int rc = edmd_advance(ctx, ncoll, INFINITY, EDMD_F_LOG | EDMD_F_COUNT_NORMAL, (int64_t)1 << 60, nullptr);
   if (rc) return rc;
-  rc = edmd_advance(ctx, ncoll, INFINITY, EDMD_F_LOG | EDMD_F_COUNT_NORMAL, (int64_t)1 << 60, nullptr);
-  if (rc) return rc;
-  uint64_t nl = 0;
-  CK(sync_copy(ctx, &nl, &ctx->st[s].nlog, 8, cudaMemcpyDeviceToHost));
-  if ((int64_t)nl > ctx->log_cap) return set_err(ctx, EDMD_ERR_CAPACITY, "collision log overflow");
-  *nlog = (int64_t)nl;
+  std::vector<uint64_t> nl(ctx->nsys);
+  CK(sync_copy2d(ctx, nl.data(), 8, &ctx->st[0].nlog, sizeof(SysState), 8, ctx->nsys, cudaMemcpyDeviceToHost));
+  int64_t most = 0;
+  for (uint64_t v : nl) {
+    const int64_t n = (int64_t)v - from;
+    if (n > room) return set_err(ctx, EDMD_ERR_CAPACITY, "collision log overflow");
+    most = n > most ? n : most;
+  }
+  if (longest) *longest = s >= 0 ? (int64_t)nl[s] - from : most;
   return EDMD_OK;
 }
+
+// The differentiation drivers' logs hold the collisions of a whole call up to
+// this size, and leave each system's public log length as it was.
+constexpr int64_t LOG_ALL_BYTES = (int64_t)2 << 30;
+
+// log lengths put back at the end of a call
+struct LogLengths {
+  edmd_ctx* ctx;
+  uint64_t* saved = nullptr;
+  explicit LogLengths(edmd_ctx* c) : ctx(c) {}
+  cudaError_t save() {
+    cudaError_t e = dalloc(&saved, ctx->nsys);
+    return e != cudaSuccess ? e : cudaMemcpy2DAsync(saved, 8, &ctx->st[0].nlog, sizeof(SysState), 8, ctx->nsys,
+                                                    cudaMemcpyDeviceToDevice, ctx->stream);
+  }
+  ~LogLengths() {
+    if (!saved) return;
+    k_set_log<<<(ctx->nsys + 127) / 128, 128, 0, ctx->stream>>>(ctx->ds, ctx->nsys, 0, saved);
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(saved);
+  }
+};
+
+// What a tangent driver's chunks alternate between: two halves of the logs and
+// the chunk's end times and log ends.  The tangent map and the QR of a chunk
+// run on a second stream beside the next chunk's forward run; the forward run
+// after that waits until the map has read the half it is going to write.
+struct Chunks {
+  double* tq[2] = {nullptr, nullptr};
+  uint64_t* nend[2] = {nullptr, nullptr};
+  cudaEvent_t ran[2] = {nullptr, nullptr}, mapped[2] = {nullptr, nullptr};
+  ~Chunks() {
+    for (int k = 0; k < 2; k++) {
+      if (tq[k]) cudaFree(tq[k]);
+      if (nend[k]) cudaFree(nend[k]);
+      if (ran[k]) cudaEventDestroy(ran[k]);
+      if (mapped[k]) cudaEventDestroy(mapped[k]);
+    }
+  }
+  cudaError_t make(int nsys) {
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < 2 && e == cudaSuccess; k++) {
+      e = dalloc(&tq[k], nsys);
+      if (e == cudaSuccess) e = dalloc(&nend[k], nsys);
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ran[k], cudaEventDisableTiming);
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&mapped[k], cudaEventDisableTiming);
+    }
+    return e;
+  }
+};
 
 constexpr int GRAM_BLOCKS = 1024;
 
@@ -553,7 +734,9 @@ static int cholqr(edmd_ctx* ctx, double* T, double* tl, int N, int K, const doub
     k_gram<<<blocks, 1024, 0, st>>>(T, tl, N, K, tqp, Gp);
     k_gram_sum<<<1, 1024, 0, st>>>(Gp, blocks, K, G);
     k_chol<<<1, 32, 0, st>>>(G, K, Rinv, logdiag, accumulate ? 1 : 0, fail);
-    k_apply_rinv<<<(N + 127) / 128, 128, 0, st>>>(T, tl, N, K, tqp, Rinv);
+    const int rb = (4 * N + RINV_THREADS - 1) / RINV_THREADS;
+    if (K <= 16) k_apply_rinv<16><<<rb, RINV_THREADS, 0, st>>>(T, tl, N, K, tqp, Rinv);
+    else k_apply_rinv<32><<<rb, RINV_THREADS, 0, st>>>(T, tl, N, K, tqp, Rinv);
     CK(cudaGetLastError());
   }
   return EDMD_OK;
@@ -566,10 +749,10 @@ extern "C" int edmd_tangent_run(edmd_ctx* ctx, int32_t s, int32_t K, int64_t n_c
   if (ctx->engine != EDMD_ENGINE_WARP) return set_err(ctx, EDMD_ERR_ARG, "tangents need the warp engine");
   const int N = ctx->hs[s].B.N;
   int64_t chunk = qr_every > 0 ? qr_every : (n_coll > 0 ? n_coll : 1);
-  int rc = edmd_set_log_capacity(ctx, chunk + 16);
+  const int64_t half = chunk + 16;
+  int rc = edmd_set_log_capacity(ctx, n_coll > chunk ? 2 * half : half);
   if (rc) return rc;
   double *T = nullptr, *tl = nullptr, *G = nullptr, *Gp = nullptr, *Rinv = nullptr, *logdiag = nullptr;
-  double* tqd = nullptr;
   int* fail = nullptr;
   CK(dalloc(&T, (size_t)4 * N * K));
   CK(dalloc(&tl, N));
@@ -578,17 +761,12 @@ extern "C" int edmd_tangent_run(edmd_ctx* ctx, int32_t s, int32_t K, int64_t n_c
   CK(dalloc(&Rinv, K * K));
   CK(dalloc(&logdiag, K));
   CK(dalloc(&fail, 1));
-  CK(dalloc(&tqd, 1));
-  struct Free { void* p[8]; ~Free() { for (void* q : p) if (q) cudaFree(q); } } guard{{T, tl, G, Gp, Rinv, logdiag, fail, tqd}};
-  // as in the batched form: each chunk's QR on a second stream beside the
-  // next chunk's forward run, at the chunk's end time copied on the device
+  struct Free { void* p[7]; ~Free() { for (void* q : p) if (q) cudaFree(q); } } guard{{T, tl, G, Gp, Rinv, logdiag, fail}};
+  Chunks ch;
+  CK(ch.make(1));
   if (!ctx->stream2) CK(cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking));
-  struct Ev {
-    cudaEvent_t e = nullptr;
-    ~Ev() { if (e) cudaEventDestroy(e); }
-  } ea, eq;
-  CK(cudaEventCreateWithFlags(&ea.e, cudaEventDisableTiming));
-  CK(cudaEventCreateWithFlags(&eq.e, cudaEventDisableTiming));
+  cudaStream_t st2 = ctx->stream2;
+  struct Idle { edmd_ctx* c; ~Idle() { cudaStreamSynchronize(c->stream2); } } idle{ctx};   // before the frees
   CK(call_begin(ctx));
   double t0;
   if ((rc = current_time(ctx, s, &t0))) return rc;
@@ -606,29 +784,34 @@ extern "C" int edmd_tangent_run(edmd_ctx* ctx, int32_t s, int32_t K, int64_t n_c
   k_fill<<<(N + 255) / 256, 256, 0, ctx->stream>>>(tl, N, t0);
   CK(cudaMemsetAsync(logdiag, 0, K * sizeof(double), ctx->stream));
   CK(cudaMemsetAsync(fail, 0, 4, ctx->stream));
-  k_sys_times<<<1, 32, 0, ctx->stream>>>(ctx->ds + s, 1, tqd);
-  if (!tangent_io && (rc = cholqr(ctx, T, tl, N, K, tqd, G, Gp, Rinv, logdiag, fail, false, ctx->stream)))
+  k_sys_times<<<1, 32, 0, ctx->stream>>>(ctx->ds + s, 1, ch.tq[0], nullptr);
+  if (!tangent_io &&
+      (rc = cholqr(ctx, T, tl, N, K, ch.tq[0], G, Gp, Rinv, logdiag, fail, false, ctx->stream)))
     return rc;
-  CK(cudaEventRecord(eq.e, ctx->stream));
-  int64_t done = 0;
-  while (done < n_coll) {
+  // the tangent vectors are the second stream's from here on
+  CK(cudaEventRecord(ch.ran[0], ctx->stream));
+  CK(cudaStreamWaitEvent(st2, ch.ran[0], 0));
+  int64_t done = 0, last = 0;
+  for (int c = 0; done < n_coll; c ^= 1) {
     int64_t want = n_coll - done < chunk ? n_coll - done : chunk;
     int64_t nl = 0;
-    if ((rc = advance_logged(ctx, s, want, &nl))) return rc;
-    CK(cudaStreamWaitEvent(ctx->stream, eq.e, 0));             // the previous QR is done
-    k_tangent_apply<<<1, 32, 0, ctx->stream>>>((const edmd_log_entry*)ctx->hs[s].log, nl, ctx->hs[s].d, T, tl, K);
+    const int64_t from = c ? half : 0;
+    if (done >= 2 * chunk) CK(cudaStreamWaitEvent(ctx->stream, ch.mapped[c], 0));
+    if ((rc = advance_logged(ctx, want, from, half, s, &nl))) return rc;
+    k_sys_times<<<1, 32, 0, ctx->stream>>>(ctx->ds + s, 1, ch.tq[c], nullptr);
+    CK(cudaEventRecord(ch.ran[c], ctx->stream));
+    CK(cudaStreamWaitEvent(st2, ch.ran[c], 0));
+    k_tangent_apply<<<1, 32, 0, st2>>>((const edmd_log_entry*)ctx->hs[s].log + from, nl, ctx->hs[s].d, T, tl, K);
     CK(cudaGetLastError());
-    if (qr_every > 0) {
-      k_sys_times<<<1, 32, 0, ctx->stream>>>(ctx->ds + s, 1, tqd);
-      CK(cudaEventRecord(ea.e, ctx->stream));
-      CK(cudaStreamWaitEvent(ctx->stream2, ea.e, 0));
-      if ((rc = cholqr(ctx, T, tl, N, K, tqd, G, Gp, Rinv, logdiag, fail, true, ctx->stream2))) return rc;
-      CK(cudaEventRecord(eq.e, ctx->stream2));
-    }
+    if (qr_every > 0 && (rc = cholqr(ctx, T, tl, N, K, ch.tq[c], G, Gp, Rinv, logdiag, fail, true, st2))) return rc;
+    CK(cudaEventRecord(ch.mapped[c], st2));
     done += want;
+    last = from;
     if (nl < want) break;     // the run ended early (tmax or t_stop)
   }
-  CK(cudaStreamWaitEvent(ctx->stream, eq.e, 0));
+  CK(cudaEventRecord(ch.ran[0], st2));
+  CK(cudaStreamWaitEvent(ctx->stream, ch.ran[0], 0));
+  if (last) k_log_front<<<ctx->nsys, 128, 0, ctx->stream>>>(ctx->ds, last);
   {
     int hf = 0;
     CK(sync_copy(ctx, &hf, fail, 4, cudaMemcpyDeviceToHost));
@@ -667,8 +850,15 @@ extern "C" int edmd_msd_gradient(edmd_ctx* ctx, int32_t s, int64_t n_coll, int64
   if (ctx->engine != EDMD_ENGINE_WARP) return set_err(ctx, EDMD_ERR_ARG, "adjoints need the warp engine");
   const int N = ctx->hs[s].B.N;
   const double Lx = ctx->hs[s].B.Lx, Ly = ctx->hs[s].B.Ly;
-  int rc = edmd_set_log_capacity(ctx, ckpt_every + 16);
+  // one logged forward run, or (a long one) checkpointed segments run twice
+  bool whole = n_coll < LOG_ALL_BYTES / ((int64_t)sizeof(edmd_log_entry) * ctx->nsys) - 16;
+  int rc = whole ? edmd_set_log_capacity(ctx, n_coll + 16) : EDMD_OK;
+  if (rc) { whole = false; cudaGetLastError(); }         // no room for it
+  if (!whole) rc = edmd_set_log_capacity(ctx, ckpt_every + 16);
   if (rc) return rc;
+  LogLengths lengths(ctx);
+  CK(lengths.save());
+  int64_t nlog_all = 0;
   double *A = nullptr, *ta = nullptr, *px = nullptr, *py = nullptr;
   CK(dalloc(&A, 4 * (size_t)N));
   CK(dalloc(&ta, N));
@@ -684,15 +874,16 @@ extern "C" int edmd_msd_gradient(edmd_ctx* ctx, int32_t s, int64_t n_coll, int64
   CK(cudaMemcpyAsync(y0.data(), py, N * 8, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   // forward sweep: exact engine checkpoints at every segment boundary
-  const int64_t nseg = (n_coll + ckpt_every - 1) / ckpt_every;
+  const int64_t nseg = whole ? 0 : (n_coll + ckpt_every - 1) / ckpt_every;
   std::vector<int64_t> seglen(nseg);
+  if (whole && (rc = advance_logged(ctx, n_coll, 0, n_coll + 16, s, &nlog_all))) return rc;
   for (int64_t g = 0; g < nseg; g++) {
     if ((rc = edmd_checkpoint_save(ctx, (int32_t)g))) return rc;
     seglen[g] = (g == nseg - 1) ? n_coll - g * ckpt_every : ckpt_every;
     rc = edmd_advance(ctx, seglen[g], INFINITY, EDMD_F_COUNT_NORMAL, (int64_t)1 << 60, nullptr);
     if (rc) return rc;
   }
-  if ((rc = edmd_checkpoint_save(ctx, (int32_t)nseg))) return rc;
+  if (!whole && (rc = edmd_checkpoint_save(ctx, (int32_t)nseg))) return rc;
   if ((rc = current_time(ctx, s, &T))) return rc;
   if (t_obs >= 0) {
     if (t_obs < T) return set_err(ctx, EDMD_ERR_ARG, "t_obs precedes the last processed event");
@@ -723,19 +914,21 @@ extern "C" int edmd_msd_gradient(edmd_ctx* ctx, int32_t s, int64_t n_coll, int64
   msd /= N;
   CK(cudaMemcpyAsync(A, hA.data(), hA.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
   k_fill<<<(N + 255) / 256, 256, 0, ctx->stream>>>(ta, N, T);
-  // reverse sweep: recompute each segment from its checkpoint, then its adjoint
+  // reverse sweep over the log; else recompute each segment from its checkpoint, then its adjoint
+  const edmd_log_entry* const log = (const edmd_log_entry*)ctx->hs[s].log;
+  if (whole) k_adjoint<<<1, 32, 0, ctx->stream>>>(log, nlog_all, ctx->hs[s].d, A, ta);
   for (int64_t g = nseg - 1; g >= 0; g--) {
     if ((rc = edmd_checkpoint_restore(ctx, (int32_t)g))) return rc;
     int64_t nl = 0;
-    if ((rc = advance_logged(ctx, s, seglen[g], &nl))) return rc;
-    k_adjoint_segment<<<1, 1, 0, ctx->stream>>>((const edmd_log_entry*)ctx->hs[s].log, nl, ctx->hs[s].d, A, ta);
-    CK(cudaGetLastError());
+    if ((rc = advance_logged(ctx, seglen[g], 0, ckpt_every + 16, s, &nl))) return rc;
+    k_adjoint<<<1, 32, 0, ctx->stream>>>(log, nl, ctx->hs[s].d, A, ta);
   }
+  CK(cudaGetLastError());
   k_adjoint_finish<<<(N + 127) / 128, 128, 0, ctx->stream>>>(N, A, ta, t0);
   CK(cudaMemcpyAsync(hA.data(), A, hA.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   // leave the engine at the end of the run
-  if ((rc = edmd_checkpoint_restore(ctx, (int32_t)nseg))) return rc;
+  if (!whole && (rc = edmd_checkpoint_restore(ctx, (int32_t)nseg))) return rc;
   // u = r(t) - r(0) also depends on the initial positions directly
   for (int i = 0; i < N; i++) {
     if (g_x) g_x[i] = hA[4 * i + 0] - 2.0 * (ux[i] - mx) / N;
@@ -774,28 +967,18 @@ int batch_index(edmd_ctx* ctx, BatchIndex& bi) {
   return EDMD_OK;
 }
 
-// one advance of every system with the collision log; EDMD_ERR_CAPACITY when
-// a system logged more than the log holds
-int advance_logged_all(edmd_ctx* ctx, int64_t ncoll) {
-  int rc = edmd_clear_log(ctx);
-  if (rc) return rc;
-  rc = edmd_advance(ctx, ncoll, INFINITY, EDMD_F_LOG | EDMD_F_COUNT_NORMAL, (int64_t)1 << 60, nullptr);
-  if (rc) return rc;
-  std::vector<uint64_t> nl(ctx->nsys);
-  CK(sync_copy2d(ctx, nl.data(), 8, &ctx->st[0].nlog, sizeof(SysState), 8, ctx->nsys, cudaMemcpyDeviceToHost));
-  for (uint64_t v : nl)
-    if ((int64_t)v > ctx->log_cap) return set_err(ctx, EDMD_ERR_CAPACITY, "collision log overflow");
-  return EDMD_OK;
-}
-
 // CholQR2 of every system's tangent block at the times tqs, on stream st
 int cholqr_b(edmd_ctx* ctx, const BatchIndex& bi, double* T, double* tl, int K, double* G, double* Rinv,
              double* logdiag, int* fail, bool accumulate, const double* tqs, cudaStream_t st) {
-  const int64_t TN = ctx->total_N;
+  // all pairs of a system in one block, or (few systems) spread over blocks
+  const int pair_warps = (K * (K + 1) / 2 + 31) / 32, split = std::max(1, std::min(pair_warps, 152 / ctx->nsys));
+  const int warps = std::max((pair_warps + split - 1) / split, (4 * K + 31) / 32);
   for (int pass = 0; pass < 2; pass++) {    // CholQR2: the second pass restores orthogonality
-    k_gram_b<<<ctx->nsys, 1024, 0, st>>>(ctx->ds, bi.doff, T, tl, K, tqs, G);
+    k_gram_b<<<dim3(ctx->nsys, (pair_warps + warps - 1) / warps), 32 * warps, 0, st>>>(ctx->ds, bi.doff, T, tl, K, tqs, G);
     k_chol_b<<<ctx->nsys, 32, 0, st>>>(G, ctx->nsys, K, Rinv, logdiag, accumulate ? 1 : 0, fail);
-    k_apply_rinv_b<<<(unsigned)((TN + 127) / 128), 128, 0, st>>>(bi.doff, bi.dsys, TN, T, tl, K, tqs, Rinv);
+    const dim3 rb((4 * ctx->maxN + RINV_THREADS - 1) / RINV_THREADS, ctx->nsys);
+    if (K <= 16) k_apply_rinv_b<16><<<rb, RINV_THREADS, 0, st>>>(ctx->ds, bi.doff, T, tl, K, tqs, Rinv);
+    else k_apply_rinv_b<32><<<rb, RINV_THREADS, 0, st>>>(ctx->ds, bi.doff, T, tl, K, tqs, Rinv);
     CK(cudaGetLastError());
   }
   return EDMD_OK;
@@ -824,11 +1007,12 @@ extern "C" int edmd_tangent_run_batch(edmd_ctx* ctx, int32_t K, int64_t n_coll, 
   const int64_t TN = ctx->total_N;
   const int nsys = ctx->nsys;
   const int64_t chunk = qr_every > 0 ? qr_every : (n_coll > 0 ? n_coll : 1);
-  int rc = edmd_set_log_capacity(ctx, chunk + 16);
+  const int64_t half = chunk + 16;
+  int rc = edmd_set_log_capacity(ctx, n_coll > chunk ? 2 * half : half);
   if (rc) return rc;
   BatchIndex bi;
   if ((rc = batch_index(ctx, bi))) return rc;
-  double *T = nullptr, *tl = nullptr, *G = nullptr, *Rinv = nullptr, *logdiag = nullptr, *tqs = nullptr;
+  double *T = nullptr, *tl = nullptr, *G = nullptr, *Rinv = nullptr, *logdiag = nullptr;
   int* fail = nullptr;
   CK(dalloc(&T, (size_t)4 * TN * K));
   CK(dalloc(&tl, TN));
@@ -836,18 +1020,12 @@ extern "C" int edmd_tangent_run_batch(edmd_ctx* ctx, int32_t K, int64_t n_coll, 
   CK(dalloc(&Rinv, (size_t)nsys * K * K));
   CK(dalloc(&logdiag, (size_t)nsys * K));
   CK(dalloc(&fail, nsys));
-  CK(dalloc(&tqs, nsys));
-  struct Free { void* p[7]; ~Free() { for (void* q : p) if (q) cudaFree(q); } } guard{{T, tl, G, Rinv, logdiag, fail, tqs}};
-  // the QR of a chunk runs on a second stream beside the next chunk's forward
-  // run (which does not touch the tangent vectors); the next tangent map
-  // waits for it
+  struct Free { void* p[6]; ~Free() { for (void* q : p) if (q) cudaFree(q); } } guard{{T, tl, G, Rinv, logdiag, fail}};
+  Chunks ch;
+  CK(ch.make(nsys));
   if (!ctx->stream2) CK(cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking));
-  struct Ev {
-    cudaEvent_t e = nullptr;
-    ~Ev() { if (e) cudaEventDestroy(e); }
-  } ea, eq;
-  CK(cudaEventCreateWithFlags(&ea.e, cudaEventDisableTiming));
-  CK(cudaEventCreateWithFlags(&eq.e, cudaEventDisableTiming));
+  cudaStream_t st2 = ctx->stream2;
+  struct Idle { edmd_ctx* c; ~Idle() { cudaStreamSynchronize(c->stream2); } } idle{ctx};   // before the frees
   const unsigned gs = (unsigned)((nsys + 127) / 128);
   // system s starts from the vectors edmd_tangent_run draws from seed + s
   // (drawn on the host before the timed part of the call)
@@ -873,25 +1051,30 @@ extern "C" int edmd_tangent_run_batch(edmd_ctx* ctx, int32_t K, int64_t n_coll, 
   k_fill_sys_time<<<(unsigned)((TN + 255) / 256), 256, 0, ctx->stream>>>(ctx->ds, bi.dsys, TN, tl);
   CK(cudaMemsetAsync(logdiag, 0, (size_t)nsys * K * sizeof(double), ctx->stream));
   CK(cudaMemsetAsync(fail, 0, nsys * sizeof(int), ctx->stream));
-  k_sys_times<<<gs, 128, 0, ctx->stream>>>(ctx->ds, nsys, tqs);
-  if ((rc = cholqr_b(ctx, bi, T, tl, K, G, Rinv, logdiag, fail, false, tqs, ctx->stream))) return rc;
-  CK(cudaEventRecord(eq.e, ctx->stream));
-  for (int64_t done = 0; done < n_coll;) {
+  k_sys_times<<<gs, 128, 0, ctx->stream>>>(ctx->ds, nsys, ch.tq[0], nullptr);
+  if ((rc = cholqr_b(ctx, bi, T, tl, K, G, Rinv, logdiag, fail, false, ch.tq[0], ctx->stream))) return rc;
+  // the tangent vectors are the second stream's from here on
+  CK(cudaEventRecord(ch.ran[0], ctx->stream));
+  CK(cudaStreamWaitEvent(st2, ch.ran[0], 0));
+  int64_t done = 0, last = 0;
+  for (int c = 0; done < n_coll; c ^= 1) {
     const int64_t want = n_coll - done < chunk ? n_coll - done : chunk;
-    if ((rc = advance_logged_all(ctx, want))) return rc;
-    CK(cudaStreamWaitEvent(ctx->stream, eq.e, 0));             // the previous QR is done
-    k_tangent_apply_b<<<nsys, 32, 0, ctx->stream>>>(ctx->ds, bi.doff, T, tl, K);
+    const int64_t from = c ? half : 0;
+    if (done >= 2 * chunk) CK(cudaStreamWaitEvent(ctx->stream, ch.mapped[c], 0));
+    if ((rc = advance_logged(ctx, want, from, half, -1, nullptr))) return rc;
+    k_sys_times<<<gs, 128, 0, ctx->stream>>>(ctx->ds, nsys, ch.tq[c], ch.nend[c]);   // the chunk's end
+    CK(cudaEventRecord(ch.ran[c], ctx->stream));
+    CK(cudaStreamWaitEvent(st2, ch.ran[c], 0));
+    k_tangent_apply_b<<<nsys, 32, 0, st2>>>(ctx->ds, bi.doff, T, tl, K, from, ch.nend[c]);
     CK(cudaGetLastError());
-    if (qr_every > 0) {
-      k_sys_times<<<gs, 128, 0, ctx->stream>>>(ctx->ds, nsys, tqs);   // the chunk's end times
-      CK(cudaEventRecord(ea.e, ctx->stream));
-      CK(cudaStreamWaitEvent(ctx->stream2, ea.e, 0));
-      if ((rc = cholqr_b(ctx, bi, T, tl, K, G, Rinv, logdiag, fail, true, tqs, ctx->stream2))) return rc;
-      CK(cudaEventRecord(eq.e, ctx->stream2));
-    }
+    if (qr_every > 0 && (rc = cholqr_b(ctx, bi, T, tl, K, G, Rinv, logdiag, fail, true, ch.tq[c], st2))) return rc;
+    CK(cudaEventRecord(ch.mapped[c], st2));
     done += want;
+    last = from;
   }
-  CK(cudaStreamWaitEvent(ctx->stream, eq.e, 0));
+  CK(cudaEventRecord(ch.ran[0], st2));
+  CK(cudaStreamWaitEvent(ctx->stream, ch.ran[0], 0));
+  if (last) k_log_front<<<nsys, 128, 0, ctx->stream>>>(ctx->ds, last);
   if ((rc = check_fail(ctx, fail))) return rc;
   if (lyap_out) {
     std::vector<double> ld((size_t)nsys * K);
@@ -911,8 +1094,14 @@ extern "C" int edmd_msd_gradient_batch(edmd_ctx* ctx, int64_t n_coll, int64_t ck
   if (ctx->engine != EDMD_ENGINE_WARP) return set_err(ctx, EDMD_ERR_ARG, "adjoints need the warp engine");
   const int64_t TN = ctx->total_N;
   const int nsys = ctx->nsys;
-  int rc = edmd_set_log_capacity(ctx, ckpt_every + 16);
+  // one logged forward run, or (a long one) checkpointed segments run twice
+  bool whole = n_coll < LOG_ALL_BYTES / ((int64_t)sizeof(edmd_log_entry) * nsys) - 16;
+  int rc = whole ? edmd_set_log_capacity(ctx, n_coll + 16) : EDMD_OK;
+  if (rc) { whole = false; cudaGetLastError(); }         // no room for it
+  if (!whole) rc = edmd_set_log_capacity(ctx, ckpt_every + 16);
   if (rc) return rc;
+  LogLengths lengths(ctx);
+  CK(lengths.save());
   BatchIndex bi;
   if ((rc = batch_index(ctx, bi))) return rc;
   double *A = nullptr, *ta = nullptr, *x0 = nullptr, *y0 = nullptr, *x1 = nullptr, *y1 = nullptr;
@@ -924,33 +1113,35 @@ extern "C" int edmd_msd_gradient_batch(edmd_ctx* ctx, int64_t n_coll, int64_t ck
       guard{{A, ta, x0, y0, x1, y1, dux, duy, t0, msd}};
   CK(call_begin(ctx));
   const unsigned gT = (unsigned)((TN + 127) / 128);
-  k_sys_times<<<(nsys + 127) / 128, 128, 0, ctx->stream>>>(ctx->ds, nsys, t0);
+  k_sys_times<<<(nsys + 127) / 128, 128, 0, ctx->stream>>>(ctx->ds, nsys, t0, nullptr);
   k_positions_now_b<<<gT, 128, 0, ctx->stream>>>(ctx->ds, bi.doff, bi.dsys, TN, x0, y0);
   CK(cudaGetLastError());
   // forward sweep: exact engine checkpoints at every segment boundary
-  const int64_t nseg = (n_coll + ckpt_every - 1) / ckpt_every;
+  const int64_t nseg = whole ? 0 : (n_coll + ckpt_every - 1) / ckpt_every;
   std::vector<int64_t> seglen(nseg);
+  if (whole && (rc = advance_logged(ctx, n_coll, 0, n_coll + 16, -1, nullptr))) return rc;
   for (int64_t g = 0; g < nseg; g++) {
     if ((rc = edmd_checkpoint_save(ctx, (int32_t)g))) return rc;
     seglen[g] = (g == nseg - 1) ? n_coll - g * ckpt_every : ckpt_every;
     rc = edmd_advance(ctx, seglen[g], INFINITY, EDMD_F_COUNT_NORMAL, (int64_t)1 << 60, nullptr);
     if (rc) return rc;
   }
-  if ((rc = edmd_checkpoint_save(ctx, (int32_t)nseg))) return rc;
+  if (!whole && (rc = edmd_checkpoint_save(ctx, (int32_t)nseg))) return rc;
   k_positions_now_b<<<gT, 128, 0, ctx->stream>>>(ctx->ds, bi.doff, bi.dsys, TN, x1, y1);
   k_msd_b<<<nsys, 256, 0, ctx->stream>>>(ctx->ds, bi.doff, x0, y0, x1, y1, A, ta, dux, duy, msd);
   CK(cudaGetLastError());
-  // reverse sweep: recompute each segment from its checkpoint, then its adjoint
+  // reverse sweep over the logs; else recompute each segment from its checkpoint, then its adjoint
+  if (whole) k_adjoint_b<<<nsys, 32, 0, ctx->stream>>>(ctx->ds, bi.doff, A, ta);
   for (int64_t g = nseg - 1; g >= 0; g--) {
     if ((rc = edmd_checkpoint_restore(ctx, (int32_t)g))) return rc;
-    if ((rc = advance_logged_all(ctx, seglen[g]))) return rc;
-    k_adjoint_segment_b<<<(nsys + 63) / 64, 64, 0, ctx->stream>>>(ctx->ds, bi.doff, nsys, A, ta);
-    CK(cudaGetLastError());
+    if ((rc = advance_logged(ctx, seglen[g], 0, ckpt_every + 16, -1, nullptr))) return rc;
+    k_adjoint_b<<<nsys, 32, 0, ctx->stream>>>(ctx->ds, bi.doff, A, ta);
   }
+  CK(cudaGetLastError());
   k_adjoint_finish_b<<<gT, 128, 0, ctx->stream>>>(bi.dsys, TN, A, ta, t0);
   CK(cudaGetLastError());
   // leave the engine at the end of the run
-  if ((rc = edmd_checkpoint_restore(ctx, (int32_t)nseg))) return rc;
+  if (!whole && (rc = edmd_checkpoint_restore(ctx, (int32_t)nseg))) return rc;
   std::vector<double> hA(4 * (size_t)TN), hx(TN), hy(TN);
   CK(sync_copy(ctx, hA.data(), A, hA.size() * 8, cudaMemcpyDeviceToHost));
   CK(sync_copy(ctx, hx.data(), dux, TN * 8, cudaMemcpyDeviceToHost));

@@ -107,3 +107,37 @@ def test_round_selection_at_other_time_scales(edmd, energy, t0, t1):
     same(a.state(0), b.state(0))
     a.close()
     b.close()
+
+
+# one lane, both row-register builds at their edges, all columns; qr_every leaves an odd and an even number of chunks
+@pytest.mark.parametrize("K,n_coll", [(1, 60), (16, 100), (17, 80), (32, 100)])
+def test_tangent_batch_equals_single_systems(edmd, K, n_coll):
+    starts = [start(edmd, N, 0.60, 2) for N in (33, 120, 200)]
+    eng = edmd.Engine(starts)
+    lyap = eng.tangent_batch(K, n_coll, 20, seed=5)
+    eng.close()
+    for s, st in enumerate(starts):
+        one = edmd.Engine([st])
+        _, ref = one.tangent(K, n_coll, 20, seed=5 + s)
+        assert len(one.log(0)) == 20                      # the last chunk's collisions
+        one.close()
+        # the two forms add a Gram matrix's rows in another order: 2 QRs of 20 collisions each, condition ~1e3
+        np.testing.assert_allclose(lyap[s], ref, rtol=1e-9, atol=1e-9 * np.abs(ref).max())
+
+
+def test_gradient_of_a_run_too_long_for_one_log(edmd):
+    """4096 systems x 8300 collisions exceed the log kept for a whole call: the checkpointed sweep, against single systems."""
+    starts = [start(edmd, 12 + 2 * (k % 3), 0.5, k % 3 + 1, tmax=1e9) for k in range(3)]
+    eng = edmd.Engine([starts[k % 3] for k in range(4096)])
+    msd, g = eng.msd_gradient_batch(8300, ckpt_every=4150)
+    off = np.cumsum([0] + eng.N)
+    eng.close()
+    for s in range(3):
+        one = edmd.Engine([starts[s]])
+        m1, g1 = one.msd_gradient(8300, ckpt_every=1000)
+        one.close()
+        for q in (s, s + 3 * 1364):
+            a, b = off[q], off[q + 1]
+            np.testing.assert_allclose(msd[q], m1, rtol=1e-12)
+            for k in ("vx", "vy", "x", "y"):
+                np.testing.assert_allclose(g[k][a:b], g1[k], rtol=1e-9, atol=1e-9 * np.abs(g1[k]).max())
