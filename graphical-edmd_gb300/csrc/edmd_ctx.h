@@ -60,6 +60,8 @@ struct edmd_ctx {
   bool round_dirty = false;         // queue order lost: set by the round engine, cleared by a restage
   bool any_additive = false;        // some system uses additive contact (EDMD_CONTACT_ADDITIVE)
   std::vector<char> ckpt_dirty;     // round_dirty of each checkpoint
+  void* pcf = nullptr;              // g(r): histogram and bin steps of up to pcf_bins bins
+  int pcf_bins = 0;
   char* pin = nullptr;              // two page-locked buffers of host_copies, and their events
   cudaEvent_t pin_ev[2] = {nullptr, nullptr};
   std::string err;

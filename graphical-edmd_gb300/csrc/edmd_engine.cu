@@ -1355,10 +1355,11 @@ extern "C" int edmd_device_info(char* name, int32_t cap, int32_t* sm_count) {
 
 
 constexpr int64_t PIN_BYTES = (int64_t)4 << 20;      // one staging buffer
-// Smaller lists are copied directly: starting the threads costs ~0.4 ms (10^5
-// disks, 4.8 MB back: 0.6 ms staged, 0.19 ms direct into arrays of a reused
-// heap), and arrays that small are rarely new to the device.
-constexpr int64_t PIN_LEAST = (int64_t)16 << 20;
+// Smaller lists are copied directly; below PIN_THREADS the calling thread moves
+// the pieces itself, since starting threads costs ~0.4 ms.  10^5 disks (4.8 MB)
+// back: 0.2 ms direct into arrays the device has used before, 3.2 ms into
+// others (a program that takes new arrays every time alternates); staged 0.4 ms.
+constexpr int64_t PIN_LEAST = (int64_t)1 << 20, PIN_THREADS = (int64_t)16 << 20;
 
 cudaError_t host_copies(edmd_ctx* ctx, const std::vector<HostCopy>& list, bool to_device) {
   const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
@@ -1410,7 +1411,7 @@ cudaError_t host_copies(edmd_ctx* ctx, const std::vector<HostCopy>& list, bool t
     else memcpy((char*)pieces[p].host + lo, pin + lo, hi - lo);
   };
   std::vector<std::thread> pool;
-  const int want = host_threads(total, (int64_t)2 << 20) / 2;
+  const int want = total < PIN_THREADS ? 0 : host_threads(total, PIN_THREADS) / 2;
   std::atomic<int> workers{0};                       // fixed before the first piece opens
   for (int k = 0; k < want; k++) {
     try {
@@ -1906,6 +1907,7 @@ extern "C" int edmd_destroy(edmd_ctx* ctx) {
   for (void* p : ctx->ckpt)
     if (p) cudaFree(p);
   if (ctx->logbuf) cudaFree(ctx->logbuf);
+  if (ctx->pcf) cudaFree(ctx->pcf);
   if (ctx->pin) cudaFreeHost(ctx->pin);
   for (cudaEvent_t e : ctx->pin_ev)
     if (e) cudaEventDestroy(e);

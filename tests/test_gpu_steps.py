@@ -141,3 +141,22 @@ def test_gradient_of_a_run_too_long_for_one_log(edmd):
             np.testing.assert_allclose(msd[q], m1, rtol=1e-12)
             for k in ("vx", "vy", "x", "y"):
                 np.testing.assert_allclose(g[k][a:b], g1[k], rtol=1e-9, atol=1e-9 * np.abs(g1[k]).max())
+
+
+# wide and narrow bins (lattice distances fall on their edges at the start), a reach that is no multiple of the bin
+@pytest.mark.parametrize("dr,max_r,coll", [(0.5, 6.0, 0), (3.0, 7.7, 0), (0.004, 12.0, 2000), (0.05, 9.99, 2000)])
+def test_pcf_bins(edmd, oracle, dr, max_r, coll):
+    s = start(edmd, 3000, 0.60, 9)
+    eng = edmd.Engine([s])
+    o = oracle.Oracle(arrays={k: s[k] for k in ("x", "y", "vx", "vy", "rad", "m", "type")}, Lx=s["Lx"], Ly=s["Ly"])
+    if coll:
+        eng.advance(max_coll=coll)
+        eng.sync()
+        o.run(coll, cap=1)
+        o.sync()
+    for _ in range(2):                                    # the second call reuses the workspace
+        r, g = eng.pcf(0, dr, max_r)
+        ro, go = o.pcf(dr, max_r)
+        np.testing.assert_array_equal(r, ro)
+        np.testing.assert_array_equal(g, go)
+    eng.close()
