@@ -355,38 +355,6 @@ __device__ __forceinline__ double crossing_time_i(const Box& B, const Disk& p, i
   return t + ty;
 }
 
-// One axis of crossingEventNormal (src/EDMD.c:2405-2482): the time to the
-// wall of cell (cx, cy) the disk moves towards along x (ydim false) or y, and
-// the direction code.  Branch-free over the axis, with the same operations
-// as crossing_time_i, so lanes working on different axes share instructions.
-__device__ __forceinline__ double axis_time(const Box& B, const Disk& p, int cx, int cy, bool ydim, int* dir) {
-  const double pos = ydim ? p.y : p.x, v = ydim ? p.vy : p.vx;
-  const double cs = ydim ? B.cys : B.cxs, hL = ydim ? B.hLy : B.hLx, L = ydim ? B.Ly : B.Lx;
-  const int c = ydim ? cy : cx;
-  const bool neg = is_neg(v);
-  double a = (neg ? c : 1 + c) * cs - pos;
-  *dir = (ydim ? 3 : 1) + (neg ? 0 : 1);
-  if (ge_pos(a, hL)) a = a - L;
-  else if (lt_neg(a, hL)) a = a + L;
-  return div_rn(a, v);
-}
-
-// crossing_time_i with the two divisions on two lanes of a full warp: the
-// lane with (lane & xmask) == 0 takes the x axis of its disk, its partner
-// lane ^ xmask the y axis; both lanes return the disk's crossing
-__device__ __forceinline__ double crossing_time_lanes(const Box& B, const Disk& p, int cx, int cy, double t,
-                                                      int lane, int xmask, int* dir) {
-  const bool ydim = (lane & xmask) != 0;
-  int d;
-  const double ta = axis_time(B, p, cx, cy, ydim, &d);
-  const double tb = __shfl_xor_sync(0xffffffffu, ta, xmask);
-  const int db = __shfl_xor_sync(0xffffffffu, d, xmask);
-  const double tx = ydim ? tb : ta, ty = ydim ? ta : tb;
-  const bool ux = lt_i(tx, ty);
-  *dir = ux ? (ydim ? db : d) : (ydim ? d : db);
-  return t + (ux ? tx : ty);
-}
-
 // (int)(dt / dtP) of addEventToQueue without the FP64 division when provably
 // equal: |dt*rdtP - fl(dt/dtP)| <= 3*q*2^-53 < 1e-9 for q < 2^22, so the floor
 // is unchanged unless q is within 1e-9 of an integer (then divide exactly).

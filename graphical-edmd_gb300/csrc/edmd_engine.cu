@@ -16,7 +16,7 @@
 //                ascending counter.
 // The keys live in a 32-ary tournament tree (level 0 = one leaf per disk, the
 // minimum of its crossing and collision events, plus three special events);
-// each tree level is fixed by one coalesced 32-wide load and a warp butterfly.
+// each tree level is fixed by one coalesced load and hardware reductions.
 // Collision prediction packs the candidates of the 3x3 neighbour cells of the
 // (up to two) disks that changed into the lanes of the warp.
 #include "edmd_lanes.cuh"

@@ -30,9 +30,6 @@ struct Grp {
   template <class T> __device__ __forceinline__ T shfl_xor(T v, int o) const {
     return __shfl_xor_sync(mask, v, o, GW);
   }
-  template <class T> __device__ __forceinline__ T shfl_up(T v, int o) const {
-    return __shfl_up_sync(mask, v, o, GW);
-  }
   __device__ __forceinline__ void sync() const { __syncwarp(mask); }
   __device__ __forceinline__ bool any(bool p) const { return __any_sync(mask, p); }
   __device__ __forceinline__ uint32_t min_u32(uint32_t v) const { return __reduce_min_sync(mask, v); }

@@ -1,6 +1,6 @@
 // edmd_round.cu -- round-parallel event engine: the causally independent events
-// of one large system, or of a whole batch, processed at once, one warp or one
-// thread per event.
+// of one large system, or of a whole batch, processed at once, one warp per
+// event.
 //
 // Every disk has one pending event: the earlier of its crossing event
 // (crossingEventNormal, src/EDMD.c:2405) and its collision event
@@ -20,8 +20,8 @@
 //      next screenshot, t_stop and its collision budget) that is the window
 //      minimum at both of its footprint cells: no earlier pending event lies
 //      within r cells, and selected events are more than r cells apart;
-//   3. the selected events are processed, one warp each or (rounds of many
-//      events) one thread each, with the arithmetic of the serial engines;
+//   3. the selected events are processed, one warp each (one thread each where
+//      the flags ask for it), with the arithmetic of the serial engines;
 //   4. the cell minima around them are recomputed, and systems with nothing
 //      left before their screenshot pass it (every disk free-flown to it).
 // Events created inside a round can still precede a processed event (a chain
@@ -620,9 +620,9 @@ struct EvResult {
 // One selected event g of system s processed by a group of GW lanes:
 // doTheCollisionNormal (src/EDMD.c:3542, elastic rule 3802-3827), its stale
 // branch (3553-3556) or doTheCrossing (2501).  The lanes hold the roles of
-// edmd_lanes.cuh, so an event's scalar FP64 work (and, with GW = 8, that of the
-// four events of a warp) shares its instructions; `on` is false in a group
-// without an event, which follows along on event g without storing anything.
+// edmd_lanes.cuh, so an event's scalar FP64 work shares its instructions;
+// `on` is false in a group without an event, which follows along on event g
+// without storing anything.
 template <int GW, bool ONE>
 __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& A, int s, int64_t g, bool on,
                                               LaneScratch* W, const Grp<GW>& G, EvResult& res) {
@@ -1707,16 +1707,15 @@ static int run_rounds(edmd_ctx* ctx, const std::vector<uint64_t>& tgt, double t_
   A.pnext = R->nsafe + 2;
   A.active = R->active; A.lim = R->lim; A.scale = R->scale; A.target = R->target; A.freeze = R->freeze;
   A.maxsafe = R->active + 1; A.thread_kernel = 1;
-  // one thread per event needs enough events to keep every SM busy with one
-  // lane each: the cells of small systems stay in L2, so 4096 events do; the
-  // events of a large system are far apart, each cell list walk misses L2,
-  // and below ~16k events a warp's 32 lanes per event hide that latency
-  // better (4096-system batch: mixed 2.6e7 coll/s, warp-only 2.4e7,
-  // thread-only 2.0e7; 10^6 disks, 8k events a round: warp 3.0e7, thread
-  // 2.1e7; 4*10^6 disks, 22k events a round: thread 3.2e7, warp 2.9e7)
+  // A warp per event at every size: with the event's scalar work spread over
+  // its lanes it beats one thread per event in batches as well (coll/s, mixed
+  // rule from 4096 or 16384 events a round against warps: 512 systems of
+  // 256-1024 disks 1.9e7 / 3.0e7, 2048 of them 3.2e7 / 4.3e7, 12 of 3-6*10^4
+  // 2.5e7 / 5.0e7, 3 of 5*10^5 5.0e7 / 6.6e7).  The FP32 screen exists in the
+  // thread kernel, so it keeps its thresholds with that flag.
   A.thr_min = (flags & EDMD_F_ROUND_THREAD) ? 0
-            : (flags & EDMD_F_ROUND_WARP) ? INT32_MAX
-            : ctx->nsys > 1 ? (TN / ctx->nsys <= 65536 ? 4096 : 16384) : (flags & EDMD_F_SCREEN) ? 16384 : INT32_MAX;
+            : (flags & EDMD_F_ROUND_WARP) || !(flags & EDMD_F_SCREEN) ? INT32_MAX
+            : TN / ctx->nsys <= 65536 ? 4096 : 16384;
   A.tlast = R->tlast; A.cnt = R->cnt; A.shp = R->shp; A.sht = R->sht; A.epoch = R->epoch; A.tsys = R->tsys; A.tx0 = R->tx0; A.ty0 = R->ty0; A.violations = R->viol;
   const unsigned gd = (unsigned)((TN + 255) / 256);
   // the serial queue keys are still in the event records only when the

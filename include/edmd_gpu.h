@@ -178,13 +178,13 @@ int edmd_advance(edmd_ctx* ctx, int64_t max_coll, double t_stop, uint32_t flags,
  * call is always the serial result and *violations_out counts the discarded
  * ones.
  * Rounds are grid-wide (selection over every tile, one kernel per step);
- * EDMD_F_ROUND_BLOCK runs them inside one block per system instead.  A round
- * of many events runs one thread per event (from 4096 events when the systems
- * average at most 65536 disks, else from 16384), a smaller one one warp per
- * event; EDMD_F_ROUND_THREAD / EDMD_F_ROUND_WARP force either.  EDMD_F_SCREEN
- * lets the thread path reject separating pairs in FP32 first, with a bound on
- * the FP32 error that keeps every FP64 decision.  All choices give the same
- * results.
+ * EDMD_F_ROUND_BLOCK runs them inside one block per system instead.  An event
+ * runs on one warp; EDMD_F_ROUND_THREAD runs one thread per event instead.
+ * EDMD_F_SCREEN lets that thread path reject separating pairs in FP32 first,
+ * with a bound on the FP32 error that keeps every FP64 decision; without
+ * EDMD_F_ROUND_WARP it also sends rounds of many events to the thread path
+ * (from 4096 events when the systems average at most 65536 disks, else from
+ * 16384).  All choices give the same results.
  * EDMD_F_TRACE records collisions in processing order.  After this call
  * edmd_advance refuses the context until edmd_load_state restages it. */
 int edmd_advance_rounds(edmd_ctx* ctx, int64_t max_coll, double t_stop, uint32_t flags,
