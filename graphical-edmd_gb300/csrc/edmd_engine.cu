@@ -87,12 +87,10 @@ __device__ __forceinline__ int grp_argmin(const Node& n, const Grp<GW>& G) {
 }
 
 // this lane's child of node `par` of level h-1 (the least of its 32 / GW
-// children), with the nodes at ia and ib taken from na and nb
+// children), with the nodes at ia and ib taken from na and nb (T, cnt: that level)
 template <int GW>
-__device__ __forceinline__ Node child_node(const SysDev& S, int h, int par, int ia, const Node& na, int ib,
+__device__ __forceinline__ Node child_node(const Node* __restrict__ T, int cnt, int par, int ia, const Node& na, int ib,
                                            const Node& nb, const Grp<GW>& G) {
-  const int cnt = S.lev_cnt[h - 1];
-  const Node* __restrict__ T = S.tree + S.lev_off[h - 1];
   Node c = empty_node(0x7fffffff);
 #pragma unroll
   for (int k = 0; k < 32; k += GW) {
@@ -104,6 +102,11 @@ __device__ __forceinline__ Node child_node(const SysDev& S, int h, int par, int 
     if (GW == 32 || node_less(m, c)) c = m;
   }
   return c;
+}
+template <int GW>
+__device__ __forceinline__ Node child_node(const SysDev& S, int h, int par, int ia, const Node& na, int ib,
+                                           const Node& nb, const Grp<GW>& G) {
+  return child_node(S.tree + S.lev_off[h - 1], S.lev_cnt[h - 1], par, ia, na, ib, nb, G);
 }
 
 __device__ __forceinline__ Node ev_node(const Ev& e, int idx) {
@@ -440,6 +443,193 @@ __device__ void do_growstop(const SysDev& S, SysState& R, const Grp<GW>& G, Warp
   tree_rebuild(S, G);
 }
 
+// offset of the next crossing of the lane's disk and its direction
+// (src/EDMD.c:2405-2482), one axis per lane
+template <int GW>
+__device__ __forceinline__ double next_crossing(const Box& B, const Grp<GW>& G, int c, double p, double v, int* dir) {
+  const bool ydim = G.lane & 2;
+  const bool neg = is_neg(v);
+  const double a = near_image((neg ? c : 1 + c) * (ydim ? B.cys : B.cxs) - p, ydim ? B.hLy : B.hLx,
+                              ydim ? B.Ly : B.Lx);
+  const double ta = div_rn(a, v);
+  const int da = (ydim ? 3 : 1) + (neg ? 0 : 1);
+  const double tb = G.shfl_xor(ta, 2);
+  const int db = G.shfl_xor(da, 2);
+  const bool ux = lt_i(ydim ? tb : ta, ydim ? ta : tb);
+  *dir = ux == ydim ? db : da;
+  return ux == ydim ? tb : ta;
+}
+
+// ---------------------------------------------------------------- two warps on one system
+
+// What the two warps of a system exchange (k_run_pair): the first runs the
+// event loop, the second does beside it whatever does not need the outcome of
+// the event, or is not needed before the next one.
+struct Aside : Flock {
+  // the event (first warp): disk i (or an order below), disk j of a collision
+  // or the direction of a crossing, the partner's counter, the time, and the
+  // calendar: paulTime of bucket k, the event's bucket b
+  int i, j;
+  bool coll, grow;
+  uint32_t ca, b;
+  double t, P;
+  uint64_t k;
+  double p[4], v[4];             // outcome (first warp): coordinate and velocity of the lane roles
+  Node leaf[2];                  // the changed leaves (first warp)
+  double tc[2];                  // next crossings (second warp): offset from t, direction
+  int dir[2];
+  double Pb;                     // paulTime of bucket b (second warp)
+  Node rest;                     // least of the leaves that the event leaves alone (second warp)
+  int self[2];                   // where disk i's candidates hold j, and j's hold i (-1: they don't)
+  Node sibs[MAXLEV][2];          // least sibling of each path node, by level
+  int off[MAXLEV], cnt[MAXLEV];  // the tree's levels
+};
+constexpr int ASIDE_END = -1, ASIDE_FLUSH = -2;
+
+// Both warps of a block meet here, three times an event: [A] the event is
+// known, [B] its outcome is, and the candidates are flown, [C] the crossings
+// and the rest of the tree are.  Neither leaves the event loop between A and C.
+__device__ __forceinline__ void pair_barrier() {
+  __syncwarp();
+  asm volatile("barrier.sync 1, 64;" ::: "memory");
+}
+
+// after this the tree in memory is up to date (first warp)
+__device__ __forceinline__ void pair_flush(Aside* as, int lane) {
+  if (lane == 0) as->i = ASIDE_FLUSH;
+  pair_barrier();
+  pair_barrier();                             // i has been read
+}
+
+// The second warp.  Between A and B: the candidates of the disks that change,
+// flown to the event's time.  It reads the state before the event, into which
+// the first warp stores nothing until B; what the event changes is known: a
+// crossing disk's cell, and the colliding disks' own records, which the first
+// warp fills in (self).  Between B and C, while the first warp solves the pairs:
+// the next crossings, the calendar's walk to the event, the paths of the last
+// event's leaves in the tree, and the least siblings along this event's paths.
+// Their minimum and the new leaves are all the first warp needs for the next
+// event, so the tree itself is one event late (pair_flush).
+__device__ __forceinline__ void run_aside(const SysDev& S, Grp<32> G, Aside* as) {
+  const int lane = G.lane;
+  const bool odd = lane & 1, ydim = lane & 2;
+  const Box& B = S.B;
+  int li = -1, lj = -1;                       // the last event's leaves
+  const int nlev = S.nlev;
+  for (int h = lane; h < nlev; h += 32) { as->off[h] = S.lev_off[h]; as->cnt[h] = S.lev_cnt[h]; }
+  G.sync();
+  auto fix_paths = [&]() {
+    if (li < 0) return;
+    Node na = as->leaf[0], nb = as->leaf[1];
+    if (lane == 0) S.tree[li] = na;
+    if (lane == 1 && lj >= 0) S.tree[lj] = nb;
+    int ia = li, ib = lj;
+#pragma unroll 1
+    for (int h = 1; h < nlev; h++) {
+      Node* T = S.tree + as->off[h];
+      const Node sa = as->sibs[h][0], sb = as->sibs[h][1];
+      ia >>= 5;
+      ib >>= 5;                               // -1: one path (left)
+      if (ib == ia) {
+        if (node_less(nb, na)) na = nb;
+        ib = -1;
+      }
+      if (node_less(sa, na)) na = sa;
+      if (ib >= 0 && node_less(sb, nb)) nb = sb;
+      if (lane == 0) T[ia] = na;
+      if (lane == 1 && ib >= 0) T[ib] = nb;
+    }
+    li = -1;
+    G.sync();
+  };
+  for (;;) {
+    pair_barrier();                                                    // A
+    const int i = as->i;
+    if (i < 0) {
+      fix_paths();
+      if (i == ASIDE_END) break;
+      pair_barrier();
+      continue;
+    }
+    const bool coll = as->coll, grow = as->grow;
+    const double t = as->t;
+    const int w = as->j;
+    const bool stale = coll && S.d[w].coll != as->ca;
+    const int j = coll && !stale ? w : -1;
+    const int my = odd && j >= 0 ? j : i;
+    int c = (ydim ? S.cy : S.cx)[my];
+    if (!coll && ydim == (w >= 3)) {
+      const int n = ydim ? B.Nyc : B.Nxc;
+      c = w & 1 ? (c == 0 ? n - 1 : c - 1) : (c + 1 == n ? 0 : c + 1);
+    }
+    int tot = 0, tot0 = 0;
+    bool corrupt = false;
+    const bool spill = gather(S, i, j, G.shfl(c, 0), G.shfl(c, 1), G.shfl(c, 2), G.shfl(c, 3), G, as, &tot, &tot0,
+                              &corrupt, [](int) {});
+    corrupt = G.any(corrupt);
+    if (lane < 2) as->self[lane] = -1;
+    if (lane == 0) { as->tot = tot; as->tot0 = tot0; as->spill = spill; as->corrupt = corrupt; }
+    G.sync();
+    if (!spill)
+      for (int f = lane >> 1; f < tot; f += 16) {
+        const int p = as->comp[f], y = lane & 1;
+        const Disk* P = S.d + p;
+        Flown& F = as->cand[f];
+        const double vel = (&P->vx)[y], lat = t - P->tl;
+        F.p[y] = (&P->x)[y] + lat * vel;
+        F.v[y] = vel;
+        double rad = P->rad, vr = 0;
+        if (grow) { vr = S.vr[p]; rad = rad + lat * vr; }
+        if (!y) {
+          F.rad = rad; F.vr = vr; F.coll = P->coll; F.id = p;
+          if (p == (f < tot0 ? j : i)) as->self[f < tot0 ? 0 : 1] = f;
+        }
+      }
+    pair_barrier();                                                    // B
+    if (!stale) {
+      int dir;
+      const double tc = next_crossing(B, G, c, as->p[lane & 3], as->v[lane & 3], &dir);
+      if (lane < 2) { as->tc[lane] = tc; as->dir[lane] = dir; }
+    }
+    double P = as->P;
+    for (uint64_t k = as->k; k < as->b; k++) P += B.dtP;
+    if (lane == 0) as->Pb = P;
+    fix_paths();
+    // a level's nodes are loaded while those of the level below are compared
+    Node rest = empty_node(0x7fffffff);
+    const Node none = rest;
+    int ia = i, ib = j;
+    auto load = [&](int h, Node& ca, Node& cb) {
+      const Node* T = S.tree + as->off[h - 1];
+      const int cnt = as->cnt[h - 1], pa = ia >> 5, pb = ib >> 5;
+      ca = child_node(T, cnt, pa, ia, none, ib, none, G);
+      const bool apart = pb >= 0 && pb != pa;
+      if (apart) cb = child_node(T, cnt, pb, ib, none, -1, none, G);
+      ia = pa;
+      ib = apart ? pb : -1;
+      return apart;
+    };
+    Node ca, cb = none, da, db = none;
+    bool apart = load(1, ca, cb), next = false;
+#pragma unroll 1
+    for (int h = 1; h < nlev; h++) {
+      if (h + 1 < nlev) next = load(h + 1, da, db);
+      int src = grp_argmin(ca, G);
+      if (lane == src) as->sibs[h][0] = ca;
+      if (node_less(ca, rest)) rest = ca;
+      if (apart) {
+        src = grp_argmin(cb, G);
+        if (lane == src) as->sibs[h][1] = cb;
+        if (node_less(cb, rest)) rest = cb;
+      }
+      ca = da; cb = db; apart = next;
+    }
+    if (lane == grp_argmin(rest, G)) as->rest = rest;
+    li = i; lj = j;
+    pair_barrier();                                                    // C
+  }
+}
+
 // ---------------------------------------------------------------- run loop
 
 // what ends a stretch of disk events
@@ -456,9 +646,11 @@ enum { END_STOP, END_SPECIAL, END_SHARE };
 // of the loop, and everything rare is left to serve_special.
 // ADD = false: a context without additive-contact systems (the rule's
 // switch compiled out of the pair solves and the collision rule)
-template <int GW, bool ADD, bool GROW>
+// PAIR: a second warp works beside this one (run_aside).
+template <int GW, bool ADD, bool GROW, bool PAIR>
 __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int64_t max_coll, const Grp<GW>& G,
-                                          WarpSmem* sm, int64_t& logged, int64_t& nev, int64_t share_end, int* special) {
+                                          WarpSmem* sm, Aside* as, int64_t& logged, int64_t& nev, int64_t share_end,
+                                          int* special) {
   const int lane = G.lane;
   const bool odd = lane & 1, ydim = lane & 2;
   const Box& B = S.B;
@@ -478,6 +670,8 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
   }
   G.sync();
   const int root = S.lev_off[S.nlev - 1];
+  Node top;                                   // PAIR: the root
+  if constexpr (PAIR) top = S.tree[root];
   uint64_t ncoll = 0, nstale = 0, npair = 0, nlog = st->nlog;
   const uint64_t ntrace0 = st->ntrace;
   const int64_t nev0 = nev;
@@ -492,24 +686,28 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
       else end = END_SHARE;
       break;
     }
-    Node r;
+    Node r = top;
     int guard = 0;
     for (;;) {
-      r = S.tree[root];
+      if constexpr (!PAIR) r = S.tree[root];
       if (r.b == BINF || (uint64_t)r.b >= Q.next_wrap) {
         if (r.b == BINF && Q.ovf == NIL) { status = EDMD_ERR_BUDGET; break; }
         while (Q.k < Q.next_wrap) { Q.P += B.dtP; Q.k++; }
+        if constexpr (PAIR) pair_flush(as, lane);
         Q = do_wrap(S, Q, G);
+        if constexpr (PAIR) r = S.tree[root];
         if (Q.ovf == OVF_CORRUPT) { Q.ovf = NIL; status = EDMD_ERR_BUDGET; break; }
         if (++guard > (1 << 20)) { status = EDMD_ERR_BUDGET; break; }
         continue;
       }
-      while (Q.k < (uint64_t)r.b) { Q.P += B.dtP; Q.k++; }
       break;
     }
     if (status != EDMD_OK) break;
     const int e = r.idx;
     const Ev E = S.ev[e];
+    // the calendar's walk to the event: by the second warp if that runs it
+    if (!PAIR || e >= 2 * N || le_i(A.t_stop, E.t))
+      while (Q.k < (uint64_t)r.b) { Q.P += B.dtP; Q.k++; }
     if (le_i(A.t_stop, E.t)) { stop = EDMD_STOP_TIME; break; }
     t = E.t;
     nev++;
@@ -521,6 +719,14 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
     {
       const bool coll = e >= N;
       const int i = coll ? e - N : e, j = coll ? E.j : i;
+      if constexpr (PAIR) {
+        if (lane == 0) {
+          as->i = i; as->j = E.j; as->coll = coll; as->grow = GROW; as->ca = E.ca; as->t = t;
+          as->P = Q.P; as->k = Q.k; as->b = r.b;
+        }
+        if (Q.k < (uint64_t)r.b) Q.k = r.b;
+        pair_barrier();                                                // A
+      }
       const int my = odd ? j : i;
       Disk* const D = S.d + my;
       Own own;
@@ -544,6 +750,13 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
       }
       const bool stale = coll && E.ca != G.shfl(hits, 1);
       const bool two = coll && !stale;       // a second disk changes
+      // the state is stored only after the second warp has read it
+      auto outcome = [&]() {
+        if constexpr (PAIR) {
+          if (lane < 4) { as->p[lane] = own.p; as->v[lane] = own.v; }
+          pair_barrier();                                              // B
+        }
+      };
       if (two) {
         // ---------------- collision (doTheCollisionNormal 3542 / Grow 3465)
         if ((A.flags & EDMD_F_TRACE) && S.trace && (int64_t)(ntrace0 + ncoll) < S.trace_cap) {
@@ -597,6 +810,7 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
           const double delta = 0;
           own.v += flip(collKernel * mo * dr - 2 * mo * inv * delta * dr, odd);
         }
+        outcome();
         if (lane < 4) {
           *axis_pos(D, ydim) = own.p;
           *axis_vel(D, ydim) = own.v;
@@ -607,6 +821,7 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
           }
         }
       } else if (stale) {
+        outcome();
         if (lane == 0 || lane == 2) *axis_pos(D, ydim) = own.p;
         if (lane == 0) {
           D->tl = t;
@@ -623,6 +838,7 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
           else { if (own.c + 1 == n) { own.c = 0; wrap = 1; } else own.c += 1; }
         }
         const int to = G.shfl(own.c, 2) * B.Nxc + G.shfl(own.c, 0);
+        outcome();
         if (lane == 0 || lane == 2) {
           *axis_pos(D, ydim) = own.p;
           (ydim ? S.cy : S.cx)[i] = own.c;
@@ -659,23 +875,30 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
         }
         Q.ovf = G.shfl(first, 0);
       }
-      // the next crossing (src/EDMD.c:2405-2482): one axis per lane
+      // the next crossing and collision
       double tc = 0;
       int dir = 0;
-      if (!stale) {
-        const bool neg = is_neg(own.v);
-        const double a = near_image((neg ? own.c : 1 + own.c) * (ydim ? B.cys : B.cxs) - own.p, ydim ? B.hLy : B.hLx,
-                                    ydim ? B.Ly : B.Lx);
-        const double ta = div_rn(a, own.v);
-        const int da = (ydim ? 3 : 1) + (neg ? 0 : 1);
-        const double tb = G.shfl_xor(ta, 2);
-        const int db = G.shfl_xor(da, 2);
-        const bool ux = lt_i(ydim ? tb : ta, ydim ? ta : tb);
-        tc = ux == ydim ? tb : ta;
-        dir = ux == ydim ? db : da;
+      Next nx;
+      if constexpr (PAIR) {
+        if (two && lane < 4) {                  // the colliding disks as each other's candidates
+          const int f = as->self[odd ? 0 : 1];
+          if (f >= 0) {
+            Flown& F = as->cand[f];
+            F.p[ydim ? 1 : 0] = own.p; F.v[ydim ? 1 : 0] = own.v;
+            if (!ydim) { F.rad = own.rad; F.coll = hits + 1; }
+          }
+        }
+        G.sync();
+        nx = predict2<GW, ADD, GROW, GW, true>(S, t, i, two ? j : -1, own, &npair, G, sm, &ovl, &oa, &ob, [](int) {}, [](int) { return 0; }, as);
+        pair_barrier();                                                // C
+        tc = as->tc[lane & 1];
+        dir = as->dir[lane & 1];
+        Q.P = as->Pb;
+      } else {
+        if (!stale) tc = next_crossing(B, G, own.c, own.p, own.v, &dir);
+        G.sync();
+        nx = predict2<GW, ADD, GROW, GW>(S, t, i, two ? j : -1, own, &npair, G, sm, &ovl, &oa, &ob, [](int) {}, [](int) { return 0; });
       }
-      G.sync();
-      const Next nx = predict2<GW, ADD, GROW, GW>(S, t, i, two ? j : -1, own, &npair, G, sm, &ovl, &oa, &ob, [](int) {}, [](int) { return 0; });
       // addEventToQueue (src/EDMD.c:2144): lanes 0 and 1 take the crossings of
       // the two disks, lanes 2 and 3 their collisions; in that order they get
       // the insertion counters and join the overflow list
@@ -712,10 +935,19 @@ __device__ __forceinline__ int run_events(const SysDev& S, const RunArgs& A, int
         o.b = G.shfl_xor(n.b, 2); o.idx = G.shfl_xor(n.idx, 2);
         if (node_less(o, n)) n = o;
       }
-      path_update(S, i, two ? j : -1, shfl_node(n, 0, G), shfl_node(n, 1, G), G);
+      if constexpr (PAIR) {
+        // the root: the changed leaves (lanes 0 and 1) and all others (lane 2)
+        if (lane < 2) as->leaf[lane] = n;
+        if (lane == 2) n = as->rest;
+        if (lane > 2 || (lane == 1 && !two)) n = empty_node(0x7fffffff);
+        top = shfl_node(n, grp_argmin(n, G), G);
+      } else {
+        path_update(S, i, two ? j : -1, shfl_node(n, 0, G), shfl_node(n, 1, G), G);
+      }
     }
     if (ovl) { status = oa == OVL_CORRUPT ? EDMD_ERR_BUDGET : EDMD_ERR_OVERLAP; break; }
   }
+  if constexpr (PAIR) pair_flush(as, lane);
   const double vir = G.shfl(ctl, virial_lane<GW>(lane & 3));
   if (lane < 4) st->collT[lane] = vir;
   if (lane == 0) {
@@ -785,15 +1017,15 @@ __device__ __noinline__ bool serve_special(const SysDev& S, uint32_t flags, int 
 
 // the event loop of one system, at most `share` events of it; true when the
 // call is done with the system
-template <int GW, bool ADD = true>
+template <int GW, bool ADD = true, bool PAIR = false>
 __device__ bool run_system(const SysDev& S, const RunArgs& A, const Grp<GW>& G, WarpSmem* sm, RunProgress& pr,
-                           int64_t share) {
+                           int64_t share, Aside* as = nullptr) {
   if (S.st->status != EDMD_OK) return true;
   const int64_t share_end = A.max_events - pr.nev > share ? pr.nev + share : A.max_events;
   for (;;) {
     int special = 0, end;
-    if (S.st->grow) end = run_events<GW, ADD, true>(S, A, A.max_coll, G, sm, pr.logged, pr.nev, share_end, &special);
-    else end = run_events<GW, ADD, false>(S, A, A.max_coll, G, sm, pr.logged, pr.nev, share_end, &special);
+    if (S.st->grow) end = run_events<GW, ADD, true, PAIR>(S, A, A.max_coll, G, sm, as, pr.logged, pr.nev, share_end, &special);
+    else end = run_events<GW, ADD, false, PAIR>(S, A, A.max_coll, G, sm, as, pr.logged, pr.nev, share_end, &special);
     if (end == END_SHARE) return false;
     if (end != END_SPECIAL || !serve_special<GW, ADD>(S, A.flags, special, G, sm)) return true;
   }
@@ -881,6 +1113,34 @@ k_run(const SysDev* __restrict__ sys, RunArgs A) {
   }
 }
 
+// Two warps per system, one system per block.  An event is one chain of
+// dependent instructions (64 cycles for each FP64 one, 106 for a load that hits
+// L1), so a context of few systems leaves the GPU idle whatever its lanes do;
+// run_aside takes ~40 % of the chain off it: of ~10.5k cycles per event the
+// neighbour lists and candidates were 2.4k, the crossings 1.0k, the tree 1.4k to
+// 2.0k and the calendar 0.2k.  Measured, one warp / two (600 collisions a
+// system, ms): 1 system of 1000 disks 6.2 / 4.9, 304 of 128-512 7.1 / 5.7, 912
+// 8.2 / 6.9, 1064 of 64-1024 8.9 / 7.4, 1216 8.4 / 7.5; with registers for 10
+// blocks per SM 1520 of 128-512 9.1 / 8.7 but 304 6.0, and 1824 10.1 / 10.1.
+constexpr int PAIR_PER_SM = 8;
+template <bool ADD>
+__global__ void __launch_bounds__(64, PAIR_PER_SM) k_run_pair(const SysDev* __restrict__ sys, RunArgs A) {
+  __shared__ WarpSmem smem;
+  __shared__ Aside as;
+  const Grp<32> G(threadIdx.x);
+  const int p = blockIdx.x;
+  if (p >= A.nrun) return;                    // both warps
+  const SysDev& S = sys[A.order ? A.order[p] : p];
+  if (threadIdx.x < 32) {
+    RunProgress pr{0, 0};
+    run_system<32, ADD, true>(S, A, G, &smem, pr, A.max_events, &as);
+    if (G.lane == 0) as.i = ASIDE_END;
+    pair_barrier();                           // A, the last
+  } else {
+    run_aside(S, G, &as);
+  }
+}
+
 __global__ void k_waiting(RunArgs A) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < A.nwait) A.waiting[k] = A.nrun + k;
@@ -888,25 +1148,27 @@ __global__ void k_waiting(RunArgs A) {
   if (k == 0) { A.ticket[0] = 0; A.ticket[1] = (unsigned)A.nwait; }
 }
 
-// How nsys systems are run with gw lanes each: kernel and warps per block.
-// Measured with 32 lanes (203 disks alone / 192 growth starts / 1824 < 2600
-// mixed systems, ms; every build has the same event loop):
+// How nsys systems are run with gw lanes each: kernel, warps and systems of a
+// block.  With 32 lanes up to eight systems per SM get two warps each
+// (k_run_pair; `pair`: unless they would not all be resident).  One warp each,
+// measured (203 disks alone / 192 growth starts / 1824 < 2600 mixed systems,
+// ms; every build has the same event loop):
 //   3 blocks per SM, 168 registers: 1.41 / 15.2 / 36
 //   4 blocks, 128 registers:        1.45 / 15.5 / 40.5 (2432 warps, a second wave)
 //   5 blocks, 102 registers:        1.50 / 16.4 / 30.2 (3040 warps)
 //   6 blocks, 85 registers:         1.58 / 17.6 / 32.2
 // so systems that all find a warp at three blocks per SM run there, without
-// spills, and larger batches at five.  Few enough for one warp in each SM
-// sub-partition, they are spread over the SMs in one-warp blocks.
+// spills, and larger batches at five.
 using RunKernel = void (*)(const SysDev*, RunArgs);
-struct RunShape { RunKernel kernel; int warps; };
-RunShape run_shape(int gw, bool additive, int nsys, int nsm) {
-  if (gw == 4) return {k_run<4, true, 4>, WARPS_PER_BLOCK};
-  if (gw == 8) return {k_run<8, true, 4>, WARPS_PER_BLOCK};
-  if (gw == 16) return {k_run<16, true, 4>, WARPS_PER_BLOCK};
-  if (nsys <= 3 * WARPS_PER_BLOCK * nsm)
-    return {additive ? k_run<32, true, 3> : k_run<32, false, 3>, nsys <= 4 * nsm ? 1 : WARPS_PER_BLOCK};
-  return {additive ? k_run<32, true, 5> : k_run<32, false, 5>, WARPS_PER_BLOCK};
+struct RunShape { RunKernel kernel; int warps, systems; };   // a block's warps and systems
+RunShape run_shape(int gw, bool additive, int nsys, int nsm, bool pair = true) {
+  const int W = WARPS_PER_BLOCK;
+  if (gw == 4) return {k_run<4, true, 4>, W, W * 8};
+  if (gw == 8) return {k_run<8, true, 4>, W, W * 4};
+  if (gw == 16) return {k_run<16, true, 4>, W, W * 2};
+  if (pair && nsys <= PAIR_PER_SM * nsm) return {additive ? k_run_pair<true> : k_run_pair<false>, 2, 1};
+  if (nsys <= 3 * W * nsm) return {additive ? k_run<32, true, 3> : k_run<32, false, 3>, W, W};
+  return {additive ? k_run<32, true, 5> : k_run<32, false, 5>, W, W};
 }
 
 // ---------------------------------------------------------------- shared-memory kernel
@@ -1663,10 +1925,14 @@ extern "C" int edmd_load_state(edmd_ctx* ctx, const double* x, const double* y, 
 // k_run on `nsys` places on the context's stream, with the tables of waiting
 // systems when they exceed the resident lane groups
 static int run_launch(edmd_ctx* ctx, RunArgs A, int nsys, int gw, int nsm) {
-  const RunShape shape = run_shape(gw, ctx->any_additive, nsys, nsm);
-  const int per_block = shape.warps * (32 / gw);
+  RunShape shape = run_shape(gw, ctx->any_additive, nsys, nsm);
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shape.kernel, 32 * shape.warps, 0));
+  if (shape.systems == 1 && per_sm * nsm < nsys) {
+    shape = run_shape(gw, ctx->any_additive, nsys, nsm, false);
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shape.kernel, 32 * shape.warps, 0));
+  }
+  const int per_block = shape.systems;
   const int grid = std::max(1, std::min(per_sm * nsm, (nsys + per_block - 1) / per_block));
   A.nrun = std::min(nsys, grid * per_block);
   A.nwait = nsys - A.nrun;

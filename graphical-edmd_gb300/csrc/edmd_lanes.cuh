@@ -94,16 +94,15 @@ __device__ __forceinline__ void best_merge(uint64_t& bk, int& bo, int& bp, uint3
 // candidates of an event (about 6 per disk) still fit one pass of a warp.
 // Same operations and roundings as coll_time_normal_i / coll_time_grow (the
 // sums of two products commute).  Every lane of the group takes part; `act`
-// marks the pairs that count.
+// marks the pairs that count.  The candidate comes flown to t: coordinate and
+// velocity along the lane's axis, radius, growth rate.
 template <int GW, bool ADD, bool GROW>
-__device__ __forceinline__ double pair_time_lanes(const Box& B, const Grp<GW>& G, bool act, double p1, double v1,
-                                                  double rad1, double vr1, const Disk* P, const double* vr2p,
-                                                  double t, bool* ovl) {
+__device__ __forceinline__ double pair_time_flown(const Box& B, const Grp<GW>& G, bool act, double p1, double v1,
+                                                  double rad1, double vr1, double p2, double vel, double rad2,
+                                                  double vr2, bool* ovl) {
   const bool y = G.lane & 1;
-  const double pos = (&P->x)[y ? 1 : 0], vel = (&P->vx)[y ? 1 : 0], rad2 = P->rad;
-  const double lat2 = t - P->tl;
   const double dv = vel - v1;
-  const double d = near_image((pos + lat2 * vel) - p1, y ? B.hLy : B.hLx, y ? B.Ly : B.Lx);
+  const double d = near_image(p2 - p1, y ? B.hLy : B.hLx, y ? B.Ly : B.Lx);
   double b = d * dv, v2 = dv * dv, d2 = d * d;
   b += G.shfl_xor(b, 1);
   v2 += G.shfl_xor(v2, 1);
@@ -119,9 +118,8 @@ __device__ __forceinline__ double pair_time_lanes(const Box& B, const Grp<GW>& G
     if (is_neg(det)) return NEVER;
     return div_rn(-b - sqrt_rn(det), v2);
   } else {
-  const double vr2 = *vr2p;
   const double dvr = vr1 + vr2;
-  const double dr = contact(B, rad1, rad2 + lat2 * vr2);
+  const double dr = contact(B, rad1, rad2);
   b -= dvr * dr;
   const double den = v2 - dvr * dvr, gap = d2 - dr * dr;
   const double det = b * b - den * gap;
@@ -141,6 +139,22 @@ __device__ __forceinline__ double pair_time_lanes(const Box& B, const Grp<GW>& G
   if (gap < -0.01) *ovl = true;
   return NEVER;
   }
+}
+
+// the same with the candidate's record, flown here
+template <int GW, bool ADD, bool GROW>
+__device__ __forceinline__ double pair_time_lanes(const Box& B, const Grp<GW>& G, bool act, double p1, double v1,
+                                                  double rad1, double vr1, const Disk* P, const double* vr2p,
+                                                  double t, bool* ovl) {
+  const bool y = G.lane & 1;
+  const double pos = (&P->x)[y ? 1 : 0], vel = (&P->vx)[y ? 1 : 0];
+  const double lat2 = t - P->tl;
+  double rad2 = P->rad, vr2 = 0;
+  if constexpr (GROW) {
+    vr2 = *vr2p;
+    rad2 = rad2 + lat2 * vr2;
+  }
+  return pair_time_flown<GW, ADD, GROW>(B, G, act, p1, v1, rad1, vr1, pos + lat2 * vel, vel, rad2, vr2, ovl);
 }
 
 // group-relative lane of the least (time key, scan order), word by word like
@@ -164,26 +178,21 @@ __device__ __forceinline__ int best_lane(uint64_t k, int o, const Grp<GW>& G) {
   return __ffs(q) - 1;
 }
 
-// collisionEventNormal / Grow (src/EDMD.c:2829 / 3104) for disks a0 and a1
-// (a1 may be -1), both current at t, whose lane roles hold `own`: scan the
-// 3x3 neighbour cells, dy outer and dx inner, list order, keep the first
-// strict minimum.  The (disk, cell) walks are tasks t = 0..8 (a0's cells in
-// scan order) and 9..17 (a1's): task t runs on lane t % GW, a lane with two
-// tasks walks both lists at once.  The candidates are then packed over the
-// group in task order and solved by two lanes each.
-// `on_cell(cell)` is called for every cell scanned, by the lane that walks it;
-// `tag_of(p)` gives 0..3 for a candidate, loaded beside its record.
-// ORD: lanes the naming order of overlapping pairs refers to.
-template <int GW, bool ADD, bool GROW, int ORD, class F, class T>
-__device__ __forceinline__ Next predict2(const SysDev& S, double t, int a0, int a1, const Own& own,
-                                         uint64_t* npair, const Grp<GW>& G, LaneScratch* sm, bool* ovl, int* ovl_a,
-                                         int* ovl_b, F&& on_cell, T&& tag_of) {
+// The candidates of the disks a0 at cell (X0, Y0) and a1 (may be -1) at
+// (X1, Y1): the 3x3 neighbour cells, dy outer and dx inner, list order.  The
+// (disk, cell) walks are tasks t = 0..8 (a0's cells in scan order) and 9..17
+// (a1's): task t runs on lane t % GW, a lane with two tasks walks both lists
+// at once.  The candidates are then packed over the group in task order, *tot
+// of them, *tot0 for a0.  True when a list is longer than MAXC (nothing
+// packed).  `on_cell(cell)` is called for every cell scanned, by the lane that
+// walks it; *corrupt is set on a lane whose list is longer than the system.
+template <int GW, class F>
+__device__ __forceinline__ bool gather(const SysDev& S, int a0, int a1, int X0, int X1, int Y0, int Y1,
+                                       const Grp<GW>& G, LaneScratch* sm, int* tot, int* tot0, bool* corrupt,
+                                       F&& on_cell) {
   const Box& B = S.B;
   const int lane = G.lane;
-  const double dinit = GROW ? 10000000 : NEVER;
-  const uint32_t coll0 = S.d[0].coll;
   const int ntask = a1 >= 0 ? 18 : 9;
-  const int X0 = G.shfl(own.c, 0), X1 = G.shfl(own.c, 1), Y0 = G.shfl(own.c, 2), Y1 = G.shfl(own.c, 3);
   // the tasks of this lane: t = lane + k GW, k < NT (a warp: one task per
   // lane; 16 lanes: two; 8 lanes: three; 4 lanes: five)
   constexpr int NT = (18 + GW - 1) / GW;
@@ -200,7 +209,6 @@ __device__ __forceinline__ Next predict2(const SysDev& S, double t, int a0, int 
     if (u < ntask) on_cell(hc[k]);
     ct[k] = 0;
   }
-  bool lcorrupt = false;
   {
     int guard = 0;                   // the lists hold N disks in all
     bool more = true;
@@ -216,16 +224,73 @@ __device__ __forceinline__ Next predict2(const SysDev& S, double t, int a0, int 
         }
       }
     }
-    // a list longer than N is corrupt: reported like an overlap, with the
-    // marker OVL_CORRUPT in place of the first disk (EDMD_ERR_BUDGET)
 #pragma unroll
     for (int k = 0; k < NT; k++)
-      if (pt[k] != NIL) lcorrupt = true;
+      if (pt[k] != NIL) *corrupt = true;
   }
   bool over = false;
 #pragma unroll
   for (int k = 0; k < NT; k++) over |= ct[k] > MAXC;
-  const bool spill = G.any(over);
+  if (G.any(over)) return true;
+  // exclusive prefix of the counts (at most 7) in task order, bit by bit
+  int ex[NT];
+  int base = 0;
+  const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+  for (int k = 0; k < NT; k++) {
+    const unsigned c0 = G.ballot(ct[k] & 1), c1 = G.ballot(ct[k] & 2), c2 = G.ballot(ct[k] & 4);
+    ex[k] = base + __popc(c0 & below) + 2 * __popc(c1 & below) + 4 * __popc(c2 & below);
+    base += __popc(c0) + 2 * __popc(c1) + 4 * __popc(c2);
+  }
+  // a0's candidates are tasks 0..8: their count is the prefix at task 9
+  *tot0 = G.shfl(ex[9 / GW], 9 % GW);
+  *tot = base;
+#pragma unroll
+  for (int k = 0; k < NT; k++) {
+    const int u = lane + k * GW;
+    for (int m = 0; m < ct[k]; m++) {
+      sm->comp[ex[k] + m] = sm->reg[u * MAXC + m];
+      sm->ord[ex[k] + m] = (int16_t)(qt[k] * MAXC + m);
+    }
+  }
+  G.sync();
+  return false;
+}
+
+// Candidates found and flown to the event's time by another warp (gather): the
+// prediction is then left with the pair solves.
+struct Flown { double p[2], v[2], rad, vr; uint32_t coll; int32_t id; };
+struct Flock : LaneScratch {
+  Flown cand[2 * 9 * MAXC];
+  int tot, tot0;
+  bool spill, corrupt;
+};
+
+// collisionEventNormal / Grow (src/EDMD.c:2829 / 3104) for disks a0 and a1
+// (a1 may be -1), both current at t, whose lane roles hold `own`: of the
+// candidates (gather) keep the first strict minimum, each solved by two lanes.
+// `tag_of(p)` gives 0..3 for a candidate, loaded beside its record.
+// ORD: lanes the naming order of overlapping pairs refers to.
+// FLOWN: the candidates come from `flock`.
+template <int GW, bool ADD, bool GROW, int ORD, bool FLOWN = false, class F, class T>
+__device__ __forceinline__ Next predict2(const SysDev& S, double t, int a0, int a1, const Own& own,
+                                         uint64_t* npair, const Grp<GW>& G, LaneScratch* sm, bool* ovl, int* ovl_a,
+                                         int* ovl_b, F&& on_cell, T&& tag_of, const Flock* flock = nullptr) {
+  const Box& B = S.B;
+  const int lane = G.lane;
+  const double dinit = GROW ? 10000000 : NEVER;
+  const uint32_t coll0 = S.d[0].coll;
+  const int ntask = a1 >= 0 ? 18 : 9;
+  const int X0 = G.shfl(own.c, 0), X1 = G.shfl(own.c, 1), Y0 = G.shfl(own.c, 2), Y1 = G.shfl(own.c, 3);
+  // a list longer than N is corrupt: reported like an overlap, with the
+  // marker OVL_CORRUPT in place of the first disk (EDMD_ERR_BUDGET)
+  bool lcorrupt = false, spill;
+  int tot = 0, tot0 = 0;
+  if constexpr (FLOWN) {
+    tot = flock->tot; tot0 = flock->tot0; spill = flock->spill; lcorrupt = flock->corrupt;
+  } else {
+    spill = gather(S, a0, a1, X0, X1, Y0, Y1, G, sm, &tot, &tot0, &lcorrupt, on_cell);
+  }
   uint64_t bd0 = cand_key(dinit), bd1 = bd0;
   int bo0 = -1, bo1 = -1, bp0 = 0, bp1 = 0;
   uint32_t bc0 = 0, bc1 = 0;
@@ -233,30 +298,7 @@ __device__ __forceinline__ Next predict2(const SysDev& S, double t, int a0, int 
   // candidates have when each takes a lane of its own
   uint32_t lk = 0xffffffffu;
   int la = -1, lb = -1;
-  int tot;
   if (!spill) {
-    // exclusive prefix of the counts (at most 7) in task order, bit by bit
-    int ex[NT];
-    int base = 0;
-    const unsigned below = (1u << lane) - 1u;
-#pragma unroll
-    for (int k = 0; k < NT; k++) {
-      const unsigned c0 = G.ballot(ct[k] & 1), c1 = G.ballot(ct[k] & 2), c2 = G.ballot(ct[k] & 4);
-      ex[k] = base + __popc(c0 & below) + 2 * __popc(c1 & below) + 4 * __popc(c2 & below);
-      base += __popc(c0) + 2 * __popc(c1) + 4 * __popc(c2);
-    }
-    // a0's candidates are tasks 0..8: their count is the prefix at task 9
-    const int tot0 = G.shfl(ex[9 / GW], 9 % GW);
-    tot = base;
-#pragma unroll
-    for (int k = 0; k < NT; k++) {
-      const int u = lane + k * GW;
-      for (int m = 0; m < ct[k]; m++) {
-        sm->comp[ex[k] + m] = sm->reg[u * MAXC + m];
-        sm->ord[ex[k] + m] = (int16_t)(qt[k] * MAXC + m);
-      }
-    }
-    G.sync();
     for (int f0 = 0; f0 < tot; f0 += GW / 2) {
       const int f = f0 + (lane >> 1);
       const bool act = f < tot;
@@ -264,13 +306,22 @@ __device__ __forceinline__ Next predict2(const SysDev& S, double t, int a0, int 
       const int src = (g1 ? 1 : 0) | ((lane & 1) << 1);
       const double p1 = G.shfl(own.p, src), v1 = G.shfl(own.v, src), rad1 = G.shfl(own.rad, src);
       const double vr1 = GROW ? G.shfl(own.vr, src) : 0.0;
-      const int p = act ? sm->comp[f] : a0;
-      const int o = act ? (int)sm->ord[f] << 2 | tag_of(p) : 0;
-      const Disk* P = S.d + p;
-      const uint32_t pc = P->coll;
+      int p, o;
+      uint32_t pc;
+      double dt;
       bool ov = false;
-      const uint64_t kd =
-          cand_key(pair_time_lanes<GW, ADD, GROW>(B, G, act, p1, v1, rad1, vr1, P, S.vr + p, t, &ov));
+      if constexpr (FLOWN) {
+        const Flown& P = flock->cand[act ? f : 0];
+        p = P.id; o = (int)flock->ord[act ? f : 0] << 2; pc = P.coll;
+        dt = pair_time_flown<GW, ADD, GROW>(B, G, act, p1, v1, rad1, vr1, P.p[lane & 1], P.v[lane & 1], P.rad, P.vr, &ov);
+      } else {
+        p = act ? sm->comp[f] : a0;
+        o = act ? (int)sm->ord[f] << 2 | tag_of(p) : 0;
+        const Disk* P = S.d + p;
+        pc = P->coll;
+        dt = pair_time_lanes<GW, ADD, GROW>(B, G, act, p1, v1, rad1, vr1, P, S.vr + p, t, &ov);
+      }
+      const uint64_t kd = cand_key(dt);
       if (ov) {
         const uint32_t k = ((uint32_t)(f % ORD) << 16) | (0xffffu - (uint32_t)f);
         if (k < lk) { lk = k; la = g1 ? a1 : a0; lb = p; }

@@ -70,7 +70,7 @@ def test_crowded_cells(edmd, oracle, per_cell):
 
 
 # number of systems around one warp per SM sub-partition, one block of four warps at three per SM, and the five-block build
-@pytest.mark.parametrize("nsys", [3, 610, 1830, 3100])
+@pytest.mark.parametrize("nsys", [3, 610, 1216, 1217, 1830, 3100])
 def test_batch_sizes_share_one_result(edmd, oracle, nsys):
     starts = [start(edmd, 40 + 2 * (k % 5), 0.5, k % 5 + 1) for k in range(5)]
     eng = edmd.Engine([starts[k % 5] for k in range(nsys)])
@@ -86,6 +86,31 @@ def test_batch_sizes_share_one_result(edmd, oracle, nsys):
             for k in KEYS:
                 np.testing.assert_array_equal(st[k][off[s]:off[s + 1]], ost[k])
     eng.close()
+
+
+# 20 disks: a tree of two levels and a box of few cells; 29 / 30: two and three levels; 200: cells of their own
+@pytest.mark.parametrize("N,additive", [(20, False), (29, False), (30, True), (200, False), (200, True)])
+def test_two_warps_equal_one(edmd, N, additive):
+    """Few systems have two warps each: growth, samples, calendar wraps and stops of every kind as with 16 lanes."""
+    kw = dict(tmax=1e9, dtime=0.4, dtime_thermo=0.3, contact=edmd.CONTACT_ADDITIVE if additive else edmd.CONTACT_NONADDITIVE)
+    res = []
+    for lanes in (16, 32):
+        s = edmd.grow_start(N, 0.45, 11)
+        s["desc"] = edmd.default_desc(s["N"], s["Lx"], s["Ly"], vr_base=s["vr_base"], **kw)
+        edmd.set_warp_group(lanes)
+        try:
+            eng = edmd.Engine([s, s])
+            for k in range(1, 30):
+                eng.advance(max_coll=k * 7 if k % 3 else 2 ** 62, t_stop=1.7 * k if k % 3 == 0 else float("inf"))
+            eng.sync()
+            c = {k: v for k, v in eng.counters(1).items()}
+            res.append((eng.state(1), c, eng.thermo(1)))
+            eng.close()
+        finally:
+            edmd.set_warp_group(32)
+    same(res[0][0], res[1][0])
+    assert res[0][1] == res[1][1]
+    np.testing.assert_array_equal(res[0][2], res[1][2])
 
 
 @pytest.mark.parametrize("energy,t0,t1", [(1.0, 0.0, 0.02), (1.0, 70.0, 70.6), (1e6, 0.0, 0.0006), (1e-6, 3000.0, 3100.0)])
