@@ -40,6 +40,7 @@
 // have been given (new_rank), other new ones rank after inherited ones; two
 // valid mutual events give bit-identical velocities in either order since
 // the collision rule is odd in (dx, dy) and in (dvx, dvy).
+#include <algorithm>
 #include <cstdio>
 #include <cstdint>
 #include <cstring>
@@ -1637,7 +1638,11 @@ cudaError_t enqueue_round(edmd_ctx* ctx, const RoundBufs* R, const RoundArgs& A0
   A.nsafe_next = R->nsafe + ((k + 1) & 1);
   A.thread_kernel = with_thread ? 1 : 0;
   const bool one = ctx->nsys == 1;
-  const unsigned tgrid = (unsigned)(R->ntiles < nsm * 8 ? R->ntiles : nsm * 8);
+  // a block per tile: a block spends most of a tile at its barriers, waiting for
+  // the warp whose event is being checked, so the next tile of a block that
+  // holds several starts late (10^6 disks, 2,130 tiles on 1,216 blocks: 49.1 ms
+  // against 47.1; 4*10^6 disks, 8,500 tiles: 104.3 against 97.8)
+  const unsigned tgrid = (unsigned)std::min<int64_t>(R->ntiles, nsm * 64);
   switch (A.radius) {
 #define SEL_CASE(R) \
     case R: \
