@@ -33,7 +33,9 @@ struct edmd_ctx {
   SysDev* ds = nullptr;
   int64_t* doff = nullptr;          // first disk of each system
   unsigned long long* bad = nullptr;  // first bad disk of a staged state
-  // device arrays shared by all systems (each system owns a slice)
+  // device arrays shared by all systems (each system owns a slice), in one
+  // allocation
+  char* slab = nullptr;
   Disk* d = nullptr; double* vr = nullptr;
   int32_t *cx = nullptr, *cy = nullptr, *prv = nullptr, *crossX = nullptr, *crossY = nullptr;
   int32_t* head = nullptr;
