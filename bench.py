@@ -86,18 +86,20 @@ DIFF_N, DIFF_PHI, DIFF_SEED, DIFF_COLL = 1024, 0.60, 11, 10000
 # configuration (workload, engine, lanes per system)
 PROFILED = {
     ("batched", "warp", 32): dict(
-        kernel="k_run<32, false>", dram_bytes_per_collision=5765.0, fp64_pipe_active=0.543,
-        capture="ncu --set full --clock-control none -k regex:k_run -s 4 -c 1 python bench.py --workload batched "
+        kernel="k_run<32, false, 5>", dram_bytes_per_collision=6434.0, fp64_pipe_active=0.514,
+        capture="ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,"
+                "sm__pipe_fp64_cycles_active.avg.pct_of_peak_sustained_active --clock-control none -k regex:k_run "
+                "-s 4 -c 1 python bench.py --workload batched "
                 "--nsys 4096 --coll 2000 --steps 1 --warmup 3 --no-cpu-baseline --no-secondary --no-tune "
-                "(dram__bytes_read.sum + dram__bytes_write.sum = 47.23 GB for 8.192e6 collisions)"),
+                "(dram__bytes_read.sum + dram__bytes_write.sum = 52.71 GB for 8.192e6 collisions)"),
     ("single_large", "round", None): dict(
-        kernel="k_select<4> + k_process + k_recompute_barrier", dram_bytes_per_collision=4990.0,
-        fp64_pipe_active=0.606,
+        kernel="k_select<4> + k_process + k_recompute_barrier", dram_bytes_per_collision=4625.0,
+        fp64_pipe_active=0.641,
         capture="ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum --cache-control none "
                 "--clock-control none -k regex:'k_select|k_process$|k_recompute_barrier' -s 480 -c 60 python bench.py "
                 "--workload single_large --coll 300000 --steps 1 --warmup 3 --no-cpu-baseline --no-secondary "
-                "(20 rounds in the middle of a call, warm caches: 19.76 MB per round, over the workload's mean "
-                "of 3960 collisions per round; FP64 pipe of k_process from one --set full capture of a round)"),
+                "(20 rounds in the middle of a call, warm caches: 18.32 MB per round, over the workload's mean "
+                "of 3960 collisions per round; FP64 pipe of k_process in the same rounds)"),
 }
 
 

@@ -1,9 +1,10 @@
-// edmd_engine.cu -- serial-exact event engine (one warp per system) and the C ABI.
+// edmd_engine.cu -- serial-exact event engine (one or two warps per system) and the C ABI.
 //
-// Each system is advanced by one warp that pops events in exactly the order of
-// the reference's queue (src/EDMD.c:2144-2327: a calendar of N buckets of
-// width 5/N plus an overflow bucket, feeding an unbalanced BST whose in-order
-// ties go to the later insertion).  That order is emulated by the key
+// Each system is advanced by a warp (with a second one beside it in contexts of
+// few systems) that pops events in exactly the order of the reference's queue
+// (src/EDMD.c:2144-2327: a calendar of N buckets of width 5/N plus an overflow
+// bucket, feeding an unbalanced BST whose in-order ties go to the later
+// insertion).  That order is emulated by the key
 //     (b, t, tie)
 // b   = absolute calendar bucket in which the event enters the BST,
 // t   = event time,
@@ -1932,12 +1933,8 @@ extern "C" int edmd_load_state(edmd_ctx* ctx, const double* x, const double* y, 
   return stage_all(ctx, x, y, vx, vy, rad, m, nullptr, true);
 }
 
-// EDMD_F_SMEM: the systems whose engine state fits one block's shared memory
-// go to k_run_smem on a second stream, the others to k_run on the context's
-// stream; both start after e0 and the context's stream waits for the second
-// one before e1.
-// k_run on `nsys` places on the context's stream, with the tables of waiting
-// systems when they exceed the resident lane groups
+// the event loop on `nsys` places on the context's stream, with the tables of
+// waiting systems when they exceed the resident lane groups
 static int run_launch(edmd_ctx* ctx, RunArgs A, int nsys, int gw, int nsm) {
   RunShape shape = run_shape(gw, ctx->any_additive, nsys, nsm);
   int per_sm = 0;
@@ -1964,6 +1961,10 @@ static int run_launch(edmd_ctx* ctx, RunArgs A, int nsys, int gw, int nsm) {
   return EDMD_OK;
 }
 
+// EDMD_F_SMEM: the systems whose engine state fits one block's shared memory
+// go to k_run_smem on a second stream, the others to k_run on the context's
+// stream; both start after e0 and the context's stream waits for the second
+// one before e1.
 static int advance_smem_split(edmd_ctx* ctx, RunArgs A, int nsm) {
   int dev = 0, optin = 0;
   CK(cudaGetDevice(&dev));

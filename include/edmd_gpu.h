@@ -51,8 +51,8 @@ extern "C" {
                                    then run the warp engine's event loop, the faster
                                    one at every size measured.  The differentiation
                                    calls need EDMD_ENGINE_WARP */
-#define EDMD_ENGINE_WARP    1   /* one warp per system: single large systems  */
-#define EDMD_ENGINE_LANE    2   /* one thread per system: large batches, N <= 32766 */
+#define EDMD_ENGINE_WARP    1   /* one or two warps per system               */
+#define EDMD_ENGINE_LANE    2   /* one thread per system, N <= 32766          */
 
 /* edmd_advance flags */
 #define EDMD_F_STOP_AT_SCREEN  1u  /* return after each screenshot event      */
@@ -287,9 +287,10 @@ int edmd_tangent_run(edmd_ctx* ctx, int32_t sys, int32_t K, int64_t n_coll, int6
                      uint64_t seed, double* tangent_io, double* lyap_out);
 
 /* Adjoint of the final mean-square displacement.  Advances n_coll accepted
- * collisions from the current state, with exact engine checkpoints every
- * ckpt_every collisions; the reverse pass recomputes each segment from its
- * checkpoint and applies the transposed collision and free-flight maps.
+ * collisions from the current state and applies the transposed collision and
+ * free-flight maps backwards over their log.  A run whose log takes more than
+ * 2 GiB is logged in segments instead: exact engine checkpoints every ckpt_every
+ * collisions, and the reverse pass recomputes each segment from its checkpoint.
  * The observable is taken at t_obs (>= the time of the last processed event;
  * t_obs < 0 means that time): msd_out = (1/N) sum |u_i - <u>|^2 with u the
  * minimum-image displacement; g_vx, g_vy (g_x, g_y) receive d MSD / d v(0)
@@ -309,8 +310,9 @@ int edmd_tangent_run_batch(edmd_ctx* ctx, int32_t K, int64_t n_coll, int64_t qr_
                            double* lyap_out);
 
 /* Batched adjoint of the final mean-square displacement of every system: the
- * forward sweep with whole-context checkpoints every ckpt_every collisions
- * and the reverse sweep one thread per system.  The observable of system s is
+ * forward sweep (whole-context checkpoints every ckpt_every collisions when the
+ * logs take more than 2 GiB together) and the reverse sweep one warp per
+ * system.  The observable of system s is
  * taken at the time of its last processed event; msd_out (nsys) and the
  * gradients (total N, concatenated in system order like edmd_get_states) may
  * be NULL.  No reference counterpart.  Warp engine. */
