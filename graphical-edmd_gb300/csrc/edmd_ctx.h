@@ -61,6 +61,7 @@ struct edmd_ctx {
   void* round = nullptr;            // buffers of the round-parallel engine (edmd_round.cu)
   bool round_dirty = false;         // queue order lost: set by the round engine, cleared by a restage
   bool any_additive = false;        // some system uses additive contact (EDMD_CONTACT_ADDITIVE)
+  bool any_few_cells = false;       // some system has fewer than three cells along an axis
   std::vector<char> ckpt_dirty;     // round_dirty of each checkpoint
   void* pcf = nullptr;              // g(r): histogram and bin steps of up to pcf_bins bins
   int pcf_bins = 0;

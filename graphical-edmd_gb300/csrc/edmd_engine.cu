@@ -482,7 +482,8 @@ struct Aside : Flock {
   int dir[2];
   double Pb;                     // paulTime of bucket b (second warp)
   Node rest;                     // least of the leaves that the event leaves alone (second warp)
-  int self[2];                   // where disk i's candidates hold j, and j's hold i (-1: they don't)
+  int self[2];                   // where disk i's candidates hold j, and j's hold i (-1: they don't); one place
+                                 // each, since a 3x3 scan of at least three cells an axis meets a disk once
   Node sibs[MAXLEV][2];          // least sibling of each path node, by level
   int off[MAXLEV], cnt[MAXLEV];  // the tree's levels
 };
@@ -1152,7 +1153,10 @@ __global__ void k_waiting(RunArgs A) {
 
 // How nsys systems are run with gw lanes each: kernel, warps and systems of a
 // block.  With 32 lanes up to eight systems per SM get two warps each
-// (k_run_pair; `pair`: unless they would not all be resident).  One warp each,
+// (k_run_pair; `pair`: unless they would not all be resident, or one has fewer
+// than three cells along an axis: its 3x3 scans meet a colliding partner more
+// than once, and the second warp's list holds one place for it, while the
+// one-warp loop reads every candidate after the collision).  One warp each,
 // measured (203 disks alone / 192 growth starts / 1824 < 2600 mixed systems,
 // ms; every build has the same event loop):
 //   3 blocks per SM, 168 registers: 1.41 / 15.2 / 36
@@ -1161,9 +1165,10 @@ __global__ void k_waiting(RunArgs A) {
 //   6 blocks, 85 registers:         1.58 / 17.6 / 32.2
 // so systems that all find a warp at three blocks per SM run there, without
 // spills, and larger batches at five.
+bool few_cells(const Box& B) { return B.Nxc < 3 || B.Nyc < 3; }
 using RunKernel = void (*)(const SysDev*, RunArgs);
 struct RunShape { RunKernel kernel; int warps, systems; };   // a block's warps and systems
-RunShape run_shape(int gw, bool additive, int nsys, int nsm, bool pair = true) {
+RunShape run_shape(int gw, bool additive, int nsys, int nsm, bool pair) {
   const int W = WARPS_PER_BLOCK;
   if (gw == 4) return {k_run<4, true, 4>, W, W * 8};
   if (gw == 8) return {k_run<8, true, 4>, W, W * 4};
@@ -1831,6 +1836,7 @@ extern "C" int edmd_create(int32_t nsys, const edmd_system_desc* desc, const dou
     B.hLx = D.Lx / 2; B.hLy = D.Ly / 2;                      // boxConstantHelper 679-714
     B.Nyc = (int)(B.hLy); B.Nxc = (int)(B.hLx);
     if (B.Nxc < 1 || B.Nyc < 1) return set_err(ctx, EDMD_ERR_ARG, "box smaller than one cell");
+    if (few_cells(B)) ctx->any_few_cells = true;
     B.cxs = D.Lx / B.Nxc; B.cys = D.Ly / B.Nyc;
     B.cxf = 1 / B.cxs; B.cyf = 1 / B.cys;
     B.dtP = 5.0 / (double)D.N;
@@ -1936,7 +1942,7 @@ extern "C" int edmd_load_state(edmd_ctx* ctx, const double* x, const double* y, 
 // the event loop on `nsys` places on the context's stream, with the tables of
 // waiting systems when they exceed the resident lane groups
 static int run_launch(edmd_ctx* ctx, RunArgs A, int nsys, int gw, int nsm) {
-  RunShape shape = run_shape(gw, ctx->any_additive, nsys, nsm);
+  RunShape shape = run_shape(gw, ctx->any_additive, nsys, nsm, !ctx->any_few_cells);
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shape.kernel, 32 * shape.warps, 0));
   if (shape.systems == 1 && per_sm * nsm < nsys) {
@@ -2390,7 +2396,7 @@ extern "C" int edmd_run_noalloc(const edmd_system_desc* desc, double* x, double*
   k_noalloc_stage<<<1, 32, 0, st>>>(dsys, x, y, vx, vy, rad, m, D.first_screen, D.first_thermo);
   if (cudaError_t qe = init_queues(dsys, 1, N, true, st); qe != cudaSuccess)
     return noalloc_fail(EDMD_ERR_CUDA, cudaGetErrorString(qe));
-  const RunShape shape = run_shape(32, B.additive != 0, 1, 1);
+  const RunShape shape = run_shape(32, B.additive != 0, 1, 1, !few_cells(B));
   shape.kernel<<<1, 32 * shape.warps, 0, st>>>(dsys, A);
   k_sync<<<dim3((N + 255) / 256, 1), 256, 0, st>>>(dsys);
   k_noalloc_out<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(dsys, x, y, vx, vy);
