@@ -55,8 +55,7 @@ struct edmd_ctx {
   std::vector<size_t> ckpt_parts;   // bytes of each array in a snapshot
   uint16_t* cal = nullptr;          // calendars of the thread-per-system engine
   uint16_t* mask = nullptr;
-  int engine = 0;                   // EDMD_ENGINE_WARP or EDMD_ENGINE_LANE, as reported
-  bool calendar = false;            // events run by the thread-per-system loop on its calendars
+  int engine = 0;                   // EDMD_ENGINE_WARP or EDMD_ENGINE_LANE
   int64_t total_C = 0;
   void* round = nullptr;            // buffers of the round-parallel engine (edmd_round.cu)
   bool round_dirty = false;         // queue order lost: set by the round engine, cleared by a restage

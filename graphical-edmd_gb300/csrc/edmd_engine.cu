@@ -1798,8 +1798,8 @@ static int stage_all(edmd_ctx* ctx, const double* x, const double* y, const doub
   k_links<<<gd, 256, 0, sm>>>(ctx->ds);
   k_heads<<<gd, 256, 0, sm>>>(ctx->ds);
   CK(cudaGetLastError());
-  CK(init_queues(ctx->ds, nsys, ctx->maxN, !ctx->calendar, sm));
-  if (ctx->calendar) CK(lane_build(ctx->ds, nsys, sm));
+  CK(init_queues(ctx->ds, nsys, ctx->maxN, ctx->engine == EDMD_ENGINE_WARP, sm));
+  if (ctx->engine == EDMD_ENGINE_LANE) CK(lane_build(ctx->ds, nsys, sm));
   return report_status(ctx, "initial configuration");
 }
 
@@ -1860,17 +1860,21 @@ extern "C" int edmd_create(int32_t nsys, const edmd_system_desc* desc, const dou
   ctx->total_N = TN; ctx->total_C = TC;
   ctx->engine = g_engine;
   if (ctx->engine == EDMD_ENGINE_AUTO) {
-    // Contexts of many small systems count as EDMD_ENGINE_LANE, but run the
-    // warp engine's event loop: measured on GB300 (300 collisions a call) it
-    // gives 1.65e8 / 1.55e8 / 1.31e8 coll/s on 16384 systems of 96 / 256 /
-    // 1024 disks against 1.10e8 / 1.07e8 / 1.00e8 for one thread per system,
-    // 1.75e8 against 1.62e8 on 32768 of 96 and 1.77e8 against 1.54e8 on 60000;
-    // and the thread loop's calendars cost 2 KB per disk.
-    const bool many = nsys >= 16384 && 2 * (int64_t)ctx->maxN + NSPECIAL <= 65535 &&
+    // One thread per system issues each FP64 instruction for up to 32 systems,
+    // but needs enough of them to hide its dependent loads; the warp loop is
+    // full from ~3000 systems on.  Hex starts at phi 0.55, 1000 collisions a
+    // call, one warp / one thread per system in 1e8 coll/s:
+    //   systems   96 disks     256          1024         64-1024 mixed
+    //   16384     1.77 / 1.25  1.70 / 1.20  1.50 / 1.14  1.66 / 1.18
+    //   24576     1.77 / 1.70  1.68 / 1.63  1.50 / 1.54  1.65 / 1.62
+    //   28672     1.77 / 1.89  1.65 / 1.85  -            1.64 / 1.83
+    //   32768     1.77 / 2.03  1.64 / 2.03  -            1.63 / 1.98
+    // (150 collisions after a restart, whose calendars take longer to build:
+    // 24576 x 256 46.7 / 51.6 ms, 28672 54.3 / 56.8, 32768 61.3 / 61.8).  The
+    // calendars cost 1 KB per disk.
+    const bool many = nsys >= 28672 && 2 * (int64_t)ctx->maxN + NSPECIAL <= 65535 &&
                       TN * (int64_t)(CAL_SUB * CAL_LINE * 2 + 2) <= ((int64_t)32 << 30);
     ctx->engine = many ? EDMD_ENGINE_LANE : EDMD_ENGINE_WARP;
-  } else {
-    ctx->calendar = ctx->engine == EDMD_ENGINE_LANE;
   }
   if (ctx->engine == EDMD_ENGINE_LANE && 2 * (int64_t)ctx->maxN + NSPECIAL > 65535)
     return set_err(ctx, EDMD_ERR_ARG, "thread-per-system engine supports N <= 32766");
@@ -1904,7 +1908,7 @@ extern "C" int edmd_create(int32_t nsys, const edmd_system_desc* desc, const dou
   arrays();
   CK(dalloc(&ctx->slab, bytes));
   arrays();
-  if (ctx->calendar) {
+  if (ctx->engine == EDMD_ENGINE_LANE) {
     CK(dalloc(&ctx->cal, (size_t)TN * CAL_SUB * CAL_LINE));
     CK(dalloc(&ctx->mask, (size_t)TN));
   }
@@ -1922,7 +1926,7 @@ extern "C" int edmd_create(int32_t nsys, const edmd_system_desc* desc, const dou
     S.trace_cap = trace_cap;
     S.rows = ctx->rows + (size_t)s * rows_cap * 9;
     S.rows_cap = rows_cap;
-    if (ctx->calendar) {
+    if (ctx->engine == EDMD_ENGINE_LANE) {
       S.cal = ctx->cal + (size_t)o * CAL_SUB * CAL_LINE;
       S.mask = ctx->mask + o;
       S.invw = CAL_SUB / S.B.dtP;
@@ -2032,7 +2036,7 @@ extern "C" int edmd_advance(edmd_ctx* ctx, int64_t max_coll, double t_stop, uint
   A.order = nullptr; A.waiting = nullptr; A.ticket = nullptr; A.progress = nullptr;
   A.nwait = 0; A.nrun = ctx->nsys;
   ctx->last_launches = 0;
-  if (ctx->calendar) {
+  if (ctx->engine == EDMD_ENGINE_LANE) {
     CK(cudaEventRecord(ctx->e0, ctx->stream));
     CK(lane_run_launch(ctx->ds, A, g_lane_threads, ctx->stream));
     ctx->last_launches = 1;
@@ -2040,9 +2044,9 @@ extern "C" int edmd_advance(edmd_ctx* ctx, int64_t max_coll, double t_stop, uint
     int dev = 0, nsm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    const int gw = ctx->engine == EDMD_ENGINE_LANE ? 32 : g_group;     // lanes per system: 4, 8, 16 or 32
+    const int gw = g_group;                     // lanes per system: 4, 8, 16 or 32
     int rc;
-    if ((flags & EDMD_F_SMEM) && gw == 32 && ctx->engine == EDMD_ENGINE_WARP) {
+    if ((flags & EDMD_F_SMEM) && gw == 32) {
       rc = advance_smem_split(ctx, A, nsm);
     } else {
       CK(cudaEventRecord(ctx->e0, ctx->stream));

@@ -2,10 +2,10 @@
 
 Every engine and launch shape of the serial-exact event loop gives
 bit-identical trajectories (the reference's event order), so the choice is a
-pure speed question: the warp engine with 32 lanes won on every batch measured
-so far, narrower groups trade FP64 issue against divergence, the shared-memory
-kernel memory latency against resident systems, and the thread-per-system
-engine needs tens of thousands of systems to come near.  `tune` times each
+pure speed question: the warp engine with 32 lanes won on every batch of up to
+~24000 systems measured so far, the thread-per-system engine from ~28000 on;
+narrower groups trade FP64 issue against divergence and the shared-memory
+kernel memory latency against resident systems.  `tune` times each
 candidate on the batch itself -- a fresh context from the given states, one
 untimed warm-up call and `reps` timed calls of `coll` accepted collisions per
 system (CUDA events on the context's stream) -- and returns the fastest.

@@ -46,11 +46,11 @@ extern "C" {
 #define EDMD_STOP_GROW      5   /* stopped right after the growth stop        */
 
 /* engines (edmd_set_engine) */
-#define EDMD_ENGINE_AUTO    0   /* EDMD_ENGINE_LANE for contexts of at least 16384
-                                   systems of N <= 32766, else EDMD_ENGINE_WARP; both
-                                   then run the warp engine's event loop, the faster
-                                   one at every size measured.  The differentiation
-                                   calls need EDMD_ENGINE_WARP */
+#define EDMD_ENGINE_AUTO    0   /* EDMD_ENGINE_LANE for contexts of at least 28672
+                                   systems of N <= 32766 whose calendars (1 KB a
+                                   disk) take at most 32 GiB, faster there; else
+                                   EDMD_ENGINE_WARP.  The differentiation calls need
+                                   EDMD_ENGINE_WARP */
 #define EDMD_ENGINE_WARP    1   /* one or two warps per system               */
 #define EDMD_ENGINE_LANE    2   /* one thread per system, N <= 32766          */
 
