@@ -148,8 +148,9 @@ extern "C" int edmd_get_pcf(edmd_ctx* ctx, int32_t s, double dr, double max_r, d
   unsigned long long* hist = (unsigned long long*)ctx->pcf;
   CK(cudaMemsetAsync(hist, 0, nb * sizeof(unsigned long long), ctx->stream));
   // cells are distinct up to the reach (and a block's counts fit 32 bits)
+  std::vector<double> step;                // to the device: kept until the copy back
   if (2 * kx + 1 <= B.Nxc && 2 * ky + 1 <= B.Nyc && B.N < (1 << 25)) {
-    std::vector<double> step(nb + 1);
+    step.resize(nb + 1);
     step[0] = 0;
     for (int b = 1; b <= nb; b++)
       step[b] = first_above(b * dr * (b * dr), [&](double d2) { return (int)(std::sqrt(d2) / dr) >= b; });
