@@ -147,9 +147,11 @@ extern "C" int edmd_get_pcf(edmd_ctx* ctx, int32_t s, double dr, double max_r, d
   }
   unsigned long long* hist = (unsigned long long*)ctx->pcf;
   CK(cudaMemsetAsync(hist, 0, nb * sizeof(unsigned long long), ctx->stream));
-  // cells are distinct up to the reach (and a block's counts fit 32 bits)
+  // cells are distinct up to the reach, a block's counts fit 32 bits, and bins
+  // are wide enough for the FP32 estimate (d2 below 2^-126, which it takes for
+  // zero, lies in bin 0) and for first_above (b dr b dr is a normal number)
   std::vector<double> step;                // to the device: kept until the copy back
-  if (2 * kx + 1 <= B.Nxc && 2 * ky + 1 <= B.Nyc && B.N < (1 << 25)) {
+  if (2 * kx + 1 <= B.Nxc && 2 * ky + 1 <= B.Nyc && B.N < (1 << 25) && dr >= 1e-12) {
     step.resize(nb + 1);
     step[0] = 0;
     for (int b = 1; b <= nb; b++)
