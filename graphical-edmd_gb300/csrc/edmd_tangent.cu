@@ -553,6 +553,8 @@ static int upload_sysdev(edmd_ctx* ctx) {
 
 extern "C" int edmd_set_log_capacity(edmd_ctx* ctx, int64_t cap) {
   if (!ctx || cap < 0) return EDMD_ERR_ARG;
+  if (cap > INT64_MAX / (int64_t)sizeof(edmd_log_entry) / ctx->nsys)   // its bytes are no number
+    return set_err(ctx, EDMD_ERR_CUDA, "collision log: out of memory");
   if (cap > ctx->log_cap) {
     if (ctx->logbuf) cudaFree(ctx->logbuf);
     ctx->logbuf = nullptr;
@@ -748,7 +750,8 @@ extern "C" int edmd_tangent_run(edmd_ctx* ctx, int32_t s, int32_t K, int64_t n_c
     return EDMD_ERR_ARG;
   if (ctx->engine != EDMD_ENGINE_WARP) return set_err(ctx, EDMD_ERR_ARG, "tangents need the warp engine");
   const int N = ctx->hs[s].B.N;
-  int64_t chunk = qr_every > 0 ? qr_every : (n_coll > 0 ? n_coll : 1);
+  const int64_t most = n_coll > 0 ? n_coll : 1;
+  const int64_t chunk = qr_every > 0 && qr_every < most ? qr_every : most;
   const int64_t half = chunk + 16;
   int rc = edmd_set_log_capacity(ctx, n_coll > chunk ? 2 * half : half);
   if (rc) return rc;
@@ -848,6 +851,7 @@ extern "C" int edmd_msd_gradient(edmd_ctx* ctx, int32_t s, int64_t n_coll, int64
                                  double* g_x, double* g_y) {
   if (!ctx || s < 0 || s >= ctx->nsys || n_coll < 1 || ckpt_every < 1) return EDMD_ERR_ARG;
   if (ctx->engine != EDMD_ENGINE_WARP) return set_err(ctx, EDMD_ERR_ARG, "adjoints need the warp engine");
+  ckpt_every = std::min(ckpt_every, n_coll);
   const int N = ctx->hs[s].B.N;
   const double Lx = ctx->hs[s].B.Lx, Ly = ctx->hs[s].B.Ly;
   // one logged forward run, or (a long one) checkpointed segments run twice
@@ -1006,7 +1010,8 @@ extern "C" int edmd_tangent_run_batch(edmd_ctx* ctx, int32_t K, int64_t n_coll, 
   if (ctx->engine != EDMD_ENGINE_WARP) return set_err(ctx, EDMD_ERR_ARG, "tangents need the warp engine");
   const int64_t TN = ctx->total_N;
   const int nsys = ctx->nsys;
-  const int64_t chunk = qr_every > 0 ? qr_every : (n_coll > 0 ? n_coll : 1);
+  const int64_t most = n_coll > 0 ? n_coll : 1;
+  const int64_t chunk = qr_every > 0 && qr_every < most ? qr_every : most;
   const int64_t half = chunk + 16;
   int rc = edmd_set_log_capacity(ctx, n_coll > chunk ? 2 * half : half);
   if (rc) return rc;
@@ -1092,6 +1097,7 @@ extern "C" int edmd_msd_gradient_batch(edmd_ctx* ctx, int64_t n_coll, int64_t ck
                                        double* g_vx, double* g_vy, double* g_x, double* g_y) {
   if (!ctx || n_coll < 1 || ckpt_every < 1) return EDMD_ERR_ARG;
   if (ctx->engine != EDMD_ENGINE_WARP) return set_err(ctx, EDMD_ERR_ARG, "adjoints need the warp engine");
+  ckpt_every = std::min(ckpt_every, n_coll);
   const int64_t TN = ctx->total_N;
   const int nsys = ctx->nsys;
   // one logged forward run, or (a long one) checkpointed segments run twice
