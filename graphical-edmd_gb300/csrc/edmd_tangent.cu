@@ -700,7 +700,8 @@ struct LogLengths {
 // What a tangent driver's chunks alternate between: two halves of the logs and
 // the chunk's end times and log ends.  The tangent map and the QR of a chunk
 // run on a second stream beside the next chunk's forward run; the forward run
-// after that waits until the map has read the half it is going to write.
+// after that waits until the map has read the half it is going to write (one
+// half: see chunk_logs).
 struct Chunks {
   double* tq[2] = {nullptr, nullptr};
   uint64_t* nend[2] = {nullptr, nullptr};
@@ -724,6 +725,15 @@ struct Chunks {
     return e;
   }
 };
+
+// Logs of two halves for a run of several chunks; of one where there is no room
+// for two: a chunk's forward run then waits for the map of the one before.
+static int chunk_logs(edmd_ctx* ctx, int64_t half, bool several, bool* two) {
+  *two = several && half <= INT64_MAX / 2 && edmd_set_log_capacity(ctx, 2 * half) == EDMD_OK;
+  if (*two) return EDMD_OK;
+  cudaGetLastError();
+  return edmd_set_log_capacity(ctx, half);
+}
 
 constexpr int GRAM_BLOCKS = 1024;
 
@@ -753,8 +763,6 @@ extern "C" int edmd_tangent_run(edmd_ctx* ctx, int32_t s, int32_t K, int64_t n_c
   const int64_t most = n_coll > 0 ? n_coll : 1;
   const int64_t chunk = qr_every > 0 && qr_every < most ? qr_every : most;
   const int64_t half = chunk + 16;
-  int rc = edmd_set_log_capacity(ctx, n_coll > chunk ? 2 * half : half);
-  if (rc) return rc;
   double *T = nullptr, *tl = nullptr, *G = nullptr, *Gp = nullptr, *Rinv = nullptr, *logdiag = nullptr;
   int* fail = nullptr;
   CK(dalloc(&T, (size_t)4 * N * K));
@@ -767,6 +775,9 @@ extern "C" int edmd_tangent_run(edmd_ctx* ctx, int32_t s, int32_t K, int64_t n_c
   struct Free { void* p[7]; ~Free() { for (void* q : p) if (q) cudaFree(q); } } guard{{T, tl, G, Gp, Rinv, logdiag, fail}};
   Chunks ch;
   CK(ch.make(1));
+  bool two = false;
+  int rc = chunk_logs(ctx, half, n_coll > chunk, &two);
+  if (rc) return rc;
   if (!ctx->stream2) CK(cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking));
   cudaStream_t st2 = ctx->stream2;
   struct Idle { edmd_ctx* c; ~Idle() { cudaStreamSynchronize(c->stream2); } } idle{ctx};   // before the frees
@@ -798,8 +809,8 @@ extern "C" int edmd_tangent_run(edmd_ctx* ctx, int32_t s, int32_t K, int64_t n_c
   for (int c = 0; done < n_coll; c ^= 1) {
     int64_t want = n_coll - done < chunk ? n_coll - done : chunk;
     int64_t nl = 0;
-    const int64_t from = c ? half : 0;
-    if (done >= 2 * chunk) CK(cudaStreamWaitEvent(ctx->stream, ch.mapped[c], 0));
+    const int64_t from = two && c ? half : 0;
+    if (done > (two ? chunk : 0)) CK(cudaStreamWaitEvent(ctx->stream, ch.mapped[two ? c : c ^ 1], 0));
     if ((rc = advance_logged(ctx, want, from, half, s, &nl))) return rc;
     k_sys_times<<<1, 32, 0, ctx->stream>>>(ctx->ds + s, 1, ch.tq[c], nullptr);
     CK(cudaEventRecord(ch.ran[c], ctx->stream));
@@ -1013,8 +1024,7 @@ extern "C" int edmd_tangent_run_batch(edmd_ctx* ctx, int32_t K, int64_t n_coll, 
   const int64_t most = n_coll > 0 ? n_coll : 1;
   const int64_t chunk = qr_every > 0 && qr_every < most ? qr_every : most;
   const int64_t half = chunk + 16;
-  int rc = edmd_set_log_capacity(ctx, n_coll > chunk ? 2 * half : half);
-  if (rc) return rc;
+  int rc = EDMD_OK;
   BatchIndex bi;
   if ((rc = batch_index(ctx, bi))) return rc;
   double *T = nullptr, *tl = nullptr, *G = nullptr, *Rinv = nullptr, *logdiag = nullptr;
@@ -1028,6 +1038,8 @@ extern "C" int edmd_tangent_run_batch(edmd_ctx* ctx, int32_t K, int64_t n_coll, 
   struct Free { void* p[6]; ~Free() { for (void* q : p) if (q) cudaFree(q); } } guard{{T, tl, G, Rinv, logdiag, fail}};
   Chunks ch;
   CK(ch.make(nsys));
+  bool two = false;
+  if ((rc = chunk_logs(ctx, half, n_coll > chunk, &two))) return rc;
   if (!ctx->stream2) CK(cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking));
   cudaStream_t st2 = ctx->stream2;
   struct Idle { edmd_ctx* c; ~Idle() { cudaStreamSynchronize(c->stream2); } } idle{ctx};   // before the frees
@@ -1064,8 +1076,8 @@ extern "C" int edmd_tangent_run_batch(edmd_ctx* ctx, int32_t K, int64_t n_coll, 
   int64_t done = 0, last = 0;
   for (int c = 0; done < n_coll; c ^= 1) {
     const int64_t want = n_coll - done < chunk ? n_coll - done : chunk;
-    const int64_t from = c ? half : 0;
-    if (done >= 2 * chunk) CK(cudaStreamWaitEvent(ctx->stream, ch.mapped[c], 0));
+    const int64_t from = two && c ? half : 0;
+    if (done > (two ? chunk : 0)) CK(cudaStreamWaitEvent(ctx->stream, ch.mapped[two ? c : c ^ 1], 0));
     if ((rc = advance_logged(ctx, want, from, half, -1, nullptr))) return rc;
     k_sys_times<<<gs, 128, 0, ctx->stream>>>(ctx->ds, nsys, ch.tq[c], ch.nend[c]);   // the chunk's end
     CK(cudaEventRecord(ch.ran[c], ctx->stream));

@@ -29,3 +29,43 @@ def test_intervals_longer_than_any_log(edmd):
     for r in res[1:]:
         for a, b in zip(r, res[0]):
             np.testing.assert_array_equal(a, b)
+
+
+def test_chunks_whose_logs_have_no_room_for_two(edmd):
+    """One log of 1.7e11 bytes fits the GPU, two of them do not: chunks one after the other (the runs end at tmax, soon)."""
+    s = start(edmd, 60, 3, tmax=3.0)
+    for batch in (False, True):
+        res = []
+        for every, most in ((10 ** 6, 2 * 10 ** 6), (3 * 10 ** 9, 6 * 10 ** 9)):
+            eng = edmd.Engine([s])
+            lyap = eng.tangent_batch(3, most, every, seed=4)[0] if batch else eng.tangent(3, most, every, seed=4)[1]
+            res.append((lyap, eng.counters(0)["ncol"]))
+            eng.close()
+        assert res[0][1] == res[1][1] > 100
+        np.testing.assert_array_equal(res[0][0], res[1][0])
+
+
+def crowd_out(leave):
+    """Takes the GPU's memory up to `leave` bytes (given back with the returned tensor)."""
+    import torch
+    return torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda:0")
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_one_log_gives_the_exponents_of_two(edmd, batch):
+    """340 MB of log a chunk, and 500 MB left: every chunk's log is read before the next chunk writes it."""
+    import torch
+    s = [start(edmd, 60 + 20 * (k % 3), 3 + k % 3) for k in range(2000)]
+    res = []
+    for full in (False, True):
+        eng = edmd.Engine(s)
+        hog = crowd_out(500 << 20) if full else None
+        try:
+            res.append(eng.tangent_batch(2, 10000, 3000, seed=4) if batch else eng.tangent(2, 10000, 3000, seed=4, s=7)[1])
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+        n = len(eng.log(7))
+        assert n == 1000                                  # the last chunk's collisions
+        eng.close()
+    np.testing.assert_array_equal(res[0], res[1])
