@@ -735,6 +735,16 @@ static int chunk_logs(edmd_ctx* ctx, int64_t half, bool several, bool* two) {
   return edmd_set_log_capacity(ctx, half);
 }
 
+// The last chunk's collisions at the front of the logs when a run ends, also by
+// an error (declared before what waits for the second stream).
+struct LastChunk {
+  edmd_ctx* ctx;
+  int64_t from = 0;
+  ~LastChunk() {
+    if (from) k_log_front<<<ctx->nsys, 128, 0, ctx->stream>>>(ctx->ds, from);
+  }
+};
+
 constexpr int GRAM_BLOCKS = 1024;
 
 // CholQR2 of one system's tangent block at the time *tqp, on stream st
@@ -780,6 +790,7 @@ extern "C" int edmd_tangent_run(edmd_ctx* ctx, int32_t s, int32_t K, int64_t n_c
   if (rc) return rc;
   if (!ctx->stream2) CK(cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking));
   cudaStream_t st2 = ctx->stream2;
+  LastChunk last{ctx};
   struct Idle { edmd_ctx* c; ~Idle() { cudaStreamSynchronize(c->stream2); } } idle{ctx};   // before the frees
   CK(call_begin(ctx));
   double t0;
@@ -805,12 +816,13 @@ extern "C" int edmd_tangent_run(edmd_ctx* ctx, int32_t s, int32_t K, int64_t n_c
   // the tangent vectors are the second stream's from here on
   CK(cudaEventRecord(ch.ran[0], ctx->stream));
   CK(cudaStreamWaitEvent(st2, ch.ran[0], 0));
-  int64_t done = 0, last = 0;
+  int64_t done = 0;
   for (int c = 0; done < n_coll; c ^= 1) {
     int64_t want = n_coll - done < chunk ? n_coll - done : chunk;
     int64_t nl = 0;
     const int64_t from = two && c ? half : 0;
     if (done > (two ? chunk : 0)) CK(cudaStreamWaitEvent(ctx->stream, ch.mapped[two ? c : c ^ 1], 0));
+    last.from = from;
     if ((rc = advance_logged(ctx, want, from, half, s, &nl))) return rc;
     k_sys_times<<<1, 32, 0, ctx->stream>>>(ctx->ds + s, 1, ch.tq[c], nullptr);
     CK(cudaEventRecord(ch.ran[c], ctx->stream));
@@ -820,12 +832,10 @@ extern "C" int edmd_tangent_run(edmd_ctx* ctx, int32_t s, int32_t K, int64_t n_c
     if (qr_every > 0 && (rc = cholqr(ctx, T, tl, N, K, ch.tq[c], G, Gp, Rinv, logdiag, fail, true, st2))) return rc;
     CK(cudaEventRecord(ch.mapped[c], st2));
     done += want;
-    last = from;
     if (nl < want) break;     // the run ended early (tmax or t_stop)
   }
   CK(cudaEventRecord(ch.ran[0], st2));
   CK(cudaStreamWaitEvent(ctx->stream, ch.ran[0], 0));
-  if (last) k_log_front<<<ctx->nsys, 128, 0, ctx->stream>>>(ctx->ds, last);
   {
     int hf = 0;
     CK(sync_copy(ctx, &hf, fail, 4, cudaMemcpyDeviceToHost));
@@ -1042,6 +1052,7 @@ extern "C" int edmd_tangent_run_batch(edmd_ctx* ctx, int32_t K, int64_t n_coll, 
   if ((rc = chunk_logs(ctx, half, n_coll > chunk, &two))) return rc;
   if (!ctx->stream2) CK(cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking));
   cudaStream_t st2 = ctx->stream2;
+  LastChunk last{ctx};
   struct Idle { edmd_ctx* c; ~Idle() { cudaStreamSynchronize(c->stream2); } } idle{ctx};   // before the frees
   const unsigned gs = (unsigned)((nsys + 127) / 128);
   // system s starts from the vectors edmd_tangent_run draws from seed + s
@@ -1073,11 +1084,12 @@ extern "C" int edmd_tangent_run_batch(edmd_ctx* ctx, int32_t K, int64_t n_coll, 
   // the tangent vectors are the second stream's from here on
   CK(cudaEventRecord(ch.ran[0], ctx->stream));
   CK(cudaStreamWaitEvent(st2, ch.ran[0], 0));
-  int64_t done = 0, last = 0;
+  int64_t done = 0;
   for (int c = 0; done < n_coll; c ^= 1) {
     const int64_t want = n_coll - done < chunk ? n_coll - done : chunk;
     const int64_t from = two && c ? half : 0;
     if (done > (two ? chunk : 0)) CK(cudaStreamWaitEvent(ctx->stream, ch.mapped[two ? c : c ^ 1], 0));
+    last.from = from;
     if ((rc = advance_logged(ctx, want, from, half, -1, nullptr))) return rc;
     k_sys_times<<<gs, 128, 0, ctx->stream>>>(ctx->ds, nsys, ch.tq[c], ch.nend[c]);   // the chunk's end
     CK(cudaEventRecord(ch.ran[c], ctx->stream));
@@ -1087,11 +1099,9 @@ extern "C" int edmd_tangent_run_batch(edmd_ctx* ctx, int32_t K, int64_t n_coll, 
     if (qr_every > 0 && (rc = cholqr_b(ctx, bi, T, tl, K, G, Rinv, logdiag, fail, true, ch.tq[c], st2))) return rc;
     CK(cudaEventRecord(ch.mapped[c], st2));
     done += want;
-    last = from;
   }
   CK(cudaEventRecord(ch.ran[0], st2));
   CK(cudaStreamWaitEvent(ctx->stream, ch.ran[0], 0));
-  if (last) k_log_front<<<nsys, 128, 0, ctx->stream>>>(ctx->ds, last);
   if ((rc = check_fail(ctx, fail))) return rc;
   if (lyap_out) {
     std::vector<double> ld((size_t)nsys * K);

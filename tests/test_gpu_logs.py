@@ -69,3 +69,20 @@ def test_one_log_gives_the_exponents_of_two(edmd, batch):
         assert n == 1000                                  # the last chunk's collisions
         eng.close()
     np.testing.assert_array_equal(res[0], res[1])
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_a_run_that_fails_leaves_its_last_chunk(edmd, batch):
+    """Two disks meet at t = 0.05 (the first chunk); the collision at t = 0.1 finds an overlap (the second)."""
+    from conftest import line_overlap_state
+    s = line_overlap_state(edmd)
+    s["x"][4], s["vx"][3], s["vx"][4] = 4.05, 1.0, 0.0
+    s["vy"][3] = s["vy"][4] = 0.0
+    eng = edmd.Engine([s])
+    with pytest.raises(edmd.EngineError) as e:
+        eng.tangent_batch(1, 5, 1, seed=2) if batch else eng.tangent(1, 5, 1, seed=2)
+    assert e.value.code == edmd.ERR_OVERLAP
+    log = eng.log(0)
+    eng.close()
+    assert len(log) == 1 and {int(log["i"][0]), int(log["j"][0])} == {1, 2}
+    assert abs(log["t"][0] - 0.1) < 1e-12
