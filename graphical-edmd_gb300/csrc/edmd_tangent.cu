@@ -675,9 +675,21 @@ static int advance_logged(edmd_ctx* ctx, int64_t ncoll, int64_t from, int64_t ro
   return EDMD_OK;
 }
 
-// The differentiation drivers' logs hold the collisions of a whole call up to
-// this size, and leave each system's public log length as it was.
-constexpr int64_t LOG_ALL_BYTES = (int64_t)2 << 30;
+// The gradient drivers log the collisions of the whole call (one forward run)
+// where that takes no more memory than the checkpoints and the segment's log of
+// a run in segments of ckpt_every, or at most LOG_FREE_BYTES, and never more
+// than LOG_ALL_BYTES; else they run in segments (twice as long).  The log stays
+// with the context, as the checkpoints do.
+constexpr int64_t LOG_ALL_BYTES = (int64_t)2 << 30, LOG_FREE_BYTES = (int64_t)64 << 20;
+static bool log_whole(edmd_ctx* ctx, int64_t n_coll, int64_t ckpt_every) {
+  std::vector<std::pair<void*, size_t>> parts;
+  state_parts(ctx, parts);
+  double state = 0;
+  for (auto& p : parts) state += (double)align_up(p.second, 256);
+  const double entry = (double)sizeof(edmd_log_entry) * ctx->nsys, all = entry * (n_coll + 16.0);
+  const double segments = entry * (ckpt_every + 16.0) + state * (double)((n_coll - 1) / ckpt_every + 2);
+  return all <= (double)LOG_ALL_BYTES && all <= std::max((double)LOG_FREE_BYTES, segments);
+}
 
 // log lengths put back at the end of a call
 struct LogLengths {
@@ -875,8 +887,8 @@ extern "C" int edmd_msd_gradient(edmd_ctx* ctx, int32_t s, int64_t n_coll, int64
   ckpt_every = std::min(ckpt_every, n_coll);
   const int N = ctx->hs[s].B.N;
   const double Lx = ctx->hs[s].B.Lx, Ly = ctx->hs[s].B.Ly;
-  // one logged forward run, or (a long one) checkpointed segments run twice
-  bool whole = n_coll < LOG_ALL_BYTES / ((int64_t)sizeof(edmd_log_entry) * ctx->nsys) - 16;
+  // one logged forward run, or checkpointed segments run twice
+  bool whole = log_whole(ctx, n_coll, ckpt_every);
   int rc = whole ? edmd_set_log_capacity(ctx, n_coll + 16) : EDMD_OK;
   if (rc) { whole = false; cudaGetLastError(); }         // no room for it
   if (!whole) rc = edmd_set_log_capacity(ctx, ckpt_every + 16);
@@ -1122,8 +1134,8 @@ extern "C" int edmd_msd_gradient_batch(edmd_ctx* ctx, int64_t n_coll, int64_t ck
   ckpt_every = std::min(ckpt_every, n_coll);
   const int64_t TN = ctx->total_N;
   const int nsys = ctx->nsys;
-  // one logged forward run, or (a long one) checkpointed segments run twice
-  bool whole = n_coll < LOG_ALL_BYTES / ((int64_t)sizeof(edmd_log_entry) * nsys) - 16;
+  // one logged forward run, or checkpointed segments run twice
+  bool whole = log_whole(ctx, n_coll, ckpt_every);
   int rc = whole ? edmd_set_log_capacity(ctx, n_coll + 16) : EDMD_OK;
   if (rc) { whole = false; cudaGetLastError(); }         // no room for it
   if (!whole) rc = edmd_set_log_capacity(ctx, ckpt_every + 16);

@@ -288,9 +288,11 @@ int edmd_tangent_run(edmd_ctx* ctx, int32_t sys, int32_t K, int64_t n_coll, int6
 
 /* Adjoint of the final mean-square displacement.  Advances n_coll accepted
  * collisions from the current state and applies the transposed collision and
- * free-flight maps backwards over their log.  A run whose log takes more than
- * 2 GiB is logged in segments instead: exact engine checkpoints every ckpt_every
- * collisions, and the reverse pass recomputes each segment from its checkpoint.
+ * free-flight maps backwards over their log, or, where that log would take more
+ * than 64 MiB and more than the memory of the following (or more than 2 GiB),
+ * logs in segments: exact engine checkpoints every ckpt_every collisions (slots
+ * 0, 1, ... of edmd_checkpoint_save), and the reverse pass recomputes each
+ * segment from its checkpoint.  Logs and checkpoints stay with the context.
  * The observable is taken at t_obs (>= the time of the last processed event;
  * t_obs < 0 means that time): msd_out = (1/N) sum |u_i - <u>|^2 with u the
  * minimum-image displacement; g_vx, g_vy (g_x, g_y) receive d MSD / d v(0)
@@ -310,9 +312,9 @@ int edmd_tangent_run_batch(edmd_ctx* ctx, int32_t K, int64_t n_coll, int64_t qr_
                            double* lyap_out);
 
 /* Batched adjoint of the final mean-square displacement of every system: the
- * forward sweep (whole-context checkpoints every ckpt_every collisions when the
- * logs take more than 2 GiB together) and the reverse sweep one warp per
- * system.  The observable of system s is
+ * forward sweep (whole-context checkpoints every ckpt_every collisions under the
+ * rule of edmd_msd_gradient, for all logs together) and the reverse sweep one
+ * warp per system.  The observable of system s is
  * taken at the time of its last processed event; msd_out (nsys) and the
  * gradients (total N, concatenated in system order like edmd_get_states) may
  * be NULL.  No reference counterpart.  Warp engine. */

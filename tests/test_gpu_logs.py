@@ -86,3 +86,51 @@ def test_a_run_that_fails_leaves_its_last_chunk(edmd, batch):
     eng.close()
     assert len(log) == 1 and {int(log["i"][0]), int(log["j"][0])} == {1, 2}
     assert abs(log["t"][0] - 0.1) < 1e-12
+
+
+def same_gradient(a, b):
+    np.testing.assert_array_equal(a[0], b[0])
+    for k in KEYS:
+        np.testing.assert_array_equal(a[1][k], b[1][k], err_msg=k)
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_long_intervals_bound_a_gradients_memory(edmd, batch):
+    """64 systems x 19000 collisions (68 MB of log): in five segments, whose log and checkpoints take half of that, and as one."""
+    import torch
+    s = [start(edmd, 200, 3 + k % 2) for k in range(64)]
+    res, took = [], []
+    for every in (3800, 100):
+        eng = edmd.Engine(s)
+        eng.tangent_batch(1, 4, 2)                        # (kernels loaded, second stream made)
+        free = torch.cuda.mem_get_info()[0]
+        res.append(eng.msd_gradient_batch(19000, ckpt_every=every) if batch else eng.msd_gradient(19000, ckpt_every=every, s=5))
+        took.append(free - torch.cuda.mem_get_info()[0])
+        res[-1] += (eng.state(5),)
+        eng.close()
+    same_gradient(res[0], res[1])
+    assert np.isfinite(res[0][1]["vx"]).all() and np.abs(res[0][1]["vx"]).max() > 0
+    for k in KEYS:
+        np.testing.assert_array_equal(res[0][2][k], res[1][2][k])
+    assert took[0] < 45 << 20 and took[1] > 55 << 20, took
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_a_gradient_without_room_for_its_log(edmd, batch):
+    """230 MB of log asked for and 130 MB left: the segments' checkpoints are there already, and the result is the same."""
+    import torch
+    s = [start(edmd, 100, 3 + k % 2) for k in range(1024)]
+    res = []
+    for full in (False, True):
+        eng = edmd.Engine(s)
+        for k in range(22):
+            eng.checkpoint_save(k)
+        eng.msd_gradient_batch(2, ckpt_every=1)           # (kernels loaded)
+        hog = crowd_out(130 << 20) if full else None
+        try:
+            res.append(eng.msd_gradient_batch(4000, ckpt_every=200) if batch else eng.msd_gradient(4000, ckpt_every=200, s=5))
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+        eng.close()
+    same_gradient(res[0], res[1])
