@@ -1990,9 +1990,9 @@ static int advance_smem_split(edmd_ctx* ctx, RunArgs A, int nsm) {
   if (!ctx->smem_list) {
     CK(dalloc(&ctx->smem_list, ctx->nsys));
     CK(dalloc(&ctx->smem_work, 1));
-    CK(cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&ctx->e2, cudaEventDisableTiming));
   }
+  if (!ctx->stream2) CK(cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking));
   if (!rest.empty())
     CK(cudaMemcpyAsync(ctx->order, rest.data(), rest.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
                        ctx->stream));
