@@ -2235,7 +2235,7 @@ extern "C" int edmd_get_last_launches(const edmd_ctx* ctx, int64_t* n) {
 // that owns every device buffer and forbids cudaMalloc/cudaFree after start-up.
 // The caller passes its own device arrays (the state in and out); everything
 // the engine needs besides them -- the system descriptor, cell lists, event
-// records, the tournament tree, the scalar state and the work counter -- lives
+// records, the tournament tree and the scalar state -- lives
 // in the file-scope array below, which every GPU that loads this library keeps
 // until the process exits.
 namespace {
@@ -2370,7 +2370,6 @@ extern "C" int edmd_run_noalloc(const edmd_system_desc* desc, double* x, double*
   auto take = [&](size_t bytes) { unsigned char* r = base + off; off += align_up(bytes, 256); return r; };
   size_t N = D.N, E = 2 * N + NSPECIAL, C = (size_t)B.Nxc * B.Nyc;
   SysDev* dsys = (SysDev*)take(sizeof(SysDev));
-  int32_t* work = (int32_t*)take(sizeof(int32_t));
   S.st = (SysState*)take(sizeof(SysState));
   S.d = (Disk*)take(N * sizeof(Disk));
   S.vr = (double*)take(N * 8);

@@ -605,7 +605,7 @@ __device__ __forceinline__ void cnt_addf(const RoundArgs& A, int s, int stripe, 
   atomicAdd((double*)&A.cnt[((int64_t)s * NSTRIPE + stripe) * NCNT + k], v);
 }
 
-// outcome of one processed event, the same on all lanes of its group but for
+// outcome of one processed event, the same on all lanes of its warp but for
 // `dc` (lanes 0..7: one cell each whose minimum can have changed, or -1) and
 // `ct` (lane virial_lane(k): virial term k)
 struct EvResult {
@@ -618,15 +618,13 @@ struct EvResult {
   int a, ob;
 };
 
-// One selected event g of system s processed by a group of GW lanes:
+// One selected event g of system s processed by a warp:
 // doTheCollisionNormal (src/EDMD.c:3542, elastic rule 3802-3827), its stale
 // branch (3553-3556) or doTheCrossing (2501).  The lanes hold the roles of
-// edmd_lanes.cuh, so an event's scalar FP64 work shares its instructions;
-// `on` is false in a group without an event, which follows along on event g
-// without storing anything.
-template <int GW, bool ONE>
-__device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& A, int s, int64_t g, bool on,
-                                              LaneScratch* W, const Grp<GW>& G, EvResult& res) {
+// edmd_lanes.cuh, so an event's scalar FP64 work shares its instructions.
+template <bool ONE>
+__device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& A, int s, int64_t g,
+                                              LaneScratch* W, const Grp<32>& G, EvResult& res) {
   const Box& B = S.B;
   const int N = B.N, gl = G.lane;
   const bool odd = gl & 1, ydim = gl & 2;
@@ -664,8 +662,8 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
     const double msum = m + c.mo;
     const double inv = (__double_as_longlong(msum) == 0x4000000000000000ll ? 0.5 : div_rn(1.0, msum)) * (1 + S.res);
     double dx, dy;
-    elastic_lanes<GW, true>(B, G, own, m, c, inv, res.ct, &dx, &dy);
-    if (on && gl < 4) {
+    elastic_lanes<32, true>(B, G, own, m, c, inv, res.ct, &dx, &dy);
+    if (gl < 4) {
       *axis_pos(D, ydim) = own.p;
       *axis_vel(D, ydim) = own.v;
       if (!ydim) {
@@ -673,7 +671,7 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
         D->coll = hits + 1;
       }
     }
-    if (on && (A.flags & EDMD_F_TRACE) && S.trace && gl == 0) {
+    if ((A.flags & EDMD_F_TRACE) && S.trace && gl == 0) {
       const unsigned long long k = atomicAdd((unsigned long long*)&S.st->ntrace, 1ull);
       if ((int64_t)k < S.trace_cap) {
         edmd_collision* tr = (edmd_collision*)S.trace + k;
@@ -689,7 +687,7 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
     }
     const int to = cell_of(B, G.shfl(own.c, 0), G.shfl(own.c, 2));
     if (cross) wc1 = to;
-    if (on && (gl == 0 || gl == 2)) {
+    if (gl == 0 || gl == 2) {
       *axis_pos(D, ydim) = own.p;
       if (cross) {
         (ydim ? S.cy : S.cx)[a] = own.c;
@@ -697,7 +695,7 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
       }
       if (!ydim) D->tl = t;
     }
-    if (on && cross && gl == 0) {
+    if (cross && gl == 0) {
       // unlink from the old cell, relink at the head of the new one
       const int pv = S.prv[a], nx = D->nxt;
       if (pv == NIL) S.head[ca] = nx;
@@ -716,7 +714,7 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
   uint64_t lw_old = 0, lr_old = 0;
   {
     const int c = gl == 0 ? ca : wc1;
-    if (on && gl < 2 && c >= 0) {
+    if (gl < 2 && c >= 0) {
       lr_old = A.lr[base + c];
       lw_old = atomicMax((unsigned long long*)&A.lw[base + c], (unsigned long long)clk);
     }
@@ -737,17 +735,15 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
     dir = ux == ydim ? db : da;
   }
   __syncwarp();
-  uint64_t lw_seen[(18 + GW - 1) / GW] = {};
-  int seen = 0;
+  uint64_t lw_seen = 0;
   res.npair = 0;
   res.ovl = false;
   res.a = a;
   res.ob = -1;
-  const Next nx = predict2<GW, true, false, 32>(S, t, a, two ? j : -1, own, &res.npair, G, W, &res.ovl, &res.a,
+  const Next nx = predict2<32, true, false, 32>(S, t, a, two ? j : -1, own, &res.npair, G, W, &res.ovl, &res.a,
                                                 &res.ob, [&](int cell) {
-    // stamps of the cells read
-    if (!on) return;
-    lw_seen[seen++] = A.lw[base + cell];
+    // stamps of the cells read, one cell a lane
+    lw_seen = A.lw[base + cell];
     atomicMax((unsigned long long*)&A.lr[base + cell], (unsigned long long)clk);
   }, [&](int p) { return (int)A.drank[dbase + p]; });
   if (res.ovl && res.a == OVL_CORRUPT) { res.a = a; res.ob = OB_CORRUPT; }
@@ -764,9 +760,9 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
   ev.j = ydim ? nx.partner : dir;
   ev.ca = ydim ? nx.ca : 0;
   ev.st = ST_QUEUED;
-  if (on && mine) S.ev[(ydim ? N : 0) + my] = ev;
+  if (mine) S.ev[(ydim ? N : 0) + my] = ev;
   uint8_t rank = 0;
-  if (on && mine && ydim) {
+  if (mine && ydim) {
     rank = new_rank(S, A, dbase, my, odd ? a : two ? j : -1, ev.t, nx.partner, nx.tag, clk);
     A.drank[gm] = rank;
   }
@@ -780,7 +776,7 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
   const int wayc = G.shfl(way, odd ? 1 : 0), rk = G.shfl((int)rank, odd ? 3 : 2);
   const int own_cell = cell_of(B, X, Y);
   const int c2 = hit ? pcell : target_cell(B, X, Y, wayc);
-  const bool changed = on && (!odd || two);
+  const bool changed = !odd || two;
   if (changed && gl < 4) {
     Att* const at = A.att + gm;
     if (!ydim) {
@@ -803,10 +799,7 @@ __device__ __forceinline__ void process_event(const SysDev& S, const RoundArgs& 
   }
   res.dc = dc;
   res.ncol = two; res.ncross = cross; res.nstale = stale;
-  bool bad = lw_old > clk || lr_old > clk;
-#pragma unroll
-  for (int k = 0; k < (18 + GW - 1) / GW; k++) bad |= lw_seen[k] > clk;
-  res.bad = G.any(bad);
+  res.bad = G.any(lw_old > clk || lr_old > clk || lw_seen > clk);
   if (A.flags & EDMD_F_SCREEN) {             // the FP32 shadows serve the thread path's screen only
     G.sync();
     if (changed && gl < 2) shadow_write(A, gm, B, S.d[my], S.cx[my], S.cy[my], A.epoch[s]);
@@ -1163,58 +1156,48 @@ __device__ __forceinline__ void list_min(const SysDev& S, const RoundArgs& A, in
   }
 }
 
-// the selected events w .. w + 32 / GW - 1 by the groups of a warp: the event,
-// its system's counters (one of NSTRIPE stripes, to spread the atomics), its
-// dirty cells, its errors
-template <int GW, bool ONE>
-__device__ __forceinline__ void run_event(const SysDev* __restrict__ sys, const RoundArgs& A, int w, int nsafe,
-                                          int stripe, LaneScratch* W, const Grp<GW>& G) {
-  const int n = w + (threadIdx.x & 31) / GW;
-  const bool on = n < nsafe;
-  const int64_t g = A.safe[on ? n : w];
+// the selected event n by a warp: the event, its system's counters (one of
+// NSTRIPE stripes, to spread the atomics), its dirty cells, its errors
+template <bool ONE>
+__device__ __forceinline__ void run_event(const SysDev* __restrict__ sys, const RoundArgs& A, int n, int stripe,
+                                          LaneScratch* W, const Grp<32>& G) {
+  const int64_t g = A.safe[n];
   const int s = sys_index<ONE>(A, g);
   const SysDev& S = sys_of<ONE>(sys, A, s);
   EvResult r;
-  process_event<GW, ONE>(S, A, s, g, on, W, G, r);
-  if (on) {
-    if (r.ncol && G.lane >= virial_lane<GW>(0) && G.lane < virial_lane<GW>(0) + 4)
-      cnt_addf(A, s, stripe, C_CT0 + (G.lane & 3), r.ct);
-    if (G.lane < MAXDIRTY) A.dcell[(int64_t)n * MAXDIRTY + G.lane] = r.dc;
-    if (G.lane == 0) {
-      cnt_add(A, s, stripe, r.ncol ? C_NCOL : r.ncross ? C_NCROSS : C_NSTALE, 1ull);
-      cnt_add(A, s, stripe, C_NPAIR, r.npair);
-      atomicMax((unsigned long long*)&A.cnt[((int64_t)s * NSTRIPE + stripe) * NCNT + C_TLAST],
-                (unsigned long long)r.key);
-      if (r.bad) atomicAdd(A.violations, 1ull);
-      if (r.ovl) {
-        SysState* R = S.st;
-        R->err_a = r.a;
-        R->err_b = r.ob;
-        R->status = r.ob == OB_CORRUPT ? EDMD_ERR_BUDGET : EDMD_ERR_OVERLAP;
-      }
+  process_event<ONE>(S, A, s, g, W, G, r);
+  if (r.ncol && G.lane >= virial_lane<32>(0) && G.lane < virial_lane<32>(0) + 4)
+    cnt_addf(A, s, stripe, C_CT0 + (G.lane & 3), r.ct);
+  if (G.lane < MAXDIRTY) A.dcell[(int64_t)n * MAXDIRTY + G.lane] = r.dc;
+  if (G.lane == 0) {
+    cnt_add(A, s, stripe, r.ncol ? C_NCOL : r.ncross ? C_NCROSS : C_NSTALE, 1ull);
+    cnt_add(A, s, stripe, C_NPAIR, r.npair);
+    atomicMax((unsigned long long*)&A.cnt[((int64_t)s * NSTRIPE + stripe) * NCNT + C_TLAST],
+              (unsigned long long)r.key);
+    if (r.bad) atomicAdd(A.violations, 1ull);
+    if (r.ovl) {
+      SysState* R = S.st;
+      R->err_a = r.a;
+      R->err_b = r.ob;
+      R->status = r.ob == OB_CORRUPT ? EDMD_ERR_BUDGET : EDMD_ERR_OVERLAP;
     }
   }
 }
 
-// The selected events of a round, GW lanes each: a warp an event (GW = 32), or
-// four events a warp.
-template <int GW, int MINB, bool ONE>
+// The selected events of a round, a warp each.
+template <int MINB, bool ONE>
 __global__ void __launch_bounds__(32, MINB) k_process(const SysDev* __restrict__ sys, const __grid_constant__ RoundArgs A) {
-  constexpr int PER = 32 / GW;
-  __shared__ LaneScratch scr[PER];
-  const int lane = threadIdx.x & 31;
-  const Grp<GW> G(lane);
-  LaneScratch* W = &scr[lane / GW];
+  __shared__ LaneScratch scr;
+  const Grp<32> G(threadIdx.x);
   const int nsafe = *A.nsafe;
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicMax(A.maxsafe, nsafe);
   if (A.thread_kernel && nsafe >= A.thr_min) return;   // k_process_thread takes the round
   const int stripe = blockIdx.x & (NSTRIPE - 1);
-  const int wave = gridDim.x * PER;
-  // one resident wave: each warp takes the events at its own index, then the
+  // one resident wave: each warp takes the event at its own index, then the
   // warps that finish first take the rest from a counter (a grid of one
   // block per event would mostly launch blocks that find nothing to do)
-  for (int w = blockIdx.x * PER; w < nsafe; w = next_chunk(A, lane, wave, PER, nsafe)) {
-    run_event<GW, ONE>(sys, A, w, nsafe, stripe, W, G);
+  for (int n = blockIdx.x; n < nsafe; n = next_chunk(A, G.lane, gridDim.x, 1, nsafe)) {
+    run_event<ONE>(sys, A, n, stripe, &scr, G);
     __syncwarp();
   }
 }
@@ -1387,7 +1370,7 @@ __global__ void __launch_bounds__(32 * BWPB, 4) k_block_rounds(const SysDev* __r
       }
       for (int e = wid; e < n; e += BWPB) {
         EvResult r;
-        process_event<32, false>(S, A, s, evl[e], true, &scr[wid], Grp<32>(lane), r);
+        process_event<false>(S, A, s, evl[e], &scr[wid], Grp<32>(lane), r);
         if (r.ncol && lane >= virial_lane<32>(0) && lane < virial_lane<32>(0) + 4) atomicAdd(&c_ct[lane & 3], r.ct);
         if (lane < MAXDIRTY && r.dc >= 0) dl[atomicAdd(&ndl, 1)] = r.dc;
         if (lane == 0) {
@@ -1656,8 +1639,8 @@ cudaError_t enqueue_round(edmd_ctx* ctx, const RoundBufs* R, const RoundArgs& A0
   }
   // one resident wave of each event kernel: one-warp blocks, 20 per SM (k_process)
   // and 16 per SM (k_process_thread), measured best
-  if (one) k_process<32, 20, true><<<nsm * 20, 32, 0, st>>>(ctx->ds, A);
-  else k_process<32, 20, false><<<nsm * 20, 32, 0, st>>>(ctx->ds, A);
+  if (one) k_process<20, true><<<nsm * 20, 32, 0, st>>>(ctx->ds, A);
+  else k_process<20, false><<<nsm * 20, 32, 0, st>>>(ctx->ds, A);
   if (with_thread) k_process_thread<<<nsm * 16, 32, 0, st>>>(ctx->ds, A);
   const int nbar = ctx->nsys < nsm * 8 ? ctx->nsys : nsm * 8;
   if (one) k_recompute_barrier<true><<<nsm * 8, 256, 0, st>>>(ctx->ds, A, nbar);
