@@ -1034,11 +1034,15 @@ __device__ bool run_system(const SysDev& S, const RunArgs& A, const Grp<GW>& G, 
   }
 }
 
-// Events a system runs before it makes room for a waiting one, ~5 ms: measured
-// on 3100 mixed systems x 1200 collisions 1.18e8 coll/s with 64 and 256, 1.05e8
-// with 1024 (too coarse at the end of the launch).  A call of at most 256
-// collisions takes a system whole: 16384 systems of 96 disks x 150 collisions
-// (257 events each) 16.1 ms against 18.2 ms cut at 256.
+// Events a system runs before it makes room for a waiting one.  Turns of 256 are
+// ~5 ms and leave little of the launch's end to a part of the groups; measured
+// against 1024 (ms): 3100 systems of 64-1024 disks, 257 / 400 / 1200 collisions
+// 6.4 / 9.3 / 24.8 against 6.9 / 11.1 / 28.7; 4096 of 256-1024 disks 7.6 / 11.6 /
+// 31.7 against 8.5 / 13.3 / 33.6; 16384 of 96 disks 24.1 / 36.8 / 111.3 against
+// 25.2 / 38.7 / 111.0; for one unit of time 37.8, 45.2 and 19.3 against 37.9, 46.9
+// and 19.7.  A call of at most 256 collisions takes turns of 1024, in which most
+// systems end (1.7 events a collision at phi 0.55): 16384 of 96 disks, 150
+// collisions 16.1 ms against 18.2 in turns of 256.
 __device__ __forceinline__ int64_t share_of(int64_t max_coll) { return max_coll <= 256 ? 1024 : 256; }
 
 // The place whose system a lane group runs next, -1 when there is none.  A

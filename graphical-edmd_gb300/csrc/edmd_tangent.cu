@@ -1007,8 +1007,11 @@ int batch_index(edmd_ctx* ctx, BatchIndex& bi) {
 // CholQR2 of every system's tangent block at the times tqs, on stream st
 int cholqr_b(edmd_ctx* ctx, const BatchIndex& bi, double* T, double* tl, int K, double* G, double* Rinv,
              double* logdiag, int* fail, bool accumulate, const double* tqs, cudaStream_t st) {
-  // all pairs of a system in one block, or (few systems) spread over blocks
-  const int pair_warps = (K * (K + 1) / 2 + 31) / 32, split = std::max(1, std::min(pair_warps, 152 / ctx->nsys));
+  // all pairs of a system in one block, or (fewer systems than SMs) spread over blocks
+  int dev = 0, nsm = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const int pair_warps = (K * (K + 1) / 2 + 31) / 32, split = std::max(1, std::min(pair_warps, nsm / ctx->nsys));
   const int warps = std::max((pair_warps + split - 1) / split, (4 * K + 31) / 32);
   for (int pass = 0; pass < 2; pass++) {    // CholQR2: the second pass restores orthogonality
     k_gram_b<<<dim3(ctx->nsys, (pair_warps + warps - 1) / warps), 32 * warps, 0, st>>>(ctx->ds, bi.doff, T, tl, K, tqs, G);
