@@ -3,8 +3,6 @@
 Produces, in this directory:
   libedmd_gpu.so  C ABI of include/edmd_gpu.h + include/edmd_host.h
   edmd            drop-in command-line driver (host/edmd_main.c), rpath to the .so
-and, only with `python build.py probe`, the measurement tool peak_probe
-(probe/peak_probe.cu: FP64 issue rate and load latency).
 
 All CUDA is compiled for sm_103a only, with --fmad=false so that no
 floating-point multiply-add is contracted (the event arithmetic must round
@@ -13,7 +11,6 @@ compiled in parallel; no cmake.
 """
 import os
 import subprocess
-import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -84,16 +81,5 @@ def build(verbose=False):
     return lib
 
 
-def build_probe():
-    """The FP64/FP32 issue-rate and load-latency microbenchmark behind the
-    engines' FP64 roofline (not part of the library): ./peak_probe."""
-    src = os.path.join(HERE, "probe", "peak_probe.cu")
-    exe = os.path.join(HERE, "peak_probe")
-    if _newer(exe, [src, __file__]):
-        _run_all([[_nvcc(), "-gencode", "arch=compute_103a,code=sm_103a", "-O3", "-o", exe, src]])
-    return exe
-
-
 if __name__ == "__main__":
-    print(build_probe() if sys.argv[1:] == ["probe"] else build(verbose=True))
-    sys.exit(0)
+    print(build(verbose=True))
