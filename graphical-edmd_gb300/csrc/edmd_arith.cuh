@@ -2,13 +2,13 @@
 // division and square root, bit for bit the IEEE results of `a / b` and
 // `sqrt(x)`, and the event calendar's repeated additions in closed form.
 //
-// GB300 issues one FP64 warp instruction per ~76 cycles and SM sub-partition
-// (dependent latency ~38), and the compiler's FP64 division and square root
-// are chains of about nine of them.  Measured on GB300 (one dependent chain /
-// 16 warps per SM, cycles per operation and warp, 19 of loop overhead
-// included): a / b 575 / 2245, div_rn 267 / 532; sqrt(x) 654 / 2602, sqrt_rn
-// 280 / 497.  The event kernels are bound by FP64 issue and by the latency of
-// the pair solve, so both figures count.
+// GB300 issues one FP64 warp instruction per 64 cycles from one warp, dependent
+// or not, and one per 76 cycles and SM sub-partition with all four busy; the
+// compiler's FP64 division and square root are chains of about nine of them.
+// Measured on GB300 (one dependent chain / 16 warps per SM, cycles per operation
+// and warp, loop included): a / b 575 / 2245, div_rn 267 / 532; sqrt(x) 654 /
+// 2602, sqrt_rn 280 / 497.  The event kernels are bound by FP64 issue and by the
+// latency of the pair solve, so both figures count.
 //
 // Method: long division (and digit-by-digit square root) of the 53-bit
 // significands in two digits, each estimated with a 31-bit reciprocal (root)

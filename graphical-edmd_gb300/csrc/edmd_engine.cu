@@ -1165,10 +1165,10 @@ __global__ void k_waiting(RunArgs A) {
 // ms; every build has the same event loop):
 //   3 blocks per SM, 168 registers: 1.41 / 15.2 / 36
 //   4 blocks, 128 registers:        1.45 / 15.5 / 40.5 (2432 warps, a second wave)
-//   5 blocks, 102 registers:        1.50 / 16.4 / 30.2 (3040 warps)
-//   6 blocks, 85 registers:         1.58 / 17.6 / 32.2
-// so systems that all find a warp at three blocks per SM run there, without
-// spills, and larger batches at five.
+//   5 blocks, 96 registers:         1.50 / 16.4 / 30.2 (3040 warps)
+//   6 blocks, 80 registers:         1.58 / 17.6 / 32.2
+// so systems that all find a warp at three blocks per SM run there (8 bytes of
+// spill stores), and larger batches at five (476 bytes).
 bool few_cells(const Box& B) { return B.Nxc < 3 || B.Nyc < 3; }
 using RunKernel = void (*)(const SysDev*, RunArgs);
 struct RunShape { RunKernel kernel; int warps, systems; };   // a block's warps and systems
