@@ -17,6 +17,8 @@
  *     message readable with edmd_last_error(ctx).
  *   - Systems are independent; arrays passed for several systems are the
  *     per-system arrays concatenated in system order.
+ *   - A context that has copied 1 MB or more from or to pageable host arrays
+ *     keeps 8 MB of page-locked host memory until it is destroyed.
  *   - Device loops are bounded: a call that would exceed its event budget
  *     returns EDMD_ERR_BUDGET instead of spinning.
  */
@@ -136,7 +138,11 @@ typedef struct edmd_ctx edmd_ctx;
  * starts.  Positions must lie in [0,L); radii must be zero or normal
  * positive below 2^1020 (EDMD_ERR_ARG otherwise).  trace_cap is the per-system
  * capacity of the collision trace (0 disables tracing).  *out is set even when
- * the call fails, so that edmd_last_error can be read; destroy it either way. */
+ * the call fails, so that edmd_last_error can be read; destroy it either way.
+ * In a box of fewer than three cells (of at least 2 x 2) along an axis, the
+ * nearest image of a cell's wall can lie behind a disk that moves along that
+ * axis; its crossings are then scheduled in the past, as the reference's are,
+ * and the clock may not advance: give edmd_advance a max_events there. */
 int edmd_create(int32_t nsys, const edmd_system_desc* desc,
                 const double* x, const double* y, const double* vx, const double* vy,
                 const double* rad, const double* m, const double* vr,
